@@ -98,12 +98,11 @@ void decode_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n) {
     need(n >= 1 && n <= 0x7fffffff, "empty token list (the count must be between 1 and 2^31 - 1)");
     check_tokens(m, tokens, n);
     RSV_CUDA(cudaSetDevice(m.device));
-    if (!m.prof_on && m.persistent_available(1)) {
+    if (!m.prof_on && m.stream_available()) {
         m.ensure_workspace(1, 1, 1);
         ensure_tok_list(m, (size_t)n);
         RSV_CUDA(cudaMemcpyAsync(m.ws.tok_list, tokens, (size_t)n * sizeof(uint32_t), cudaMemcpyHostToDevice, m.stream));
-        const int slot0 = 0;
-        m.run_persistent(st, 1, &slot0, (int)n, true, false, nullptr, nullptr, 0);  // all n tokens in one launch, head on the last
+        m.run_stream(st, 0, (int)n, true, false, nullptr, nullptr, 0);  // all n tokens in one launch, head on the last
         return;
     }
     StepPlan with_head = decode_plan(1, true), no_head = decode_plan(1, false);
@@ -191,14 +190,13 @@ std::unique_ptr<rsv_ticket> selfloop_submit(Model& m, State& st, const uint32_t*
         else
             engine_argmax(m, m.ws.logits, B, m.ws.tokens, t.seq, t.cnt, (int)n);
     };
-    if (!m.prof_on && B <= 4 && m.persistent_available(B)) {
-        // up to 4 sessions: the persistent kernel runs whole steps (and, for arg-max, the whole self-loop) in one launch
-        int slots[4] = {0, 1, 2, 3};
+    if (!m.prof_on && B == 1 && m.stream_available()) {
+        // one session: the weight-streaming kernel runs whole steps (and, for arg-max, the whole self-loop) in one launch
         if (!sp) {
-            m.run_persistent(st, B, slots, (int)n, false, true, t.seq, t.cnt, (int)n);
+            m.run_stream(st, 0, (int)n, false, true, t.seq, t.cnt, (int)n);
         } else {
             for (int64_t round = 0; round < n; ++round) {
-                m.run_persistent(st, B, slots, 1, false, false, nullptr, nullptr, 0);
+                m.run_stream(st, 0, 1, false, false, nullptr, nullptr, 0);
                 engine_sample(m, m.ws.logits, B, t.sampler, t.seq, (int)n, t.cnt, m.ws.tokens, t.seq, t.cnt, (int)n);
             }
         }

@@ -40,7 +40,7 @@
 #include <cstddef>
 
 #include "kernels.cuh"
-#include "tc_linear.cuh"
+#include "tc_ptx.cuh"
 
 namespace rsv {
 

@@ -7,8 +7,7 @@
 
 #include "kernels.cuh"
 #include "safetensors.hpp"
-#include "tc_linear.cuh"
-#include "decode_persistent.cuh"
+#include "rows_linear.cuh"
 #include "decode_stream_layout.hpp"
 #include "wkv_rows.cuh"
 #include "wkv_seq.cuh"
@@ -57,6 +56,33 @@ static void launch_pdl(Model& m, void (*kernel)(KArgs...), dim3 grid, dim3 block
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = m.use_pdl ? 1 : 0;
+    RSV_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(std::forward<Args>(args))...));
+}
+
+// The same as a launch of thread-block clusters of `cluster` CTAs.
+template <typename... KArgs, typename... Args>
+static void launch_pdl_cluster(Model& m, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, Args&&... args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = m.stream;
+    cudaLaunchAttribute at[2];
+    memset(at, 0, sizeof(at));
+    int n = 0;
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = (unsigned)cluster;
+    at[n].val.clusterDim.y = 1;
+    at[n].val.clusterDim.z = 1;
+    ++n;
+    if (m.use_pdl) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
     RSV_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(std::forward<Args>(args))...));
 }
 
@@ -180,49 +206,40 @@ struct Loader {
             L.wtype = W_F16;
             if (t.dtype == "F16") {
                 L.w = upload(t.data, t.nbytes);
-                prepare_tc_f16(L, (const uint16_t*)t.data);
+                prepare_tc_f16(L);
             } else {
                 auto h = to_f16_bits(t);
                 L.w = upload(h.data(), h.size() * 2);
-                prepare_tc_f16(L, h.data());
+                prepare_tc_f16(L);
             }
         }
         return L;
     }
-    // int8: the tensor-core path needs one (scale, zero) per output row (all groups of a row equal) and
-    // M, K multiples of 128; other files keep tc_ok = false and run on the SIMT kernel.
+    // int8: files with one (scale, zero) per output row (all groups of a row equal) keep them as two vectors; others keep the words
+    // transposed, so that the 128 output rows of a tile read a group's words together.
     void prepare_tc_i8(LinearW& L, const uint32_t* sz_host) {
         const int KG = L.K / 128;
-        if (L.M % kTcTileM || L.K % kTcKBlockBytes) return;
-        std::vector<float> sc(L.M), zr(L.M);
-        for (int m = 0; m < L.M; ++m) {
-            const uint32_t w0 = sz_host[(size_t)m * KG];
-            for (int g = 1; g < KG; ++g)
-                if (sz_host[(size_t)m * KG + g] != w0) return;
-            sc[m] = half_bits_to_float((uint16_t)(w0 & 0xFFFFu));
-            zr[m] = half_bits_to_float((uint16_t)(w0 >> 16));
-        }
-        L.wscale = (float*)upload(sc.data(), sc.size() * 4);
-        L.wzero = (float*)upload(zr.data(), zr.size() * 4);
-        L.Mpad = L.M;
-        L.Kpad = L.K;
-        L.w_tc = L.w;
-        encode_kmajor_map(&L.amap, true, L.w_tc, L.Mpad, L.Kpad, kTcTileM);
-        L.tc_ok = true;
-    }
-    // fp16: zero-pad to [Mpad = ceil128(M), Kpad = ceil64(K)] when the shape needs it (only small matrices do).
-    void prepare_tc_f16(LinearW& L, const uint16_t* w_host) {
-        L.Mpad = (int)round_up(L.M, kTcTileM);
-        L.Kpad = (int)round_up(L.K, 64);
-        if (L.Mpad == L.M && L.Kpad == L.K) {
-            L.w_tc = L.w;
+        bool per_row = true;
+        for (int m = 0; m < L.M && per_row; ++m)
+            for (int g = 1; g < KG && per_row; ++g) per_row = sz_host[(size_t)m * KG + g] == sz_host[(size_t)m * KG];
+        if (per_row) {
+            std::vector<float> sc(L.M), zr(L.M);
+            for (int m = 0; m < L.M; ++m) {
+                sc[m] = half_bits_to_float((uint16_t)(sz_host[(size_t)m * KG] & 0xFFFFu));
+                zr[m] = half_bits_to_float((uint16_t)(sz_host[(size_t)m * KG] >> 16));
+            }
+            L.wscale = (float*)upload(sc.data(), sc.size() * 4);
+            L.wzero = (float*)upload(zr.data(), zr.size() * 4);
         } else {
-            std::vector<uint16_t> pad((size_t)L.Mpad * L.Kpad, 0);
-            for (int m = 0; m < L.M; ++m) memcpy(&pad[(size_t)m * L.Kpad], &w_host[(size_t)m * L.K], (size_t)L.K * 2);
-            L.w_tc = upload(pad.data(), pad.size() * 2);
+            std::vector<uint32_t> t((size_t)KG * L.M);
+            for (int m = 0; m < L.M; ++m)
+                for (int g = 0; g < KG; ++g) t[(size_t)g * L.M + m] = sz_host[(size_t)m * KG + g];
+            L.szt = (uint32_t*)upload(t.data(), t.size() * 4);
         }
-        encode_kmajor_map(&L.amap, false, L.w_tc, L.Mpad, L.Kpad, kTcTileM);
-        L.tc_ok = true;
+        encode_kmajor_map(&L.amap, true, L.w, L.M, L.K, kTcTileM);
+    }
+    void prepare_tc_f16(LinearW& L) {
+        encode_kmajor_map(&L.amap, false, L.w, L.M, L.K, kTcTileM);  // boxes past the matrix read zeros
     }
     // Low-rank pair member.  The file holds either [in,out] or [out,in] (src/model.rs:564-581 accepts
     // both, first match wins when in == out); HBM always holds [out,in] fp16.
@@ -245,7 +262,7 @@ struct Loader {
         L.K = in_dim;
         L.wtype = W_F16;
         L.w = upload(oi.data(), oi.size() * 2);
-        prepare_tc_f16(L, oi.data());
+        prepare_tc_f16(L);
         return L;
     }
 };
@@ -306,8 +323,6 @@ std::unique_ptr<Model> Model::load(const std::string& path, int device) {
     if (c.n_embd % 8 || c.ffn_hidden % 8) throw std::runtime_error("n_embd and ffn_hidden must be multiples of 8");
 
     m->num_sms = prop.multiProcessorCount;
-    if (const char* e = getenv("RSV_NO_PERSISTENT"))
-        if (*e && *e != '0') m->use_persistent = false;
     if (const char* e = getenv("RSV_NO_STREAM"))
         if (*e && *e != '0') m->use_stream = false;
     if (const char* e = getenv("RSV_NO_GRAPH"))
@@ -403,7 +418,7 @@ std::unique_ptr<Model> Model::create_bare(int device) {
 }
 
 static void free_workspace(Workspace& w) {
-    void* ptrs[] = {w.x, w.x2, w.delta, w.xmix, w.r, w.k, w.v, w.w, w.a, w.g, w.yg, w.xb, w.mid, w.h, w.vfirst, w.xn, w.logits, w.staging, w.tokens, w.row_meta, w.seg_meta, w.out_rows, w.samp_temp, w.samp_cnt};
+    void* ptrs[] = {w.x, w.x2, w.delta, w.r, w.k, w.v, w.w, w.a, w.g, w.yg, w.xb, w.mid, w.h, w.vfirst, w.logits, w.staging_t, w.staging_c, w.ymax, w.hmax, w.tokens, w.row_meta, w.seg_meta, w.out_rows, w.samp_temp, w.samp_cnt};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     int* status = w.status;
@@ -414,14 +429,8 @@ static void free_workspace(Workspace& w) {
     w.tok_pos = pos;
     w.tok_list = keep.tok_list;
     w.tok_list_cap = keep.tok_list_cap;
-    w.tc_b = keep.tc_b;
-    w.tc_b_bytes = keep.tc_b_bytes;
-    w.tc_xscale = keep.tc_xscale;
-    w.tc_tsum = keep.tc_tsum;
-    w.tc_rows = keep.tc_rows;
-    w.tc_partials = keep.tc_partials;
-    w.tc_cnt = keep.tc_cnt;
-    w.tc_partials_bytes = keep.tc_partials_bytes;
+    w.op_mem = keep.op_mem;
+    w.op_bytes = keep.op_bytes;
 }
 
 Model::~Model() {
@@ -432,19 +441,11 @@ Model::~Model() {
     if (ws.tok_pos) cudaFree(ws.tok_pos);
     if (ws.tok_list) cudaFree(ws.tok_list);
     for (void* p : allocs) cudaFree(p);
-    for (void* p : {(void*)ws.tc_b, (void*)ws.tc_xscale, (void*)ws.tc_tsum, ws.tc_partials, (void*)ws.tc_cnt})
-        if (p) cudaFree(p);
-    for (void* p : {pctx.d_layers, pctx.d_maps, (void*)pctx.x, (void*)pctx.yg, (void*)pctx.vfirst, (void*)pctx.cand_val, (void*)pctx.cand_idx, (void*)pctx.rkv, (void*)pctx.mid, (void*)pctx.hbuf,
-                    (void*)pctx.grid_bar})
+    for (void* p : {(void*)ws.op_mem})
         if (p) cudaFree(p);
     for (void* p : {sctx.d_layers, sctx.wstream, sctx.hstream, (void*)sctx.x, (void*)sctx.yg, (void*)sctx.vfirst, (void*)sctx.rkv, (void*)sctx.mid, (void*)sctx.hbuf, (void*)sctx.cand_val,
                     (void*)sctx.cand_idx, (void*)sctx.grid_bar, (void*)sctx.dbg})
         if (p) cudaFree(p);
-    for (int i = 0; i < 5; ++i) {
-        if (pctx.region_data[i]) cudaFree(pctx.region_data[i]);
-        if (pctx.region_meta[i]) cudaFree(pctx.region_meta[i]);
-        if (pctx.region_cnt[i]) cudaFree(pctx.region_cnt[i]);
-    }
     if (pinned) cudaFreeHost(pinned);
     for (int i = 0; i < kPinRing; ++i)
         if (pin_ev[i]) cudaEventDestroy(pin_ev[i]);
@@ -458,12 +459,6 @@ Model::~Model() {
 State::~State() {
     if (model) {
         cudaSetDevice(model->device);
-        // the persistent kernel's device layer table may point into this state: a later state that cudaMalloc places at the
-        // same addresses (with another batch, hence other per-layer strides) must not be taken for it
-        if (model->pctx.bound_tmix == tmix_x) {
-            model->pctx.bound_tmix = model->pctx.bound_wkv = model->pctx.bound_cmix = nullptr;
-            model->pctx.bound_cap = -1;
-        }
     }
     for (float* p : {tmix_x, wkv, cmix_x, v_first})
         if (p) cudaFree(p);
@@ -484,7 +479,6 @@ void Model::ensure_workspace(int rows, int outs, int segs) {
     fa(ws.x, R * C);
     fa(ws.x2, R * C);
     fa(ws.delta, R * C);
-    fa(ws.xmix, 6 * R * C);
     fa(ws.r, R * C);
     fa(ws.k, R * C);
     fa(ws.v, R * C);
@@ -496,9 +490,11 @@ void Model::ensure_workspace(int rows, int outs, int segs) {
     fa(ws.mid, R * (size_t)cfg.mids());
     fa(ws.h, R * F);
     fa(ws.vfirst, R * C);
-    fa(ws.xn, (size_t)outs * C);
     fa(ws.logits, (size_t)outs * V);
-    fa(ws.staging, (size_t)segs * C);
+    fa(ws.ymax, R * 2 * (size_t)cfg.n_head);
+    fa(ws.hmax, R * ((F + kRlTileM - 1) / kRlTileM));
+    fa(ws.staging_t, (size_t)segs * C);
+    fa(ws.staging_c, (size_t)segs * C);
     fa(ws.samp_temp, (size_t)outs * V);
     RSV_CUDA(cudaMalloc(&ws.samp_cnt, std::max<size_t>((size_t)outs * V, 4) * sizeof(uint32_t)));
     RSV_CUDA(cudaMalloc(&ws.tokens, R * sizeof(uint32_t)));
@@ -623,260 +619,205 @@ void run_linear_simt(Model& m, const char* name, const LinReq* reqs, int n, int 
 
 
 // ---- tensor-core path ---------------------------------------------------------------------------
-void ensure_tc_buffers(Model& m, size_t b_bytes, size_t rows, size_t partial_bytes) {
-    Workspace& w = m.ws;
-    if (!w.tc_cnt) {
-        RSV_CUDA(cudaMalloc(&w.tc_cnt, (size_t)kTcMaxSplit * kTcEpiWarps * sizeof(int)));
-        RSV_CUDA(cudaMemsetAsync(w.tc_cnt, 0, (size_t)kTcMaxSplit * kTcEpiWarps * sizeof(int), m.stream));
+// Row tiles of a step: at most 64 activation rows each (32 with per-group int8 weights), of equal size.
+struct RowTiles {
+    int R = 0, rt = 0, n = 0, nt8 = 0, nt16 = 0;
+    int nt(int fmt) const { return fmt == RL_F16 ? nt16 : nt8; }
+    size_t image_bytes(int fmt, int K) const { return (size_t)n * ((K + rl_kelems(fmt) - 1) / rl_kelems(fmt)) * nt(fmt) * 128; }
+};
+RowTiles row_tiles(int R, bool per_group) {
+    RowTiles t;
+    t.R = R;
+    const int most = per_group ? kRlMaxRowsG : kRlMaxRows;
+    t.n = (R + most - 1) / most;
+    t.rt = (R + t.n - 1) / t.n;
+    t.nt8 = (int)round_up((size_t)t.rt * rl_cols(RL_I8), 16);
+    t.nt16 = (int)round_up((size_t)t.rt * rl_cols(RL_F16), 16);
+    return t;
+}
+int rl_fmt(const LinearW& W) { return W.wtype != W_INT8 ? RL_F16 : W.row_scaled() ? RL_I8 : RL_I8G; }
+
+// Carves a step's operands out of one block of device memory.
+struct OperandCarver {
+    uint8_t* base = nullptr;
+    size_t used = 0;
+    template <typename T>
+    T* take(size_t n) {
+        T* p = reinterpret_cast<T*>(base + used);
+        used += round_up(n * sizeof(T), 1024);
+        return p;
     }
-    if (b_bytes <= w.tc_b_bytes && rows <= w.tc_rows && partial_bytes <= w.tc_partials_bytes) return;
+    RlOperandOut operand(const RowTiles& t, int fmt, int K, const float* mix = nullptr, int tparts = 1) {
+        RlOperandOut o;
+        memset(&o, 0, sizeof(o));
+        o.mix = mix;
+        o.fmt = fmt;
+        o.nt = t.nt(fmt);
+        o.kblocks = (K + rl_kelems(fmt) - 1) / rl_kelems(fmt);
+        o.img = take<uint8_t>(t.image_bytes(fmt, K));
+        o.xscale = take<float>((size_t)t.R);
+        o.tparts = tparts;
+        if (fmt == RL_I8) o.tsum = take<long long>((size_t)t.R * tparts);
+        if (fmt == RL_I8G) o.tgrp = take<float>((size_t)t.R * o.kblocks);
+        return o;
+    }
+};
+void ensure_operand_memory(Model& m, size_t bytes) {
+    Workspace& w = m.ws;
+    if (bytes <= w.op_bytes) return;
     RSV_CUDA(cudaStreamSynchronize(m.stream));
-    if (b_bytes > w.tc_b_bytes) {
-        if (w.tc_b) cudaFree(w.tc_b);
-        w.tc_b = nullptr;
-        w.tc_b_bytes = 0;
-        const size_t nb = b_bytes + b_bytes / 4;
-        RSV_CUDA(cudaMalloc(&w.tc_b, nb));
-        RSV_CUDA(cudaMemsetAsync(w.tc_b, 0, nb, m.stream));
-        w.tc_b_bytes = nb;
-    }
-    if (rows > w.tc_rows) {
-        if (w.tc_xscale) cudaFree(w.tc_xscale);
-        if (w.tc_tsum) cudaFree(w.tc_tsum);
-        w.tc_xscale = nullptr;
-        w.tc_tsum = nullptr;
-        w.tc_rows = 0;
-        const size_t nr = rows + rows / 4;
-        RSV_CUDA(cudaMalloc(&w.tc_xscale, nr * sizeof(float)));
-        RSV_CUDA(cudaMalloc(&w.tc_tsum, nr * sizeof(long long)));
-        w.tc_rows = nr;
-    }
-    if (partial_bytes > w.tc_partials_bytes) {
-        if (w.tc_partials) cudaFree(w.tc_partials);
-        w.tc_partials = nullptr;
-        w.tc_partials_bytes = 0;
-        const size_t np = partial_bytes + partial_bytes / 4;
-        RSV_CUDA(cudaMalloc(&w.tc_partials, np));
-        w.tc_partials_bytes = np;
-    }
+    if (w.op_mem) cudaFree(w.op_mem);
+    w.op_mem = nullptr;
+    w.op_bytes = 0;
+    const size_t nb = bytes + bytes / 4;
+    RSV_CUDA(cudaMalloc(&w.op_mem, nb));
+    RSV_CUDA(cudaMemsetAsync(w.op_mem, 0, nb, m.stream));
+    w.op_bytes = nb;
 }
 
-constexpr int kTcDigits = 4;  // base-128 digits of the fixed-point activations (P = 27 bits)
-
-// One launch group of the tensor-core path: all requests share the weight kind (int8 or fp16).  A stage of a layer has up to
-// two groups; their activation operands are prepared by one launch, then each group's GEMM is launched.
-struct TcRegion {
-    const float* x;
-    int ldx, K, Kpad;
-    size_t off;  // bytes from the group's base in the operand buffer
-    int row0;    // first scale / sum row of the region inside the group
-};
-struct TcGroup {
-    bool i8 = false;
-    int n = 0, R = 0, D = 0, ncols = 0, NT = 0, ncols_pad = 0, rows = 0, U = 0, G = 0;
-    LinReq reqs[kTcMaxProblems];
-    std::vector<TcRegion> regions;
-    int region_of[kTcMaxProblems];
-    size_t b_bytes = 0, b_base = 0, partial_bytes = 0;
-    int row_base = 0;
-    TcLaunch L;
+// One linear layer of a launch.  Its operand is a prepared image (`op`), or fp32 activations the kernel converts itself.
+struct RlReq {
+    const LinearW* W;
+    const RlOperandOut* op;
+    float* y;
+    int ldy;
+    int epi;
+    const float* bias = nullptr;
+    float* y2 = nullptr;
+    float* ymax = nullptr;
+    const float* x = nullptr;  // op == nullptr: activations [R, ldx]
+    int ldx = 0;
 };
 
-void tc_plan_group(Model& m, TcGroup& g) {
-    const bool i8 = g.i8;
-    const int n = g.n, R = g.R;
-    g.D = i8 ? kTcDigits : 2;
-    g.ncols = R * g.D;
-    g.NT = 16;
-    while (g.NT < g.ncols && g.NT < 256) g.NT <<= 1;
-    g.ncols_pad = (int)round_up(g.ncols, g.NT);
-    const size_t es = i8 ? 1 : 2;
-    // B operand regions (requests that read the same activations share one)
-    for (int i = 0; i < n; ++i) {
-        const LinearW& W = *g.reqs[i].W;
-        int found = -1;
-        for (size_t j = 0; j < g.regions.size(); ++j)
-            if (g.regions[j].x == g.reqs[i].x && g.regions[j].K == W.K && g.regions[j].Kpad == W.Kpad && g.regions[j].ldx == g.reqs[i].ldx) found = (int)j;
-        if (found < 0) {
-            g.regions.push_back(TcRegion{g.reqs[i].x, g.reqs[i].ldx, W.K, W.Kpad, g.b_bytes, g.rows});
-            found = (int)g.regions.size() - 1;
-            g.b_bytes += round_up((size_t)g.ncols_pad * W.Kpad * es, 1024);
-            g.rows += R;
-        }
-        g.region_of[i] = found;
-    }
-    // units, tiles, CTA count
-    TcLaunch& L = g.L;
-    memset(&L, 0, sizeof(L));
-    int U = 0, T = 0;
-    const int n_tiles = g.ncols_pad / g.NT;
-    for (int i = 0; i < n; ++i) {
-        const LinearW& W = *g.reqs[i].W;
-        TcProb& P = L.p[i];
-        P.M = W.M;
-        P.kblocks = (int)((size_t)W.Kpad * es / kTcKBlockBytes);
-        P.ncols = g.ncols;
-        P.n_tiles = n_tiles;
-        P.unit0 = U;
-        P.tile0 = T;
-        const int mtiles = W.Mpad / kTcTileM;
-        U += mtiles * n_tiles * P.kblocks;
-        T += mtiles * n_tiles;
-        L.amap[i] = W.amap;
-    }
-    // CTA count.  A tile cut between CTAs costs a partial-sum round trip through global memory and a serial sum over its
-    // pieces, which at few rows outweighs the idle SMs: a CTA gets about a K = 2560 int8 tile's worth of K blocks (20), and the
-    // piece length divides the shortest tile of the group, so that cuts fall on tile boundaries or split a tile evenly
-    // (3B shape, 64 rows: 7.4 -> 5.7 ms per step against one unit range per SM).
-    int kb_min = L.p[0].kblocks;
-    for (int i = 1; i < n; ++i) kb_min = std::min(kb_min, L.p[i].kblocks);
-    int upc = kb_min;
-    while (upc > 30 && upc % 2 == 0) upc /= 2;  // K = 10240 tiles (80 K blocks) in four pieces: measured best of 1, 2, 4, 8
-    int G = std::min(m.num_sms, std::max(1, U / upc));
-    // Short reductions (the rank back-projections: 1-5 K blocks per tile), where a cut tile's partial-sum round trip is longer
-    // than the tile itself, and launches with at least a tile per SM (many rows): CTAs get whole tiles, balanced by their K
-    // blocks, and no tile is cut (256 rows: 10.9 -> 10.4 ms per step; 512-row prefill chunks 2 % faster).
-    int kb_max = 0;
-    for (int i = 0; i < n; ++i) kb_max = std::max(kb_max, L.p[i].kblocks);
-    const bool snap = (kb_max <= 8 || T >= m.num_sms) && std::min(m.num_sms, T) + 1 <= kTcMaxSplit;
-    if (snap) {
-        G = std::min(m.num_sms, T);
-        std::vector<int> tk;
-        tk.reserve((size_t)T);
-        for (int i = 0; i < n; ++i)
-            for (int t = (i + 1 < n ? L.p[i + 1].tile0 : T) - L.p[i].tile0; t > 0; --t) tk.push_back(L.p[i].kblocks);
-        int ti = 0, u = 0;
-        for (int c = 0; c < G; ++c) {
-            L.split_unit[c] = u;
-            const int left = G - c;  // CTAs still to be served, this one included: each gets at least one tile
-            const double target = (double)(U - u) / left;
-            int taken = 0;
-            while (ti < T && T - ti > left - 1) {
-                if (taken > 0 && taken + 0.5 * tk[ti] > target) break;
-                taken += tk[ti++];
-            }
-            u += taken;
-        }
-        if (u != U || ti != T) throw std::runtime_error("tc_linear: tile assignment does not cover the launch");
-        L.split_unit[G] = U;
-        L.snap = 1;
-    }
-    // tiles cut by a CTA boundary keep partial sums; the epilogue warp that arrives last on a sub-block finishes it
-    int pmax = 1, nsplit = 0;
-    for (int c = 1; c < G && !snap; ++c) {
-        const int bnd = tc_cta_begin(c, U, G);
-        int pi = 0;
-        while (pi + 1 < n && bnd >= L.p[pi + 1].unit0) ++pi;
-        const TcProb& P = L.p[pi];
-        const int local = bnd - P.unit0;
-        if (local % P.kblocks == 0) continue;  // boundary falls between tiles
-        const int tile_first = bnd - local % P.kblocks;
-        if (nsplit > 0 && L.split_unit[nsplit - 1] == tile_first) {
-            // same tile cut again
-        } else {
-            if (nsplit >= kTcMaxSplit) throw std::runtime_error("tc_linear: too many split tiles");
-            L.split_unit[nsplit++] = tile_first;
-        }
-        pmax = std::max(pmax, tc_cta_of_unit(tile_first + P.kblocks - 1, U, G) - tc_cta_of_unit(tile_first, U, G) + 1);
-    }
-    g.partial_bytes = (size_t)nsplit * pmax * g.NT * kTcTileM * 4;
-    g.U = U;
-    g.G = G;
-    L.nprob = n;
-    L.total_units = U;
-    L.nt = g.NT;
-    L.is_i8 = i8;
-    L.pmax = pmax;
-    L.grid = G;
-    L.nsplit = nsplit;
+constexpr size_t kRlHalfSm = 111 * 1024;  // dynamic shared memory of a CTA that leaves room for a second one on its SM
+
+// How many CTAs share a tile's K.  The step's launches are short (few tiles, weights prefetched behind the previous kernel), so a
+// launch wants about one CTA per half SM and few K blocks per CTA, but no second wave.
+int rl_split(const Model& m, int jobs, int kb_min, int kb_max) {
+    int s = 1;
+    while (s < kRlMaxSplit && 2 * s <= kb_min && jobs * 2 * s <= 2 * m.num_sms && kb_max / s > 5) s *= 2;
+    return s;
 }
 
-void tc_launch_group(Model& m, const char* name, TcGroup& g) {
-    Workspace& w = m.ws;
-    TcLaunch& L = g.L;
-    for (int i = 0; i < g.n; ++i) {
-        const TcRegion& rg = g.regions[g.region_of[i]];
-        const LinReq& q = g.reqs[i];
-        encode_kmajor_map(&L.bmap[i], g.i8, w.tc_b + g.b_base + rg.off, g.ncols_pad, rg.Kpad, g.NT);
-        TcProb& P = L.p[i];
-        P.R = g.R;
-        P.D = g.D;
-        P.wscale = q.W->wscale;
-        P.wzero = q.W->wzero;
-        P.xscale = w.tc_xscale + g.row_base + rg.row0;
-        P.tsum = w.tc_tsum + g.row_base + rg.row0;
-        P.y = q.y;
-        P.y2 = q.y2;
-        P.bias = q.bias;
-        P.aux = q.aux;
-        P.ldy = q.ldy;
-        P.ldaux = q.ldaux;
-        P.epi = q.epi;
-    }
-    const size_t stage_bytes = (size_t)kTcTileM * kTcKBlockBytes + (size_t)g.NT * kTcKBlockBytes;
-    L.nstages = (int)std::min<size_t>(8, (200 * 1024) / stage_bytes);
-    L.partials = w.tc_partials;
-    L.tile_cnt = w.tc_cnt;
-    L.status = w.status;
-    const size_t smem = (size_t)L.nstages * stage_bytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
+template <bool GROUPED, bool BUILD>
+void rl_launch(Model& m, const char* name, const RlLaunch& L, int ctas, size_t smem) {
     static bool configured[16] = {false};
     if (!configured[m.device & 15]) {
-        RSV_CUDA(cudaFuncSetAttribute(tc_linear_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        RSV_CUDA(cudaFuncSetAttribute(tc_linear_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        RSV_CUDA(cudaFuncSetAttribute(rows_linear_kernel<GROUPED, BUILD>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         configured[m.device & 15] = true;
     }
     LAUNCH(m, name) {
-        if (g.i8)
-            launch_pdl(m, tc_linear_kernel<true>, dim3(g.G), dim3(kTcThreads), smem, L);
-        else
-            launch_pdl(m, tc_linear_kernel<false>, dim3(g.G), dim3(kTcThreads), smem, L);
-        check_launch("tc_linear");
+        launch_pdl_cluster(m, rows_linear_kernel<GROUPED, BUILD>, dim3(ctas), dim3(kRlThreads), smem, L.split, L);
+        check_launch("rows_linear");
     }
 }
 
-void run_linear_tc(Model& m, const char* name, const LinReq* reqs, int n, int R) {
-    TcGroup ga, gb;
-    ga.i8 = true;
-    gb.i8 = false;
-    ga.R = gb.R = R;
+void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const RowTiles& t) {
+    if (n < 1 || n > kRlMaxProb) throw std::runtime_error("rows_linear: too many problems in one launch");
+    RlLaunch L;
+    memset(&L, 0, sizeof(L));
+    const bool build = reqs[0].op == nullptr;
+    bool grouped = false, row8 = false;
+    int jobs = 0, kb_min = 1 << 30, kb_max = 0, nt_max = 0;
     for (int i = 0; i < n; ++i) {
-        TcGroup& g = reqs[i].W->wtype == W_INT8 ? ga : gb;
-        if (g.n >= kTcMaxProblems) throw std::runtime_error("tc_linear: too many problems in one group");
-        g.reqs[g.n++] = reqs[i];
-    }
-    if (ga.n) tc_plan_group(m, ga);
-    if (gb.n) tc_plan_group(m, gb);
-    gb.b_base = ga.b_bytes;  // the fp16 group's operands follow the int8 group's
-    gb.row_base = ga.rows;
-    if (ga.regions.size() + gb.regions.size() > (size_t)kTcMaxRegions) throw std::runtime_error("tc_linear: too many operand regions");
-    ensure_tc_buffers(m, ga.b_bytes + gb.b_bytes, (size_t)(ga.rows + gb.rows), std::max(ga.partial_bytes, gb.partial_bytes));
-    Workspace& w = m.ws;
-    // operand preparation: one launch for every activation operand of the stage
-    {
-        TcPrepLaunch PL;
-        memset(&PL, 0, sizeof(PL));
-        int nr = 0;
-        for (TcGroup* g : {&ga, &gb})
-            for (const TcRegion& rg : g->regions)
-                PL.r[nr++] = TcPrepRegion{rg.x, w.tc_b + g->b_base + rg.off, w.tc_xscale + g->row_base + rg.row0, w.tc_tsum + g->row_base + rg.row0,
-                                          rg.ldx, rg.K, rg.Kpad, g->i8 ? 1 : 0};
-        LAUNCH(m, "tc_prepare") {
-            const dim3 grid(R, (unsigned)nr);
-            const dim3 block((size_t)R * nr < 2 * (size_t)m.num_sms ? kPrepThreadsWide : kPrepThreads);
-            launch_pdl(m, tc_prepare_kernel<kTcDigits>, grid, block, 0, PL);
-            check_launch("tc_prepare");
+        const RlReq& q = reqs[i];
+        const LinearW& W = *q.W;
+        RlProb& P = L.p[i];
+        P.fmt = rl_fmt(W);
+        grouped = grouped || P.fmt == RL_I8G;
+        row8 = row8 || P.fmt == RL_I8;
+        if ((q.op == nullptr) != build) throw std::runtime_error("rows_linear: prepared and unprepared operands in one launch");
+        if (q.op) {
+            P.bimg = q.op->img;
+            P.xscale = q.op->xscale;
+            P.tsum = q.op->tsum;
+            P.tgrp = q.op->tgrp;
+            P.tparts = q.op->tparts;
         }
+        P.wscale = W.wscale;
+        P.wzero = W.wzero;
+        P.szt = W.szt;
+        P.x = q.x;
+        P.y = q.y;
+        P.y2 = q.y2;
+        P.bias = q.bias;
+        P.ymax = q.ymax;
+        P.ldx = q.ldx;
+        P.ldy = q.ldy;
+        P.epi = q.epi;
+        P.M = W.M;
+        P.K = W.K;
+        P.kblocks = (W.K + rl_kelems(P.fmt) - 1) / rl_kelems(P.fmt);
+        P.job0 = jobs;
+        L.amap[i] = W.amap;
+        jobs += (W.M + kRlTileM - 1) / kRlTileM * t.n;
+        kb_min = std::min(kb_min, P.kblocks);
+        kb_max = std::max(kb_max, P.kblocks);
+        nt_max = std::max(nt_max, t.nt(P.fmt));
     }
-    std::string nm = std::string(name) + "_tc";
-    if (ga.n) tc_launch_group(m, nm.c_str(), ga);
-    if (gb.n) tc_launch_group(m, nm.c_str(), gb);
+    if (grouped && row8) throw std::runtime_error("rows_linear: per-row and per-group int8 weights in one launch");
+    if (grouped && t.rt > kRlMaxRowsG) throw std::runtime_error("rows_linear: row tile too large for per-group weights");
+    L.nprob = n;
+    L.R = t.R;
+    L.rt = t.rt;
+    L.n_tiles = t.n;
+    L.nt8 = t.nt8;
+    L.nt16 = t.nt16;
+    L.status = m.ws.status;
+    L.split = build ? 1 : rl_split(m, jobs, kb_min, kb_max);  // a kernel that builds its operands has to see whole rows
+    while ((1 << L.log_split) < L.split) ++L.log_split;
+    L.f16_halves = grouped || row8;
+    int nk = 0;
+    for (int i = 0; i < n; ++i) {
+        const int sk = L.p[i].fmt == RL_F16 && L.f16_halves ? std::min(L.split, 2) : L.split;
+        nk = std::max(nk, (L.p[i].kblocks + sk - 1) / sk);
+    }
+    const size_t stage = kRlABytes + (build ? 0 : (size_t)nt_max * 128), bbuf = build ? (size_t)nk * nt_max * 128 : 0, tg = grouped ? round_up((size_t)nk * t.rt * 4, 16) : 0;
+    const size_t recv = (size_t)L.split * ((t.rt + L.split - 1) / L.split) * kRlTileM * 8;  // partial sums reuse the ring
+    int stages = std::min(nk, kRlMaxStages);
+    while (stages > 2 && stages * stage + bbuf + tg + 1024 > kRlHalfSm) --stages;
+    L.ring = (int)std::max(stages * stage, round_up(recv, 1024));
+    const size_t smem = L.ring + bbuf + tg + 1024;
+    if (smem > 200 * 1024) throw std::runtime_error("rows_linear: operands do not fit in shared memory");
+    int cols = 32;
+    while (cols < (grouped ? 2 * t.nt8 : nt_max)) cols *= 2;
+    L.tmem_cols = cols;
+    if (build)
+        rl_launch<false, true>(m, name, L, jobs, smem);
+    else if (grouped)
+        rl_launch<true, false>(m, name, L, jobs * L.split, smem);
+    else
+        rl_launch<false, false>(m, name, L, jobs * L.split, smem);
 }
 
-void run_linear(Model& m, const char* name, const LinReq* reqs, int n, int R) {
-    bool tc = R >= m.tc_min_rows;
-    for (int i = 0; i < n; ++i) tc = tc && reqs[i].W->tc_ok;
-    if (!tc) return run_linear_simt(m, name, reqs, n, R);
-    run_linear_tc(m, name, reqs, n, R);
+// Short fp16 rows (the rank-space vectors) of few sessions are converted inside the GEMM.
+bool rl_builds(const LinearW& W, const RowTiles& t) { return t.n == 1 && t.R <= 16 && rl_fmt(W) == RL_F16 && (size_t)((W.K + 63) / 64) * t.nt16 * 128 <= 44 * 1024; }
+
+void launch_ln_operands(Model& m, const char* name, const LnOperandsArgs& A) {
+    const int threads = std::max(kLnSumThreads, (int)round_up((size_t)(A.C / 8), 32));
+    if (threads > kLnMaxThreads) throw std::runtime_error("n_embd too large for the LayerNorm kernel");
+    // few rows: a CTA per (row, output), each repeating the row statistics; as rows fill the GPU a CTA takes several outputs (more
+    // than two CTAs per SM would have to wait for the predecessor's to leave)
+    const int gy = std::max(1, std::min(A.nout, 2 * m.num_sms / std::max(A.R, 1)));
+    const size_t smem = (size_t)A.C * 4 * (A.rows ? 2 : 1);
+    if (smem > 40 * 1024) RSV_CUDA(cudaFuncSetAttribute(ln_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 8 * kLnMaxThreads * 4));
+    LAUNCH(m, name) {
+        launch_pdl(m, ln_operands_kernel, dim3(A.R + A.nseg, gy), dim3(threads), smem, A);
+        check_launch("ln_operands");
+    }
+}
+int known_parts(int K) { return (K + 8 * kOpThreads - 1) / (8 * kOpThreads); }
+void launch_operand_known(Model& m, const float* x, int ldx, int K, const float* amax, int parts, const RowTiles& t, const RlOperandOut& o) {
+    LAUNCH(m, "operand_known") {
+        launch_pdl(m, operand_known_kernel, dim3(t.R, known_parts(K)), dim3(kOpThreads), 0, x, ldx, K, amax, parts, t.rt, o);
+        check_launch("operand_known");
+    }
+}
+void launch_operand_rows(Model& m, const OperandRowsArgs& A) {
+    LAUNCH(m, "operand_rows") {
+        launch_pdl(m, operand_rows_kernel, dim3((A.R * A.n + kOpThreads / 32 - 1) / (kOpThreads / 32)), dim3(kOpThreads), 0, A);
+        check_launch("operand_rows");
+    }
 }
 }  // namespace
 
@@ -885,13 +826,43 @@ void run_linear(Model& m, const char* name, const LinReq* reqs, int n, int R) {
 // ------------------------------------------------------------------------------------------------
 void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     const int R = (int)plan.rows.size(), S = (int)plan.segs.size(), O = (int)plan.out_rows.size();
-    const int C = cfg.n_embd, H = cfg.n_head, F = cfg.ffn_hidden, V = cfg.vocab, MIDS = cfg.mids();
+    const int C = cfg.n_embd, H = cfg.n_head, F = cfg.ffn_hidden, V = cfg.vocab, MIDS = cfg.mids(), NL = cfg.n_layer;
     if (R == 0) return;
     RSV_CUDA(cudaSetDevice(device));
-    const size_t RC = (size_t)R * C;
-    float* xm[6];
-    for (int i = 0; i < 6; ++i) xm[i] = ws.xmix + i * RC;  // order: r, w, k, v, a, g
-    float* staging = plan.multi_row_segments ? ws.staging : nullptr;
+    const LayerW& L0 = layers[0];
+    bool per_group = false;
+    for (const LayerW& L : layers)
+        for (const LinearW* W : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv}) per_group = per_group || rl_fmt(*W) == RL_I8G;
+    const RowTiles t = row_tiles(R, per_group), to = row_tiles(std::max(O, 1), rl_fmt(head) == RL_I8G);
+    // Operands of a layer; the matrices of one kind have the same format in every layer of the files the loader accepts, and where
+    // they do not, the operand is carved again.
+    OperandCarver cv;
+    struct LayerOps {
+        RlOperandOut r, w, k, v, a, g, vr, mid[4], y, x2, h;
+    };
+    auto carve_layer = [&](const LayerW& L, LayerOps& o) {
+        cv.used = 0;
+        o.r = cv.operand(t, rl_fmt(L.Wr), C, L.x_r);
+        o.k = cv.operand(t, rl_fmt(L.Wk), C, L.x_k);
+        o.v = cv.operand(t, rl_fmt(L.Wv), C, L.x_v);
+        o.w = cv.operand(t, RL_F16, C, L.x_w);
+        o.a = cv.operand(t, RL_F16, C, L.x_a);
+        o.g = cv.operand(t, RL_F16, C, L.x_g);
+        o.vr = rl_fmt(L.Wv) == RL_F16 ? o.v : cv.operand(t, RL_F16, C, L.x_v);
+        const int mids[4] = {cfg.w_mid, cfg.a_mid, cfg.g_mid, cfg.v_mid};
+        for (int i = 0; i < 4; ++i) o.mid[i] = cv.operand(t, RL_F16, mids[i]);
+        o.y = cv.operand(t, rl_fmt(L.Wo), C, nullptr, known_parts(C));
+        o.x2 = cv.operand(t, rl_fmt(L.Wfk), C, L.ffn_x_k);
+        o.h = cv.operand(t, rl_fmt(L.Wfv), F, nullptr, known_parts(F));
+    };
+    LayerOps ops;
+    carve_layer(L0, ops);
+    const size_t layer_bytes = cv.used;
+    RlOperandOut head_op = cv.operand(to, rl_fmt(head), C);
+    ensure_operand_memory(*this, cv.used);
+    cv.base = ws.op_mem;
+    cv.used = layer_bytes;
+    head_op = cv.operand(to, rl_fmt(head), C);
 
     LAUNCH(*this, "embed_ln0") {
         embed_ln0_kernel<<<R, kRowThreads, 0, stream>>>(emb, ln0_w, ln0_b, use_cursor ? ws.tok_list : ws.tokens, use_cursor ? ws.tok_pos : nullptr, R, C, V,
@@ -902,60 +873,105 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     // linear layer before it (x_cur + pending -> x_alt) so that no linear epilogue has to read-modify-write x.
     float *x_cur = ws.x, *x_alt = ws.x2;
     const float* pending = nullptr;
-    // few rows: several CTAs share a row of the LayerNorm + shift kernels (each recomputes the row statistics, then handles a
-    // slice of the channels), so that the step's latency does not hang on R single CTAs
-    // (a thread's channels are handled one after the other, each a dependent round of loads: five CTAs per row keep that to two rounds)
-    const int ln_split = std::max(R <= 512 ? 5 : 1, std::min(10, (2 * num_sms) / std::max(R, 1)));
     const size_t lay_x = (size_t)st.cap * C, lay_s = (size_t)st.cap * H * kHeadSize * kHeadSize;
-    for (int l = 0; l < cfg.n_layer; ++l) {
+    // LayerNorm + token shift: commits the shift states staged by the block before (`from` -> `to_state`), stages its own
+    auto ln_args = [&](const float* lw, const float* lb, float* shift_state, float* staging, const float* from, float* to_state) {
+        LnOperandsArgs A;
+        memset(&A, 0, sizeof(A));
+        A.x_in = x_cur;
+        A.delta = pending;
+        A.x_out = pending ? x_alt : nullptr;
+        A.lw = lw;
+        A.lb = lb;
+        A.rows = ws.row_meta;
+        A.shift_state = shift_state;
+        A.staging = staging;
+        A.commit_src = from;
+        A.commit_dst = to_state;
+        A.segs = ws.seg_meta;
+        A.R = R;
+        A.C = C;
+        A.rt = t.rt;
+        A.nseg = from ? S : 0;
+        return A;
+    };
+    float* vgate_buf = ws.xb;
+    for (int l = 0; l < NL; ++l) {
         const LayerW& L = layers[l];
+        carve_layer(L, ops);
+        if (cv.used > layer_bytes) throw std::runtime_error("layers of one model differ in their weight formats");
         float* tmix_x = st.tmix_x + l * lay_x;
         float* cmix_x = st.cmix_x + l * lay_x;
         float* wkv = st.wkv + l * lay_s;
-        LAUNCH(*this, "ln_shift6") {
-            MixPtrs mp{{L.x_r, L.x_w, L.x_k, L.x_v, L.x_a, L.x_g}};
-            launch_pdl(*this, ln_shift_kernel<6>, dim3(R, ln_split), dim3(kRowThreads), 0, x_cur, pending, x_alt, L.ln1_w, L.ln1_b, mp, ws.row_meta, R, C, tmix_x, staging, ws.xmix);
-            check_launch("ln_shift6");
+        {
+            LnOperandsArgs A = ln_args(L.ln1_w, L.ln1_b, tmix_x, ws.staging_t, l ? ws.staging_c : nullptr, l ? cmix_x - lay_x : nullptr);
+            const RlOperandOut* out[7] = {&ops.r, &ops.k, &ops.v, &ops.w, &ops.a, &ops.g, &ops.vr};
+            const bool shared_v = ops.vr.img == ops.v.img;
+            A.nout = l == 0 || shared_v ? 6 : 7;
+            for (int i = 0; i < A.nout; ++i) A.out[i] = *out[i];
+            launch_ln_operands(*this, "ln_shift6", A);
         }
         if (pending) {
             std::swap(x_cur, x_alt);
             pending = nullptr;
         }
-        if (staging) LAUNCH(*this, "commit_shift") {
-                launch_pdl(*this, commit_shift_kernel, dim3(S), dim3(256), 0, staging, ws.seg_meta, C, tmix_x);
-                check_launch("commit_shift");
-            }
-        float* vgate = l == 0 ? nullptr : ws.xb;  // xb is free until ln_shift1
+        float* vgate = l == 0 ? nullptr : vgate_buf;
         {
             // r, k, v and the four rank-space projections in one launch
             float* mw = ws.mid;
             float* ma = mw + cfg.w_mid;
             float* mv = ma + cfg.a_mid;
             float* mg = mv + cfg.v_mid;
-            LinReq q[7] = {
-                {&L.Wr, xm[0], C, ws.r, C, EPI_STORE},
-                {&L.Wk, xm[2], C, ws.k, C, EPI_STORE},
-                {&L.Wv, xm[3], C, ws.v, C, EPI_STORE, nullptr, nullptr, 0, l == 0 ? ws.vfirst : nullptr},
-                {&L.w1, xm[1], C, mw, MIDS, EPI_TANH},
-                {&L.a1, xm[4], C, ma, MIDS, EPI_STORE},
-                {&L.g1, xm[5], C, mg, MIDS, EPI_SIGMOID},
-                {&L.v1, xm[3], C, mv, MIDS, EPI_STORE},
+            RlReq q[7] = {
+                {&L.Wr, &ops.r, ws.r, C, EPI_STORE},
+                {&L.Wk, &ops.k, ws.k, C, EPI_STORE},
+                {&L.Wv, &ops.v, ws.v, C, EPI_STORE, nullptr, l == 0 ? ws.vfirst : nullptr},
+                {&L.w1, &ops.w, mw, MIDS, EPI_TANH},
+                {&L.a1, &ops.a, ma, MIDS, EPI_STORE},
+                {&L.g1, &ops.g, mg, MIDS, EPI_SIGMOID},
+                {&L.v1, &ops.vr, mv, MIDS, EPI_STORE},
             };
-            run_linear(*this, "linear_rkv_rank", q, l == 0 ? 6 : 7, R);
-            // back-projections: decay w, a, gate g and (layers > 0) the v-lerp gate; all plain stores
-            LinReq q2[4] = {
-                {&L.w2, mw, MIDS, ws.w, C, EPI_DECAY, L.w0},
-                {&L.a2, ma, MIDS, ws.a, C, EPI_SIGMOID_BIAS, L.a0},
-                {&L.g2, mg, MIDS, ws.g, C, EPI_STORE},
-                {&L.v2, mv, MIDS, vgate, C, EPI_SIGMOID_BIAS, L.v0},
+            run_rows_linear(*this, "linear_rkv_rank", q, l == 0 ? 6 : 7, t);
+            // back-projections: decay w, a, gate g and (layers > 0) the v-lerp gate
+            const int nb = l == 0 ? 3 : 4;
+            const LinearW* Wb[4] = {&L.w2, &L.a2, &L.g2, &L.v2};
+            const float* src[4] = {mw, ma, mg, mv};
+            bool build = true;
+            for (int i = 0; i < nb; ++i) build = build && rl_builds(*Wb[i], t);
+            if (!build) {
+                OperandRowsArgs A;
+                memset(&A, 0, sizeof(A));
+                A.R = R;
+                A.rt = t.rt;
+                A.n = nb;
+                for (int i = 0; i < nb; ++i) {
+                    A.x[i] = src[i];
+                    A.ldx[i] = MIDS;
+                    A.K[i] = Wb[i]->K;
+                    A.out[i] = ops.mid[i];
+                }
+                launch_operand_rows(*this, A);
+            }
+            RlReq q2[4] = {
+                {&L.w2, &ops.mid[0], ws.w, C, EPI_DECAY, L.w0},
+                {&L.a2, &ops.mid[1], ws.a, C, EPI_SIGMOID_BIAS, L.a0},
+                {&L.g2, &ops.mid[2], ws.g, C, EPI_STORE},
+                {&L.v2, &ops.mid[3], vgate, C, EPI_SIGMOID_BIAS, L.v0},
             };
-            run_linear(*this, "linear_rank_back", q2, l == 0 ? 3 : 4, R);
+            if (build)
+                for (int i = 0; i < nb; ++i) {
+                    q2[i].op = nullptr;
+                    q2[i].x = src[i];
+                    q2[i].ldx = MIDS;
+                }
+            run_rows_linear(*this, "linear_rank_back", q2, nb, t);
         }
+        int yparts = H;  // maxima a row of yg comes with
         LAUNCH(*this, "wkv7") {
             const int n_items = H * S;
             if (plan.multi_row_segments) {
                 // prefill chunks: vectors built by preparation warps, only state-dependent work in the per-token chain (wkv_seq.cuh)
-// few (head, segment) pairs: a head over two CTAs
+                // few (head, segment) pairs: a head over two CTAs
                 if (H * S <= num_sms) {
                     launch_pdl(*this, wkv7_seq_kernel<2>, dim3(2 * H, S), dim3(kWsThreads), 0, ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, ws.g,
                                L.k_k, L.k_a, L.r_k, L.lnx_w, L.lnx_b, wkv, l == 0 ? st.v_first : nullptr, ws.yg, H, C, ws.status);
@@ -964,7 +980,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
                                L.k_k, L.k_a, L.r_k, L.lnx_w, L.lnx_b, wkv, l == 0 ? st.v_first : nullptr, ws.yg, H, C, ws.status);
                 }
                 launch_pdl(*this, wkv7_finish_kernel, dim3((R * H + kWsFinishThreads / 32 - 1) / (kWsFinishThreads / 32)), dim3(kWsFinishThreads), 0, ws.r, ws.k,
-                           ws.v, vgate, ws.vfirst, ws.a, ws.g, L.k_a, L.r_k, L.lnx_w, L.lnx_b, ws.yg, R, H, C);
+                           ws.v, vgate, ws.vfirst, ws.a, ws.g, L.k_a, L.r_k, L.lnx_w, L.lnx_b, ws.yg, R, H, C, ws.ymax);
             } else if (n_items >= 4 * num_sms) {
                 // many (session, head) pairs: one state row per lane, states staged by TMA (wkv_rows.cuh)
                 const size_t rows_total = (size_t)cfg.n_layer * st.cap * H * kHeadSize;
@@ -982,46 +998,60 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
                 const int ctas = std::min((n_items + kWrPairs - 1) / kWrPairs, num_sms);
                 launch_pdl(*this, wkv7_rows_kernel, dim3(ctas), dim3(kWrThreads), kWrSmemBytes, st.wkv_map, (long long)l * st.cap * H * kHeadSize, ws.seg_meta,
                            n_items, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, ws.g, L.k_k, L.k_a, L.r_k, L.lnx_w, L.lnx_b,
-                           l == 0 ? st.v_first : nullptr, ws.yg, H, C, ws.status);
+                           l == 0 ? st.v_first : nullptr, ws.yg, H, C, ws.status, ws.ymax);
+                yparts = 2 * H;
             } else {
                 launch_pdl(*this, wkv7_kernel, dim3(H, S), dim3(kWkvThreads), 0, ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, ws.g, L.k_k, L.k_a,
-                           L.r_k, L.lnx_w, L.lnx_b, wkv, l == 0 ? st.v_first : nullptr, ws.yg, H, C);
+                           L.r_k, L.lnx_w, L.lnx_b, wkv, l == 0 ? st.v_first : nullptr, ws.yg, H, C, ws.ymax);
             }
             check_launch("wkv7");
         }
+        // a linear layer on activations whose row maxima their producer collected
+        auto linear_known = [&](const char* name, RlReq q, const float* x, int ldx, const float* amax, int parts, const RlOperandOut& op) {
+            launch_operand_known(*this, x, ldx, q.W->K, amax, parts, t, op);
+            q.op = &op;
+            run_rows_linear(*this, name, &q, 1, t);
+        };
+        linear_known("linear_att_out", RlReq{&L.Wo, nullptr, ws.delta, C, EPI_STORE}, ws.yg, C, ws.ymax, yparts, ops.y);
+        pending = ws.delta;
         {
-            LinReq q = {&L.Wo, ws.yg, C, ws.delta, C, EPI_STORE};
-            run_linear(*this, "linear_att_out", &q, 1, R);
-            pending = ws.delta;
-        }
-        LAUNCH(*this, "ln_shift1") {
-            MixPtrs mp{{L.ffn_x_k, nullptr, nullptr, nullptr, nullptr, nullptr}};
-            launch_pdl(*this, ln_shift_kernel<1>, dim3(R, ln_split), dim3(kRowThreads), 0, x_cur, pending, x_alt, L.ln2_w, L.ln2_b, mp, ws.row_meta, R, C, cmix_x, staging, ws.xb);
-            check_launch("ln_shift1");
+            LnOperandsArgs A = ln_args(L.ln2_w, L.ln2_b, cmix_x, ws.staging_c, ws.staging_t, tmix_x);
+            A.nout = 1;
+            A.out[0] = ops.x2;
+            launch_ln_operands(*this, "ln_shift1", A);
         }
         std::swap(x_cur, x_alt);
         pending = nullptr;
-        if (staging) LAUNCH(*this, "commit_shift") {
-                launch_pdl(*this, commit_shift_kernel, dim3(S), dim3(256), 0, staging, ws.seg_meta, C, cmix_x);
-                check_launch("commit_shift");
-            }
         {
-            LinReq q = {&L.Wfk, ws.xb, C, ws.h, F, EPI_RELU2};
-            run_linear(*this, "linear_ffn_key", &q, 1, R);
-            LinReq q2 = {&L.Wfv, ws.h, F, ws.delta, C, EPI_STORE};
-            run_linear(*this, "linear_ffn_value", &q2, 1, R);
-            pending = ws.delta;
+            RlReq q = {&L.Wfk, &ops.x2, ws.h, F, EPI_RELU2};
+            q.ymax = ws.hmax;
+            run_rows_linear(*this, "linear_ffn_key", &q, 1, t);
         }
+        linear_known("linear_ffn_value", RlReq{&L.Wfv, nullptr, ws.delta, C, EPI_STORE}, ws.h, F, ws.hmax, (F + kRlTileM - 1) / kRlTileM, ops.h);
+        pending = ws.delta;
+    }
+    LAUNCH(*this, "commit_shift") {
+        launch_pdl(*this, commit_shift_kernel, dim3(S), dim3(256), 0, ws.staging_c, ws.seg_meta, C, st.cmix_x + (size_t)(NL - 1) * lay_x);
+        check_launch("commit_shift");
     }
     ws.final_x = x_cur;
     ws.final_delta = pending;
     if (O) {
-        LAUNCH(*this, "ln_out") {
-            ln_rows_kernel<<<O, kRowThreads, 0, stream>>>(x_cur, pending, ln_out_w, ln_out_b, ws.out_rows, C, ws.xn);
-            check_launch("ln_out");
-        }
-        LinReq q = {&head, ws.xn, C, ws.logits, V, EPI_STORE};
-        run_linear(*this, "linear_head", &q, 1, O);
+        LnOperandsArgs A;
+        memset(&A, 0, sizeof(A));
+        A.x_in = x_cur;
+        A.delta = pending;
+        A.lw = ln_out_w;
+        A.lb = ln_out_b;
+        A.row_map = ws.out_rows;
+        A.R = O;
+        A.C = C;
+        A.rt = to.rt;
+        A.nout = 1;
+        A.out[0] = head_op;
+        launch_ln_operands(*this, "ln_out", A);
+        RlReq q = {&head, &head_op, ws.logits, V, EPI_STORE};
+        run_rows_linear(*this, "linear_head", &q, 1, to);
     }
     if (use_cursor) LAUNCH(*this, "advance_cursor") {
             advance_cursor_kernel<<<1, 1, 0, stream>>>(ws.tok_pos);
@@ -1029,345 +1059,6 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         }
 }
 
-
-// ------------------------------------------------------------------------------------------------
-// persistent decode kernel: host side
-// ------------------------------------------------------------------------------------------------
-namespace {
-
-DpMat make_dpmat(const LinearW& W, int map_index) {
-    DpMat d;
-    d.map = map_index;
-    d.M = W.M;
-    d.mtiles = W.Mpad / kTcTileM;
-    d.is_i8 = W.wtype == W_INT8;
-    d.kblocks = (int)((size_t)W.Kpad * (d.is_i8 ? 1 : 2) / kTcKBlockBytes);
-    d.K = W.K;
-    d.wscale = W.wscale;
-    d.wzero = W.wzero;
-    return d;
-}
-struct HostProb {
-    int mtiles, kblocks;
-};
-// largest number of CTAs that share one tile, and per CTA the largest numbers of operand tiles, units, runs and
-// problem shares, for one phase shape (the device builds its tables with the same formulas)
-struct PhaseShape {
-    int pmax = 1, btiles = 0, tiles = 0, units = 0, runs = 0, shares = 0;
-};
-PhaseShape phase_shape(const std::vector<HostProb>& probs, int G) {
-    PhaseShape ps;
-    int U = 0;
-    std::vector<int> unit0;
-    for (auto& q : probs) {
-        unit0.push_back(U);
-        U += q.mtiles * q.kblocks;
-    }
-    G = dp_choose_ge(unit0.data(), (int)unit0.size(), U, G);  // CTAs that take part in the phase (same rule as on the device)
-    int u0 = 0;
-    for (auto& q : probs) {
-        for (int t = 0; t < q.mtiles; ++t) {
-            const int first = u0 + t * q.kblocks;
-            ps.pmax = std::max(ps.pmax, tc_cta_of_unit(first + q.kblocks - 1, U, G) - tc_cta_of_unit(first, U, G) + 1);
-        }
-        u0 += q.mtiles * q.kblocks;
-        ps.tiles += q.mtiles;
-    }
-    for (int c = 0; c < G; ++c) {
-        const int ub = tc_cta_begin(c, U, G), ue = tc_cta_begin(c + 1, U, G);
-        int need = 0, p0 = 0, runs = 0, shares = 0;
-        for (auto& q : probs) {
-            const int lo = std::max(ub, p0), hi = std::min(ue, p0 + q.mtiles * q.kblocks);
-            if (hi > lo) {
-                need += std::min(hi - lo, q.kblocks);
-                ++shares;
-                runs += (hi - 1 - p0) / q.kblocks - (lo - p0) / q.kblocks + 1;
-            }
-            p0 += q.mtiles * q.kblocks;
-        }
-        ps.btiles = std::max(ps.btiles, need);
-        ps.units = std::max(ps.units, ue - ub);
-        ps.runs = std::max(ps.runs, runs);
-        ps.shares = std::max(ps.shares, shares);
-    }
-    return ps;
-}
-
-}  // namespace
-
-bool Model::persistent_available(int nb) {
-    if (!use_persistent || nb < 1 || nb > kDpMaxNB) return false;
-    if (nb == 1 && stream_available()) return true;  // one session: the weight-streaming kernel
-    PersistentCtx& pc = pctx;
-    if (pc.tried) return pc.ok;
-    pc.tried = true;
-    auto fail = [&](const std::string& why) {
-        pc.why = why;
-        pc.ok = false;
-        return false;
-    };
-    RSV_CUDA(cudaSetDevice(device));
-    int coop = 0;
-    RSV_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
-    if (!coop) return fail("device does not support cooperative launches");
-    if (!head.tc_ok) return fail("head matrix cannot take the tensor-core path");
-    for (const LayerW& L : layers)
-        for (const LinearW* W : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv, &L.w1, &L.a1, &L.v1, &L.g1})
-            if (!W->tc_ok) return fail("a weight matrix cannot take the tensor-core path (int8 files need one scale/zero per output row)");
-    const int L = cfg.n_layer, C = cfg.n_embd;
-    // tensor maps and per-layer tables
-    std::vector<CUtensorMap> maps;
-    std::vector<DpLayer> dl(L);
-    auto add = [&](const LinearW& W) {
-        maps.push_back(W.amap);
-        return make_dpmat(W, (int)maps.size() - 1);
-    };
-    for (int l = 0; l < L; ++l) {
-        const LayerW& Lw = layers[l];
-        DpLayer& d = dl[l];
-        memset(&d, 0, sizeof(d));
-        d.mat[DM_WR] = add(Lw.Wr);
-        d.mat[DM_WK] = add(Lw.Wk);
-        d.mat[DM_WV] = add(Lw.Wv);
-        d.mat[DM_WO] = add(Lw.Wo);
-        d.mat[DM_WFK] = add(Lw.Wfk);
-        d.mat[DM_WFV] = add(Lw.Wfv);
-        d.mat[DM_W1] = add(Lw.w1);
-        d.mat[DM_A1] = add(Lw.a1);
-        d.mat[DM_V1] = add(Lw.v1);
-        d.mat[DM_G1] = add(Lw.g1);
-        d.w2 = (const __half*)Lw.w2.w;
-        d.a2 = (const __half*)Lw.a2.w;
-        d.v2 = (const __half*)Lw.v2.w;
-        d.g2 = (const __half*)Lw.g2.w;
-        d.ln1_w = Lw.ln1_w;
-        d.ln1_b = Lw.ln1_b;
-        d.ln2_w = Lw.ln2_w;
-        d.ln2_b = Lw.ln2_b;
-        d.lnx_w = Lw.lnx_w;
-        d.lnx_b = Lw.lnx_b;
-        d.x_r = Lw.x_r;
-        d.x_w = Lw.x_w;
-        d.x_k = Lw.x_k;
-        d.x_v = Lw.x_v;
-        d.x_a = Lw.x_a;
-        d.x_g = Lw.x_g;
-        d.ffn_x_k = Lw.ffn_x_k;
-        d.w0 = Lw.w0;
-        d.a0 = Lw.a0;
-        d.v0 = Lw.v0;
-        d.r_k = Lw.r_k;
-        d.k_k = Lw.k_k;
-        d.k_a = Lw.k_a;
-    }
-    DpParams P;
-    memset(&P, 0, sizeof(P));
-    P.head = add(head);
-    const int G = num_sms;
-    // phase shapes (layer 0 has no v1 problem; all layers share the matrix shapes)
-    auto hp = [&](const DpMat& d) { return HostProb{d.mtiles, d.kblocks}; };
-    const DpLayer& d0 = dl[0];
-    std::vector<HostProb> p1a = {hp(d0.mat[DM_WR]), hp(d0.mat[DM_WK]), hp(d0.mat[DM_WV]), hp(d0.mat[DM_W1]), hp(d0.mat[DM_A1]), hp(d0.mat[DM_G1])};
-    std::vector<HostProb> p1b = p1a;
-    p1b.push_back(hp(d0.mat[DM_V1]));
-    int pmax[5], tiles[5], btiles = 0, max_units = 8, max_runs = 0, max_shares = 0;
-    {
-        const PhaseShape a = phase_shape(p1a, G), b = phase_shape(p1b, G);
-        pmax[0] = std::max(a.pmax, b.pmax);
-        tiles[0] = b.tiles;
-        btiles = std::max(a.btiles, b.btiles);
-        max_units += a.units + b.units;
-        max_runs = std::max(a.runs, b.runs);
-        max_shares = std::max(a.shares, b.shares);
-    }
-    const DpMat* single[4] = {&d0.mat[DM_WO], &d0.mat[DM_WFK], &d0.mat[DM_WFV], &P.head};
-    for (int i = 0; i < 4; ++i) {
-        const PhaseShape a = phase_shape({hp(*single[i])}, G);
-        pmax[i + 1] = a.pmax;
-        tiles[i + 1] = a.tiles;
-        btiles = std::max(btiles, a.btiles);
-        max_units += a.units;
-        max_runs = std::max(max_runs, a.runs);
-        max_shares = std::max(max_shares, a.shares);
-    }
-    if (max_runs > kDpMaxRuns || max_shares > kDpMaxShares) return fail("schedule tables of the persistent kernel are too small for this shape");
-    if (btiles > 255) return fail("too many operand tiles per CTA for this shape");
-    if (C > 16 * kDpWorkers) return fail("n_embd too large for the persistent kernel's register-resident LayerNorm");
-    if ((C + G - 1) / G + 1 > kDpMaxSlice) return fail("n_embd too large for the persistent kernel's per-CTA slice of the residual stream");
-    // shared memory: ring + operand tiles + barriers + worker scratch
-    const size_t fixed = (size_t)btiles * kDpBTile + 1024 /*alignment*/ + 2048 /*barriers, small scratch*/ + (size_t)btiles * kDpMaxNB * 8 +
-                         (size_t)cfg.mids() * 4 + 8 * 64 * 4 + (size_t)kDpMaxNB * kDpMaxSlice * 4 + 2 * sizeof(DpLayer) + DV_COUNT * sizeof(DpVar) + (size_t)max_units * sizeof(DpUnit);
-    const size_t budget = 227 * 1024;
-    if (fixed + 3 * (size_t)kDpATile > budget) return fail("operand tiles do not fit in shared memory for this shape");
-    const int nstages = (int)std::min<size_t>(10, (budget - fixed) / kDpATile);
-    pc.smem = fixed + (size_t)nstages * kDpATile;
-    pc.grid = G;
-    pc.nstages = nstages;
-    pc.btiles = btiles;
-    RSV_CUDA(cudaFuncSetAttribute(decode_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pc.smem));
-    int per_sm = 0;
-    RSV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_persistent_kernel, kDpThreads, pc.smem));
-    if (per_sm < 1) return fail("persistent kernel does not fit on an SM");
-    // device tables and scratch
-    RSV_CUDA(cudaMalloc(&pc.d_layers, dl.size() * sizeof(DpLayer)));
-    RSV_CUDA(cudaMalloc(&pc.d_maps, maps.size() * sizeof(CUtensorMap)));
-    RSV_CUDA(cudaMemcpy(pc.d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
-    RSV_CUDA(cudaMalloc(&pc.x, (size_t)kDpMaxNB * C * 4));
-    RSV_CUDA(cudaMalloc(&pc.yg, (size_t)kDpMaxNB * C * 4));
-    RSV_CUDA(cudaMalloc(&pc.vfirst, (size_t)kDpMaxNB * C * 4));
-    RSV_CUDA(cudaMalloc(&pc.rkv, (size_t)kDpMaxNB * 3 * C * 4));
-    RSV_CUDA(cudaMalloc(&pc.mid, (size_t)kDpMaxNB * cfg.mids() * 4));
-    RSV_CUDA(cudaMalloc(&pc.hbuf, (size_t)kDpMaxNB * cfg.ffn_hidden * 4));
-    RSV_CUDA(cudaMemsetAsync(pc.mid, 0, (size_t)kDpMaxNB * cfg.mids() * 4, stream));
-    RSV_CUDA(cudaMalloc(&pc.cand_val, (size_t)G * kDpMaxNB * 4));
-    RSV_CUDA(cudaMalloc(&pc.cand_idx, (size_t)G * kDpMaxNB * 4));
-    RSV_CUDA(cudaMalloc(&pc.grid_bar, 4));
-#ifdef RSV_DP_DEBUG
-    RSV_CUDA(cudaMalloc(&pc.dbg, (64 + 8 * 1024) * sizeof(long long)));
-    RSV_CUDA(cudaMemsetAsync(pc.dbg, 0, (64 + 8 * 1024) * sizeof(long long), stream));
-#endif
-    RSV_CUDA(cudaMemsetAsync(pc.vfirst, 0, (size_t)kDpMaxNB * C * 4, stream));
-    for (int i = 0; i < 5; ++i) {
-        const size_t runs = (size_t)tiles[i] * pmax[i];
-        RSV_CUDA(cudaMalloc(&pc.region_data[i], runs * kDpN * 128 * 4));
-        RSV_CUDA(cudaMalloc(&pc.region_meta[i], runs * kDpWarps * sizeof(DpRunMeta)));
-        RSV_CUDA(cudaMalloc(&pc.region_cnt[i], (size_t)tiles[i] * kDpWarps * sizeof(int)));
-        pc.region_cnt_bytes[i] = (size_t)tiles[i] * kDpWarps * sizeof(int);
-        RSV_CUDA(cudaMemsetAsync(pc.region_data[i], 0, runs * kDpN * 128 * 4, stream));
-        RSV_CUDA(cudaMemsetAsync(pc.region_meta[i], 0, runs * kDpWarps * sizeof(DpRunMeta), stream));
-        RSV_CUDA(cudaMemsetAsync(pc.region_cnt[i], 0, (size_t)tiles[i] * kDpWarps * sizeof(int), stream));
-        pc.region_pmax[i] = pmax[i];
-    }
-    // layer tables need the state pointers of the call: only the state-independent part is stored here
-    pc.params_template.resize(sizeof(DpParams) + dl.size() * sizeof(DpLayer));
-    P.maps = (const CUtensorMap*)pc.d_maps;
-    P.layers = (const DpLayer*)pc.d_layers;
-    P.emb = emb;
-    P.ln0_w = ln0_w;
-    P.ln0_b = ln0_b;
-    P.lno_w = ln_out_w;
-    P.lno_b = ln_out_b;
-    P.L = L;
-    P.C = C;
-    P.H = cfg.n_head;
-    P.F = cfg.ffn_hidden;
-    P.V = cfg.vocab;
-    P.wm = cfg.w_mid;
-    P.am = cfg.a_mid;
-    P.vm = cfg.v_mid;
-    P.gm = cfg.g_mid;
-    P.x = pc.x;
-    P.yg = pc.yg;
-    P.vfirst = pc.vfirst;
-    P.rkv = pc.rkv;
-    P.mid = pc.mid;
-    P.hbuf = pc.hbuf;
-    for (int i = 0; i < 5; ++i) {
-        P.reg[i].data = (uint32_t*)pc.region_data[i];
-        P.reg[i].meta = (DpRunMeta*)pc.region_meta[i];
-        P.reg[i].cnt = pc.region_cnt[i];
-        P.reg[i].pmax = pmax[i];
-    }
-    P.dbg = pc.dbg;
-    P.cand_val = pc.cand_val;
-    P.cand_idx = pc.cand_idx;
-    P.grid_bar = pc.grid_bar;
-    P.status = ws.status;
-    P.nstages = nstages;
-    P.btiles = btiles;
-    P.max_units = max_units;
-    memcpy(pc.params_template.data(), &P, sizeof(P));
-    memcpy(pc.params_template.data() + sizeof(P), dl.data(), dl.size() * sizeof(DpLayer));
-    pc.ok = true;
-    return true;
-}
-
-void Model::run_persistent(State& st, int nb, const int* slots, int n_tokens, bool tok_from_list, bool argmax_feed, uint32_t* seq_dev, int* seq_cnt_dev,
-                           int seq_cap) {
-    if (nb == 1 && stream_available()) return run_stream(st, slots[0], n_tokens, tok_from_list, argmax_feed, seq_dev, seq_cnt_dev, seq_cap);
-    if (!persistent_available(nb)) throw std::runtime_error("persistent decode path unavailable: " + pctx.why);
-    PersistentCtx& pc = pctx;
-    RSV_CUDA(cudaSetDevice(device));
-    const int L = cfg.n_layer, C = cfg.n_embd, H = cfg.n_head;
-    ensure_workspace(std::max(nb, 1), std::max(nb, 1), std::max(nb, 1));
-    DpParams P;
-    memcpy(&P, pc.params_template.data(), sizeof(P));
-    // the device layer table carries the state pointers: rewrite it only when another state is used
-    if (pc.bound_tmix != st.tmix_x || pc.bound_wkv != st.wkv || pc.bound_cmix != st.cmix_x || pc.bound_cap != st.cap) {
-        std::vector<DpLayer> dl(L);
-        memcpy(dl.data(), pc.params_template.data() + sizeof(P), dl.size() * sizeof(DpLayer));
-        const size_t lay_x = (size_t)st.cap * C, lay_s = (size_t)st.cap * H * kHeadSize * kHeadSize;
-        for (int l = 0; l < L; ++l) {
-            dl[l].tmix_x = st.tmix_x + l * lay_x;
-            dl[l].cmix_x = st.cmix_x + l * lay_x;
-            dl[l].wkv = st.wkv + l * lay_s;
-        }
-        RSV_CUDA(cudaStreamSynchronize(stream));  // earlier launches may still read the table
-        RSV_CUDA(cudaMemcpyAsync(pc.d_layers, dl.data(), dl.size() * sizeof(DpLayer), cudaMemcpyHostToDevice, stream));
-        RSV_CUDA(cudaStreamSynchronize(stream));  // `dl` is a local pageable buffer
-        pc.bound_tmix = st.tmix_x;
-        pc.bound_wkv = st.wkv;
-        pc.bound_cmix = st.cmix_x;
-        pc.bound_cap = st.cap;
-    }
-    P.nb = nb;
-    for (int b = 0; b < kDpMaxNB; ++b) P.slot[b] = b < nb ? slots[b] : 0;
-    P.state_vfirst = st.v_first;
-    P.tokens = ws.tokens;
-    P.tok_list = ws.tok_list;
-    P.seq = seq_dev;
-    P.seq_cnt = seq_cnt_dev;
-    P.seq_cap = seq_cap;
-    P.logits = ws.logits;
-    P.status = ws.status;
-    P.n_tokens = n_tokens;
-    P.tok_from_list = tok_from_list ? 1 : 0;
-    P.argmax_feed = argmax_feed ? 1 : 0;
-    RSV_CUDA(cudaMemsetAsync(pc.grid_bar, 0, 4, stream));
-    void* args[] = {&P};
-    LAUNCH(*this, "decode_persistent") {
-        RSV_CUDA(cudaLaunchCooperativeKernel((const void*)decode_persistent_kernel, dim3(pc.grid), dim3(kDpThreads), args, pc.smem, stream));
-    }
-#ifdef RSV_DP_DEBUG
-    if (pc.dbg && n_tokens >= 2) {
-        std::vector<long long> hv(64 + 8 * 1024);
-        long long* h = hv.data();
-        RSV_CUDA(cudaStreamSynchronize(stream));
-        RSV_CUDA(cudaMemcpy(h, pc.dbg, hv.size() * sizeof(long long), cudaMemcpyDeviceToHost));
-        const char* names[7] = {"phase start", "stats done", "operands done", "runs drained", "barrier done", "x slice done", "barrier b done"};
-        long long t0 = h[0];
-        fprintf(stderr, "[persistent kernel, CTA 0, token 1, layer 1] times in us since P1 start\n");
-        for (int ph = 0; ph < 4; ++ph) {
-            if (ph == 1) fprintf(stderr, "  heads done %.2f, barrier 2 done %.2f\n", (h[40] - t0) / 1e3, (h[41] - t0) / 1e3);
-            for (int i = 0; i < 7; ++i)
-                if (h[ph * 10 + i]) fprintf(stderr, "  phase %d %-14s %.2f\n", ph, names[i], (h[ph * 10 + i] - t0) / 1e3);
-        }
-        {
-            const char* nm[5] = {"operands done", "partials stored", "arrivals returned", "finishing done", "barrier left"};
-            const long long p3 = h[10];  // CTA 0, phase 3 start
-            for (int k = 0; k < 5; ++k) {
-                long long mn = 1LL << 62, mx = 0, sum = 0;
-                int amx = -1, n = 0;
-                for (int c = 0; c < pc.grid && c < 1024; ++c) {
-                    const long long v = h[64 + c * 8 + k];
-                    if (!v) continue;
-                    ++n;
-                    sum += v - p3;
-                    if (v < mn) mn = v;
-                    if (v > mx) {
-                        mx = v;
-                        amx = c;
-                    }
-                }
-                if (n) fprintf(stderr, "  att.output phase, all CTAs: %-18s min %.2f avg %.2f max %.2f (CTA %d) [us since CTA 0 entered the phase]\n", nm[k], (mn - p3) / 1e3, sum / 1e3 / n, (mx - p3) / 1e3, amx);
-            }
-        }
-        fprintf(stderr, "  ffn.key operands: loads start %.2f, values loaded %.2f, scale set %.2f, digits written %.2f\n", (h[63] - t0) / 1e3, (h[60] - t0) / 1e3, (h[61] - t0) / 1e3, (h[62] - t0) / 1e3);
-        fprintf(stderr, "  ffn.key phase: producer issued its %lld tiles from %.2f to %.2f; MMA thread started %.2f, last issue %.2f, waited %.2f us for tiles/accumulators\n",
-                h[53], (h[55] - t0) / 1e3, (h[56] - t0) / 1e3, (h[50] - t0) / 1e3, (h[51] - t0) / 1e3, h[52] / 1e3);
-    }
-#endif
-}
 
 // ------------------------------------------------------------------------------------------------
 // batch-1 weight-streaming decode kernel: host side
@@ -1400,7 +1091,7 @@ void dispatch_stream(int cmax, const DsParams& P, int grid, size_t smem, cudaStr
 }  // namespace
 
 bool Model::stream_available() {
-    if (!use_persistent || !use_stream) return false;
+    if (!use_stream) return false;
     StreamCtx& sc = sctx;
     if (sc.tried) return sc.ok;
     sc.tried = true;
@@ -1658,12 +1349,6 @@ void Model::check_status() {
     const int s = sw[0];
     if (s) {
         RSV_CUDA(cudaMemsetAsync(ws.status, 0, 2 * sizeof(int), stream));
-        if (s & (2 | 4 | 32)) {
-            // a kernel that gave up on a wait may have left arrival counters non-zero: the next launch must start from zero
-            if (ws.tc_cnt) RSV_CUDA(cudaMemsetAsync(ws.tc_cnt, 0, (size_t)kTcMaxSplit * kTcEpiWarps * sizeof(int), stream));
-            for (int i = 0; i < 5; ++i)
-                if (pctx.region_cnt[i]) RSV_CUDA(cudaMemsetAsync(pctx.region_cnt[i], 0, pctx.region_cnt_bytes[i], stream));
-        }
         if (s & 32) {
             static const char* const site[5] = {"a wait", "a chunk of weight rows", "room in the ring", "a grid barrier", "a chunk of a head's rows"};
             const int k = sw[1] & 15;
@@ -1671,8 +1356,7 @@ void Model::check_status() {
                                      std::to_string((sw[1] >> 20) & 255) + ", index " + std::to_string((sw[1] >> 4) & 0xFFFF) + ")");
         }
         if (s & 16) throw std::runtime_error("WKV kernel gave up waiting for a staged state (device status bit 4)");
-        if (s & 8) throw std::runtime_error("persistent decode kernel: schedule tables too small for this shape (device status bit 3)");
-        if (s & 4) throw std::runtime_error("persistent decode kernel gave up waiting on a barrier (device status bit 2)");
+        if (s & 8) throw std::runtime_error("weight-streaming decode kernel: chunk table too small for this shape (device status bit 3)");
         if (s & 2) throw std::runtime_error("tensor-core kernel gave up waiting on a barrier (device status bit 1)");
         if (s & 1) throw std::runtime_error("token id out of range (>= vocab); the embedding row 0 was used instead");
         throw std::runtime_error("device status word = " + std::to_string(s));
@@ -1795,13 +1479,13 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
     const int sms = prop.multiProcessorCount, n_items = H * nseg;
     if (variant == 0) variant = T > 1 ? (n_items <= sms ? 3 : 4) : (n_items >= 4 * sms ? 2 : 1);
     if (variant == 1) {
-        wkv7_kernel<<<dim3(H, nseg), kWkvThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C);
+        wkv7_kernel<<<dim3(H, nseg), kWkvThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C, nullptr);
     } else if (variant == 2) {
         CUtensorMap map;
         encode_state_map(&map, state, (size_t)nseg * H * kHeadSize);
         RSV_CUDA(cudaFuncSetAttribute(wkv7_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWrSmemBytes));
         const int ctas = std::min((n_items + kWrPairs - 1) / kWrPairs, sms);
-        wkv7_rows_kernel<<<ctas, kWrThreads, kWrSmemBytes>>>(map, 0LL, sm, n_items, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, nullptr, yg, H, C, status);
+        wkv7_rows_kernel<<<ctas, kWrThreads, kWrSmemBytes>>>(map, 0LL, sm, n_items, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, nullptr, yg, H, C, status, nullptr);
     } else if (variant == 3 || variant == 4) {
         if (variant == 3)
             wkv7_seq_kernel<2><<<dim3(2 * H, nseg), kWsThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C, status);
@@ -1809,7 +1493,7 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
             wkv7_seq_kernel<4><<<dim3(H, nseg), kWsThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C, status);
         check_launch("wkv7_seq");
         wkv7_finish_kernel<<<(R * H + kWsFinishThreads / 32 - 1) / (kWsFinishThreads / 32), kWsFinishThreads>>>(r, k, v, vgate, vfirst, a, g, k_a, r_k, lnx_w, lnx_b, yg,
-                                                                                                              R, H, C);
+                                                                                                              R, H, C, nullptr);
     } else {
         throw std::runtime_error("wkv7: variant must be 0 (automatic), 1 (token kernel), 2 (row-per-lane kernel), 3 or 4 (sequence kernel, head over two CTAs / one CTA)");
     }
@@ -1841,16 +1525,32 @@ void engine_op_linear(Model& m, int path, int wtype, const void* w_host, const u
             ld.prepare_tc_i8(W, sz_host);
         } else {
             W.w = ld.upload(w_host, (size_t)M * K * 2);
-            ld.prepare_tc_f16(W, (const uint16_t*)w_host);
+            ld.prepare_tc_f16(W);
         }
-        if (path == 1 && !W.tc_ok) throw std::runtime_error("op_linear: this matrix cannot take the tensor-core path (needs one scale/zero per row, M and K multiples of 128)");
+        if (path == 1 && wtype == W_INT8 && (!W.row_scaled() || M % kTcTileM)) throw std::runtime_error("op_linear: this matrix cannot take the tensor-core path (needs one scale/zero per row, M and K multiples of 128)");
         RSV_CUDA(cudaMalloc(&dx, (size_t)R * K * 4));
         RSV_CUDA(cudaMalloc(&dy, (size_t)R * M * 4));
         RSV_CUDA(cudaMemcpyAsync(dx, x_host, (size_t)R * K * 4, cudaMemcpyHostToDevice, m.stream));
-        LinReq q = {&W, dx, K, dy, M, EPI_STORE};
         if (path == 1) {
-            run_linear_tc(m, "op_linear", &q, 1, R);
+            const RowTiles t = row_tiles(R, false);
+            OperandCarver cv;
+            cv.operand(t, rl_fmt(W), K);
+            ensure_operand_memory(m, cv.used);
+            cv.base = m.ws.op_mem;
+            cv.used = 0;
+            OperandRowsArgs A;
+            memset(&A, 0, sizeof(A));
+            A.R = R;
+            A.rt = t.rt;
+            A.n = 1;
+            A.x[0] = dx;
+            A.ldx[0] = A.K[0] = K;
+            A.out[0] = cv.operand(t, rl_fmt(W), K);
+            launch_operand_rows(m, A);
+            RlReq q = {&W, &A.out[0], dy, M, EPI_STORE};
+            run_rows_linear(m, "op_linear", &q, 1, t);
         } else {
+            LinReq q = {&W, dx, K, dy, M, EPI_STORE};
             run_linear_simt(m, "op_linear_simt", &q, 1, R);
         }
         RSV_CUDA(cudaMemcpyAsync(y_host, dy, (size_t)R * M * 4, cudaMemcpyDeviceToHost, m.stream));

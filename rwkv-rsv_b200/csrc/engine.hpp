@@ -29,13 +29,13 @@ struct LinearW {
     void* w = nullptr;         // fp16 [M,K] or u8 [M,K]
     uint32_t* sz = nullptr;    // int8: [M,K/128] (fp16 scale | fp16 zero << 16), the reference container
     size_t bytes() const { return wtype == W_INT8 ? (size_t)M * K + (size_t)M * (K / 128) * 4 : (size_t)M * K * 2; }
-    // tensor-core path (tcgen05): A operand = the same bytes (or a zero-padded copy when M % 128 or the K pitch
-    // does not fit), one (scale, zero) pair per output row for int8, and the TMA descriptor of the A operand
-    bool tc_ok = false;
-    int Mpad = 0, Kpad = 0;
-    void* w_tc = nullptr;
+    // tensor-core path (tcgen05): A operand = the same bytes through a TMA descriptor (tiles that reach past the matrix read
+    // zeros); int8 files with one (scale, zero) pair per output row keep them as fp32 vectors, others the container's words
+    // transposed to [K/128][M]
     float *wscale = nullptr, *wzero = nullptr;
+    uint32_t* szt = nullptr;
     CUtensorMap amap;
+    bool row_scaled() const { return wtype == W_INT8 && wscale; }
 };
 
 struct LayerW {
@@ -50,17 +50,13 @@ struct LayerW {
 struct Workspace {
     int rows = 0, outs = 0, segs = 0;  // capacities
     const float *final_x = nullptr, *final_delta = nullptr;  // after forward_rows: the last layer's residual stream of row i is final_x[i] + final_delta[i]
-    float *x = nullptr, *x2 = nullptr, *delta = nullptr, *xmix = nullptr, *r = nullptr, *k = nullptr, *v = nullptr, *w = nullptr, *a = nullptr, *g = nullptr;
-    float *yg = nullptr, *xb = nullptr, *mid = nullptr, *h = nullptr, *vfirst = nullptr, *xn = nullptr, *logits = nullptr, *staging = nullptr;
-    // tensor-core linear path: B operands, per-row scales, fixed-point sums, split-K partials (grown on demand)
-    uint8_t* tc_b = nullptr;
-    size_t tc_b_bytes = 0;
-    float* tc_xscale = nullptr;
-    long long* tc_tsum = nullptr;
-    size_t tc_rows = 0;
-    void* tc_partials = nullptr;
-    int* tc_cnt = nullptr;
-    size_t tc_partials_bytes = 0;
+    float *x = nullptr, *x2 = nullptr, *delta = nullptr, *r = nullptr, *k = nullptr, *v = nullptr, *w = nullptr, *a = nullptr, *g = nullptr;
+    float *yg = nullptr, *xb = nullptr, *mid = nullptr, *h = nullptr, *vfirst = nullptr, *logits = nullptr;
+    float *staging_t = nullptr, *staging_c = nullptr;  // new shift states of the step's segments until they are committed
+    // operands of the tensor-core layers (operands.cuh) with their scales and sums, carved per step from one block
+    uint8_t* op_mem = nullptr;
+    size_t op_bytes = 0;
+    float *ymax = nullptr, *hmax = nullptr;  // [rows][parts] maxima of the time-mix output (per head) and of the ffn hidden vector (per M tile)
     float* samp_temp = nullptr;      // [outs, V] sampler work area
     uint32_t* samp_cnt = nullptr;    // [outs, V] penalty histogram
     uint32_t* tokens = nullptr;    // [rows] input token of every row (device-resident between self-loop rounds)
@@ -71,29 +67,6 @@ struct Workspace {
     int* out_rows = nullptr;
     int* status = nullptr;   // bit 0: token id out of range
     int* tok_pos = nullptr;  // cursor into tok_list
-};
-
-// Device-side tables and scratch of the persistent decode kernel (built on first use).
-struct PersistentCtx {
-    bool tried = false, ok = false;
-    std::string why;            // reason when the model cannot take the persistent path
-    void* d_layers = nullptr;   // DpLayer[L]
-    void* d_maps = nullptr;     // CUtensorMap[]
-    float *x = nullptr, *yg = nullptr, *vfirst = nullptr, *cand_val = nullptr;
-    int* cand_idx = nullptr;
-    unsigned* grid_bar = nullptr;
-    long long* dbg = nullptr;  // builds with -DRSV_DP_DEBUG: phase time stamps of the persistent kernel
-    void* region_data[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    void* region_meta[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    int* region_cnt[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    size_t region_cnt_bytes[5] = {0, 0, 0, 0, 0};
-    float *rkv = nullptr, *mid = nullptr, *hbuf = nullptr;
-    int region_pmax[5] = {1, 1, 1, 1, 1};
-    int grid = 0, nstages = 0, btiles = 0;
-    size_t smem = 0;
-    std::vector<char> params_template;  // DpParams with everything but the per-call fields
-    const float *bound_tmix = nullptr, *bound_wkv = nullptr, *bound_cmix = nullptr;  // state whose pointers the device layer table holds
-    int64_t bound_cap = -1;                                                           // and its slot capacity (the per-layer strides)
 };
 
 // Device-side tables and scratch of the batch-1 weight-streaming decode kernel (built on first use).
@@ -166,20 +139,10 @@ struct Model {
     int num_sms = 148;
     bool use_pdl = true;     // launch the per-layer kernels of the batched path as programmatic dependents (RSV_NO_PDL=1 disables)
     bool use_graphs = true;  // replay self-loop rounds from a captured CUDA graph (RSV_NO_GRAPH=1 disables)
-    int tc_min_rows = 5;  // packed steps with at least this many rows use the tensor-core linear path
-
-    bool use_persistent = true;  // batch <= 4 decode goes through the persistent kernel (RSV_NO_PERSISTENT=1 disables)
-    PersistentCtx pctx;
-    bool use_stream = true;  // one session: the row-owner weight-streaming kernel (RSV_NO_STREAM=1 falls back to the tensor-core persistent kernel)
+    bool use_stream = true;  // one session: the row-owner weight-streaming kernel (RSV_NO_STREAM=1 sends it through the batched path)
     StreamCtx sctx;
     bool stream_available();
     void run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bool argmax_feed, uint32_t* seq_dev, int* seq_cnt_dev, int seq_cap);
-    // Persistent decode: n_tokens steps for nb <= 4 sessions (slots[b] of `st`) in one cooperative launch.
-    // Returns false (with pctx.why set) when this model cannot take that path.
-    bool persistent_available(int nb);
-    void run_persistent(State& st, int nb, const int* slots, int n_tokens, bool tok_from_list, bool argmax_feed, uint32_t* seq_dev, int* seq_cnt_dev,
-                        int seq_cap);
-
     static std::unique_ptr<Model> create_bare(int device);  // stream + events only (operator-level entry points)
 
     static std::unique_ptr<Model> load(const std::string& path, int device);

@@ -16,6 +16,9 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// maximum of |v| over a warp (non-negative floats compare as their bits; NaN counts as 0)
+__device__ __forceinline__ float warp_absmax(float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fabsf(v), 0.f)))); }
+
 // Sum over a whole CTA of NW warps; every thread returns the same value, summed in a fixed order.
 template <int NW>
 __device__ __forceinline__ float block_sum(float v, float* red) {
@@ -42,25 +45,6 @@ __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
 template <int I>
 __device__ __forceinline__ float byte_to_float(uint32_t word) {
     return __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u + I)) - 8388608.0f;
-}
-
-// ------------------------------------------------------------------------------------------------
-// LayerNorm of one row held in global memory, two-pass variance exactly as src/model.rs:625-635:
-// mean = sum/n ; var = sum((x-mean)^2)/n + eps ; out = (x-mean)/sqrt(var)*w + b.
-// Returns (mean, inv_std) to every thread of the CTA.
-// ------------------------------------------------------------------------------------------------
-template <int NT>
-__device__ __forceinline__ void row_stats(const float* __restrict__ x, int C, float eps, float* red, float& mean, float& inv_std) {
-    float s = 0.f;
-    for (int i = threadIdx.x; i < C; i += NT) s += x[i];
-    mean = block_sum<NT / 32>(s, red) / (float)C;
-    float q = 0.f;
-    for (int i = threadIdx.x; i < C; i += NT) {
-        float d = x[i] - mean;
-        q += d * d;
-    }
-    float var = block_sum<NT / 32>(q, red) / (float)C + eps;
-    inv_std = 1.0f / sqrtf(var);
 }
 
 // x[r] = LN0(emb[token[r]]).  Stands in for the reference's load-time emb_ln table plus
@@ -96,97 +80,13 @@ __global__ void __launch_bounds__(kRowThreads) embed_ln0_kernel(const __half* __
 // Advances the device-side token cursor used by the token-by-token decode path.
 __global__ void advance_cursor_kernel(int* pos) { *pos += 1; }
 
-// LayerNorm + token shift.  NMIX=6: ln1 and the six time-mix lerps; NMIX=1: ln2 and the channel-mix
-// lerp.  Stands in for norm_lerp6(_batch), cmix_norm_lerp(_batch), rwkv_seq_shift(_batch) and
-// rwkv_copy_token(_batch) (src/backend_cuda.rs:2412-2549, 1505-1640, 4313-4406); math per
-// src/model.rs:402-411, 487-490: out_m = cur + mix_m * (prev - cur), state <- cur.
-// The residual add of the preceding linear layer is folded in: when `delta` is given the row's input is
-// x_in + delta (src/model.rs:484, 495) and that sum is written to x_out, a different buffer, because
-// row r also needs row r-1's sum while another CTA produces it.
-// `prev` is the LayerNorm of row r-1 when that row is the session's previous token (recomputed here
-// with the same code, hence the same bits) and the slot's shift state otherwise.  When a step holds
-// multi-row segments the new shift state goes to `staging` (one row per segment) and is committed by
-// commit_shift_kernel afterwards, because the segment's first row still has to read the old state.
-struct MixPtrs {
-    const float* m[6];
-};
-template <int NT>
-__device__ __forceinline__ void row_stats2(const float* __restrict__ x, const float* __restrict__ d, int C, float eps, float* red, float& mean,
-                                           float& inv_std) {
-    float s = 0.f;
-    for (int i = threadIdx.x; i < C; i += NT) s += d ? x[i] + d[i] : x[i];
-    mean = block_sum<NT / 32>(s, red) / (float)C;
-    float q = 0.f;
-    for (int i = threadIdx.x; i < C; i += NT) {
-        const float t = (d ? x[i] + d[i] : x[i]) - mean;
-        q += t * t;
-    }
-    const float var = block_sum<NT / 32>(q, red) / (float)C + eps;
-    inv_std = 1.0f / sqrtf(var);
-}
-template <int NMIX>
-__global__ void __launch_bounds__(kRowThreads) ln_shift_kernel(const float* __restrict__ x_in, const float* __restrict__ delta, float* __restrict__ x_out,
-                                                               const float* __restrict__ lw, const float* __restrict__ lb, MixPtrs mix,
-                                                               const RowMeta* __restrict__ rows, int R, int C, float* __restrict__ shift_state,
-                                                               float* __restrict__ staging, float* __restrict__ out) {
-    __shared__ float red[kRowThreads / 32];
-    pdl_launch_dependents();
-    pdl_wait();
-    x_in = pdl_fresh(x_in);
-    delta = pdl_fresh(delta);
-    shift_state = pdl_fresh(shift_state);
-    const int r = blockIdx.x;
-    const RowMeta rm = rows[r];
-    const float* xr = x_in + (size_t)r * C;
-    const float* dr = delta ? delta + (size_t)r * C : nullptr;
-    float mean, inv_std, pmean = 0.f, pinv = 0.f;
-    row_stats2<kRowThreads>(xr, dr, C, kLnEps, red, mean, inv_std);
-    if (rm.has_prev) row_stats2<kRowThreads>(xr - C, dr ? dr - C : nullptr, C, kLnEps, red, pmean, pinv);
-    // gridDim.y CTAs share a row: each has the full-row statistics and writes the channels [c_lo, c_hi)
-    const int c_lo = (int)(((long long)blockIdx.y * C) / gridDim.y), c_hi = (int)(((long long)(blockIdx.y + 1) * C) / gridDim.y);
-    for (int i = c_lo + threadIdx.x; i < c_hi; i += kRowThreads) {
-        const float wi = lw[i], bi = lb[i];
-        const float xv = dr ? xr[i] + dr[i] : xr[i];
-        if (dr) x_out[(size_t)r * C + i] = xv;
-        const float cur = (xv - mean) * inv_std * wi + bi;
-        float prev;
-        if (rm.has_prev) {
-            const float xp = dr ? xr[i - C] + dr[i - C] : xr[i - C];
-            prev = (xp - pmean) * pinv * wi + bi;
-        } else {
-            prev = shift_state[(size_t)rm.slot * C + i];
-        }
-#pragma unroll
-        for (int m = 0; m < NMIX; ++m) out[((size_t)m * R + r) * C + i] = cur + mix.m[m][i] * (prev - cur);
-        if (rm.is_last) {
-            if (staging)
-                staging[(size_t)rm.seg * C + i] = cur;
-            else
-                shift_state[(size_t)rm.slot * C + i] = cur;
-        }
-    }
-}
+// Shift states staged by the step's last block -> the sessions' slots (earlier ones are committed by ln_operands_kernel).
 __global__ void commit_shift_kernel(const float* __restrict__ staging, const SegMeta* __restrict__ segs, int C, float* __restrict__ shift_state) {
     pdl_launch_dependents();
     pdl_wait();
     staging = pdl_fresh(staging);
     const SegMeta sg = segs[blockIdx.x];
     for (int i = threadIdx.x; i < C; i += blockDim.x) shift_state[(size_t)sg.slot * C + i] = staging[(size_t)blockIdx.x * C + i];
-}
-
-// Plain LayerNorm of selected rows (ln_out before the head; src/model.rs:507, rwkv_norm at
-// src/backend_cuda.rs:2555-2610).  out[o] = LN(x[out_rows[o]] (+ delta[out_rows[o]])).
-__global__ void __launch_bounds__(kRowThreads) ln_rows_kernel(const float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ lw,
-                                                              const float* __restrict__ lb, const int* __restrict__ out_rows, int C,
-                                                              float* __restrict__ out) {
-    __shared__ float red[kRowThreads / 32];
-    const size_t row = (size_t)out_rows[blockIdx.x];
-    const float* xr = x + row * C;
-    const float* dr = delta ? delta + row * C : nullptr;
-    float mean, inv_std;
-    row_stats2<kRowThreads>(xr, dr, C, kLnEps, red, mean, inv_std);
-    for (int i = threadIdx.x; i < C; i += kRowThreads)
-        out[(size_t)blockIdx.x * C + i] = ((dr ? xr[i] + dr[i] : xr[i]) - mean) * inv_std * lw[i] + lb[i];
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -449,10 +349,10 @@ __global__ void __launch_bounds__(kWkvThreads, 4) wkv7_kernel(const SegMeta* __r
                                                               const float* __restrict__ g, const float* __restrict__ k_k, const float* __restrict__ k_a,
                                                               const float* __restrict__ r_k, const float* __restrict__ lnx_w, const float* __restrict__ lnx_b,
                                                               float* __restrict__ state, float* __restrict__ v_first_state, float* __restrict__ yg, int H,
-                                                              int C) {
+                                                              int C, float* __restrict__ ymax) {
     constexpr int N = kHeadSize;
     __shared__ __align__(16) float s_vec[kWkvThreads / 32][5][N];  // per warp: kk, w, b, k~, r
-    __shared__ float red_a[kWkvThreads / 32], red_b[kWkvThreads / 32];
+    __shared__ float red_a[kWkvThreads / 32], red_b[kWkvThreads / 32], red_m[kWkvThreads / 32];
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, i = tid >> 2, quad = tid & 3;
     pdl_launch_dependents();
     // The segment table and this layer's state were last written before the step's first kernel (plan upload, the previous
@@ -468,6 +368,10 @@ __global__ void __launch_bounds__(kWkvThreads, 4) wkv7_kernel(const SegMeta* __r
         S[4 * jj + 2] = t.z;
         S[4 * jj + 3] = t.w;
     }
+    const int hc = h * N;
+    const float kkc0 = k_k[hc + lane], kkc1 = k_k[hc + lane + 32], kac0 = k_a[hc + lane], kac1 = k_a[hc + lane + 32];
+    const float rkc0 = r_k[hc + lane], rkc1 = r_k[hc + lane + 32];
+    const float gw = lnx_w[hc + i], gb = lnx_b[hc + i];
     pdl_wait();
     r = pdl_fresh(r);
     k = pdl_fresh(k);
@@ -477,10 +381,6 @@ __global__ void __launch_bounds__(kWkvThreads, 4) wkv7_kernel(const SegMeta* __r
     w = pdl_fresh(w);
     a = pdl_fresh(a);
     g = pdl_fresh(g);
-    const int hc = h * N;
-    const float kkc0 = k_k[hc + lane], kkc1 = k_k[hc + lane + 32], kac0 = k_a[hc + lane], kac1 = k_a[hc + lane + 32];
-    const float rkc0 = r_k[hc + lane], rkc1 = r_k[hc + lane + 32];
-    const float gw = lnx_w[hc + i], gb = lnx_b[hc + i];
     float(*sv)[N] = s_vec[warp];
     WkvIn nxt = wkv_load_inputs(r, k, v, vgate, vfirst, w, a, g, (size_t)sg.start * C + hc, lane, i);
     for (int t = 0; t < sg.len; ++t) {
@@ -549,9 +449,19 @@ __global__ void __launch_bounds__(kWkvThreads, 4) wkv7_kernel(const SegMeta* __r
         __syncthreads();
         const float var = (((red_b[0] + red_b[1]) + (red_b[2] + red_b[3])) + ((red_b[4] + red_b[5]) + (red_b[6] + red_b[7]))) / (float)N + kGnEps;
         const float inv_std = 1.0f / sqrtf(var);
+        const float out = (d * inv_std * gw + gb + srk * vj) * gj;
+        const float om = warp_absmax(out);
+        if (lane == 0) red_m[warp] = om;
         if (quad == 0) {
-            yg[hb + i] = (d * inv_std * gw + gb + srk * vj) * gj;
+            yg[hb + i] = out;
             if (v_first_state && t == sg.len - 1) v_first_state[(size_t)sg.slot * C + hc + i] = vj;
+        }
+        if (ymax) {  // the head's part of the row maximum: the scale of the next linear layer's operand needs no pass of its own
+            __syncthreads();
+            if (warp == 0) {
+                const float hm = warp_absmax(lane < kWkvThreads / 32 ? red_m[lane] : 0.f);
+                if (lane == 0) ymax[(size_t)(sg.start + t) * H + h] = hm;
+            }
         }
     }
 #pragma unroll

@@ -1,0 +1,383 @@
+// Activation operands of the tensor-core linear layers (rows_linear.cuh), and the LayerNorm + token-shift kernel that produces most
+// of them.
+//
+// An operand is what an activation matrix x[R, K] becomes before it meets weights on the tensor cores:
+//   int8 weights: t = rint(x / e 2^27), e = 2^ceil(log2 max|x_r|) per row r, as four signed base-128 digits = four int8 columns;
+//   fp16 weights: x / e split into hi + lo fp16 halves = two columns.
+// It is stored as the image of the shared-memory tiles the GEMM reads: [row tile][128-byte block of K][column][128 bytes] with the
+// 16-byte chunks of a column permuted as the 128-byte swizzle wants them (chunk ^ (column mod 8)), so that a tile is one untiled
+// bulk copy and needs no tensor map, and the same code can write it straight to shared memory inside the GEMM.
+// Besides the image a row leaves its scale (xscale), and for int8 the exact sum of its t: over the row (tsum; one (scale, zero) per
+// weight row) or per group of 128 (tgrp; one per weight row and group).
+#pragma once
+#include "kernels.cuh"
+
+namespace rsv {
+
+enum RlFmt : int { RL_F16 = 0, RL_I8 = 1, RL_I8G = 2 };  // fp16; int8 with one (scale, zero) per row; int8 with one per row and group of 128
+constexpr int kRlDigits = 4;
+constexpr int kRlP = 7 * kRlDigits - 1;  // fixed-point bits
+
+// columns an activation row takes in an operand tile
+__host__ __device__ inline int rl_cols(int fmt) { return fmt == RL_F16 ? 2 : kRlDigits; }
+// K elements in a 128-byte block
+__host__ __device__ inline int rl_kelems(int fmt) { return fmt == RL_F16 ? 64 : 128; }
+
+// smallest ex with 2^ex >= amax (0 for an all-zero or non-finite row)
+__device__ __forceinline__ int rl_scale_exp(float amax) {
+    const uint32_t b = __float_as_uint(amax);
+    if (!(amax > 0.f && amax < 3.0e38f)) return 0;
+    const int ex = (int)(b >> 23) - 127 + ((b & 0x7FFFFFu) ? 1 : 0);
+    return max(-99, min(99, ex));
+}
+__device__ __forceinline__ float rl_pow2(int n) { return __int_as_float((n + 127) << 23); }  // -126 <= n <= 127
+// fp32 scale of a row: what one unit of its fixed-point (int8) or normalised (fp16) values is worth
+__device__ __forceinline__ float rl_xscale(int fmt, int ex) { return rl_pow2(fmt == RL_F16 ? ex : ex - kRlP); }
+__device__ __forceinline__ float rl_mult(int fmt, int ex) { return rl_pow2(fmt == RL_F16 ? -ex : kRlP - ex); }
+
+__device__ __forceinline__ void rl_load8(float (&v)[8], const float* p) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(p)), b = __ldcg(reinterpret_cast<const float4*>(p + 4));
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+
+// Eight consecutive elements (K index kin .. kin + 7 inside a block, a multiple of 8) of the activation row whose first column in
+// the tile is n0.  Returns the sum of the fixed-point values (int8; 0 for fp16).  `tile`: global or shared memory.
+__device__ __forceinline__ int rl_put8(int fmt, uint8_t* tile, int n0, int kin, const float (&v)[8], float mult) {
+    if (fmt == RL_F16) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float a = v[2 * i] * mult, b = v[2 * i + 1] * mult;
+            a = fminf(fmaxf(a, -1.0f), 1.0f);
+            b = fminf(fmaxf(b, -1.0f), 1.0f);
+            const __half2 h = __floats2half2_rn(a, b);
+            const float2 hf = __half22float2(h);
+            const __half2 l = __floats2half2_rn(a - hf.x, b - hf.y);
+            hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+            lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+        }
+        const int chunk = kin >> 3;
+        *reinterpret_cast<uint4*>(tile + n0 * 128 + ((chunk ^ (n0 & 7)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(tile + (n0 + 1) * 128 + ((chunk ^ ((n0 + 1) & 7)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        return 0;
+    }
+    int ts = 0;
+    uint32_t dig[4][2];  // digit j of elements 0-3, 4-7
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int t = __float2int_rn(v[4 * q + i] * mult);  // NaN -> 0
+            t = max(-(1 << kRlP), min(1 << kRlP, t));
+            ts += t;
+            // biased by 64 in each of the three low digits the base-128 fields of t are its balanced digits + 64: one field per byte
+            const uint32_t u = (uint32_t)t + 64u * (1u + 128u + 16384u);
+            w[i] = (u & 0x7Fu) | ((u << 1) & 0x7F00u) | ((u << 2) & 0x7F0000u) | ((u << 3) & 0xFF000000u);
+        }
+        // 4 x 4 byte transpose: byte position (low to high) = digit 3, 2, 1, 0
+        const uint32_t a01 = __byte_perm(w[0], w[1], 0x5140), b01 = __byte_perm(w[0], w[1], 0x7362);
+        const uint32_t a23 = __byte_perm(w[2], w[3], 0x5140), b23 = __byte_perm(w[2], w[3], 0x7362);
+        auto unbias = [](uint32_t f) {  // bytes f in 0 .. 127 -> f - 64 as int8
+            const uint32_t y = f ^ 0x40404040u;
+            return y | ((y & 0x40404040u) << 1);
+        };
+        dig[3][q] = unbias(__byte_perm(a01, a23, 0x5410));
+        dig[2][q] = unbias(__byte_perm(a01, a23, 0x7632));
+        dig[1][q] = unbias(__byte_perm(b01, b23, 0x5410));
+        dig[0][q] = __byte_perm(b01, b23, 0x7632);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int n = n0 + j;
+        *reinterpret_cast<uint2*>(tile + n * 128 + (((kin >> 4) ^ (n & 7)) << 4) + (kin & 8)) = make_uint2(dig[j][0], dig[j][1]);
+    }
+    return ts;
+}
+
+// Where one operand of a step goes.
+struct RlOperandOut {
+    const float* mix;  // token-shift mix vector of the operand (null: the normalised row itself)
+    uint8_t* img;
+    float* xscale;    // [R]
+    long long* tsum;  // [R][tparts] (RL_I8)
+    float* tgrp;      // [R][kblocks] (RL_I8G)
+    int fmt, nt, kblocks, tparts;  // nt: columns of a tile
+};
+__device__ __forceinline__ uint8_t* rl_tile(const RlOperandOut& o, int rt, int r, int kb) {
+    return o.img + ((size_t)(r / rt) * o.kblocks + kb) * (size_t)(o.nt * 128);
+}
+// sum of ts over the 16 lanes that hold one group of 128 elements (|ts| <= 2^30 per lane)
+__device__ __forceinline__ long long rl_group_sum(int ts) {
+    int lo = ts & 0xFFFF, hi = ts >> 16;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+        hi += __shfl_xor_sync(0xffffffffu, hi, o);
+    }
+    return (long long)hi * 65536 + lo;
+}
+
+// ---- LayerNorm + token shift -> operands ------------------------------------------------------------------------------------
+// One CTA per row (and, with gridDim.y > 1, per output): eight channels per thread, the row lives in registers.
+//   cur = LN(x_in[r] (+ delta[r])), prev = LN of row r - 1 when that row is the session's previous token (the same code, hence the
+//   same bits) and the slot's shift state otherwise; output o = cur + mix_o (prev - cur), written as an operand.
+// Stands in for norm_lerp6(_batch), cmix_norm_lerp(_batch), rwkv_seq_shift(_batch) and rwkv_copy_token(_batch)
+// (src/backend_cuda.rs:2412-2549, 1505-1640, 4313-4406; math src/model.rs:402-411, 484-495), and, without shift, for ln_out
+// (src/model.rs:507).  `delta` is the pending residual of the linear layer before; the sum goes to x_out, another buffer, because row
+// r - 1's sum is needed too while another CTA produces it.  With multi-row segments the new shift state goes to `staging`, because a
+// segment's first row still has to read the old one; the CTAs past the rows commit the staging area of the block before this one.
+// What bounds it: at few rows the chain load -> mean -> variance -> row maximum -> digits (block-wide reductions); it writes operands instead of fp32 because the
+// conversion in a kernel of its own cost a second launch and a second such chain (8 rows, n_embd 2560: 11.0 + 9.2 us for the two kernels it replaces, CUDA events around each).
+struct LnOperandsArgs {
+    const float *x_in, *delta;
+    float* x_out;
+    const float *lw, *lb;
+    const RowMeta* rows;
+    const int* row_map;  // not null: LayerNorm of rows row_map[0 .. R), no shift
+    float *shift_state, *staging;
+    const float* commit_src;  // [nseg, C] -> commit_dst[slot of the segment]
+    float* commit_dst;
+    const SegMeta* segs;
+    int R, C, rt, nseg, nout;
+    RlOperandOut out[7];
+};
+constexpr int kLnMaxThreads = 1024;  // n_embd up to 8192
+constexpr int kLnSumThreads = 256;  // threads that take part in the row sums (the others only hold channels)
+// Sums of (x - c0) or (x - c0)^2 over the row in shared memory, and of the previous token's row when there is one: thread t adds
+// elements t, t + 256, ..., then shuffles, then the eight warps in order.  (The order is the same at every block size and number of rows.)
+template <bool SQUARE>
+__device__ __forceinline__ void ln_row_sums(const float* rows, int nrows, int C, const float (&c0)[2], float (&sum)[2], float (*red)[kLnSumThreads / 32]) {
+    if (threadIdx.x < kLnSumThreads) {
+#pragma unroll 1
+        for (int w = 0; w < nrows; ++w) {
+            const float* row = rows + (size_t)w * C + threadIdx.x;
+            const float c = w ? c0[1] : c0[0];
+            float a = 0.f;
+#pragma unroll 5
+            for (int i = threadIdx.x; i < C; i += kLnSumThreads, row += kLnSumThreads) {
+                const float d = *row - c;
+                a += SQUARE ? d * d : *row;
+            }
+            a = warp_sum(a);
+            if ((threadIdx.x & 31) == 0) red[w][threadIdx.x >> 5] = a;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        sum[w] = 0.f;
+        if (w < nrows)
+#pragma unroll
+            for (int i = 0; i < kLnSumThreads / 32; ++i) sum[w] += red[w][i];
+    }
+}
+__global__ void __launch_bounds__(kLnMaxThreads) ln_operands_kernel(const __grid_constant__ LnOperandsArgs A) {
+    extern __shared__ __align__(16) float ln_rows_smem[];  // the row and the previous token's
+    __shared__ float red[2][2][kLnSumThreads / 32];
+    __shared__ float redm[7][32];
+    __shared__ long long redt[7][32];
+    pdl_launch_dependents();
+    const int C = A.C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    if ((int)blockIdx.x >= A.R) {  // commit CTAs
+        pdl_wait();
+        if (blockIdx.y == 0) {
+            const int sg = (int)blockIdx.x - A.R;
+            float* dst = A.commit_dst + (size_t)A.segs[sg].slot * C;
+#pragma unroll 1
+            for (int i = 4 * tid; i < C; i += 4 * blockDim.x) *reinterpret_cast<float4*>(dst + i) = __ldcg(reinterpret_cast<const float4*>(A.commit_src + (size_t)sg * C + i));
+        }
+        return;
+    }
+    const int r = blockIdx.x, k0 = 8 * tid;
+    const bool on = k0 < C;
+    const int kc = on ? k0 : 0;
+    RowMeta rm{0, 0, 0, 0};
+    if (A.rows) rm = A.rows[r];
+    const size_t row = A.row_map ? (size_t)A.row_map[r] : (size_t)r;
+    const bool shift = A.rows != nullptr, pln = shift && rm.has_prev;
+    // weights: requested before the dependency wait
+    float lw[8], lb[8], mx[8];
+    rl_load8(lw, A.lw + kc);
+    rl_load8(lb, A.lb + kc);
+    const float* mix = A.out[blockIdx.y].mix;
+    if (mix) rl_load8(mx, mix + kc);
+    const int rloc = r % A.rt, rtile = r / A.rt;
+    pdl_wait();
+    const float* xr = A.x_in + row * C + kc;
+    const float* dr = A.delta ? A.delta + row * C + kc : nullptr;
+    float x[8], xp[8], d[8];
+    rl_load8(x, xr);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) xp[i] = 0.f;
+    if (shift) rl_load8(xp, pln ? xr - C : A.shift_state + (size_t)rm.slot * C + kc);
+    if (dr) {
+        rl_load8(d, dr);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] += d[i];
+        if (pln) {
+            rl_load8(d, dr - C);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) xp[i] += d[i];
+        }
+    }
+    float* xs = ln_rows_smem;
+    if (on) {
+        const float4 a = make_float4(x[0], x[1], x[2], x[3]), b = make_float4(x[4], x[5], x[6], x[7]);
+        *reinterpret_cast<float4*>(xs + k0) = a;
+        *reinterpret_cast<float4*>(xs + k0 + 4) = b;
+        if (pln) {
+            *reinterpret_cast<float4*>(xs + C + k0) = make_float4(xp[0], xp[1], xp[2], xp[3]);
+            *reinterpret_cast<float4*>(xs + C + k0 + 4) = make_float4(xp[4], xp[5], xp[6], xp[7]);
+        }
+        if (A.x_out && blockIdx.y == 0) {
+            float4* o = reinterpret_cast<float4*>(A.x_out + row * C + k0);
+            o[0] = a;
+            o[1] = b;
+        }
+    }
+    __syncthreads();
+    float mean[2] = {0.f, 0.f}, var[2];
+    ln_row_sums<false>(xs, pln ? 2 : 1, C, mean, var, red[0]);
+    mean[0] = var[0] / (float)C;
+    mean[1] = var[1] / (float)C;
+    ln_row_sums<true>(xs, pln ? 2 : 1, C, mean, var, red[1]);
+    const float inv = 1.0f / sqrtf(var[0] / (float)C + kLnEps), pinv = 1.0f / sqrtf(var[1] / (float)C + kLnEps);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        x[i] = (x[i] - mean[0]) * inv * lw[i] + lb[i];                    // cur
+        if (pln) xp[i] = (xp[i] - mean[1]) * pinv * lw[i] + lb[i];  // prev
+        xp[i] -= x[i];                                              // prev - cur
+    }
+    if (shift && rm.is_last && on && blockIdx.y == 0) {
+        float4* o = reinterpret_cast<float4*>(A.staging + (size_t)rm.seg * C + k0);
+        o[0] = make_float4(x[0], x[1], x[2], x[3]);
+        o[1] = make_float4(x[4], x[5], x[6], x[7]);
+    }
+#pragma unroll 1
+    for (int o = blockIdx.y; o < A.nout; o += gridDim.y) {
+        const RlOperandOut& O = A.out[o];
+        if (o != (int)blockIdx.y && O.mix) rl_load8(mx, O.mix + kc);
+        float v[8], am = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            v[i] = O.mix ? x[i] + mx[i] * xp[i] : x[i];
+            am = fmaxf(am, fabsf(v[i]));
+        }
+        am = warp_absmax(on ? am : 0.f);
+        if (lane == 0) redm[o][warp] = am;
+        __syncthreads();
+        const int ex = rl_scale_exp(warp_absmax(lane < nw ? redm[o][lane] : 0.f)), fmt = O.fmt, lk = fmt == RL_F16 ? 6 : 7;
+        int ts = 0;
+        if (on)
+            ts = rl_put8(fmt, O.img + ((size_t)rtile * O.kblocks + (k0 >> lk)) * (size_t)(O.nt * 128), rloc * rl_cols(fmt), k0 & ((1 << lk) - 1), v, rl_mult(fmt, ex));
+        if (fmt == RL_I8G) {
+            const long long t16 = rl_group_sum(ts);
+            if (on && (lane & 15) == 0) O.tgrp[(size_t)r * O.kblocks + k0 / 128] = (float)t16;
+        } else if (fmt == RL_I8) {
+            const int lo = __reduce_add_sync(0xffffffffu, ts & 0xFFFF), hi = __reduce_add_sync(0xffffffffu, ts >> 16);
+            if (lane == 0) redt[o][warp] = (long long)hi * 65536 + lo;
+        }
+        if (tid == 0) O.xscale[r] = rl_xscale(fmt, ex);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int o = warp; o < A.nout; o += nw)
+        if (o % (int)gridDim.y == (int)blockIdx.y && A.out[o].fmt == RL_I8) {
+            long long t = lane < nw ? redt[o][lane] : 0;
+#pragma unroll
+            for (int i = 16; i > 0; i >>= 1) t += __shfl_xor_sync(0xffffffffu, t, i);
+            if (lane == 0) A.out[o].tsum[r] = t;
+        }
+}
+
+// ---- operands of activations another kernel left in fp32 ----------------------------------------------------------------------
+// Rows whose producer left maxima of |x| over `parts` parts of the row (amax[R][parts]): elementwise, grid (rows, ceil(K / 2048)); every
+// CTA leaves the exact sum of its part of the row (tsum[R][gridDim.y]).
+constexpr int kOpThreads = 256;
+__global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* x, int ldx, int K, const float* amax, int parts, int rt,
+                                                                   const __grid_constant__ RlOperandOut O) {
+    __shared__ long long red[kOpThreads / 32];
+    __shared__ float redm[kOpThreads / 32];
+    pdl_launch_dependents();
+    const int r = blockIdx.x, k0 = ((int)blockIdx.y * kOpThreads + (int)threadIdx.x) * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_wait();
+    float v[8];
+    rl_load8(v, x + (size_t)r * ldx + (k0 < K ? k0 : 0));
+    float am = 0.f;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < parts; i += kOpThreads) am = fmaxf(am, __ldcg(amax + (size_t)r * parts + i));
+    am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)));
+    if (lane == 0) redm[warp] = am;
+    __syncthreads();
+    am = redm[lane & (kOpThreads / 32 - 1)];
+    const int ex = rl_scale_exp(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)))), kel = rl_kelems(O.fmt);
+    int ts = 0;
+    if (k0 < K) ts = rl_put8(O.fmt, rl_tile(O, rt, r, k0 / kel), (r % rt) * rl_cols(O.fmt), k0 % kel, v, rl_mult(O.fmt, ex));
+    if (O.fmt != RL_F16) {
+        const long long t16 = rl_group_sum(ts);
+        if (O.fmt == RL_I8G) {
+            if (k0 < K && (lane & 15) == 0) O.tgrp[(size_t)r * O.kblocks + k0 / 128] = (float)t16;
+        } else {
+            const long long t32 = t16 + __shfl_xor_sync(0xffffffffu, t16, 16);
+            if (lane == 0) red[warp] = t32;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                long long t = 0;
+#pragma unroll 1
+                for (int i = 0; i < kOpThreads / 32; ++i) t += red[i];
+                O.tsum[(size_t)r * gridDim.y + blockIdx.y] = t;
+            }
+        }
+    }
+    if (blockIdx.y == 0 && threadIdx.x == 0) O.xscale[r] = rl_xscale(O.fmt, ex);
+}
+
+// Short rows (the rank-space vectors; any length works): one warp per (row, matrix) finds the maximum, then converts.  Elements
+// between K and the end of the last block are written as zeros: the weights there are zero-filled by the tensor map, and 0 x NaN
+// would not be.
+struct OperandRowsArgs {
+    const float* x[4];
+    int ldx[4], K[4];
+    RlOperandOut out[4];
+    int R, rt, n;
+};
+__global__ void __launch_bounds__(kOpThreads) operand_rows_kernel(const __grid_constant__ OperandRowsArgs A) {
+    pdl_launch_dependents();
+    const int item = (int)blockIdx.x * (kOpThreads / 32) + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    pdl_wait();
+    if (item >= A.R * A.n) return;
+    const int r = item / A.n, m = item - r * A.n;
+    const RlOperandOut& O = A.out[m];
+    const float* x = A.x[m] + (size_t)r * A.ldx[m];
+    const int K = A.K[m], kel = rl_kelems(O.fmt), kend = O.kblocks * kel;
+    float am = 0.f;
+    for (int k = 4 * lane; k < K; k += 128) {
+        const float4 t = __ldcg(reinterpret_cast<const float4*>(x + k));
+        am = fmaxf(fmaxf(am, fmaxf(fabsf(t.x), fabsf(t.y))), fmaxf(fabsf(t.z), fabsf(t.w)));
+    }
+    am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)));
+    const int ex = rl_scale_exp(am);
+    const float mult = rl_mult(O.fmt, ex);
+    long long tot = 0;
+    for (int kk = 0; kk < kend; kk += 256) {  // (uniform trip count: the sums below are warp-wide)
+        const int k = kk + 8 * lane;
+        int ts = 0;
+        if (k < kend) {
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (k < K) rl_load8(v, x + k);
+            ts = rl_put8(O.fmt, rl_tile(O, A.rt, r, k / kel), (r % A.rt) * rl_cols(O.fmt), k % kel, v, mult);
+        }
+        if (O.fmt != RL_F16) {
+            const long long t16 = rl_group_sum(ts);
+            if (O.fmt == RL_I8G && k < kend && (lane & 15) == 0) O.tgrp[(size_t)r * O.kblocks + k / 128] = (float)t16;
+            tot += t16 + __shfl_xor_sync(0xffffffffu, t16, 16);
+        }
+    }
+    if (lane == 0) {
+        O.xscale[r] = rl_xscale(O.fmt, ex);
+        if (O.fmt == RL_I8) O.tsum[r] = tot;
+    }
+}
+
+}  // namespace rsv

@@ -1,0 +1,480 @@
+// Linear layers over the packed rows of a step on the 5th-generation tensor cores (sm_100a): TMA -> shared memory -> tcgen05.mma ->
+// TMEM -> epilogue.  Stands in for the reference's dequant-to-scratch + cuBLAS GEMM + epilogue pass (rwkv_dequant_int8, cublasGemmEx,
+// rwkv_gemm_epilogue; src/backend_cuda.rs:4195-4227, 1254-1368, 4613-4633) and its register-tiled batched GEMVs (gemv_variant_mb,
+// gemv_int8_rkv_stage1_batch; :3381-3554, :1665-1910).
+//
+// Arithmetic.  Weights are never converted: the u8 codes q are the A operand of tcgen05.mma.kind::i8 as they sit in HBM, the
+// activation row is four columns of signed base-128 digits of its fixed-point value t (operands.cuh).  The tensor core returns exact
+// int32 sums; Q = sum_j 128^(3-j) I_j = sum_k q_k t_k, y = e 2^-27 (s Q + z sum_k t_k): no rounding but the one of t, no dependence on
+// how K is split.  Files with one (scale, zero) per group of 128 weights (the reference's own) get a fresh accumulator per K block of
+// 128 bytes = one group: the epilogue warps fold s_g Q_g + z_g T_g into fp32 registers while the next group is multiplied.  fp16
+// weights use kind::f16 with hi + lo halves of the activations.
+//
+// Work split.  One CTA = one tile of 128 weight rows x up to 64 activation rows x one slice of K; the slices of a tile are a cluster
+// of 1, 2, 4 or 8 CTAs that exchange partial sums through distributed shared memory (each CTA finishes its share of the activation
+// rows), so that a layer with few tiles still has every SM streaming and no partial sum goes through global memory (the kernel this
+// one replaces cut tiles between persistent CTAs and paid a global round trip, an atomic and a serial sum per cut tile).  A CTA takes
+// at most half an SM (<= 112 KB shared memory, <= 256 TMEM columns): two are resident, one loads while the other finishes, and the
+// next kernel of the step becomes resident early and requests its weights before the dependency wait.
+// What bounds it: at few rows the chain operand tiles (L2) -> products -> exchange -> store behind the dependency wait, the weights
+// are there already; at 64 rows the operand tiles' L2 traffic as well (a 128-row tile re-reads them all).
+//
+// Code size is part of the design.  The kernels of a layer run for a few microseconds each, in turn, on every SM; 32 KB of code run at
+// an instruction per cycle, up to 128 KB at a third of that, more at less than a fifth (measured with straight-line kernels), and a
+// branch to a line that is not there waits for the L2.  A version of this kernel with its epilogue specialised at compile time and
+// unrolled took 150 to 345 KB and 0.5 us for thirty instructions; hence one epilogue, loops that stay loops, and one function per
+// activation.
+//
+// Roles (320 threads): warp 0 TMA producer, warp 1 MMA issuer (+ TMEM owner), warps 2-9 operand construction and epilogue (two per
+// TMEM lane quarter).  Every mbarrier wait is bounded; on expiry bit 1 of the status word is raised and the roles drain.
+#pragma once
+#include <cuda.h>
+
+#include "operands.cuh"
+#include "tc_ptx.cuh"
+
+namespace rsv {
+
+constexpr int kRlThreads = 320;
+constexpr int kRlEpiWarps = 8;
+constexpr int kRlEpiThreads = 32 * kRlEpiWarps;
+constexpr int kRlTileM = 128;
+constexpr int kRlABytes = kRlTileM * 128;
+constexpr int kRlMaxRows = 64;    // activation rows of a tile
+constexpr int kRlMaxRowsG = 32;   // the same for per-group weights: two accumulators are in use, and fp32 sums in registers
+constexpr int kRlMaxProb = 8;
+constexpr int kRlMaxStages = 8;
+constexpr int kRlMaxSplit = 8;
+
+struct RlProb {
+    const uint8_t* bimg;    // operand image; null: built in the kernel from x
+    const float* xscale;    // [R]
+    const long long* tsum;  // [R][tparts] sums over parts of a row
+    const float* tgrp;      // [R][kblocks]
+    const float *wscale, *wzero;  // RL_I8: [M]
+    const uint32_t* szt;          // RL_I8G: [kblocks][M] fp16 scale | fp16 zero << 16
+    const float* x;  // BUILD: activations [R, ldx]
+    float *y, *y2;
+    const float* bias;
+    float* ymax;  // optional: [R][M tiles] maxima of |y| over the tile's outputs (EPI_RELU2 only)
+    int ldx, ldy, epi, fmt, M, K, kblocks, job0, tparts;
+};
+struct alignas(64) RlLaunch {
+    CUtensorMap amap[kRlMaxProb];
+    RlProb p[kRlMaxProb];
+    int nprob, R, rt, n_tiles, split, log_split, nt8, nt16, ring, tmem_cols, f16_halves;  // ring: bytes of shared memory for stages
+    int* status;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void st_cluster_u64(uint32_t addr, unsigned long long v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// untiled bulk copy global -> shared memory of this CTA (16-byte aligned addresses and size)
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes),
+                 "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void rl_epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kRlEpiThreads) : "memory"); }
+
+// Four outputs at a time (independent chains), one piece of code for all epilogues (bias is 0 where there is none).
+__device__ __forceinline__ void rl_activate4(int epi, float (&a)[4], float bias) {
+    if (epi == EPI_STORE) return;
+    if (epi == EPI_RELU2) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float t = fmaxf(a[i], 0.f);
+            a[i] = t * t;
+        }
+    } else if (epi == EPI_TANH) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = tanhf(a[i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = sigmoidf_(a[i] + bias);
+        if (epi == EPI_DECAY)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = expf(a[i] * kDecayScale);
+    }
+}
+// exact integer (|q| < 2^51) -> double without the slow 64-bit conversion
+__device__ __forceinline__ double rl_ll2d(long long q) { return __longlong_as_double(0x4338000000000000LL + q) - 6755399441055744.0; }
+__device__ __forceinline__ long long rl_digits2q(int i0, int i1, int i2, int i3) {
+    return ((long long)i0 * 128 + i1) * 16384 + ((long long)i2 * 128 + i3);
+}
+
+// GROUPED: the launch's int8 problems have per-group weights (RL_I8G), else RL_I8; fp16 problems may be in either kind of launch.
+// BUILD (fp16 problems with short rows, not split along K): the operands are built here from fp32 activations, straight into shared
+// memory; a kernel of its own would cost more than every CTA converting the few rows again.
+template <bool GROUPED, bool BUILD>
+__global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid_constant__ RlLaunch L) {
+    extern __shared__ __align__(1024) uint8_t rl_raw[];
+    __shared__ __align__(8) uint64_t full[kRlMaxStages], empty[kRlMaxStages], acc_full[2], acc_empty[2], b_ready;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_abort;
+    __shared__ float s_xs[kRlMaxRows];
+    __shared__ double s_T[kRlMaxRows];
+    __shared__ uint32_t s_ymax[kRlMaxRows];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)rl_raw + 1023) & ~(uintptr_t)1023);
+    volatile int* abort_flag = &s_abort;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int S = BUILD ? 1 : L.split, rank = !BUILD && S > 1 ? (int)cluster_rank() : 0;
+    const int job = (int)blockIdx.x / S;
+    int pi = 0;
+#pragma unroll 1
+    while (pi + 1 < L.nprob && job >= L.p[pi + 1].job0) ++pi;
+    const RlProb& P = L.p[pi];
+    const int ltile = job - P.job0, mt = ltile / L.n_tiles, ntile = ltile - mt * L.n_tiles;
+    const int fmt = BUILD ? (int)RL_F16 : P.fmt, D = rl_cols(fmt), NT = fmt == RL_F16 ? L.nt16 : L.nt8;
+    const int stage_bytes = kRlABytes + (BUILD ? 0 : NT * 128), NS = min(kRlMaxStages, L.ring / stage_bytes);
+    // fp16 problems that share a launch with int8 ones are cut in two at most: their sums keep one order whatever the split
+    const int Sk = (fmt == RL_F16 && L.f16_halves) ? min(S, 2) : S;
+    const int kb0 = rank < Sk ? P.kblocks * rank / Sk : 0, nk = rank < Sk ? P.kblocks * (rank + 1) / Sk - kb0 : 0;
+    const int r0 = ntile * L.rt, nr = min(L.rt, L.R - r0), ncols = nr * D;
+    const bool grouped = GROUPED && fmt == RL_I8G;
+
+    if (threadIdx.x < kRlMaxStages) {
+        mbar_init(&full[threadIdx.x], 1);
+        mbar_init(&empty[threadIdx.x], 1);
+        if (threadIdx.x < 2) {
+            mbar_init(&acc_full[threadIdx.x], 1);
+            mbar_init(&acc_empty[threadIdx.x], kRlEpiWarps);
+        }
+        if (threadIdx.x == 0) {
+            mbar_init(&b_ready, kRlEpiWarps);
+            s_abort = 0;
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        tmem_alloc(&tmem_slot, (uint32_t)L.tmem_cols);
+        tmem_relinquish();
+    }
+    if (threadIdx.x >= 64 && threadIdx.x < 64 + kRlMaxRows) s_ymax[threadIdx.x - 64] = 0u;
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        // ---------------- producer: weight tiles before the dependency wait, operand tiles behind it ----------------
+        if (lane == 0) {
+            const int kel = rl_kelems(fmt);
+            // weights are read once per step: marked evict-first so that activations, states, vectors and the kernels' code stay in L2
+            // (several row tiles share a weight tile: then it has to stay until the others have read it)
+            const uint64_t pol = L.n_tiles == 1 ? l2_evict_first_policy() : l2_evict_normal_policy();
+            const uint32_t bbytes = BUILD ? 0u : (uint32_t)(NT * 128);
+            const uint8_t* bsrc = BUILD ? nullptr : P.bimg + ((size_t)ntile * P.kblocks + kb0) * bbytes;
+            uint32_t s = 0, par = 1;  // a fresh barrier passes a wait on parity 1
+            int j = 0, filled = 0;
+#pragma unroll 1
+            for (int step = 0; step < 2; ++step) {
+                // step 0: the first ring pass (weights only), and the tiles the ring has no room for yet are requested into L2, so that
+                // HBM works while the predecessor finishes; step 1: their operand tiles, then the rest of the ring's traffic
+                if (step == 0) {
+#pragma unroll 1
+                    for (; j < nk; ++j) {
+                        if (j < NS) {
+                            mbar_expect_tx(&full[j], kRlABytes + bbytes);
+                            tma_load_2d_hint(&L.amap[pi], &full[j], smem + (size_t)j * stage_bytes, (kb0 + j) * kel, mt * kRlTileM, pol);
+                        } else {
+                            tma_prefetch_2d(&L.amap[pi], (kb0 + j) * kel, mt * kRlTileM);
+                        }
+                    }
+                    filled = min(NS, nk);
+                    if (!BUILD) pdl_wait();
+                } else {
+#pragma unroll 1
+                    for (j = 0; j < nk; ++j) {
+                        uint8_t* dst = smem + (size_t)s * stage_bytes;
+                        if (j >= filled) {
+                            if (!mbar_wait(&empty[s], par, abort_flag)) break;
+                            mbar_expect_tx(&full[s], kRlABytes + bbytes);
+                            tma_load_2d_hint(&L.amap[pi], &full[s], dst, (kb0 + j) * kel, mt * kRlTileM, pol);
+                        }
+                        if (!BUILD) bulk_load(dst + kRlABytes, bsrc + (size_t)j * bbytes, bbytes, &full[s]);
+                        if (++s == (uint32_t)NS) {
+                            s = 0;
+                            par ^= 1u;
+                        }
+                    }
+                }
+            }
+            if (*abort_flag)  // copies in flight land before the CTA may exit
+#pragma unroll 1
+                for (int q = max(0, j - NS); q < j; ++q)
+#pragma unroll 1
+                    for (uint32_t i = 0; i < (1u << 16); ++i)
+                        if (mbar_try_wait(&full[q % NS], (uint32_t)(q / NS) & 1u)) break;
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (the warp runs convergently, one elected lane issues) ----------------
+        const uint32_t idesc = tc_idesc(fmt != RL_F16, (ncols + 15) & ~15);
+        const uint32_t smem_addr = smem_u32(smem), bbuf = smem_addr + (uint32_t)L.ring;
+        uint32_t s = 0, par = 0;
+        bool ok = true;
+        if (BUILD) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&b_ready, 0u, abort_flag));
+            tc_fence_after();
+        }
+#pragma unroll 1
+        for (int j = 0; j < nk && ok; ++j) {
+            if (grouped) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[j & 1], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_flag));
+                if (!ok) break;
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t a_addr = smem_addr + s * (uint32_t)stage_bytes, b_addr = BUILD ? bbuf + (uint32_t)(j * NT * 128) : a_addr + kRlABytes;
+            const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(b_addr);
+            const uint32_t d = tmem + (grouped ? (uint32_t)((j & 1) * NT) : 0u);
+            if (!BUILD && fmt != RL_F16) {
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<true>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, ((grouped || j == 0) && k4 == 0) ? 0u : 1u);
+            } else {
+#pragma unroll
+                for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<false>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (j == 0 && k4 == 0) ? 0u : 1u);
+            }
+            tc_commit_elect(&empty[s]);
+            if (grouped) tc_commit_elect(&acc_full[j & 1]);
+            if (++s == (uint32_t)NS) {
+                s = 0;
+                par ^= 1u;
+            }
+        }
+        if (!grouped && ok) tc_commit_elect(&acc_full[0]);
+    }
+    // epilogue warps: output row m of this thread, and which of the two warps of its lane quarter it is in
+    const bool epi = warp >= 2;
+    const int et = threadIdx.x - 64, ew = warp - 2, half = (ew >> 2) & 1, quarter = warp & 3, ml = quarter * 32 + lane, m = mt * kRlTileM + ml;
+    const bool mok = m < P.M;
+    const int sh = L.log_split, slots = (nr + S - 1) >> sh;
+    const uint32_t recv = smem_u32(smem);
+    float ws = 0.f, wz = 0.f, bias = 0.f;
+    constexpr int kGChunks = kRlMaxRowsG / 4 / 2;  // 16-column chunks (four activation rows) per warp
+    float gacc[GROUPED ? kGChunks : 1][4];
+    if (epi) {
+        if (mok) {
+            if (!BUILD && fmt == RL_I8) {
+                ws = P.wscale[m];
+                wz = P.wzero[m];
+            }
+            if (P.bias) bias = P.bias[m];
+        }
+        float* s_tg = reinterpret_cast<float*>(smem + L.ring);  // grouped: [nk][rt]
+        pdl_wait();
+        if (BUILD) {
+            // a warp per row: find the maximum, convert; elements past K are zeros (the tensor map fills the weights there with zeros)
+            uint8_t* bb = smem + L.ring;
+#pragma unroll 1
+            for (int r = ew; r < nr; r += kRlEpiWarps) {
+                const float* x = P.x + (size_t)(r0 + r) * P.ldx;
+                float am = 0.f, v[2][8];  // the row's first 512 elements stay in registers
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int k = 8 * (lane + 32 * q);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[q][e] = 0.f;
+                    if (k < P.K) rl_load8(v[q], x + k);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) am = fmaxf(am, fabsf(v[q][e]));
+                }
+#pragma unroll 1
+                for (int k = 512 + 8 * lane; k < P.K; k += 256) {
+                    float t[8];
+                    rl_load8(t, x + k);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) am = fmaxf(am, fabsf(t[e]));
+                }
+                const int ex = rl_scale_exp(warp_absmax(am));
+                const float mult = rl_mult(RL_F16, ex);
+#pragma unroll 1
+                for (int c = lane, q = 0; c < nk * 8; c += 32, ++q) {
+                    if (q >= 2) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[1][e] = 0.f;
+                        if (8 * c < P.K) rl_load8(v[1], x + 8 * c);
+                    }
+                    float t[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) t[e] = q == 0 ? v[0][e] : v[1][e];
+                    rl_put8(RL_F16, bb + (size_t)(c >> 3) * (NT * 128), 2 * r, 8 * (c & 7), t, mult);
+                }
+                if (lane == 0) s_xs[r] = rl_xscale(RL_F16, ex);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tiles are read by the tensor core
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&b_ready);
+        } else {
+            if (et < nr) {
+                s_xs[et] = __ldcg(P.xscale + r0 + et);
+                if (fmt == RL_I8) {
+                    long long t = 0;
+#pragma unroll 1
+                    for (int i = 0; i < P.tparts; ++i) t += __ldcg(P.tsum + (size_t)(r0 + et) * P.tparts + i);
+                    s_T[et] = rl_ll2d(t);
+                }
+            }
+            if (grouped)
+#pragma unroll 1
+                for (int i = et; i < nk * nr; i += kRlEpiThreads) {
+                    const int r = i / nk, kb = i - r * nk;
+                    s_tg[kb * L.rt + r] = __ldcg(P.tgrp + (size_t)(r0 + r) * P.kblocks + kb0 + kb);
+                }
+        }
+        rl_epi_sync();
+        if (grouped) {
+            // ---- per group: digit sums -> fp32, times the group's scale, plus zero x the group's activation sum ----
+#pragma unroll
+            for (int c = 0; c < (GROUPED ? kGChunks : 1); ++c)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) gacc[c][i] = 0.f;
+            uint32_t z = mok ? __ldg(P.szt + (size_t)kb0 * P.M + m) : 0u;
+#pragma unroll 1
+            for (int j = 0; j < nk; ++j) {
+                const uint32_t zc = z;
+                if (j + 1 < nk && mok) z = __ldg(P.szt + (size_t)(kb0 + j + 1) * P.M + m);
+                const float gs = __half2float(__ushort_as_half((unsigned short)(zc & 0xFFFFu))), gz = __half2float(__ushort_as_half((unsigned short)(zc >> 16)));
+                if (!__all_sync(0xffffffffu, mbar_wait_parked(&acc_full[j & 1], ((uint32_t)j >> 1) & 1u, abort_flag))) break;
+                tc_fence_after();
+                const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((j & 1) * NT);
+#pragma unroll
+                for (int c = 0; c < (GROUPED ? kGChunks : 1); ++c) {
+                    const int c0 = (2 * c + half) * 16;
+                    if (c0 < ncols) {
+                        uint32_t v[16];
+                        tmem_ld16(taddr + c0, v);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            // |digit sum| <= 2^21: pairs combine exactly in 32 bits, the two halves of Q in one fp32 fma
+                            const int hi = (int)v[4 * i] * 128 + (int)v[4 * i + 1], lo = (int)v[4 * i + 2] * 128 + (int)v[4 * i + 3];
+                            const float q = fmaf((float)hi, 16384.0f, (float)lo);
+                            gacc[c][i] = fmaf(gs, q, fmaf(gz, s_tg[j * L.rt + min((c0 >> 2) + i, nr - 1)], gacc[c][i]));
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[j & 1]);
+            }
+        } else {
+            mbar_wait_parked(&acc_full[0], 0u, abort_flag);  // a time-out shows in the abort flag
+        }
+        tc_fence_after();
+    }
+    // Exchange.  Row r of the tile is finished by CTA r mod S of the cluster (S = 1: this one); its sums land in the owner's ring as
+    // [slice][row / S][128] eight-byte words: the exact integer, the hi and lo sums of an fp16 row, or the fp32 sum of per-group weights.
+    if (S > 1) cluster_sync_all();  // every CTA of the cluster is done with its ring
+    const bool go = epi && !__any_sync(0xffffffffu, *abort_flag);
+    if (go && nk > 0) {
+        auto send = [&](int r, unsigned long long v) {
+            if (r < nr) st_cluster_u64(map_to_rank(recv + (uint32_t)(((rank * slots + (r >> sh)) * kRlTileM + ml) * 8), (uint32_t)(r & (S - 1))), v);
+        };
+        if (grouped) {
+#pragma unroll
+            for (int c = 0; c < (GROUPED ? kGChunks : 1); ++c)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) send((2 * c + half) * 4 + i, (unsigned long long)__float_as_uint(gacc[c][i]));
+        } else {
+            const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+            for (int c0 = half * 16; c0 < ncols; c0 += 32) {
+                uint32_t v[16];
+                tmem_ld16(taddr + c0, v);
+                if (BUILD || fmt == RL_F16) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) send((c0 >> 1) + i, (unsigned long long)v[2 * i] | ((unsigned long long)v[2 * i + 1] << 32));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) send((c0 >> 2) + i, (unsigned long long)rl_digits2q((int)v[4 * i], (int)v[4 * i + 1], (int)v[4 * i + 2], (int)v[4 * i + 3]));
+                }
+            }
+        }
+    }
+    if (S > 1) cluster_sync_all();
+    else if (epi) rl_epi_sync();
+    if (go) {
+        // this CTA's share of the rows: slices added in order, scaled, activated, stored (four rows at a time per thread)
+        const int mine = nr > rank ? (nr - rank + S - 1) >> sh : 0;
+        const size_t stride = (size_t)slots * kRlTileM;
+        float* y = P.y + (size_t)r0 * P.ldy + m;
+        float* y2 = P.y2 ? P.y2 + (size_t)r0 * P.ldy + m : nullptr;
+        const int epi_op = P.epi;
+#pragma unroll 1
+        for (int rl = 4 * half; rl < mine; rl += 8) {
+            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(smem) + (size_t)rl * kRlTileM + ml;
+            int off[4];  // rows past the end repeat the last one
+#pragma unroll
+            for (int i = 0; i < 4; ++i) off[i] = min(i, mine - 1 - rl) * kRlTileM;
+            float a[4];
+            if (BUILD || fmt != RL_I8) {
+                float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};  // (per-group weights: the fp32 sum is in hi, lo is zero)
+#pragma unroll 1
+                for (int s = 0; s < Sk; ++s, src += stride)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const unsigned long long t = src[off[i]];
+                        hi[i] += __uint_as_float((uint32_t)t);
+                        lo[i] += __uint_as_float((uint32_t)(t >> 32));
+                    }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = s_xs[min(rank + ((rl + i) << sh), nr - 1)] * (hi[i] + lo[i]);
+            } else {
+                long long q[4] = {0, 0, 0, 0};
+#pragma unroll 1
+                for (int s = 0; s < S; ++s, src += stride)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) q[i] += (long long)src[off[i]];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int r = min(rank + ((rl + i) << sh), nr - 1);
+                    a[i] = (float)((double)s_xs[r] * ((double)ws * rl_ll2d(q[i]) + (double)wz * s_T[r]));
+                }
+            }
+            rl_activate4(epi_op, a, bias);
+            float* yr = y + (size_t)(rank + (rl << sh)) * P.ldy;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (mok && rl + i < mine) yr[(size_t)(i << sh) * P.ldy] = a[i];
+            if (y2) {
+                float* y2r = y2 + (size_t)(rank + (rl << sh)) * P.ldy;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (mok && rl + i < mine) y2r[(size_t)(i << sh) * P.ldy] = a[i];
+            }
+            if (P.ymax) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float mx = warp_absmax(mok ? a[i] : 0.f);
+                    if (lane == 0 && rl + i < mine) atomicMax(&s_ymax[rank + ((rl + i) << sh)], __float_as_uint(mx));
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (P.ymax && go && et < nr && (et & (S - 1)) == rank) P.ymax[(size_t)(r0 + et) * ((P.M + kRlTileM - 1) / kRlTileM) + mt] = __uint_as_float(s_ymax[et]);
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(L.status, 2);
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, (uint32_t)L.tmem_cols);
+    }
+}
+
+}  // namespace rsv

@@ -14,7 +14,7 @@
 // Every mbarrier wait is bounded; on expiry bit 16 of the status word is set and the pair stops.
 #pragma once
 #include "kernels.cuh"
-#include "tc_linear.cuh"
+#include "tc_ptx.cuh"
 
 namespace rsv {
 
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kWrThreads, 1) wkv7_rows_kernel(const __grid_c
                                                                   const float* __restrict__ g, const float* __restrict__ k_k, const float* __restrict__ k_a,
                                                                   const float* __restrict__ r_k, const float* __restrict__ lnx_w,
                                                                   const float* __restrict__ lnx_b, float* __restrict__ v_first_state, float* __restrict__ yg,
-                                                                  int H, int C, int* status) {
+                                                                  int H, int C, int* status, float* __restrict__ ymax) {
     constexpr int N = kHeadSize;
     extern __shared__ __align__(1024) uint8_t wr_raw[];
     uint8_t* base = (uint8_t*)(((uintptr_t)wr_raw + 1023) & ~(uintptr_t)1023);
@@ -201,7 +201,10 @@ __global__ void __launch_bounds__(kWrThreads, 1) wkv7_rows_kernel(const __grid_c
             wr_pair_sync(pair);
             const float var = (pred[1] + pred[3]) / (float)N + kGnEps;
             const float inv_std = 1.0f / sqrtf(var);
-            yg[hb + rr] = (d * inv_std * gw + gb + srk * vj) * cur.g;
+            const float out = (d * inv_std * gw + gb + srk * vj) * cur.g;
+            yg[hb + rr] = out;
+            const float om = warp_absmax(out);
+            if (ymax && lane == 0) ymax[(size_t)(sg.start + t) * (2 * H) + 2 * h + hf] = om;  // half a head's part of the row maximum
             if (v_first_state && t == sg.len - 1) v_first_state[(size_t)sg.slot * C + hc + rr] = vj;
             cur = nx;
         }

@@ -15,7 +15,7 @@
 // Every mbarrier wait is bounded; on expiry bit 16 of the status word is set and the CTA's roles stop.
 #pragma once
 #include "kernels.cuh"
-#include "tc_linear.cuh"
+#include "tc_ptx.cuh"
 
 namespace rsv {
 
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(kWsFinishThreads) wkv7_finish_kernel(const flo
                                                                        const float* __restrict__ vgate, const float* __restrict__ vfirst,
                                                                        const float* __restrict__ a, const float* __restrict__ g, const float* __restrict__ k_a,
                                                                        const float* __restrict__ r_k, const float* __restrict__ lnx_w,
-                                                                       const float* __restrict__ lnx_b, float* yg, int R, int H, int C) {
+                                                                       const float* __restrict__ lnx_b, float* yg, int R, int H, int C, float* ymax) {
     constexpr int N = kHeadSize;
     const int lane = threadIdx.x & 31;
     const int item = blockIdx.x * (kWsFinishThreads / 32) + (threadIdx.x >> 5);
@@ -299,8 +299,11 @@ __global__ void __launch_bounds__(kWsFinishThreads) wkv7_finish_kernel(const flo
     const float inv_std = 1.0f / sqrtf(var);
     const float kt0 = k0 + kac0 * (k0 * a0 - k0), kt1 = k1 + kac1 * (k1 * a1 - k1);
     const float srk = warp_sum(r0 * kt0 * rkc0 + r1 * kt1 * rkc1);
-    yg[hb + lane] = (d0 * inv_std * gw0 + gb0 + srk * v0) * g0;
-    yg[hb + lane + 32] = (d1 * inv_std * gw1 + gb1 + srk * v1) * g1;
+    const float o0 = (d0 * inv_std * gw0 + gb0 + srk * v0) * g0, o1 = (d1 * inv_std * gw1 + gb1 + srk * v1) * g1;
+    yg[hb + lane] = o0;
+    yg[hb + lane + 32] = o1;
+    const float om = warp_absmax(fmaxf(fabsf(o0), fabsf(o1)));
+    if (ymax && lane == 0) ymax[(size_t)row * H + h] = om;
 }
 
 }  // namespace rsv

@@ -8,6 +8,7 @@
 #include "kernels.cuh"
 #include "safetensors.hpp"
 #include "rows_linear.cuh"
+#include "sample_cluster.cuh"
 #include "decode_stream_layout.hpp"
 #include "wkv_rows.cuh"
 #include "wkv_seq.cuh"
@@ -495,8 +496,10 @@ void Model::ensure_workspace(int rows, int outs, int segs) {
     fa(ws.hmax, R * ((F + kRlTileM - 1) / kRlTileM));
     fa(ws.staging_t, (size_t)segs * C);
     fa(ws.staging_c, (size_t)segs * C);
-    fa(ws.samp_temp, (size_t)outs * V);
-    RSV_CUDA(cudaMalloc(&ws.samp_cnt, std::max<size_t>((size_t)outs * V, 4) * sizeof(uint32_t)));
+    if (V > (size_t)kScMaxV) {  // the sampler of smaller vocabularies needs no work area
+        fa(ws.samp_temp, (size_t)outs * V);
+        RSV_CUDA(cudaMalloc(&ws.samp_cnt, std::max<size_t>((size_t)outs * V, 4) * sizeof(uint32_t)));
+    }
     RSV_CUDA(cudaMalloc(&ws.tokens, R * sizeof(uint32_t)));
     RSV_CUDA(cudaMemsetAsync(ws.tokens, 0, R * sizeof(uint32_t), stream));
     RSV_CUDA(cudaMalloc(&ws.row_meta, R * sizeof(RowMeta)));
@@ -1374,21 +1377,47 @@ void engine_argmax(Model& m, const float* logits_dev, int rows, uint32_t* next_t
     }
 }
 
+// Up to 65536 logits a row is a cluster of CTAs that hold it in registers (65536 logits, top-k 50 + top-p: see the table of the design
+// notes); larger vocabularies go through the one-CTA kernel and its work area.
+static void launch_sample(cudaStream_t stream, const float* logits_dev, int rows, int V, const float* sampler8_dev, const uint32_t* hist_dev, int hist_stride,
+                          const int* round_cnt_dev, float* temp_dev, uint32_t* counter_dev, uint32_t* next_tok_dev, uint32_t* seq_dev, int* seq_cnt_dev,
+                          int seq_cap, const int* row_map_dev) {
+    if (V <= kScMaxV) {
+        const int S = (V + kScSeg - 1) / kScSeg;
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3((unsigned)rows * S);
+        cfg.blockDim = dim3(kScThreads);
+        cfg.dynamicSmemBytes = hist_dev ? kScSeg * sizeof(uint32_t) : 0;
+        cfg.stream = stream;
+        cudaLaunchAttribute at[1];
+        memset(at, 0, sizeof(at));
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)S;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        RSV_CUDA(cudaLaunchKernelEx(&cfg, sample_cluster_kernel, logits_dev, V, sampler8_dev, hist_dev, hist_stride, round_cnt_dev, next_tok_dev, seq_dev, seq_cnt_dev,
+                                    seq_cap, row_map_dev, S));
+    } else {
+        sample_rows_kernel<<<rows, kSampleThreads, 0, stream>>>(logits_dev, V, sampler8_dev, hist_dev, hist_stride, round_cnt_dev, temp_dev, counter_dev, next_tok_dev,
+                                                                seq_dev, seq_cnt_dev, seq_cap, row_map_dev);
+    }
+    check_launch("sample");
+}
+
 void engine_sample(Model& m, const float* logits_dev, int rows, const float* sampler8_dev, const uint32_t* hist_dev, int hist_stride,
                    const int* round_cnt_dev, uint32_t* next_tok_dev, uint32_t* seq_dev, int* seq_cnt_dev, int seq_cap, const int* row_map_dev) {
     if (rows > m.ws.outs) throw std::runtime_error("engine_sample: more rows than the work area holds");
     LAUNCH(m, "sample") {
-        sample_rows_kernel<<<rows, kSampleThreads, 0, m.stream>>>(logits_dev, m.cfg.vocab, sampler8_dev, hist_dev, hist_stride, round_cnt_dev, m.ws.samp_temp,
-                                                                  m.ws.samp_cnt, next_tok_dev, seq_dev, seq_cnt_dev, seq_cap, row_map_dev);
-        check_launch("sample");
+        launch_sample(m.stream, logits_dev, rows, m.cfg.vocab, sampler8_dev, hist_dev, hist_stride, round_cnt_dev, m.ws.samp_temp, m.ws.samp_cnt, next_tok_dev, seq_dev,
+                      seq_cnt_dev, seq_cap, row_map_dev);
     }
 }
 
 void engine_sample_raw(cudaStream_t stream, const float* logits_dev, int rows, int V, const float* sampler8_dev, const uint32_t* hist_dev,
                        int hist_stride, float* temp_dev, uint32_t* counter_dev, uint32_t* out_dev) {
-    sample_rows_kernel<<<rows, kSampleThreads, 0, stream>>>(logits_dev, V, sampler8_dev, hist_dev, hist_stride, nullptr, temp_dev, counter_dev, out_dev,
-                                                            nullptr, nullptr, 0, nullptr);
-    check_launch("sample");
+    launch_sample(stream, logits_dev, rows, V, sampler8_dev, hist_dev, hist_stride, nullptr, temp_dev, counter_dev, out_dev, nullptr, nullptr, 0, nullptr);
 }
 
 Ticket::~Ticket() {
@@ -1626,10 +1655,8 @@ extern "C" int rsv_op_sample_static(int device, void* stream, const float* logit
             }
         });
         if (!sc.temp || !sc.cnt) throw CudaError("sample_static: cudaGetSymbolAddress failed for the static work area");
-        sample_rows_kernel<<<(unsigned)rows, kSampleThreads, 0, (cudaStream_t)stream>>>(logits_dev, (int)V, sampler8_dev, hist_stride ? hist_dev : nullptr,
-                                                                                        (int)hist_stride, nullptr, sc.temp, sc.cnt, out_dev, nullptr,
-                                                                                        nullptr, 0, nullptr);
-        check_launch("sample_static");
+        launch_sample((cudaStream_t)stream, logits_dev, (int)rows, (int)V, sampler8_dev, hist_stride ? hist_dev : nullptr, (int)hist_stride, nullptr, sc.temp, sc.cnt,
+                      out_dev, nullptr, nullptr, 0, nullptr);
         return 0;
     } catch (const CudaError& e) {
         set_last_error(e.what());

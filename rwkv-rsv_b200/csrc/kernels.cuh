@@ -491,13 +491,30 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_rows_kernel(const float
     const float* lg = logits + (size_t)row * V;
     float bv = -1e30f;
     int bi = 0;
-    for (int i = threadIdx.x; i < V; i += kArgmaxThreads) {
-        const float x = lg[i];
+    auto take = [&](float x, int i) {
         if (x > bv) {
             bv = x;
             bi = i;
         }
+    };
+    int i0 = 0;
+    if ((V & 3) == 0) {  // four 16-byte loads in flight per thread; a thread's indices ascend, so ties keep the smaller one
+        constexpr int kStep = 16 * kArgmaxThreads;
+        for (; i0 + kStep <= V; i0 += kStep) {
+            float4 v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = __ldcg(reinterpret_cast<const float4*>(lg + i0) + q * kArgmaxThreads + threadIdx.x);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = i0 + 4 * (q * kArgmaxThreads + (int)threadIdx.x);
+                take(v[q].x, i);
+                take(v[q].y, i + 1);
+                take(v[q].z, i + 2);
+                take(v[q].w, i + 3);
+            }
+        }
     }
+    for (int i = i0 + threadIdx.x; i < V; i += kArgmaxThreads) take(lg[i], i);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);

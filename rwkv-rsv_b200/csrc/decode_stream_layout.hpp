@@ -29,15 +29,16 @@ struct DsLayout {
     long long wslot = 0, hslot = 0;  // bytes of the consumption-order weight copy per (layer, CTA) and of the head's per CTA
 };
 
-// Sizes of one matrix [M, K]: pieces of at most max_piece bytes, each a multiple of 128 bytes; all CTAs, no pointers.
+// Sizes of one matrix [M, K]: 1, 2, 4, 8 or 16 pieces of K (a consumer warp's sixteenth lies inside one piece), the fewest whose
+// pieces hold at most max_piece bytes, or 16; pieces are multiples of 128 bytes.
 inline DsEntry ds_size_entry(int M, int K, int fmt, int G, int xvec, int out, int out_off, int max_piece = kDsMaxPiece) {
     DsEntry e{};
     const int row_bytes = fmt ? K : 2 * K;
-    int np = (row_bytes + max_piece - 1) / max_piece;
-    while (np <= row_bytes / 128 && row_bytes % (np * 128)) ++np;
+    int np = 1;
+    while (np < 16 && row_bytes / np > max_piece && row_bytes % (2 * np * 128) == 0) np *= 2;
     e.M = M;
     e.row_stride = row_bytes;
-    e.piece_bytes = row_bytes / std::max(np, 1);
+    e.piece_bytes = row_bytes / np;
     e.npieces = np;
     e.is_i8 = fmt;
     e.xvec = xvec;
@@ -53,10 +54,10 @@ inline void ds_layer_entries(const DsShape& s, int G, bool has_vgate, DsEntry (&
     const int C = s.C, F = s.F;
     // operand vectors of phase 1: 0 = the shifted input of the CTA's big matrix (receptance, key or value), 1 = that of its rank
     // projection
-    e[DSE_W1] = ds_size_entry(s.wm, C, 0, G, 1, DSO_MID_TANH, 0);
-    e[DSE_A1] = ds_size_entry(s.am, C, 0, G, 1, DSO_MID, s.wm);
-    e[DSE_G1] = ds_size_entry(s.gm, C, 0, G, 1, DSO_MID_SIG, s.wm + s.am + s.vm);
-    e[DSE_V1] = ds_size_entry(s.vm, C, 0, G, 1, DSO_MID, s.wm + s.am);
+    e[DSE_W1] = ds_size_entry(s.wm, C, 0, G, 1, DSO_MID_TANH, 0, kDsRankPiece);
+    e[DSE_A1] = ds_size_entry(s.am, C, 0, G, 1, DSO_MID, s.wm, kDsRankPiece);
+    e[DSE_G1] = ds_size_entry(s.gm, C, 0, G, 1, DSO_MID_SIG, s.wm + s.am + s.vm, kDsRankPiece);
+    e[DSE_V1] = ds_size_entry(s.vm, C, 0, G, 1, DSO_MID, s.wm + s.am, kDsRankPiece);
     // The rows of the four rank projections go to disjoint groups of CTAs, sized by their row counts, so that a CTA builds the
     // shifted input of one of them only.
     {
@@ -112,28 +113,34 @@ inline bool ds_layout(const DsShape& s, int G, DsLayout& out, std::string& why) 
     if (H > G) return fail("more heads than SMs");
     if (s.wm <= 0 || s.am <= 0 || s.vm <= 0 || s.gm <= 0 || s.wm % 8 || s.am % 8 || s.vm % 8 || s.gm % 8) return fail("rank dimensions must be positive multiples of 8");
     if (s.fmt < 0 || s.fmt > 2 || s.head_fmt < 0 || s.head_fmt > 2) return fail("unknown weight format");
-    if (F / 128 > kDsMaxGroups) return fail("reduction longer than 16384");
+    // a consumer warp owns a sixteenth of K in whole steps of 32 bytes, the same elements for every matrix of a phase
+    if (C % (s.fmt || s.head_fmt ? 512 : 256)) return fail("n_embd must be a multiple of 512 for int8 matrices and of 256 for fp16 ones");
+    if ((s.fmt ? F : 2 * F) / 512 > kDsMaxWarpSteps) return fail("reduction longer than 16384");
     // shared memory: ring + operand area + fixed part + rank-space vector
     const size_t budget = 227 * 1024;
     out.vec_floats = std::max(4 * C, F);
-    const size_t fixed = (size_t)out.vec_floats * 4 + sizeof(DsShared) + (size_t)s.mids() * 4 + 256;
+    const size_t fixed = (size_t)out.vec_floats * 4 + sizeof(DsShared) + 256;
     if (fixed + 64 * 1024 > budget) return fail("operand area does not fit in shared memory");
     out.ring_bytes = (int)((budget - fixed) / 128 * 128);
     out.smem = (size_t)out.ring_bytes + fixed;
     const int R = out.ring_bytes;
     // A head's back-projection rows come as three chunks (w2 + a2; v2 + half of g2; the other half of g2).  The ring hands out
-    // contiguous space in order, so what must be resident together needs its bytes plus one wrap's waste (< the largest chunk):
-    // all three when the head phase returns them together, else the first alone and then the other two.
-    const int hb_a = 64 * (s.wm + s.am) * 2, hb_b = 64 * s.vm * 2 + 32 * s.gm * 2, hb_c = 32 * s.gm * 2;
+    // contiguous space in order, so what must be resident together needs its bytes plus one wrap's waste (< the largest chunk): the
+    // consumers release the first before they wait for the other two, but the ring is best large enough for all three.
+    const int wmp = ds_pad16(s.wm), amp = ds_pad16(s.am), vmp = ds_pad16(s.vm), gmp = ds_pad16(s.gm);
+    const int hb_a = 128 * (wmp + amp), hb_b = 128 * vmp + 64 * gmp, hb_c = 64 * gmp;
     out.head_early = hb_a + hb_b + hb_c + std::max({hb_a, hb_b, hb_c}) > R;
     if (out.head_early && std::max(2 * hb_a, hb_b + hb_c + std::max(hb_b, hb_c)) > R) return fail("a head's back-projection rows do not fit in the shared-memory ring");
+    if (std::max({wmp, amp, vmp, gmp}) > kDsMaxRank) return fail("rank dimension larger than 512");
+    if (s.L < 2) return fail("fewer than two layers");  // the ordering of a layer's exchanges rests on the other layers'
+    if (wmp + amp + vmp + gmp > 4 * C) return fail("rank dimensions larger than the operand area");
     // every CTA's plan, layer with a v gate (the larger one)
     DsEntry ents[DSE_COUNT];
     ds_layer_entries(s, G, true, ents);
     const DsEntry head_e = ds_head_entry(s, G);
     for (int i = 0; i < DSE_COUNT; ++i)
-        if (ents[i].piece_bytes % 128 || ents[i].piece_bytes > kDsMaxPiece || ents[i].npieces < 1) return fail("a weight row does not split into pieces of a multiple of 128 bytes");
-    if (head_e.piece_bytes % 128 || head_e.piece_bytes > kDsMaxPiece) return fail("a head row does not split into pieces of a multiple of 128 bytes");
+        if (ents[i].piece_bytes % 128) return fail("a weight row does not split into pieces of a multiple of 128 bytes");
+    if (head_e.piece_bytes % 128) return fail("a head row does not split into pieces of a multiple of 128 bytes");
     for (int e : {DSE_W1, DSE_A1, DSE_G1, DSE_V1})
         if (ents[e].npieces * ents[e].piece_bytes != 2 * C) return fail("rank projections must be fp16 [mid, n_embd]");
     auto plan = std::make_unique<DsPlan>();
@@ -149,19 +156,8 @@ inline bool ds_layout(const DsShape& s, int G, DsLayout& out, std::string& why) 
         if (plan->en[DSE_WO] > kDsMaxSlice) return fail("too many channels per SM");
         long long rows = 0, hd = 0;
         for (int ph = 0; ph < DSP_COUNT; ++ph) {
-            int tiles = 0, part = 0, staged = 0;
-            for (int e = first[ph]; e <= last[ph]; ++e) {
-                const DsEntry& E = e == DSE_COUNT ? head_e : ents[e];
-                const int n = plan->en[e];
-                if (n <= 0) continue;
-                const int t = (n + kDsTileRows - 1) / kDsTileRows;
-                tiles += t;
-                part += t * E.npieces * kDsTileRows * (E.is_i8 == 1 ? 8 : 4);
-                if (E.is_i8 == 1) staged += n;
-            }
-            if (tiles > kDsMaxTiles) return fail("too many tiles per SM");
-            if (part > kDsPartBytes) return fail("partial sums of a phase do not fit in shared memory");
-            if (staged > kDsMaxRows) return fail("too many rows per SM");
+            for (int e = first[ph]; e <= last[ph]; ++e)
+                if (e <= DSE_V1 && plan->en[e] > kDsRankTiles * kDsTileRows) return fail("too many rank-projection rows per SM");
             for (int k = plan->ph0[ph]; k < plan->ph0[ph] + plan->phn[ph]; ++k) {
                 const DsChunk& ch = plan->ctab[k];
                 if (ch.cb % 16 || 2 * ch.cb > R) return fail("a chunk of rows does not fit twice in the shared-memory ring");
@@ -181,7 +177,7 @@ inline bool ds_layout(const DsShape& s, int G, DsLayout& out, std::string& why) 
     }
     for (int e = 0; e <= DSE_COUNT; ++e)
         if (next_row[e] != (e == DSE_COUNT ? head_e.M : ents[e].M)) return fail("the CTAs' rows do not add up to the matrix");
-    out.wslot += 128LL * s.mids();  // a head's back-projection rows
+    out.wslot += 128LL * (wmp + amp + vmp + gmp);  // a head's back-projection rows
     out.wslot = (out.wslot + 255) / 256 * 256;
     out.hslot = (out.hslot + 255) / 256 * 256;
     return true;

@@ -444,8 +444,7 @@ Model::~Model() {
     for (void* p : allocs) cudaFree(p);
     for (void* p : {(void*)ws.op_mem})
         if (p) cudaFree(p);
-    for (void* p : {sctx.d_layers, sctx.wstream, sctx.hstream, (void*)sctx.x, (void*)sctx.yg, (void*)sctx.vfirst, (void*)sctx.rkv, (void*)sctx.mid, (void*)sctx.hbuf, (void*)sctx.cand_val,
-                    (void*)sctx.cand_idx, (void*)sctx.grid_bar, (void*)sctx.dbg})
+    for (void* p : {sctx.d_layers, sctx.wstream, sctx.hstream, (void*)sctx.exchange, (void*)sctx.cand_val, (void*)sctx.cand_idx, (void*)sctx.grid_bar})
         if (p) cudaFree(p);
     if (pinned) cudaFreeHost(pinned);
     for (int i = 0; i < kPinRing; ++i)
@@ -1125,7 +1124,6 @@ bool Model::stream_available() {
         if (!ds_layout(shp, G, lay, why)) return fail(why);
     }
     const int cmax = lay.cmax, vec_floats = lay.vec_floats, ring_bytes = lay.ring_bytes;
-    const bool head_early = lay.head_early;
     sc.kl = cmax;
     sc.grid = G;
     sc.ring_bytes = ring_bytes;
@@ -1208,23 +1206,15 @@ bool Model::stream_available() {
         if (const char* e = getenv("RSV_VERBOSE"))
             if (*e && *e != '0')
                 fprintf(stderr, "[rsv] weight-streaming decode kernel: %.2f GB second copy of the weights in consumption order (%lld bytes per layer and SM); ring %d bytes%s\n",
-                        ((double)wslot * G * L + (double)hslot * G) / 1e9, wslot, ring_bytes, head_early ? ", a head's first chunk released early" : "");
+                        ((double)wslot * G * L + (double)hslot * G) / 1e9, wslot, ring_bytes, lay.head_early ? ", a head's first chunk released early" : "");
     }
-    RSV_CUDA(cudaMalloc(&sc.x, (size_t)C * 4));
-    RSV_CUDA(cudaMalloc(&sc.yg, (size_t)C * 4));
-    RSV_CUDA(cudaMalloc(&sc.vfirst, (size_t)C * 4));
-    RSV_CUDA(cudaMalloc(&sc.rkv, (size_t)3 * C * 4));
-    RSV_CUDA(cudaMalloc(&sc.mid, (size_t)std::max(cfg.mids(), 1) * 4));
-    RSV_CUDA(cudaMalloc(&sc.hbuf, (size_t)F * 4));
+    const size_t pairs = (size_t)7 * C + cfg.mids();
+    sc.exchange_bytes = pairs * 8 + (size_t)F * 4;
+    RSV_CUDA(cudaMalloc(&sc.exchange, sc.exchange_bytes));
+    RSV_CUDA(cudaMemsetAsync(sc.exchange, 0, sc.exchange_bytes, stream));  // tag 0: no launch's
     RSV_CUDA(cudaMalloc(&sc.cand_val, (size_t)G * 4));
     RSV_CUDA(cudaMalloc(&sc.cand_idx, (size_t)G * 4));
     RSV_CUDA(cudaMalloc(&sc.grid_bar, 4));
-    RSV_CUDA(cudaMemsetAsync(sc.mid, 0, (size_t)std::max(cfg.mids(), 1) * 4, stream));
-    RSV_CUDA(cudaMemsetAsync(sc.vfirst, 0, (size_t)C * 4, stream));
-#ifdef RSV_DS_DEBUG
-    RSV_CUDA(cudaMalloc(&sc.dbg, (256 + 16 * 256) * sizeof(long long)));
-    RSV_CUDA(cudaMemsetAsync(sc.dbg, 0, (256 + 16 * 256) * sizeof(long long), stream));
-#endif
     P.layers = (const DsLayer*)sc.d_layers;
     P.head = ds_head_entry(shp, G);
     bind(P.head, head, nullptr);
@@ -1242,12 +1232,13 @@ bool Model::stream_available() {
     P.am = cfg.a_mid;
     P.vm = cfg.v_mid;
     P.gm = cfg.g_mid;
-    P.x = sc.x;
-    P.yg = sc.yg;
-    P.vfirst = sc.vfirst;
-    P.rkv = sc.rkv;
-    P.mid = sc.mid;
-    P.hbuf = sc.hbuf;
+    P.xa = sc.exchange;
+    P.xb = P.xa + C;
+    P.yg = P.xb + C;
+    P.vfirst = P.yg + C;
+    P.rkv = P.vfirst + C;
+    P.mid = P.rkv + 3 * (size_t)C;
+    P.hbuf = (uint32_t*)(P.mid + cfg.mids());
     P.cand_val = sc.cand_val;
     P.cand_idx = sc.cand_idx;
     P.grid_bar = sc.grid_bar;
@@ -1256,9 +1247,7 @@ bool Model::stream_available() {
     P.hstream = (const char*)sc.hstream;
     P.hslot = sc.hslot;
     P.ring_bytes = ring_bytes;
-    P.head_early = head_early ? 1 : 0;
     P.vec_floats = vec_floats;
-    P.dbg = sc.dbg;
     sc.params_template.resize(sizeof(DsParams));
     memcpy(sc.params_template.data(), &P, sizeof(P));
     sc.ok = true;
@@ -1290,59 +1279,10 @@ void Model::run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bo
     P.n_tokens = n_tokens;
     P.tok_from_list = tok_from_list ? 1 : 0;
     P.argmax_feed = argmax_feed ? 1 : 0;
+    P.epoch = sc.epoch;
+    sc.epoch += (uint32_t)n_tokens * (uint32_t)cfg.n_layer;
     RSV_CUDA(cudaMemsetAsync(sc.grid_bar, 0, 4, stream));
     LAUNCH(*this, "decode_stream") { dispatch_stream(sc.kl, P, sc.grid, sc.smem, stream, false); }
-#ifdef RSV_DS_DEBUG
-    if (sc.dbg && n_tokens >= 2) {
-        static long long h[256 + 16 * 256];
-        RSV_CUDA(cudaStreamSynchronize(stream));
-        RSV_CUDA(cudaMemcpy(h, sc.dbg, sizeof(h), cudaMemcpyDeviceToHost));
-        const int order[15] = {0, 10, 1, 2, 11, 3, 12, 4, 5, 13, 6, 7, 14, 8, 9};
-        const char* names[15] = {"layer start", "P1 operands", "P1 rows done", "heads done", "P3 operands", "P3 rows done", "P4 operands", "P4 rows done", "P5 operands", "P5 rows done",
-                                 "barrier 5 passed", "barrier 1 passed", "barrier 2 passed", "barrier 3 passed", "barrier 4 passed"};
-        fprintf(stderr, "[decode_stream_kernel, CTA 0, token 1, layer 1] us since the layer started\n");
-        for (int i = 0; i < 15; ++i) fprintf(stderr, "  %-18s %.2f\n", names[order[i]], (h[order[i]] - h[0]) / 1e3);
-        fprintf(stderr, "  P1 prologue: loads issued %.2f, statistics done %.2f, shift / slice done %.2f\n", (h[15] - h[0]) / 1e3, (h[16] - h[0]) / 1e3, (h[17] - h[0]) / 1e3);
-        fprintf(stderr, "  producer, first chunks of the launch (ring empty), us between issues:");
-        for (int i = 1; i < 8; ++i) fprintf(stderr, " %.2f", (h[200 + i] - h[200 + i - 1]) / 1e3);
-        fprintf(stderr, "\n");
-        fprintf(stderr, "  P1 operands: magnitudes %.2f, barrier %.2f, digits written %.2f\n", (h[52] - h[0]) / 1e3, (h[53] - h[0]) / 1e3, (h[54] - h[0]) / 1e3);
-        fprintf(stderr, "  heads: vectors gathered %.2f, first chunk there %.2f, its dot products done %.2f, all three there %.2f, dot products done %.2f, state updated %.2f\n", (h[18] - h[0]) / 1e3,
-                (h[55] - h[0]) / 1e3, (h[57] - h[0]) / 1e3, (h[56] - h[0]) / 1e3, (h[19] - h[0]) / 1e3, (h[50] - h[0]) / 1e3);
-        const char* ph[4] = {"P1", "P3", "P4", "P5"};
-        for (int i = 0; i < 4; ++i)
-            fprintf(stderr, "  %s rows, consumer warp 0: %lld chunks, %.2f us waiting for them, %.2f us multiplying\n", ph[i], h[20 + 4 * i + 2], h[20 + 4 * i] / 1e3, h[20 + 4 * i + 1] / 1e3);
-        fprintf(stderr, "  producer: P1 rows issued %.2f .. %.2f, head chunk A issued %.2f, C issued %.2f, att.out issued %.2f, ffn.value issued %.2f\n", (h[40] - h[0]) / 1e3,
-                (h[41] - h[0]) / 1e3, (h[42] - h[0]) / 1e3, (h[43] - h[0]) / 1e3, (h[44] - h[0]) / 1e3, (h[45] - h[0]) / 1e3);
-        for (int w = 0; w < 16; ++w)
-            fprintf(stderr, "  P1 warp %2d: last chunk wait %.2f .. %.2f, multiplied %.2f, tile finished %.2f\n", w, (h[64 + 4 * w] - h[0]) / 1e3, (h[65 + 4 * w] - h[0]) / 1e3,
-                    (h[66 + 4 * w] - h[0]) / 1e3, h[67 + 4 * w] ? (h[67 + 4 * w] - h[0]) / 1e3 : 0.0);
-        {
-            const int ord[15] = {0, 10, 1, 2, 3, 12, 4, 5, 13, 6, 7, 14, 8, 9, -1};
-            const char* nm[15] = {"layer start", "P1 operands", "P1 rows done", "heads done", "P3 operands", "P3 rows done", "P4 operands", "P4 rows done", "P5 operands", "P5 rows done",
-                                  "barrier 5 passed", "", "barrier 2 passed", "barrier 3 passed", "barrier 4 passed"};
-            fprintf(stderr, "  all CTAs (us since CTA 0's layer start): min / mean / max (CTA)\n");
-            for (int i = 0; ord[i] >= 0; ++i) {
-                const int k = ord[i];
-                long long mn = 1LL << 62, mx = 0, sum = 0;
-                int amx = -1, n = 0;
-                for (int c = 0; c < sc.grid && c < 256; ++c) {
-                    const long long v = h[256 + c * 16 + k];
-                    if (!v) continue;
-                    ++n;
-                    sum += v - h[0];
-                    mn = std::min(mn, v);
-                    if (v > mx) {
-                        mx = v;
-                        amx = c;
-                    }
-                }
-                if (n) fprintf(stderr, "    %-18s %7.2f %7.2f %7.2f (%d)\n", nm[k], (mn - h[0]) / 1e3, sum / 1e3 / n, (mx - h[0]) / 1e3, amx);
-            }
-        }
-        RSV_CUDA(cudaMemsetAsync(sc.dbg, 0, (256 + 16 * 256) * sizeof(long long), stream));
-    }
-#endif
 }
 
 void Model::check_status() {
@@ -1352,6 +1292,10 @@ void Model::check_status() {
     const int s = sw[0];
     if (s) {
         RSV_CUDA(cudaMemsetAsync(ws.status, 0, 2 * sizeof(int), stream));
+        if ((s & 32) && sctx.exchange) {  // a launch that gave up left some of its exchanged values unwritten
+            RSV_CUDA(cudaMemsetAsync(sctx.exchange, 0, sctx.exchange_bytes, stream));
+            sctx.epoch = 1;
+        }
         if (s & 32) {
             static const char* const site[5] = {"a wait", "a chunk of weight rows", "room in the ring", "a grid barrier", "a chunk of a head's rows"};
             const int k = sw[1] & 15;
@@ -1377,8 +1321,8 @@ void engine_argmax(Model& m, const float* logits_dev, int rows, uint32_t* next_t
     }
 }
 
-// Up to 65536 logits a row is a cluster of CTAs that hold it in registers (65536 logits, top-k 50 + top-p: see the table of the design
-// notes); larger vocabularies go through the one-CTA kernel and its work area.
+// Up to 65536 logits (eight CTAs, the portable cluster size, of 8192) a row is a cluster of CTAs that hold it in registers: 25 us for
+// 65536 logits with top-k 50 + top-p against 218 us; larger vocabularies go through the one-CTA kernel and its work area.
 static void launch_sample(cudaStream_t stream, const float* logits_dev, int rows, int V, const float* sampler8_dev, const uint32_t* hist_dev, int hist_stride,
                           const int* round_cnt_dev, float* temp_dev, uint32_t* counter_dev, uint32_t* next_tok_dev, uint32_t* seq_dev, int* seq_cnt_dev,
                           int seq_cap, const int* row_map_dev) {

@@ -76,10 +76,12 @@ struct StreamCtx {
     void* d_layers = nullptr;  // DsLayer[L]
     void *wstream = nullptr, *hstream = nullptr;  // second copy of the weights in the order the kernel consumes them
     long long wslot = 0, hslot = 0;
-    float *x = nullptr, *yg = nullptr, *vfirst = nullptr, *rkv = nullptr, *mid = nullptr, *hbuf = nullptr, *cand_val = nullptr;
+    unsigned long long* exchange = nullptr;  // values the CTAs exchange (see decode_stream.cuh): xa, xb, yg, vfirst [C], rkv [3C], mid, then hbuf [F] words
+    size_t exchange_bytes = 0;
+    uint32_t epoch = 1;                      // tag of the next launch's first layer
+    float* cand_val = nullptr;
     int* cand_idx = nullptr;
     unsigned* grid_bar = nullptr;
-    long long* dbg = nullptr;
     int grid = 0, kl = 0, ring_bytes = 0, vec_floats = 0;
     size_t smem = 0;
     std::vector<char> params_template;  // DsParams with everything but the per-call fields

@@ -4,6 +4,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "engine.hpp"
@@ -117,6 +118,64 @@ constexpr int kMaxChunk = 512;  // rows per packed step on the chunk path
 
 // chunked prefill of one session; out_mode 1: logits of the very last token in ws.logits[0,:];
 // out_mode 2: every position, copied to `all_out` chunk by chunk
+// Logits of a whole chunk to the caller's memory.  A copy to pageable memory runs at what one thread of the driver moves (201 x 65536
+// logits: 53 MB, 8 ms with the first touch of the pages); here the chunk goes to pinned memory in kOutParts pieces behind its forward
+// pass, and a few threads move each piece on as soon as it has arrived, while the GPU runs the next chunk.
+class LogitsToHost {
+  public:
+    explicit LogitsToHost(Model& model) : m(model) {}
+    ~LogitsToHost() { join(); }
+    // queues the copy of `count` logits; returns while it is under way
+    void start(float* dst, size_t count) {
+        join();  // the staging area is free again
+        cudaPointerAttributes at;
+        const bool direct = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
+        if (!direct) cudaGetLastError();
+        if (direct || count < kSmall) {
+            RSV_CUDA(cudaMemcpyAsync(dst, m.ws.logits, count * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
+            return;
+        }
+        m.ensure_pinned_out(count * sizeof(float));
+        const size_t part = (count + kOutParts - 1) / kOutParts;
+        for (int i = 0; i < kOutParts; ++i) {
+            const size_t at0 = std::min(count, i * part), n = std::min(count, at0 + part) - at0;
+            if (n) RSV_CUDA(cudaMemcpyAsync(m.pinned_out + at0, m.ws.logits + at0, n * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
+            RSV_CUDA(cudaEventRecord(m.out_ev[i], m.stream));
+        }
+        const int workers = (int)std::min<unsigned>(kWorkers, std::max(1u, std::thread::hardware_concurrency() / 2));
+        failed.assign((size_t)workers, 0);
+        for (int w = 0; w < workers; ++w)
+            threads.emplace_back([this, dst, count, part, w, workers] {
+                cudaSetDevice(m.device);
+                for (int i = w; i < kOutParts; i += workers) {
+                    if (cudaEventSynchronize(m.out_ev[i]) != cudaSuccess) {
+                        failed[(size_t)w] = 1;
+                        return;
+                    }
+                    const size_t at0 = std::min(count, i * part), n = std::min(count, at0 + part) - at0;
+                    memcpy(dst + at0, m.pinned_out + at0, n * sizeof(float));
+                }
+            });
+    }
+    void finish() {
+        join();
+        RSV_CUDA(cudaStreamSynchronize(m.stream));
+        for (char f : failed) need(!f, "copy of the logits to the host failed");
+    }
+
+  private:
+    static constexpr size_t kSmall = 1u << 20;  // below 4 MB the driver's own staging is as fast as starting threads
+    static constexpr int kOutParts = Model::kOutParts;
+    static constexpr unsigned kWorkers = 8;
+    Model& m;
+    std::vector<std::thread> threads;
+    std::vector<char> failed;
+    void join() {
+        for (auto& t : threads) t.join();
+        threads.clear();
+    }
+};
+
 void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int64_t chunk, int out_mode, float* all_out) {
     need(st.model == &m, "state belongs to a different model");
     need(st.cap == 1, "this call needs a single-session state (batch == 1)");
@@ -125,6 +184,7 @@ void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int6
     RSV_CUDA(cudaSetDevice(m.device));
     const int64_t cs = std::max<int64_t>(1, std::min<int64_t>(chunk <= 0 ? kMaxChunk : chunk, out_mode == 2 ? 128 : kMaxChunk));
     const size_t V = m.cfg.vocab;
+    LogitsToHost out(m);
     for (int64_t off = 0; off < n; off += cs) {
         const int T = (int)std::min<int64_t>(cs, n - off);
         const bool last = off + T >= n;
@@ -132,11 +192,9 @@ void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int6
         m.upload_plan(p);
         RSV_CUDA(cudaMemcpyAsync(m.ws.tokens, tokens + off, (size_t)T * sizeof(uint32_t), cudaMemcpyHostToDevice, m.stream));
         m.forward_rows(st, p, false);
-        if (out_mode == 2) {
-            RSV_CUDA(cudaMemcpyAsync(all_out + (size_t)off * V, m.ws.logits, (size_t)T * V * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
-            RSV_CUDA(cudaStreamSynchronize(m.stream));
-        }
+        if (out_mode == 2) out.start(all_out + (size_t)off * V, (size_t)T * V);
     }
+    if (out_mode == 2) out.finish();
 }
 
 void fetch_logits(Model& m, float* logits_out) {
@@ -300,18 +358,8 @@ int rsv_state_new(rsv_model* mh, int64_t batch, rsv_state** out) {
         RSV_CUDA(cudaSetDevice(m.device));
         auto h = std::make_unique<rsv_state>();
         State& s = h->s;
-        s.model = &m;
-        s.cap = cap;
-        const Config& c = m.cfg;
-        const size_t nx = (size_t)c.n_layer * cap * c.n_embd, ns = (size_t)c.n_layer * cap * c.n_head * kHeadSize * kHeadSize, nv = (size_t)cap * c.n_embd;
-        RSV_CUDA(cudaMalloc(&s.tmix_x, nx * 4));
-        RSV_CUDA(cudaMalloc(&s.cmix_x, nx * 4));
-        RSV_CUDA(cudaMalloc(&s.wkv, ns * 4));
-        RSV_CUDA(cudaMalloc(&s.v_first, nv * 4));
-        RSV_CUDA(cudaMemsetAsync(s.tmix_x, 0, nx * 4, m.stream));
-        RSV_CUDA(cudaMemsetAsync(s.cmix_x, 0, nx * 4, m.stream));
-        RSV_CUDA(cudaMemsetAsync(s.wkv, 0, ns * 4, m.stream));
-        RSV_CUDA(cudaMemsetAsync(s.v_first, 0, nv * 4, m.stream));
+        s.allocate(&m, cap);
+        s.clear();
         RSV_CUDA(cudaStreamSynchronize(m.stream));
         *out = h.release();
     });
@@ -477,13 +525,8 @@ int rsv_state_reset(rsv_state* sh) {
         need(sh, "null argument");
         State& s = sh->s;
         Model& m = *s.model;
-        const Config& c = m.cfg;
         RSV_CUDA(cudaSetDevice(m.device));
-        const size_t nx = (size_t)c.n_layer * s.cap * c.n_embd, ns = (size_t)c.n_layer * s.cap * c.n_head * kHeadSize * kHeadSize;
-        RSV_CUDA(cudaMemsetAsync(s.tmix_x, 0, nx * 4, m.stream));
-        RSV_CUDA(cudaMemsetAsync(s.cmix_x, 0, nx * 4, m.stream));
-        RSV_CUDA(cudaMemsetAsync(s.wkv, 0, ns * 4, m.stream));
-        RSV_CUDA(cudaMemsetAsync(s.v_first, 0, (size_t)s.cap * c.n_embd * 4, m.stream));
+        s.clear();
         RSV_CUDA(cudaStreamSynchronize(m.stream));
     });
 }

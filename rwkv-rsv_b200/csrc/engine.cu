@@ -447,6 +447,9 @@ Model::~Model() {
     for (void* p : {sctx.d_layers, sctx.wstream, sctx.hstream, (void*)sctx.exchange, (void*)sctx.cand_val, (void*)sctx.cand_idx, (void*)sctx.grid_bar})
         if (p) cudaFree(p);
     if (pinned) cudaFreeHost(pinned);
+    if (pinned_out) cudaFreeHost(pinned_out);
+    for (cudaEvent_t e : out_ev)
+        if (e) cudaEventDestroy(e);
     for (int i = 0; i < kPinRing; ++i)
         if (pin_ev[i]) cudaEventDestroy(pin_ev[i]);
     if (ev0) cudaEventDestroy(ev0);
@@ -460,9 +463,23 @@ State::~State() {
     if (model) {
         cudaSetDevice(model->device);
     }
-    for (float* p : {tmix_x, wkv, cmix_x, v_first})
-        if (p) cudaFree(p);
+    if (wkv) cudaFree(wkv);
 }
+
+void State::allocate(Model* m, int64_t slots) {
+    model = m;
+    cap = slots;
+    const Config& c = m->cfg;
+    auto aligned = [](size_t floats) { return (floats + 63) / 64 * 64; };
+    const size_t nx = aligned((size_t)c.n_layer * cap * c.n_embd), ns = aligned((size_t)c.n_layer * cap * c.n_head * kHeadSize * kHeadSize);
+    bytes = (ns + 2 * nx + (size_t)cap * c.n_embd) * 4;
+    RSV_CUDA(cudaMalloc(&wkv, bytes));
+    tmix_x = wkv + ns;
+    cmix_x = tmix_x + nx;
+    v_first = cmix_x + nx;
+}
+
+void State::clear() { RSV_CUDA(cudaMemsetAsync(wkv, 0, bytes, model->stream)); }
 
 void Model::ensure_workspace(int rows, int outs, int segs) {
     if (rows <= ws.rows && outs <= ws.outs && segs <= ws.segs) return;
@@ -514,6 +531,17 @@ void Model::ensure_workspace(int rows, int outs, int segs) {
         pinned_bytes = need * 2;
         RSV_CUDA(cudaMallocHost(&pinned, pinned_bytes * kPinRing));
     }
+}
+
+void Model::ensure_pinned_out(size_t bytes) {
+    for (cudaEvent_t& e : out_ev)
+        if (!e) RSV_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (bytes <= pinned_out_bytes) return;
+    if (pinned_out) cudaFreeHost(pinned_out);
+    pinned_out = nullptr;
+    pinned_out_bytes = 0;
+    RSV_CUDA(cudaMallocHost(&pinned_out, bytes));
+    pinned_out_bytes = bytes;
 }
 
 void Model::upload_plan(const StepPlan& plan) {

@@ -99,9 +99,12 @@ struct Model;
 struct State {
     Model* model = nullptr;
     int64_t cap = 0;
-    float *tmix_x = nullptr, *wkv = nullptr, *cmix_x = nullptr, *v_first = nullptr;
+    float *tmix_x = nullptr, *wkv = nullptr, *cmix_x = nullptr, *v_first = nullptr;  // parts of one allocation (a device allocation costs 0.1 ms and more)
+    size_t bytes = 0;
     CUtensorMap wkv_map;      // all layers' WKV states as one 2-D tensor [layers x slots x heads x 64][64] fp32 (TMA boxes of 64 rows x 32 columns)
     bool wkv_map_ok = false;  // encoded on first use
+    void allocate(Model* m, int64_t slots);
+    void clear();  // zeros, on the model's stream
     ~State();
 };
 
@@ -131,6 +134,12 @@ struct Model {
     static constexpr int kPinRing = 4;
     void* pinned = nullptr;
     size_t pinned_bytes = 0;  // bytes per ring area
+    // pinned staging of a chunk's logits on their way to the caller (at most 128 rows), with an event per piece
+    static constexpr int kOutParts = 32;
+    float* pinned_out = nullptr;
+    size_t pinned_out_bytes = 0;
+    cudaEvent_t out_ev[kOutParts] = {};
+    void ensure_pinned_out(size_t bytes);
     cudaEvent_t pin_ev[kPinRing] = {nullptr, nullptr, nullptr, nullptr};
     int pin_next = 0;
     // profiling (clear_kernel_prof / dump_kernel_prof of the reference, src/gpu_model.rs:561-570)

@@ -176,14 +176,7 @@ int rsv_sched_new(rsv_model* mh, int64_t max_slots, int64_t chunk, int64_t max_r
         S->max_rows = (int)max_rows;
         S->seq_cap = (int)max_new_cap;
         State& st = S->st;
-        st.model = &m;
-        st.cap = max_slots;
-        const Config& c = m.cfg;
-        const size_t nx = (size_t)c.n_layer * max_slots * c.n_embd, ns = (size_t)c.n_layer * max_slots * c.n_head * kHeadSize * kHeadSize;
-        RSV_CUDA(cudaMalloc(&st.tmix_x, nx * 4));
-        RSV_CUDA(cudaMalloc(&st.cmix_x, nx * 4));
-        RSV_CUDA(cudaMalloc(&st.wkv, ns * 4));
-        RSV_CUDA(cudaMalloc(&st.v_first, (size_t)max_slots * c.n_embd * 4));
+        st.allocate(&m, max_slots);
         RSV_CUDA(cudaMalloc(&S->slot_tok, (size_t)max_slots * 4));
         RSV_CUDA(cudaMalloc(&S->slot_seq, (size_t)max_slots * max_new_cap * 4));
         RSV_CUDA(cudaMalloc(&S->slot_cnt, (size_t)max_slots * 4));

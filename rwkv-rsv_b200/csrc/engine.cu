@@ -649,16 +649,18 @@ void run_linear_simt(Model& m, const char* name, const LinReq* reqs, int n, int 
 
 
 // ---- tensor-core path ---------------------------------------------------------------------------
-// Row tiles of a step: at most 64 activation rows each (32 with per-group int8 weights), of equal size.
+// Row tiles of a step, of equal size: at most 64 activation rows each (32 with per-group int8 weights).  With fp16 weights alone and more
+// than 128 rows a tile has up to 128: its two columns per row then fill the matrix instruction as four per row of 64 do, and the
+// weights pass through L2 half as often.
 struct RowTiles {
     int R = 0, rt = 0, n = 0, nt8 = 0, nt16 = 0;
     int nt(int fmt) const { return fmt == RL_F16 ? nt16 : nt8; }
     size_t image_bytes(int fmt, int K) const { return (size_t)n * ((K + rl_kelems(fmt) - 1) / rl_kelems(fmt)) * nt(fmt) * 128; }
 };
-RowTiles row_tiles(int R, bool per_group) {
+RowTiles row_tiles(int R, bool per_group, bool int8) {
     RowTiles t;
     t.R = R;
-    const int most = per_group ? kRlMaxRowsG : kRlMaxRows;
+    const int most = per_group ? kRlMaxRowsG : int8 || R <= kRlMaxRowsF ? kRlMaxRows : kRlMaxRowsF;
     t.n = (R + most - 1) / most;
     t.rt = (R + t.n - 1) / t.n;
     t.nt8 = (int)round_up((size_t)t.rt * rl_cols(RL_I8), 16);
@@ -719,7 +721,8 @@ struct RlReq {
     int ldx = 0;
 };
 
-constexpr size_t kRlHalfSm = 111 * 1024;  // dynamic shared memory of a CTA that leaves room for a second one on its SM
+constexpr size_t kRlRingMax = 196 * 1024;  // stages of the persistent kernel, which has its SM to itself
+constexpr size_t kRlHalfSm = 109 * 1024;  // dynamic shared memory of a CTA that leaves room for a second one on its SM
 
 // How many CTAs share a tile's K.  The step's launches are short (few tiles, weights prefetched behind the previous kernel), so a
 // launch wants about one CTA per half SM and few K blocks per CTA, but no second wave.
@@ -802,6 +805,27 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
         const int sk = L.p[i].fmt == RL_F16 && L.f16_halves ? std::min(L.split, 2) : L.split;
         nk = std::max(nk, (L.p[i].kblocks + sk - 1) / sk);
     }
+    // Several full row tiles that fill the GPU without splitting K: the persistent kernel.  A tile of fewer than 16 K blocks is all
+    // epilogue (the rank back-projections: 30 us at 512 rows with a CTA per tile, 34 persistent), and fp16 tiles of 64 rows leave half of
+    // the matrix instruction's columns out.
+    if (!build && !grouped && t.n > 1 && L.split == 1 && kb_min >= 16 && (row8 || t.rt > kRlMaxRows)) {
+        const size_t st = kRlABytes + (size_t)nt_max * 128;
+        L.nt_max = nt_max;
+        L.ring = (int)(std::min<size_t>(kRlMaxStages, kRlRingMax / st) * st);
+        L.tmem_cols = 64;
+        while (L.tmem_cols < 2 * nt_max) L.tmem_cols *= 2;
+        const size_t bytes = L.ring + 1024;
+        static bool configured[16] = {false};
+        if (!configured[m.device & 15]) {
+            RSV_CUDA(cudaFuncSetAttribute(rows_linear_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRlRingMax + 1024));
+            configured[m.device & 15] = true;
+        }
+        LAUNCH(m, name) {
+            launch_pdl(m, rows_linear_persistent_kernel, dim3(std::min(jobs, m.num_sms)), dim3(kRlThreads), bytes, L, jobs);
+            check_launch("rows_linear_persistent");
+        }
+        return;
+    }
     const size_t stage = kRlABytes + (build ? 0 : (size_t)nt_max * 128), bbuf = build ? (size_t)nk * nt_max * 128 : 0, tg = grouped ? round_up((size_t)nk * t.rt * 4, 16) : 0;
     const size_t recv = (size_t)L.split * ((t.rt + L.split - 1) / L.split) * kRlTileM * 8;  // partial sums reuse the ring
     int stages = std::min(nk, kRlMaxStages);
@@ -860,10 +884,14 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     if (R == 0) return;
     RSV_CUDA(cudaSetDevice(device));
     const LayerW& L0 = layers[0];
-    bool per_group = false;
+    bool per_group = false, int8 = false;
     for (const LayerW& L : layers)
-        for (const LinearW* W : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv}) per_group = per_group || rl_fmt(*W) == RL_I8G;
-    const RowTiles t = row_tiles(R, per_group), to = row_tiles(std::max(O, 1), rl_fmt(head) == RL_I8G);
+        for (const LinearW* W : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv}) {
+            per_group = per_group || rl_fmt(*W) == RL_I8G;
+            int8 = int8 || rl_fmt(*W) == RL_I8;
+        }
+    // tw: the layer's launches with many weight tiles; t: the others, which would have too few tiles for the GPU with 128 rows each
+    const RowTiles t = row_tiles(R, per_group, true), tw = row_tiles(R, per_group, int8), to = row_tiles(std::max(O, 1), rl_fmt(head) == RL_I8G, rl_fmt(head) == RL_I8);
     // Operands of a layer; the matrices of one kind have the same format in every layer of the files the loader accepts, and where
     // they do not, the operand is carved again.
     OperandCarver cv;
@@ -872,17 +900,17 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     };
     auto carve_layer = [&](const LayerW& L, LayerOps& o) {
         cv.used = 0;
-        o.r = cv.operand(t, rl_fmt(L.Wr), C, L.x_r);
-        o.k = cv.operand(t, rl_fmt(L.Wk), C, L.x_k);
-        o.v = cv.operand(t, rl_fmt(L.Wv), C, L.x_v);
-        o.w = cv.operand(t, RL_F16, C, L.x_w);
-        o.a = cv.operand(t, RL_F16, C, L.x_a);
-        o.g = cv.operand(t, RL_F16, C, L.x_g);
-        o.vr = rl_fmt(L.Wv) == RL_F16 ? o.v : cv.operand(t, RL_F16, C, L.x_v);
+        o.r = cv.operand(tw, rl_fmt(L.Wr), C, L.x_r);
+        o.k = cv.operand(tw, rl_fmt(L.Wk), C, L.x_k);
+        o.v = cv.operand(tw, rl_fmt(L.Wv), C, L.x_v);
+        o.w = cv.operand(tw, RL_F16, C, L.x_w);
+        o.a = cv.operand(tw, RL_F16, C, L.x_a);
+        o.g = cv.operand(tw, RL_F16, C, L.x_g);
+        o.vr = rl_fmt(L.Wv) == RL_F16 ? o.v : cv.operand(tw, RL_F16, C, L.x_v);
         const int mids[4] = {cfg.w_mid, cfg.a_mid, cfg.g_mid, cfg.v_mid};
         for (int i = 0; i < 4; ++i) o.mid[i] = cv.operand(t, RL_F16, mids[i]);
         o.y = cv.operand(t, rl_fmt(L.Wo), C, nullptr, known_parts(C));
-        o.x2 = cv.operand(t, rl_fmt(L.Wfk), C, L.ffn_x_k);
+        o.x2 = cv.operand(tw, rl_fmt(L.Wfk), C, L.ffn_x_k);
         o.h = cv.operand(t, rl_fmt(L.Wfv), F, nullptr, known_parts(F));
     };
     LayerOps ops;
@@ -921,7 +949,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         A.segs = ws.seg_meta;
         A.R = R;
         A.C = C;
-        A.rt = t.rt;
+        A.rt = tw.rt;
         A.nseg = from ? S : 0;
         return A;
     };
@@ -961,7 +989,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
                 {&L.g1, &ops.g, mg, MIDS, EPI_SIGMOID},
                 {&L.v1, &ops.vr, mv, MIDS, EPI_STORE},
             };
-            run_rows_linear(*this, "linear_rkv_rank", q, l == 0 ? 6 : 7, t);
+            run_rows_linear(*this, "linear_rkv_rank", q, l == 0 ? 6 : 7, tw);
             // back-projections: decay w, a, gate g and (layers > 0) the v-lerp gate
             const int nb = l == 0 ? 3 : 4;
             const LinearW* Wb[4] = {&L.w2, &L.a2, &L.g2, &L.v2};
@@ -1003,7 +1031,15 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
                 // prefill chunks: vectors built by preparation warps, only state-dependent work in the per-token chain (wkv_seq.cuh)
                 // few (head, segment) pairs: a head over two CTAs
                 if (H * S <= num_sms) {
-                    launch_pdl(*this, wkv7_seq_kernel<2>, dim3(2 * H, S), dim3(kWsThreads), 0, ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, ws.g,
+                    // Where every CTA can have an SM to itself it asks for more than half of the shared memory, so that no two share one:
+                    // they would start in pairs as the predecessor's CTAs leave, and a pair takes a third longer (512 tokens, 40 heads).
+                    const size_t alone = 2 * H * S <= num_sms ? 120 * 1024 : 0;
+                    static bool configured[16] = {false};
+                    if (!configured[device & 15]) {
+                        RSV_CUDA(cudaFuncSetAttribute(wkv7_seq_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024));
+                        configured[device & 15] = true;
+                    }
+                    launch_pdl(*this, wkv7_seq_kernel<2>, dim3(2 * H, S), dim3(kWsThreads), alone, ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, ws.g,
                                L.k_k, L.k_a, L.r_k, L.lnx_w, L.lnx_b, wkv, l == 0 ? st.v_first : nullptr, ws.yg, H, C, ws.status);
                 } else {
                     launch_pdl(*this, wkv7_seq_kernel<4>, dim3(H, S), dim3(kWsThreads), 0, ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, ws.g,
@@ -1055,7 +1091,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         {
             RlReq q = {&L.Wfk, &ops.x2, ws.h, F, EPI_RELU2};
             q.ymax = ws.hmax;
-            run_rows_linear(*this, "linear_ffn_key", &q, 1, t);
+            run_rows_linear(*this, "linear_ffn_key", &q, 1, tw);
         }
         linear_known("linear_ffn_value", RlReq{&L.Wfv, nullptr, ws.delta, C, EPI_STORE}, ws.h, F, ws.hmax, (F + kRlTileM - 1) / kRlTileM, ops.h);
         pending = ws.delta;
@@ -1533,7 +1569,7 @@ void engine_op_linear(Model& m, int path, int wtype, const void* w_host, const u
         RSV_CUDA(cudaMalloc(&dy, (size_t)R * M * 4));
         RSV_CUDA(cudaMemcpyAsync(dx, x_host, (size_t)R * K * 4, cudaMemcpyHostToDevice, m.stream));
         if (path == 1) {
-            const RowTiles t = row_tiles(R, false);
+            const RowTiles t = row_tiles(R, false, rl_fmt(W) == RL_I8);
             OperandCarver cv;
             cv.operand(t, rl_fmt(W), K);
             ensure_operand_memory(m, cv.used);

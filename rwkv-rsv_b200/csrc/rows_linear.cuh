@@ -14,7 +14,7 @@
 // of 1, 2, 4 or 8 CTAs that exchange partial sums through distributed shared memory (each CTA finishes its share of the activation
 // rows), so that a layer with few tiles still has every SM streaming and no partial sum goes through global memory (the kernel this
 // one replaces cut tiles between persistent CTAs and paid a global round trip, an atomic and a serial sum per cut tile).  A CTA takes
-// at most half an SM (<= 112 KB shared memory, <= 256 TMEM columns): two are resident, one loads while the other finishes, and the
+// at most half an SM (<= 113 KB shared memory, <= 256 TMEM columns): two are resident, one loads while the other finishes, and the
 // next kernel of the step becomes resident early and requests its weights before the dependency wait.
 // What bounds it: at few rows the chain operand tiles (L2) -> products -> exchange -> store behind the dependency wait, the weights
 // are there already; at 64 rows the operand tiles' L2 traffic as well (a 128-row tile re-reads them all).
@@ -40,7 +40,8 @@ constexpr int kRlEpiWarps = 8;
 constexpr int kRlEpiThreads = 32 * kRlEpiWarps;
 constexpr int kRlTileM = 128;
 constexpr int kRlABytes = kRlTileM * 128;
-constexpr int kRlMaxRows = 64;    // activation rows of a tile
+constexpr int kRlMaxRows = 64;    // activation rows of a tile with int8 weights, or few rows
+constexpr int kRlMaxRowsF = 128;  // the same for fp16 weights and many rows (256 columns of operand either way)
 constexpr int kRlMaxRowsG = 32;   // the same for per-group weights: two accumulators are in use, and fp32 sums in registers
 constexpr int kRlMaxProb = 8;
 constexpr int kRlMaxStages = 8;
@@ -62,7 +63,7 @@ struct RlProb {
 struct alignas(64) RlLaunch {
     CUtensorMap amap[kRlMaxProb];
     RlProb p[kRlMaxProb];
-    int nprob, R, rt, n_tiles, split, log_split, nt8, nt16, ring, tmem_cols, f16_halves;  // ring: bytes of shared memory for stages
+    int nprob, R, rt, n_tiles, split, log_split, nt8, nt16, nt_max, ring, tmem_cols, f16_halves;  // ring: bytes of shared memory for stages
     int* status;
 };
 
@@ -110,10 +111,83 @@ __device__ __forceinline__ void rl_activate4(int epi, float (&a)[4], float bias)
             for (int i = 0; i < 4; ++i) a[i] = expf(a[i] * kDecayScale);
     }
 }
+// Lane i < 4: the warp's maximum of |a[i]| (a NaN counts as 0).
+__device__ __forceinline__ float rl_rowmax4(const float (&a)[4], bool mine, int lane) {
+    uint32_t mx = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t t = __reduce_max_sync(0xffffffffu, mine ? __float_as_uint(fmaxf(fabsf(a[i]), 0.f)) : 0u);
+        if (lane == i) mx = t;
+    }
+    return __uint_as_float(mx);
+}
 // exact integer (|q| < 2^51) -> double without the slow 64-bit conversion
 __device__ __forceinline__ double rl_ll2d(long long q) { return __longlong_as_double(0x4338000000000000LL + q) - 6755399441055744.0; }
 __device__ __forceinline__ long long rl_digits2q(int i0, int i1, int i2, int i3) {
     return ((long long)i0 * 128 + i1) * 16384 + ((long long)i2 * 128 + i3);
+}
+
+// Where a tile's outputs go: row rl of the tile to y + rl ldy (and y2), nr rows.
+struct RlOut {
+    float *y, *y2;
+    size_t ldy;
+    int nr, epi;
+    float bias;
+    bool maxima;
+};
+__device__ __forceinline__ RlOut rl_out(const RlProb& P, int r0, int nr, int m, float bias) {
+    RlOut o;
+    o.ldy = (size_t)P.ldy;
+    o.y = P.y + (size_t)r0 * P.ldy + m;
+    o.y2 = P.y2 ? P.y2 + (size_t)r0 * P.ldy + m : nullptr;
+    o.nr = nr;
+    o.epi = P.epi;
+    o.bias = bias;
+    o.maxima = P.ymax != nullptr;
+    return o;
+}
+// The sums of a tile whose K was not split, from tensor memory through the thread's registers to the output, rows rl .. rl + 3 at a time
+// (`half`: the two warps of a lane quarter take turns).  What bounds this is instructions: 8192 outputs on eight warps.
+__device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t taddr, const float* s_xs, const double2* s_xt, float* s_ymax, double ws, double wz, bool mok,
+                                          int half, int lane) {
+#pragma unroll 1
+    for (int rl = 4 * half; rl < o.nr; rl += 8) {
+        float a[4];
+        if (f16) {
+            uint32_t v[8];
+            tmem_ld8(taddr + 2 * rl, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = s_xs[rl + i] * (__uint_as_float(v[2 * i]) + __uint_as_float(v[2 * i + 1]));
+        } else {
+            uint32_t v[16];
+            tmem_ld16(taddr + 4 * rl, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double2 xt = s_xt[rl + i];
+                a[i] = (float)(xt.x * (ws * rl_ll2d(rl_digits2q((int)v[4 * i], (int)v[4 * i + 1], (int)v[4 * i + 2], (int)v[4 * i + 3])) + wz * xt.y));
+            }
+        }
+        rl_activate4(o.epi, a, o.bias);
+        const int left = o.nr - rl;
+        float* p = o.y + (size_t)rl * o.ldy;
+        if (mok) {
+            p[0] = a[0];
+            if (left > 1) p[o.ldy] = a[1];
+            if (left > 2) p[2 * o.ldy] = a[2];
+            if (left > 3) p[3 * o.ldy] = a[3];
+        }
+        if (o.y2 && mok) {
+            p = o.y2 + (size_t)rl * o.ldy;
+            p[0] = a[0];
+            if (left > 1) p[o.ldy] = a[1];
+            if (left > 2) p[2 * o.ldy] = a[2];
+            if (left > 3) p[3 * o.ldy] = a[3];
+        }
+        if (o.maxima) {
+            const float mx = rl_rowmax4(a, mok, lane);
+            if (lane < 4) s_ymax[rl + lane] = mx;  // (rows past the end have slots of their own)
+        }
+    }
 }
 
 // GROUPED: the launch's int8 problems have per-group weights (RL_I8G), else RL_I8; fp16 problems may be in either kind of launch.
@@ -125,9 +199,9 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     __shared__ __align__(8) uint64_t full[kRlMaxStages], empty[kRlMaxStages], acc_full[2], acc_empty[2], b_ready;
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
-    __shared__ float s_xs[kRlMaxRows];
-    __shared__ double s_T[kRlMaxRows];
-    __shared__ uint32_t s_ymax[kRlMaxRows];
+    __shared__ float s_xs[kRlMaxRowsF];
+    __shared__ double2 s_xt[kRlMaxRows];  // int8: the row's scale, and its sum of fixed-point values
+    __shared__ float s_ymax[4][kRlMaxRowsF];  // per lane quarter (32 weight rows)
     uint8_t* smem = (uint8_t*)(((uintptr_t)rl_raw + 1023) & ~(uintptr_t)1023);
     volatile int* abort_flag = &s_abort;
 
@@ -147,24 +221,40 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     const int r0 = ntile * L.rt, nr = min(L.rt, L.R - r0), ncols = nr * D;
     const bool grouped = GROUPED && fmt == RL_I8G;
 
-    if (threadIdx.x < kRlMaxStages) {
-        mbar_init(&full[threadIdx.x], 1);
-        mbar_init(&empty[threadIdx.x], 1);
-        if (threadIdx.x < 2) {
-            mbar_init(&acc_full[threadIdx.x], 1);
-            mbar_init(&acc_empty[threadIdx.x], kRlEpiWarps);
+    // The producer's thread sets the barriers up and requests the first ring pass of weights at once: the block's setup (tensor memory,
+    // synchronisation) is hidden behind the copies.  Tiles the ring has no room for yet are requested into L2.
+    const int kel = rl_kelems(fmt);
+    const uint32_t bbytes = BUILD ? 0u : (uint32_t)(NT * 128);
+    uint64_t pol = 0;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kRlMaxStages; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
         }
-        if (threadIdx.x == 0) {
-            mbar_init(&b_ready, kRlEpiWarps);
-            s_abort = 0;
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], kRlEpiWarps);
         }
+        mbar_init(&b_ready, kRlEpiWarps);
+        s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // weights are read once per step: marked evict-first so that activations, states, vectors and the kernels' code stay in L2
+        // (several row tiles share a weight tile: then it has to stay until the others have read it)
+        pol = L.n_tiles == 1 ? l2_evict_first_policy() : l2_evict_normal_policy();
+#pragma unroll 1
+        for (int j = 0; j < nk; ++j) {
+            if (j < NS) {
+                mbar_expect_tx(&full[j], kRlABytes + bbytes);
+                tma_load_2d_hint(&L.amap[pi], &full[j], smem + (size_t)j * stage_bytes, (kb0 + j) * kel, mt * kRlTileM, pol);
+            } else {
+                tma_prefetch_2d(&L.amap[pi], (kb0 + j) * kel, mt * kRlTileM);
+            }
+        }
     }
     if (warp == 1) {
         tmem_alloc(&tmem_slot, (uint32_t)L.tmem_cols);
         tmem_relinquish();
     }
-    if (threadIdx.x >= 64 && threadIdx.x < 64 + kRlMaxRows) s_ymax[threadIdx.x - 64] = 0u;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -172,47 +262,25 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     pdl_launch_dependents();
 
     if (warp == 0) {
-        // ---------------- producer: weight tiles before the dependency wait, operand tiles behind it ----------------
+        // ---------------- producer: operand tiles behind the dependency wait, then the rest of the ring's traffic ----------------
         if (lane == 0) {
-            const int kel = rl_kelems(fmt);
-            // weights are read once per step: marked evict-first so that activations, states, vectors and the kernels' code stay in L2
-            // (several row tiles share a weight tile: then it has to stay until the others have read it)
-            const uint64_t pol = L.n_tiles == 1 ? l2_evict_first_policy() : l2_evict_normal_policy();
-            const uint32_t bbytes = BUILD ? 0u : (uint32_t)(NT * 128);
             const uint8_t* bsrc = BUILD ? nullptr : P.bimg + ((size_t)ntile * P.kblocks + kb0) * bbytes;
+            const int filled = min(NS, nk);
             uint32_t s = 0, par = 1;  // a fresh barrier passes a wait on parity 1
-            int j = 0, filled = 0;
+            int j = 0;
+            if (!BUILD) pdl_wait();
 #pragma unroll 1
-            for (int step = 0; step < 2; ++step) {
-                // step 0: the first ring pass (weights only), and the tiles the ring has no room for yet are requested into L2, so that
-                // HBM works while the predecessor finishes; step 1: their operand tiles, then the rest of the ring's traffic
-                if (step == 0) {
-#pragma unroll 1
-                    for (; j < nk; ++j) {
-                        if (j < NS) {
-                            mbar_expect_tx(&full[j], kRlABytes + bbytes);
-                            tma_load_2d_hint(&L.amap[pi], &full[j], smem + (size_t)j * stage_bytes, (kb0 + j) * kel, mt * kRlTileM, pol);
-                        } else {
-                            tma_prefetch_2d(&L.amap[pi], (kb0 + j) * kel, mt * kRlTileM);
-                        }
-                    }
-                    filled = min(NS, nk);
-                    if (!BUILD) pdl_wait();
-                } else {
-#pragma unroll 1
-                    for (j = 0; j < nk; ++j) {
-                        uint8_t* dst = smem + (size_t)s * stage_bytes;
-                        if (j >= filled) {
-                            if (!mbar_wait(&empty[s], par, abort_flag)) break;
-                            mbar_expect_tx(&full[s], kRlABytes + bbytes);
-                            tma_load_2d_hint(&L.amap[pi], &full[s], dst, (kb0 + j) * kel, mt * kRlTileM, pol);
-                        }
-                        if (!BUILD) bulk_load(dst + kRlABytes, bsrc + (size_t)j * bbytes, bbytes, &full[s]);
-                        if (++s == (uint32_t)NS) {
-                            s = 0;
-                            par ^= 1u;
-                        }
-                    }
+            for (; j < nk; ++j) {
+                uint8_t* dst = smem + (size_t)s * stage_bytes;
+                if (j >= filled) {
+                    if (!mbar_wait(&empty[s], par, abort_flag)) break;
+                    mbar_expect_tx(&full[s], kRlABytes + bbytes);
+                    tma_load_2d_hint(&L.amap[pi], &full[s], dst, (kb0 + j) * kel, mt * kRlTileM, pol);
+                }
+                if (!BUILD) bulk_load(dst + kRlABytes, bsrc + (size_t)j * bbytes, bbytes, &full[s]);
+                if (++s == (uint32_t)NS) {
+                    s = 0;
+                    par ^= 1u;
                 }
             }
             if (*abort_flag)  // copies in flight land before the CTA may exit
@@ -328,7 +396,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
                     long long t = 0;
 #pragma unroll 1
                     for (int i = 0; i < P.tparts; ++i) t += __ldcg(P.tsum + (size_t)(r0 + et) * P.tparts + i);
-                    s_T[et] = rl_ll2d(t);
+                    s_xt[et] = make_double2((double)s_xs[et], rl_ll2d(t));
                 }
             }
             if (grouped)
@@ -378,11 +446,13 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
         }
         tc_fence_after();
     }
-    // Exchange.  Row r of the tile is finished by CTA r mod S of the cluster (S = 1: this one); its sums land in the owner's ring as
+    // K in one piece: the sums go from tensor memory through this thread's registers to the output.  Otherwise (and for per-group
+    // weights) they are exchanged: row r of the tile is finished by CTA r mod S of the cluster (S = 1: this one); its sums land in the owner's ring as
     // [slice][row / S][128] eight-byte words: the exact integer, the hi and lo sums of an fp16 row, or the fp32 sum of per-group weights.
     if (S > 1) cluster_sync_all();  // every CTA of the cluster is done with its ring
-    const bool go = epi && !__any_sync(0xffffffffu, *abort_flag);
-    if (go && nk > 0) {
+    const bool go = epi && !__any_sync(0xffffffffu, *abort_flag), direct = BUILD || (S == 1 && !grouped);
+    const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
+    if (!BUILD && go && nk > 0 && !direct) {
         auto send = [&](int r, unsigned long long v) {
             if (r < nr) st_cluster_u64(map_to_rank(recv + (uint32_t)(((rank * slots + (r >> sh)) * kRlTileM + ml) * 8), (uint32_t)(r & (S - 1))), v);
         };
@@ -392,12 +462,11 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
 #pragma unroll
                 for (int i = 0; i < 4; ++i) send((2 * c + half) * 4 + i, (unsigned long long)__float_as_uint(gacc[c][i]));
         } else {
-            const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
             for (int c0 = half * 16; c0 < ncols; c0 += 32) {
                 uint32_t v[16];
                 tmem_ld16(taddr + c0, v);
-                if (BUILD || fmt == RL_F16) {
+                if (fmt == RL_F16) {
 #pragma unroll
                     for (int i = 0; i < 8; ++i) send((c0 >> 1) + i, (unsigned long long)v[2 * i] | ((unsigned long long)v[2 * i + 1] << 32));
                 } else {
@@ -408,22 +477,31 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
         }
     }
     if (S > 1) cluster_sync_all();
-    else if (epi) rl_epi_sync();
-    if (go) {
+    else if (GROUPED && epi && !direct) rl_epi_sync();
+    const int epi_op = P.epi;
+    const double wsd = ws, wzd = wz;
+    if (go && direct) {
+        const RlOut out = rl_out(P, r0, nr, m, bias);
+        rl_finish(out, BUILD || fmt == RL_F16, taddr, s_xs, s_xt, s_ymax[quarter], wsd, wzd, mok, half, lane);
+    } else if (!BUILD && go) {
         // this CTA's share of the rows: slices added in order, scaled, activated, stored (four rows at a time per thread)
         const int mine = nr > rank ? (nr - rank + S - 1) >> sh : 0;
-        const size_t stride = (size_t)slots * kRlTileM;
-        float* y = P.y + (size_t)r0 * P.ldy + m;
-        float* y2 = P.y2 ? P.y2 + (size_t)r0 * P.ldy + m : nullptr;
-        const int epi_op = P.epi;
+        const size_t stride = (size_t)slots * kRlTileM, ystep = (size_t)P.ldy << sh;
+        const size_t y0 = (size_t)(r0 + rank + (4 * half << sh)) * P.ldy + m;
+        float *y = P.y + y0, *y2 = P.y2 ? P.y2 + y0 : nullptr;
+        const bool maxima = P.ymax != nullptr;
 #pragma unroll 1
-        for (int rl = 4 * half; rl < mine; rl += 8) {
-            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(smem) + (size_t)rl * kRlTileM + ml;
-            int off[4];  // rows past the end repeat the last one
-#pragma unroll
-            for (int i = 0; i < 4; ++i) off[i] = min(i, mine - 1 - rl) * kRlTileM;
+        for (int rl = 4 * half; rl < mine; rl += 8, y += 8 * ystep) {
+            const int left = mine - rl;  // rows past the end repeat the last one
             float a[4];
-            if (BUILD || fmt != RL_I8) {
+            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(smem) + (size_t)rl * kRlTileM + ml;
+            int r[4], off[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                off[i] = min(i, left - 1) * kRlTileM;
+                r[i] = rank + ((rl + min(i, left - 1)) << sh);
+            }
+            if (fmt != RL_I8) {
                 float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};  // (per-group weights: the fp32 sum is in hi, lo is zero)
 #pragma unroll 1
                 for (int s = 0; s < Sk; ++s, src += stride)
@@ -434,7 +512,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
                         lo[i] += __uint_as_float((uint32_t)(t >> 32));
                     }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = s_xs[min(rank + ((rl + i) << sh), nr - 1)] * (hi[i] + lo[i]);
+                for (int i = 0; i < 4; ++i) a[i] = s_xs[r[i]] * (hi[i] + lo[i]);
             } else {
                 long long q[4] = {0, 0, 0, 0};
 #pragma unroll 1
@@ -442,34 +520,222 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
 #pragma unroll
                     for (int i = 0; i < 4; ++i) q[i] += (long long)src[off[i]];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = min(rank + ((rl + i) << sh), nr - 1);
-                    a[i] = (float)((double)s_xs[r] * ((double)ws * rl_ll2d(q[i]) + (double)wz * s_T[r]));
-                }
+                for (int i = 0; i < 4; ++i) a[i] = (float)(s_xt[r[i]].x * (wsd * rl_ll2d(q[i]) + wzd * s_xt[r[i]].y));
             }
             rl_activate4(epi_op, a, bias);
-            float* yr = y + (size_t)(rank + (rl << sh)) * P.ldy;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                if (mok && rl + i < mine) yr[(size_t)(i << sh) * P.ldy] = a[i];
+                if (mok && i < left) y[i * ystep] = a[i];
             if (y2) {
-                float* y2r = y2 + (size_t)(rank + (rl << sh)) * P.ldy;
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    if (mok && rl + i < mine) y2r[(size_t)(i << sh) * P.ldy] = a[i];
+                    if (mok && i < left) y2[i * ystep] = a[i];
+                y2 += 8 * ystep;
             }
-            if (P.ymax) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float mx = warp_absmax(mok ? a[i] : 0.f);
-                    if (lane == 0 && rl + i < mine) atomicMax(&s_ymax[rank + ((rl + i) << sh)], __float_as_uint(mx));
-                }
+            if (maxima) {
+                const float mx = rl_rowmax4(a, mok, lane);
+                if (lane < min(4, left)) s_ymax[quarter][rank + ((rl + lane) << sh)] = mx;
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (P.ymax && go && et < nr && (et & (S - 1)) == rank) P.ymax[(size_t)(r0 + et) * ((P.M + kRlTileM - 1) / kRlTileM) + mt] = __uint_as_float(s_ymax[et]);
+    if (P.ymax && go && et < nr && (et & (S - 1)) == rank) P.ymax[(size_t)(r0 + et) * ((P.M + kRlTileM - 1) / kRlTileM) + mt] = fmaxf(fmaxf(s_ymax[0][et], s_ymax[1][et]), fmaxf(s_ymax[2][et], s_ymax[3][et]));
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(L.status, 2);
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, (uint32_t)L.tmem_cols);
+    }
+}
+
+// Many rows (several row tiles; per-row int8 and fp16 weights): one persistent CTA per SM takes tiles of 128 weight rows x up to 64
+// activation rows in turn, whole K.  One ring of stages runs through all of them and there are two accumulators, so the tensor core
+// works on the next tile while the epilogue warps finish the last one.  With a CTA per tile (two resident) both CTAs of an SM ran in
+// step: of a tile's 22 us at K = 2560 the tensor core worked 13 at 85 % of its rate, the rest was the first loads and the epilogue.
+// Measured, 2560 x 10240 (ffn.key): int8, 1024 rows 139 -> 94 us, 512 rows 82 -> 56 us.  What bounds it: the products (0.3 us per K block
+// and SM of 0.27 at the nominal rate), then the last turn, in which some SMs have no tile.
+struct RlCursor {
+    int job, pi, kb, nk, mt, ntile;
+    __device__ __forceinline__ void set(const RlLaunch& L, int j) {
+        job = j;
+        kb = 0;
+        while (pi + 1 < L.nprob && j >= L.p[pi + 1].job0) ++pi;  // jobs come in ascending order
+        const int lt = j - L.p[pi].job0;
+        mt = lt / L.n_tiles;
+        ntile = lt - mt * L.n_tiles;
+        nk = L.p[pi].kblocks;
+    }
+};
+__global__ void __launch_bounds__(kRlThreads, 1) rows_linear_persistent_kernel(const __grid_constant__ RlLaunch L, int jobs) {
+    extern __shared__ __align__(1024) uint8_t rl_raw[];
+    __shared__ __align__(8) uint64_t full[kRlMaxStages], empty[kRlMaxStages], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_abort;
+    __shared__ float s_xs[kRlMaxRowsF];
+    __shared__ double2 s_xt[kRlMaxRows];
+    __shared__ float s_ymax[4][kRlMaxRowsF];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)rl_raw + 1023) & ~(uintptr_t)1023);
+    volatile int* abort_flag = &s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = (int)gridDim.x;
+    const uint32_t stage_bytes = (uint32_t)(kRlABytes + L.nt_max * 128), acc_cols = (uint32_t)L.tmem_cols / 2;
+    const uint32_t NS = min((uint32_t)kRlMaxStages, (uint32_t)L.ring / stage_bytes);
+    uint32_t filled = 0;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kRlMaxStages; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&acc_full[i], 1);
+            mbar_init(&acc_empty[i], kRlEpiWarps);
+        }
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // weights of the first ring pass, before the dependency wait
+        RlCursor c;
+        c.pi = 0;
+        c.set(L, (int)blockIdx.x);
+#pragma unroll 1
+        for (; filled < NS && c.job < jobs; ++filled) {
+            const int fmt = L.p[c.pi].fmt;
+            mbar_expect_tx(&full[filled], kRlABytes + (uint32_t)(fmt == RL_F16 ? L.nt16 : L.nt8) * 128u);
+            tma_load_2d(&L.amap[c.pi], &full[filled], smem + (size_t)filled * stage_bytes, c.kb * rl_kelems(fmt), c.mt * kRlTileM);
+            if (++c.kb == c.nk) {
+                if (c.job + G >= jobs) {
+                    ++filled;
+                    break;
+                }
+                c.set(L, c.job + G);
+            }
+        }
+    }
+    if (warp == 1) {
+        tmem_alloc(&tmem_slot, (uint32_t)L.tmem_cols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();
+
+    RlCursor c;
+    c.pi = 0;
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t f = 0, s = 0, par = 1;
+            bool ok = true;
+            pdl_wait();
+#pragma unroll 1
+            for (int job = (int)blockIdx.x; job < jobs && ok; job += G) {
+                c.set(L, job);
+                const RlProb& P = L.p[c.pi];
+                const int kel = rl_kelems(P.fmt);
+                const uint32_t bbytes = (uint32_t)(P.fmt == RL_F16 ? L.nt16 : L.nt8) * 128u;
+                const uint8_t* bsrc = P.bimg + (size_t)c.ntile * c.nk * bbytes;
+#pragma unroll 1
+                for (int kb = 0; kb < c.nk; ++kb, ++f, bsrc += bbytes) {
+                    uint8_t* dst = smem + (size_t)s * stage_bytes;
+                    if (f >= filled) {
+                        if (!mbar_wait(&empty[s], par, abort_flag)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_expect_tx(&full[s], kRlABytes + bbytes);
+                        tma_load_2d(&L.amap[c.pi], &full[s], dst, kb * kel, c.mt * kRlTileM);
+                    }
+                    bulk_load(dst + kRlABytes, bsrc, bbytes, &full[s]);
+                    if (++s == NS) {
+                        s = 0;
+                        par ^= 1u;
+                    }
+                }
+            }
+            if (*abort_flag)  // copies in flight land before the CTA may exit
+#pragma unroll 1
+                for (uint32_t q = f > NS ? f - NS : 0; q < f; ++q)
+#pragma unroll 1
+                    for (uint32_t i = 0; i < (1u << 16); ++i)
+                        if (mbar_try_wait(&full[q % NS], (q / NS) & 1u)) break;
+        }
+    } else if (warp == 1) {
+        const uint32_t smem_addr = smem_u32(smem);
+        uint32_t s = 0, par = 0, it = 0;
+        bool ok = true;
+#pragma unroll 1
+        for (int job = (int)blockIdx.x; job < jobs && ok; job += G, ++it) {
+            c.set(L, job);
+            const int fmt = L.p[c.pi].fmt, nr = min(L.rt, L.R - c.ntile * L.rt);
+            const uint32_t idesc = tc_idesc(fmt != RL_F16, (nr * rl_cols(fmt) + 15) & ~15), d = tmem + (it & 1u) * acc_cols;
+            ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[it & 1u], ((it >> 1) & 1u) ^ 1u, abort_flag));
+#pragma unroll 1
+            for (int kb = 0; kb < c.nk && ok; ++kb) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t a_addr = smem_addr + s * stage_bytes;
+                const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + kRlABytes);
+                if (fmt != RL_F16) {
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<true>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb == 0 && k4 == 0) ? 0u : 1u);
+                } else {
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<false>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb == 0 && k4 == 0) ? 0u : 1u);
+                }
+                tc_commit_elect(&empty[s]);
+                if (++s == NS) {
+                    s = 0;
+                    par ^= 1u;
+                }
+            }
+            if (ok) tc_commit_elect(&acc_full[it & 1u]);
+        }
+    } else {
+        const int et = threadIdx.x - 64, half = ((warp - 2) >> 2) & 1, quarter = warp & 3, ml = quarter * 32 + lane;
+        uint32_t it = 0;
+        pdl_wait();
+        // every warp runs every turn (the block barriers below): after a time-out without waiting and without output
+#pragma unroll 1
+        for (int job = (int)blockIdx.x; job < jobs; job += G, ++it) {
+            c.set(L, job);
+            const RlProb& P = L.p[c.pi];
+            const int r0 = c.ntile * L.rt, nr = min(L.rt, L.R - r0), m = c.mt * kRlTileM + ml;
+            const bool mok = m < P.M;
+            float ws = 0.f, wz = 0.f, bias = 0.f;
+            if (mok) {
+                if (P.fmt == RL_I8) {
+                    ws = __ldg(P.wscale + m);
+                    wz = __ldg(P.wzero + m);
+                }
+                if (P.bias) bias = __ldg(P.bias + m);
+            }
+            if (et < nr) {
+                const float xs = __ldcg(P.xscale + r0 + et);
+                s_xs[et] = xs;
+                if (P.fmt == RL_I8) {
+                    long long t = 0;
+#pragma unroll 1
+                    for (int i = 0; i < P.tparts; ++i) t += __ldcg(P.tsum + (size_t)(r0 + et) * P.tparts + i);
+                    s_xt[et] = make_double2((double)xs, rl_ll2d(t));
+                }
+            }
+            rl_epi_sync();
+            if (!*abort_flag) mbar_wait_parked(&acc_full[it & 1u], (it >> 1) & 1u, abort_flag);
+            tc_fence_after();
+            if (!__any_sync(0xffffffffu, *abort_flag)) {
+                const RlOut out = rl_out(P, r0, nr, m, bias);
+                rl_finish(out, P.fmt == RL_F16, tmem + ((uint32_t)(quarter * 32) << 16) + (it & 1u) * acc_cols, s_xs, s_xt, s_ymax[quarter], (double)ws, (double)wz, mok, half, lane);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[it & 1u]);
+            rl_epi_sync();
+            if (P.ymax && et < nr)
+                P.ymax[(size_t)(r0 + et) * ((P.M + kRlTileM - 1) / kRlTileM) + c.mt] = fmaxf(fmaxf(s_ymax[0][et], s_ymax[1][et]), fmaxf(s_ymax[2][et], s_ymax[3][et]));
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
     if (threadIdx.x == 0 && *abort_flag) atomicOr(L.status, 2);
     if (warp == 1) {
         tc_fence_after();

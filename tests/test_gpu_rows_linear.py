@@ -31,6 +31,13 @@ def test_linear_tile_edges(rows, m, k, int8):
     assert np.all(np.abs(got - want) <= bound + 1e-30), float((np.abs(got - want) / bound).max())
 
 
+# enough tiles that K is not split and two CTAs share a tile of 256 weight rows: full and ragged row tiles, an odd number of 128-row
+# weight tiles, the last of them partly or wholly past the end
+@pytest.mark.parametrize("rows,m,k,int8", [(513, 2560, 1024, True), (640, 2688, 384, True), (513, 2560, 704, False), (577, 2570, 640, False)])
+def test_linear_tiles_of_a_cta_pair(rows, m, k, int8):
+    test_linear_tile_edges(rows, m, k, int8)
+
+
 @pytest.mark.parametrize("name", ["fp16", "int8", "int8g"])
 def test_step_sizes_agree_with_the_cpu_path(tiny_paths, name):
     # 16 / 17: operands built inside or outside the GEMM; 32 / 33, 64 / 65: one or two row tiles (per-group and other weights)

@@ -7,12 +7,12 @@
 //
 // Decomposition.  CTA c (one per SM) owns output rows [c M / G, (c+1) M / G) of every matrix for the WHOLE K: no
 // partial sums ever cross a CTA, so a phase is  activation vector -> dot products -> tagged stores.
-//   warp 0      producer.  Walks the fixed sequence of weight chunks this CTA will ever need - token after token, layer
+//   warp 0      producer (its warpgroup's other warps idle).  Walks the fixed sequence of weight chunks this CTA will ever need - token after token, layer
 //               after layer, phase after phase - and streams them with bulk asynchronous copies (cp.async.bulk) into a
 //               byte-granular ring in shared memory; a chunk = one tile of up to 16 rows x one piece of K, one mbarrier
 //               per chunk.  It never waits for other CTAs, only for ring space, so HBM keeps streaming while the other
 //               warps wait for activations.
-//   warps 1-16  consumers.  Warp w owns the w-th sixteenth of K of every matrix: it turns its sixteenth of the activation
+//   warps 4-19  consumers.  Warp w of them owns the w-th sixteenth of K of every matrix: it turns its sixteenth of the activation
 //               vector into operand fragments itself (LayerNorm, token shift, fixed-point digits; only the row statistics
 //               and the maximum cross warps) and multiplies its columns of every tile.  So all sixteen warps work on a
 //               tile at once, an operand is read only by the warp that wrote it, and chunks are released in the order they
@@ -44,9 +44,10 @@
 // grid barrier at the end of a token.
 // What bounds it: the dependent chain of a layer, not HBM.  Its code is therefore written once and looped (phases 1, 3, 4, 5 and the
 // head are the same code with other pointers): 32 KB of code run at an instruction per cycle, 128 KB at a third of that, more at less
-// than a fifth; and little may spill: with the shared memory taken, 544 threads' stacks do not fit L1 and every spill is an L2 round trip.
-// Measured per token at 2560 channels, 32 layers, 65536 rows of vocabulary: int8 1.40 ms (3.0 GB: 0.47 ms at copy bandwidth), fp16
-// 1.85 ms; 1.49 and 1.90 ms with a grid barrier after every phase and a tile of rows per warp.  512 channels, 12 layers: 0.09 ms (0.13).
+// than a fifth; and nothing may spill: with the shared memory taken, the threads' stacks do not fit L1 and every spill is an L2 round
+// trip (0.07 ms of a token's 1.40 with 128 bytes of spills).
+// Measured per token at 2560 channels, 32 layers, 65536 rows of vocabulary: int8 1.30 ms (3.0 GB: 0.47 ms at copy bandwidth), fp16
+// 1.83 ms; 1.49 and 1.90 ms with a grid barrier after every phase and a tile of rows per warp.  512 channels, 12 layers: 0.09 ms (0.13).
 // All waits are bounded; on expiry bit 5 of the status word is set (and the word after it says which wait), every role drains its copies in flight and exits.
 #pragma once
 #include <cstddef>
@@ -58,7 +59,11 @@ namespace rsv {
 
 constexpr int kDsConsumerWarps = 16;
 constexpr int kDsConsumers = kDsConsumerWarps * 32;  // 512
-constexpr int kDsThreads = kDsConsumers + 32;        // + producer warp
+constexpr int kDsThreads = kDsConsumers + 128;       // + the producer's warpgroup, of which one warp works
+// Registers per thread.  Seventeen warps put five on one scheduler, so a thread can be launched with 96, and the consumers spilled; the
+// producer's warpgroup gives some of its own to them (both then fit without a spill up to 2560 channels).
+constexpr int kDsLaunchRegs = 96, kDsProducerRegs = 40, kDsConsumerRegs = 104;
+static_assert(128 * kDsProducerRegs + kDsConsumers * kDsConsumerRegs <= kDsThreads * kDsLaunchRegs, "register split");
 constexpr int kDsBars = 32;                          // chunks in flight (mbarrier pairs)
 constexpr int kDsTileRows = 16;                      // rows of a tile (the m dimension of the matrix instruction)
 constexpr int kDsPad = 0;                            // bytes between the rows of a chunk
@@ -69,6 +74,7 @@ constexpr int kDsPartInt = kDsConsumerWarps * 16 + 64;  // bytes per row of part
 constexpr int kDsPartF32 = kDsConsumerWarps * 4 + 16;   // ... or one fp32 sum per warp
 constexpr int kDsPartBytes = 5 * kDsTileRows * kDsPartInt;  // partial sums of a batch of tiles
 constexpr int kDsRankTiles = 2;                      // tiles of rank-projection rows per CTA
+constexpr int kDsMergeBytes = 24 * 1024;             // a tile of at most this many bytes is one chunk
 constexpr int kDsMaxRank = 512;                      // longest rank-space vector
 constexpr int kDsMaxSlice = 32;                      // channels of the residual stream per CTA
 constexpr int kDsP = 30;                             // fixed-point bits of the activation digits
@@ -302,6 +308,7 @@ struct DsRows {
     int fmt;           // 0 fp16, 1 int8 with a (scale, zero) per row, 2 per group of 128
     int out, out_off;
     int full_bytes, last_bytes;  // bytes of a chunk of 16 rows, and of one of the last tile
+    int merged;                  // the last tile's pieces, few rows, come as one chunk: the producer takes about 0.2 us per chunk
 };
 
 // ---- shared-memory layout: [ring][operand area: vec_floats x 4 bytes][DsShared] ----------------
@@ -427,24 +434,26 @@ __device__ __forceinline__ void ds_tile_f16(float (&c)[4], uint32_t lo, uint32_t
 
 // Tiles [tile0, tile1) of one matrix: this warp's sixteenth of K of every tile, partial sums to `part_s` ([row from tile0][warp]).
 // J = the launch's index of the first chunk of tile0; a tile has np chunks, of which the warp reads one, shared with 16 / np - 1
-// neighbours.  Lanes of rows that a tile does not have read another row's data; their sums are never looked at.  Returns false after a
+// neighbours (a last tile of few rows is one chunk).  Lanes of rows that a tile does not have read another row's data; their sums are never looked at.  Returns false after a
 // timeout.
 __device__ __forceinline__ bool ds_multiply(DsShared* S, const DsRows* E, uint32_t ring_s, uint32_t vec_s, uint32_t part_s, uint32_t J, int tile0, int tile1, int w, int lane) {
     const int g = lane >> 2, t = lane & 3;
     const int np = E->np, steps = E->steps, spp = E->spp, w0 = (w * steps) >> 4, piece = (w * np) >> 4, s0 = w0 - piece * spp, ns = (((w + 1) * steps) >> 4) - w0;
-    const int fmt = E->fmt, n = E->n;
+    const int fmt = E->fmt, n = E->n, merged = E->merged ? E->tiles - 1 : -1;
     const uint32_t bb = vec_s + (uint32_t)w0 * (fmt ? 128u : 64u) + (uint32_t)(g & (fmt ? 3 : 1)) * 32u + (uint32_t)t * 8u;
     uint32_t j = J + (uint32_t)piece;
     uint32_t dst = part_s + (fmt == 1 ? (uint32_t)(g * kDsPartInt + w * 16 + t * 8) : (uint32_t)(g * kDsPartF32 + w * 4));
 #pragma unroll 1
     for (int tile = tile0; tile < tile1; ++tile, j += (uint32_t)np) {
+        const bool one = tile == merged;
+        if (one) j -= (uint32_t)piece;
         const int slot = (int)(j % kDsBars);
         const bool got = mbar_wait(&S->full[slot], (j / kDsBars) & 1u, (volatile int*)&S->abort_flag);
         if (!__all_sync(0xffffffffu, got)) {
             if (lane == 0) atomicCAS(&S->abort_where, 0, 1 | (int)((j & 0xFFFF) << 4));
             return false;
         }
-        const uint32_t base = ring_s + (uint32_t)S->ring_off[slot];
+        const uint32_t base = ring_s + (uint32_t)S->ring_off[slot] + (one ? (uint32_t)(piece * E->last_bytes) : 0u);
         const int nr = min(kDsTileRows, n - tile * kDsTileRows), nlo = min(8, nr), nhi = nr > 8 ? nr - 8 : nlo;
         const uint32_t lstep = (uint32_t)nlo * 32u, hstep = (uint32_t)nhi * 32u;
         uint32_t lo = base + (uint32_t)(s0 * nlo + min(g, nlo - 1)) * 32u + (uint32_t)t * 8u;
@@ -514,7 +523,7 @@ __device__ __forceinline__ bool ds_multiply(DsShared* S, const DsRows* E, uint32
             dst += kDsTileRows * kDsPartF32;
         }
         __syncwarp();
-        if (lane == 0) ds_arrive(&S->empty[slot], (uint32_t)np);  // 16 / np warps share the chunk; the barrier counts 16
+        if (lane == 0) ds_arrive(&S->empty[slot], one ? 1u : (uint32_t)np);  // 16 / np warps share the chunk; the barrier counts 16
     }
     return true;
 }
@@ -602,86 +611,91 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_stream_kernel(const __gr
         r.out_off = E.out_off;
         r.full_bytes = ds_chunk_bytes(E, kDsTileRows);
         r.last_bytes = ds_chunk_bytes(E, r.n - (r.tiles - 1) * kDsTileRows);
+        r.merged = r.np * r.last_bytes <= kDsMergeBytes;
         S->rows[e] = r;
         if (r.n > 0 && e <= DSE_V1) S->rank_entry = e;
         if (r.n > 0 && e >= DSE_WR && e <= DSE_WV) S->big_entry = e;
     }
     __syncthreads();
 
-    if (warp == 0) {
-        // =========================== producer ===========================
-        const uint64_t pol = l2_evict_first_policy();
-        const int R = P.ring_bytes;
-        int head = 0, used = 0;
-        uint32_t j = 0, tail = 0;
-        bool ok = true;
-        const int rank_e = S->rank_entry, big_e = S->big_entry;
-        // The weights lie in the stream in the order they are consumed: every chunk is one bulk copy from a running pointer.
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kDsProducerRegs));
+        if (warp == 0) {
+            // =========================== producer ===========================
+            const uint64_t pol = l2_evict_first_policy();
+            const int R = P.ring_bytes;
+            int head = 0, used = 0;
+            uint32_t j = 0, tail = 0;
+            bool ok = true;
+            const int rank_e = S->rank_entry, big_e = S->big_entry;
+            // The weights lie in the stream in the order they are consumed: every chunk is one bulk copy from a running pointer.
 #pragma unroll 1
-        for (int t = 0; t < P.n_tokens && ok; ++t) {
-            const bool do_head = P.argmax_feed || t == P.n_tokens - 1;
+            for (int t = 0; t < P.n_tokens && ok; ++t) {
+                const bool do_head = P.argmax_feed || t == P.n_tokens - 1;
 #pragma unroll 1
-            for (int l = 0; l < L + (do_head ? 1 : 0) && ok; ++l) {
-                const char* src = l < L ? P.wstream + ((size_t)l * G + cta) * (size_t)P.wslot : P.hstream + (size_t)cta * (size_t)P.hslot;
-                const bool has_head = l < L && ds_head_of_cta(cta, l, P.H, G) >= 0;
-                // a layer: rank rows, r / k / v rows, a head's three chunks (w2 + a2 | v2 (layers > 0) + half of g2 | the other half), att.output, ffn.key, ffn.value
+                for (int l = 0; l < L + (do_head ? 1 : 0) && ok; ++l) {
+                    const char* src = l < L ? P.wstream + ((size_t)l * G + cta) * (size_t)P.wslot : P.hstream + (size_t)cta * (size_t)P.hslot;
+                    const bool has_head = l < L && ds_head_of_cta(cta, l, P.H, G) >= 0;
+                    // a layer: rank rows, r / k / v rows, a head's three chunks (w2 + a2 | v2 (layers > 0) + half of g2 | the other half), att.output, ffn.key, ffn.value
 #pragma unroll 1
-                for (int item = 0; item < 8 && ok; ++item) {
-                    int nfull, nlast = 0, fb, lb = 0;
-                    if (item >= 2 && item <= 4) {
-                        nfull = has_head ? 1 : 0;
-                        fb = item == 2 ? 128 * (wmp + amp) : 64 * gmp + (item == 3 && l > 0 ? 128 * vmp : 0);
-                    } else {
-                        int e = l == L ? (item == 0 ? DSE_COUNT : -1) : item == 0 ? rank_e : item == 1 ? big_e : item - 5 + DSE_WO;
-                        if (e == DSE_V1 && l == 0) e = -1;
-                        if (e < 0) continue;
-                        const DsRows& E = S->rows[e];
-                        nlast = E.tiles > 0 ? E.np : 0;
-                        nfull = max(E.tiles - 1, 0) * E.np;
-                        fb = E.full_bytes;
-                        lb = E.last_bytes;
-                    }
-                    if (l == L && item > 0) break;
+                    for (int item = 0; item < 8 && ok; ++item) {
+                        int nfull, nlast = 0, fb, lb = 0;
+                        if (item >= 2 && item <= 4) {
+                            nfull = has_head ? 1 : 0;
+                            fb = item == 2 ? 128 * (wmp + amp) : 64 * gmp + (item == 3 && l > 0 ? 128 * vmp : 0);
+                        } else {
+                            int e = l == L ? (item == 0 ? DSE_COUNT : -1) : item == 0 ? rank_e : item == 1 ? big_e : item - 5 + DSE_WO;
+                            if (e == DSE_V1 && l == 0) e = -1;
+                            if (e < 0) continue;
+                            const DsRows& E = S->rows[e];
+                            nlast = E.tiles > 0 ? (E.merged ? 1 : E.np) : 0;
+                            nfull = max(E.tiles - 1, 0) * E.np;
+                            fb = E.full_bytes;
+                            lb = E.merged ? E.np * E.last_bytes : E.last_bytes;
+                        }
+                        if (l == L && item > 0) break;
 #pragma unroll 1
-                    for (int q = 0; q < nfull + nlast; ++q) {
-                        const int bytes = q < nfull ? fb : lb;
-                        // room in the ring (waiting for the oldest chunks to be released); a chunk that does not fit behind the last one goes to the start
-                        const bool wrap = head + bytes > R;
-                        const int waste = wrap ? R - head : 0;
-                        while (used + waste + bytes > R || j - tail >= (uint32_t)kDsBars) {
-                            const bool w = mbar_wait(&S->empty[tail % kDsBars], (tail / kDsBars) & 1u, abort_flag);
-                            if (!__all_sync(0xffffffffu, w)) {
-                                if (lane == 0) atomicCAS(&S->abort_where, 0, 2 | (int)((j & 0xFFFF) << 4));
-                                ok = false;
-                                break;
+                        for (int q = 0; q < nfull + nlast; ++q) {
+                            const int bytes = q < nfull ? fb : lb;
+                            // room in the ring (waiting for the oldest chunks to be released); a chunk that does not fit behind the last one goes to the start
+                            const bool wrap = head + bytes > R;
+                            const int waste = wrap ? R - head : 0;
+                            while (used + waste + bytes > R || j - tail >= (uint32_t)kDsBars) {
+                                const bool w = mbar_wait(&S->empty[tail % kDsBars], (tail / kDsBars) & 1u, abort_flag);
+                                if (!__all_sync(0xffffffffu, w)) {
+                                    if (lane == 0) atomicCAS(&S->abort_where, 0, 2 | (int)((j & 0xFFFF) << 4));
+                                    ok = false;
+                                    break;
+                                }
+                                used -= S->alloc[tail % kDsBars];
+                                ++tail;
                             }
-                            used -= S->alloc[tail % kDsBars];
-                            ++tail;
+                            if (!ok) break;
+                            if (wrap) head = 0;
+                            const int slot = (int)(j % kDsBars);
+                            if (lane == 0) {
+                                S->alloc[slot] = waste + bytes;
+                                S->ring_off[slot] = head;
+                                mbar_expect_tx(&S->full[slot], (uint32_t)bytes);  // a release: the offset is visible to whoever sees the barrier complete
+                                ds_bulk_load(ring_s + (uint32_t)head, src, (uint32_t)bytes, &S->full[slot], pol);
+                            }
+                            __syncwarp();
+                            used += waste + bytes;
+                            head += bytes;
+                            src += bytes;
+                            ++j;
                         }
-                        if (!ok) break;
-                        if (wrap) head = 0;
-                        const int slot = (int)(j % kDsBars);
-                        if (lane == 0) {
-                            S->alloc[slot] = waste + bytes;
-                            S->ring_off[slot] = head;
-                            mbar_expect_tx(&S->full[slot], (uint32_t)bytes);  // a release: the offset is visible to whoever sees the barrier complete
-                            ds_bulk_load(ring_s + (uint32_t)head, src, (uint32_t)bytes, &S->full[slot], pol);
-                        }
-                        __syncwarp();
-                        used += waste + bytes;
-                        head += bytes;
-                        src += bytes;
-                        ++j;
                     }
                 }
             }
+            // copies still in flight must land before the CTA may exit (only after an abort: otherwise every chunk was consumed)
+            if (!ok)
+                for (; tail < j; ++tail) ds_mbar_drain(&S->full[tail % kDsBars], (tail / kDsBars) & 1u);
         }
-        // copies still in flight must land before the CTA may exit (only after an abort: otherwise every chunk was consumed)
-        if (!ok)
-            for (; tail < j; ++tail) ds_mbar_drain(&S->full[tail % kDsBars], (tail / kDsBars) & 1u);
     } else {
         // =========================== consumers ===========================
-        const int wtid = threadIdx.x - 32, w = wtid >> 5;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDsConsumerRegs));
+        const int wtid = threadIdx.x - 128, w = wtid >> 5;
         uint32_t J = 0;  // chunks of this CTA consumed so far (the producer numbers them the same way)
         unsigned bar_target = 0;
         bool ok = true;
@@ -921,7 +935,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_stream_kernel(const __gr
                         const DsRows* E = which ? A : B;
                         const int e0 = which ? tile0 : 0, e1 = which ? tile1 : E->tiles;
                         ok = ok && ds_multiply(S, E, ring_s, which ? vec_s : vec_s + 4u * (uint32_t)C, which ? part_s : part_s + kDsPartBytes, J, e0, e1, w, lane);
-                        J += (uint32_t)((e1 - e0) * E->np);
+                        J += (uint32_t)((e1 - e0) * E->np - (e1 == E->tiles && E->merged ? E->np - 1 : 0));
                     }
                     if (!(ok = !ds_consumer_sync_or(!ok))) break;
                     // four lanes per row add its sixteen sums (rank rows follow the others)

@@ -1136,6 +1136,10 @@ void launch_stream(const DsParams& P, int grid, size_t smem, cudaStream_t stream
     if (configure_only) {
         RSV_CUDA(cudaFuncSetAttribute(decode_stream_kernel<CMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
+        // the consumers' larger register share (setmaxnreg) exists only if the block was launched with this much
+        cudaFuncAttributes fa;
+        RSV_CUDA(cudaFuncGetAttributes(&fa, decode_stream_kernel<CMAX>));
+        if (fa.numRegs < kDsLaunchRegs) throw std::runtime_error("weight-streaming decode kernel: built with too few registers");
         RSV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_stream_kernel<CMAX>, kDsThreads, smem));
         if (per_sm < 1) throw std::runtime_error("weight-streaming decode kernel does not fit on an SM");
         return;

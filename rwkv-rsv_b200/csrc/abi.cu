@@ -637,15 +637,24 @@ static void prefill_batch(Model& m, State& st, const uint32_t* flat, const uint3
         RSV_CUDA(cudaMalloc(&acc, (size_t)batch * C * 4));
         RSV_CUDA(cudaMemsetAsync(acc, 0, (size_t)batch * C * 4, m.stream));
     }
-    // pack chunks of several sessions into steps of at most kMaxChunk rows
-    std::vector<uint32_t> toks;
+    // Steps of at most kMaxChunk rows, shared between the sessions in proportion to what they have left.  The state update is sequential
+    // in a session's tokens, so a step takes as long as its longest chunk: filled session after session, a step of 512 rows had one or
+    // two long chains (120 us per layer for it; 20 prompts of 16 to 512 tokens).  A session that takes part gets 16 tokens at least, so that
+    // its state is not read and written for less.
+    std::vector<std::vector<uint32_t>> step_toks;  // kept until the copies are done
+    int64_t left = 0;
+    for (int64_t b = 0; b < batch; ++b) left += len[b] - done[b];
     for (;;) {
         StepPlan p;
-        toks.clear();
-        for (int64_t b = 0; b < batch && (int)p.rows.size() < kMaxChunk; ++b) {
+        std::vector<uint32_t>& toks = step_toks.emplace_back();
+        int64_t room = std::min<int64_t>(left, kMaxChunk), others = left;
+        for (int64_t b = 0; b < batch && room > 0; ++b) {
             const int64_t rem = len[b] - done[b];
             if (rem <= 0) continue;
-            const int T = (int)std::min<int64_t>(rem, kMaxChunk - (int64_t)p.rows.size());
+            const int T = (int)std::min({rem, room, std::max<int64_t>((rem * room + others - 1) / others, 16)});  // (room <= others throughout: the step is filled)
+            others -= rem;
+            room -= T;
+            left -= T;
             const int start = (int)p.rows.size(), seg = (int)p.segs.size();
             for (int r = 0; r < T; ++r) {
                 p.rows.push_back(RowMeta{(int)b, r > 0 ? 1 : 0, r == T - 1 ? 1 : 0, seg});
@@ -660,7 +669,6 @@ static void prefill_batch(Model& m, State& st, const uint32_t* flat, const uint3
         RSV_CUDA(cudaMemcpyAsync(m.ws.tokens, toks.data(), toks.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, m.stream));
         m.forward_rows(st, p, false);
         if (mean_out) engine_segment_sums(m, (int)p.segs.size(), acc);
-        RSV_CUDA(cudaStreamSynchronize(m.stream));  // `toks` is reused by the next step
     }
     m.check_status();
     if (mean_out) {

@@ -268,16 +268,26 @@ int rsv_sched_step(rsv_sched* Sp, int64_t* rows_out, int64_t* active_out) {
             Request& r = S.reqs.at(S.slot_owner[s]);
             if (r.fed == (int64_t)r.prompt.size() && r.generated < r.max_new) add_segment(r, 1, nullptr, true);
         }
-        for (int s = 0; s < S.max_slots && (int)p.rows.size() < S.max_rows; ++s) {
-            if (!S.slot_owner[s]) continue;
-            Request& r = S.reqs.at(S.slot_owner[s]);
-            const int64_t rem = (int64_t)r.prompt.size() - r.fed;
-            if (rem <= 0) continue;
-            const int T = (int)std::min<int64_t>({rem, (int64_t)S.chunk, (int64_t)S.max_rows - (int64_t)p.rows.size()});
-            if (T <= 0) break;
-            add_segment(r, T, r.prompt.data() + r.fed, r.fed + T == (int64_t)r.prompt.size());
-            r.fed += T;
-        }
+        // The state update is sequential in a session's tokens, so a step takes as long as its longest chunk: the sessions get kShare rows each,
+        // in turn, then what is left over goes to those that can use it.
+        constexpr int64_t kShare = 128;
+        std::vector<int> take((size_t)S.max_slots, 0);
+        int64_t room = (int64_t)S.max_rows - (int64_t)p.rows.size();
+        for (int64_t most : {std::min<int64_t>(kShare, S.chunk), (int64_t)S.chunk})
+            for (int s = 0; s < S.max_slots && room > 0; ++s) {
+                if (!S.slot_owner[s]) continue;
+                const Request& r = S.reqs.at(S.slot_owner[s]);
+                const int T = (int)std::min({(int64_t)r.prompt.size() - r.fed, most, room + take[s]});
+                if (T <= take[s]) continue;
+                room -= T - take[s];
+                take[s] = T;
+            }
+        for (int s = 0; s < S.max_slots; ++s)
+            if (take[s] > 0) {
+                Request& r = S.reqs.at(S.slot_owner[s]);
+                add_segment(r, take[s], r.prompt.data() + r.fed, r.fed + take[s] == (int64_t)r.prompt.size());
+                r.fed += take[s];
+            }
         const int R = (int)p.rows.size(), O = (int)p.out_rows.size();
         if (rows_out) *rows_out = R;
         if (R > 0) {

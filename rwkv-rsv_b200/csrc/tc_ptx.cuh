@@ -87,10 +87,6 @@ __device__ __forceinline__ uint64_t l2_evict_normal_policy() {
     asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-// Release / acquire fence at device scope (lighter than the sequentially consistent fence of __threadfence()).  Used as
-// "stores; __syncwarp(); lane 0: fence, atomic" on the producing side and "lane 0: atomic, fence; __syncwarp(); loads that
-// bypass L1" on the consuming side.
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
 }
@@ -100,27 +96,8 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-template <bool I8>
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    if constexpr (I8) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    }
-}
-// The same two instructions for a warp that runs its issue loop convergently: every lane computes the (identical) operands,
-// one elected lane issues.  Measured on this part with 64 back-to-back 128 x 16 x 32-byte MMAs: 38 cycles per MMA this way,
+// tcgen05.mma (u8 x s8 -> s32 or f16 x f16 -> f32) for a warp that runs its issue loop convergently: every lane computes the (identical)
+// operands, one elected lane issues.  Measured on this part with 64 back-to-back 128 x 16 x 32-byte MMAs: 38 cycles per MMA this way,
 // 56 from a single active lane with straight-line code, about 150 from a single lane inside a loop with integer divisions -
 // with one lane active the compiler cannot keep descriptors in uniform registers.
 template <bool I8>

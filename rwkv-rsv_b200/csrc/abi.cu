@@ -101,6 +101,10 @@ void decode_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n) {
     RSV_CUDA(cudaSetDevice(m.device));
     if (!m.prof_on && m.stream_available()) {
         m.ensure_workspace(1, 1, 1);
+        if (n == 1) {
+            m.run_stream(st, 0, 1, true, false, nullptr, nullptr, 0, tokens);
+            return;
+        }
         ensure_tok_list(m, (size_t)n);
         RSV_CUDA(cudaMemcpyAsync(m.ws.tok_list, tokens, (size_t)n * sizeof(uint32_t), cudaMemcpyHostToDevice, m.stream));
         m.run_stream(st, 0, (int)n, true, false, nullptr, nullptr, 0);  // all n tokens in one launch, head on the last
@@ -116,8 +120,6 @@ void decode_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n) {
 
 constexpr int kMaxChunk = 512;  // rows per packed step on the chunk path
 
-// chunked prefill of one session; out_mode 1: logits of the very last token in ws.logits[0,:];
-// out_mode 2: every position, copied to `all_out` chunk by chunk
 // Logits of a whole chunk to the caller's memory.  A copy to pageable memory runs at what one thread of the driver moves (201 x 65536
 // logits: 53 MB, 8 ms with the first touch of the pages); here the chunk goes to pinned memory in kOutParts pieces behind its forward
 // pass, and a few threads move each piece on as soon as it has arrived, while the GPU runs the next chunk.
@@ -176,6 +178,8 @@ class LogitsToHost {
     }
 };
 
+// chunked prefill of one session; out_mode 1: logits of the very last token in ws.logits[0,:];
+// out_mode 2: every position, copied to `all_out` chunk by chunk
 void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int64_t chunk, int out_mode, float* all_out) {
     need(st.model == &m, "state belongs to a different model");
     need(st.cap == 1, "this call needs a single-session state (batch == 1)");
@@ -197,9 +201,21 @@ void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int6
     if (out_mode == 2) out.finish();
 }
 
+// One row of logits and the status words, through pinned memory: two copies and one wait instead of two waits (a copy to pageable memory
+// is one).  A caller's pinned array is written directly.
 void fetch_logits(Model& m, float* logits_out) {
-    RSV_CUDA(cudaMemcpyAsync(logits_out, m.ws.logits, (size_t)m.cfg.vocab * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
-    m.check_status();  // synchronises
+    const size_t V = m.cfg.vocab;
+    cudaPointerAttributes at;
+    const bool direct = cudaPointerGetAttributes(&at, logits_out) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    if (!direct) cudaGetLastError();
+    m.ensure_pinned_out((V + 2) * sizeof(float));
+    RSV_CUDA(cudaMemcpyAsync(direct ? logits_out : m.pinned_out, m.ws.logits, V * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
+    RSV_CUDA(cudaMemcpyAsync(m.pinned_out + V, m.ws.status, 2 * sizeof(int), cudaMemcpyDeviceToHost, m.stream));
+    RSV_CUDA(cudaStreamSynchronize(m.stream));
+    int sw[2];
+    memcpy(sw, m.pinned_out + V, sizeof(sw));
+    m.judge_status(sw);
+    if (!direct) memcpy(logits_out, m.pinned_out, V * sizeof(float));
 }
 
 void pack_sampler_row(float* row, const rsv_sampler_params& sp, uint32_t seed, uint32_t hist_len) {

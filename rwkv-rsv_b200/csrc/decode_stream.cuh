@@ -135,7 +135,9 @@ struct DsParams {
     int* cand_idx;  // [G]
     unsigned* grid_bar;
     int* status;
-    int n_tokens, tok_from_list, argmax_feed;
+    int n_tokens, tok_from_list, argmax_feed;  // tok_from_list: 0 tokens[0], 1 tok_list, 2 tok0
+    uint32_t tok0;
+    unsigned bar_base;  // the grid barrier's counter when the launch begins (it only grows)
     const char* wstream;      // the layers' weights in consumption order: region (layer l, CTA c) at (l G + c) wslot
     long long wslot;
     const char* hstream;      // the head's rows in consumption order: region of CTA c at c hslot
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_stream_kernel(const __gr
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDsConsumerRegs));
         const int wtid = threadIdx.x - 128, w = wtid >> 5;
         uint32_t J = 0;  // chunks of this CTA consumed so far (the producer numbers them the same way)
-        unsigned bar_target = 0;
+        unsigned bar_target = P.bar_base;
         bool ok = true;
         const int r0o = S->rows[DSE_WO].r0, nown = S->rows[DSE_WO].n;  // this CTA's slice of the channels = its rows of att.output / ffn.value
         uint32_t lt = 0;  // layers run so far: the table of the current layer sits in S->layer[lt & 1]
@@ -742,7 +744,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_stream_kernel(const __gr
         for (int t = 0; t < P.n_tokens && ok; ++t) {
             const bool do_head = P.argmax_feed || t == P.n_tokens - 1;
             if (wtid == 0) {
-                uint32_t tk = (P.argmax_feed && t > 0) ? S->tok : (P.tok_from_list ? P.tok_list[t] : P.tokens[0]);
+                uint32_t tk = (P.argmax_feed && t > 0) ? S->tok : (P.tok_from_list == 2 ? P.tok0 : P.tok_from_list ? P.tok_list[t] : P.tokens[0]);
                 if (tk >= (uint32_t)P.V) {
                     atomicOr(P.status, 1);
                     tk = 0;

@@ -437,6 +437,7 @@ static void free_workspace(Workspace& w) {
 Model::~Model() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
+    state_pool->release(true);
     free_workspace(ws);
     if (ws.status) cudaFree(ws.status);
     if (ws.tok_pos) cudaFree(ws.tok_pos);
@@ -459,11 +460,37 @@ Model::~Model() {
     if (stream) cudaStreamDestroy(stream);
 }
 
-State::~State() {
-    if (model) {
-        cudaSetDevice(model->device);
+float* StatePool::take(size_t bytes) {
+    std::lock_guard<std::mutex> lock(mu);
+    for (size_t i = 0; i < kept.size(); ++i)
+        if (kept[i].first == bytes) {
+            float* p = kept[i].second;
+            kept.erase(kept.begin() + (long)i);
+            return p;
+        }
+    return nullptr;
+}
+void StatePool::give(size_t bytes, float* p) {
+    std::lock_guard<std::mutex> lock(mu);
+    if (open && bytes <= kMostBytes) {
+        kept.emplace_back(bytes, p);
+        if (kept.size() <= kMost) return;
+        p = kept.front().second;
+        kept.erase(kept.begin());
     }
-    if (wkv) cudaFree(wkv);
+    cudaFree(p);
+}
+void StatePool::release(bool close) {
+    std::lock_guard<std::mutex> lock(mu);
+    for (auto& k : kept) cudaFree(k.second);
+    kept.clear();
+    if (close) open = false;
+}
+
+State::~State() {
+    if (!wkv) return;
+    cudaSetDevice(pool->device);
+    pool->give(bytes, wkv);
 }
 
 void State::allocate(Model* m, int64_t slots) {
@@ -473,7 +500,15 @@ void State::allocate(Model* m, int64_t slots) {
     auto aligned = [](size_t floats) { return (floats + 63) / 64 * 64; };
     const size_t nx = aligned((size_t)c.n_layer * cap * c.n_embd), ns = aligned((size_t)c.n_layer * cap * c.n_head * kHeadSize * kHeadSize);
     bytes = (ns + 2 * nx + (size_t)cap * c.n_embd) * 4;
-    RSV_CUDA(cudaMalloc(&wkv, bytes));
+    pool = m->state_pool;
+    pool->device = m->device;
+    wkv = pool->take(bytes);
+    if (!wkv && cudaMalloc(&wkv, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        wkv = nullptr;
+        pool->release(false);
+        RSV_CUDA(cudaMalloc(&wkv, bytes));
+    }
     tmix_x = wkv + ns;
     cmix_x = tmix_x + nx;
     v_first = cmix_x + nx;
@@ -1283,6 +1318,7 @@ bool Model::stream_available() {
     RSV_CUDA(cudaMalloc(&sc.cand_val, (size_t)G * 4));
     RSV_CUDA(cudaMalloc(&sc.cand_idx, (size_t)G * 4));
     RSV_CUDA(cudaMalloc(&sc.grid_bar, 4));
+    RSV_CUDA(cudaMemsetAsync(sc.grid_bar, 0, 4, stream));
     P.layers = (const DsLayer*)sc.d_layers;
     P.head = ds_head_entry(shp, G);
     bind(P.head, head, nullptr);
@@ -1322,7 +1358,8 @@ bool Model::stream_available() {
     return true;
 }
 
-void Model::run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bool argmax_feed, uint32_t* seq_dev, int* seq_cnt_dev, int seq_cap) {
+void Model::run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bool argmax_feed, uint32_t* seq_dev, int* seq_cnt_dev, int seq_cap,
+                       const uint32_t* host_token) {
     if (!stream_available()) throw std::runtime_error("weight-streaming decode path unavailable: " + sctx.why);
     StreamCtx& sc = sctx;
     RSV_CUDA(cudaSetDevice(device));
@@ -1345,11 +1382,13 @@ void Model::run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bo
     P.logits = ws.logits;
     P.status = ws.status;
     P.n_tokens = n_tokens;
-    P.tok_from_list = tok_from_list ? 1 : 0;
+    P.tok_from_list = host_token ? 2 : tok_from_list ? 1 : 0;
+    P.tok0 = host_token ? *host_token : 0u;
     P.argmax_feed = argmax_feed ? 1 : 0;
     P.epoch = sc.epoch;
     sc.epoch += (uint32_t)n_tokens * (uint32_t)cfg.n_layer;
-    RSV_CUDA(cudaMemsetAsync(sc.grid_bar, 0, 4, stream));
+    P.bar_base = sc.bar_base;
+    sc.bar_base += (unsigned)sc.grid * (unsigned)(argmax_feed ? n_tokens : n_tokens - 1);
     LAUNCH(*this, "decode_stream") { dispatch_stream(sc.kl, P, sc.grid, sc.smem, stream, false); }
 }
 
@@ -1357,12 +1396,18 @@ void Model::check_status() {
     int sw[2] = {0, 0};  // status bits; where the weight-streaming decode kernel gave up
     RSV_CUDA(cudaMemcpyAsync(sw, ws.status, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream));
     RSV_CUDA(cudaStreamSynchronize(stream));
+    judge_status(sw);
+}
+
+void Model::judge_status(const int* sw) {
     const int s = sw[0];
     if (s) {
         RSV_CUDA(cudaMemsetAsync(ws.status, 0, 2 * sizeof(int), stream));
         if ((s & 32) && sctx.exchange) {  // a launch that gave up left some of its exchanged values unwritten
             RSV_CUDA(cudaMemsetAsync(sctx.exchange, 0, sctx.exchange_bytes, stream));
             sctx.epoch = 1;
+            RSV_CUDA(cudaMemsetAsync(sctx.grid_bar, 0, 4, stream));
+            sctx.bar_base = 0;
         }
         if (s & 32) {
             static const char* const site[5] = {"a wait", "a chunk of weight rows", "room in the ring", "a grid barrier", "a chunk of a head's rows"};

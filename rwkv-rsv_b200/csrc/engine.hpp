@@ -5,6 +5,7 @@
 #pragma once
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -79,6 +80,7 @@ struct StreamCtx {
     unsigned long long* exchange = nullptr;  // values the CTAs exchange (see decode_stream.cuh): xa, xb, yg, vfirst [C], rkv [3C], mid, then hbuf [F] words
     size_t exchange_bytes = 0;
     uint32_t epoch = 1;                      // tag of the next launch's first layer
+    unsigned bar_base = 0;      // value of the grid barrier's counter when the next launch begins
     float* cand_val = nullptr;
     int* cand_idx = nullptr;
     unsigned* grid_bar = nullptr;
@@ -94,6 +96,20 @@ struct KernelProf {
 
 struct Model;
 
+// Allocations of states that are gone, for the next ones of the same model (mapping device memory costs up to 4 ms): the last kMost of
+// at most kMostBytes each.  Shared by the model, which empties and closes it when it goes, and its states, which may outlive it.  All work
+// on a state goes through the model's stream, so the next user's clearing is ordered behind it.
+struct StatePool {
+    static constexpr size_t kMost = 2, kMostBytes = 512u << 20;
+    std::mutex mu;
+    std::vector<std::pair<size_t, float*>> kept;  // newest last
+    bool open = true;
+    int device = 0;
+    float* take(size_t bytes);
+    void give(size_t bytes, float* p);
+    void release(bool close);
+};
+
 // Session state: per layer tmix_x[cap,C], wkv[cap,H,N,N], cmix_x[cap,C], plus v_first[cap,C]
 // (src/gpu_model.rs:194-199, 3915-3963).  fp32 on the device, so back/load round-trips bit-exactly.
 struct State {
@@ -101,6 +117,7 @@ struct State {
     int64_t cap = 0;
     float *tmix_x = nullptr, *wkv = nullptr, *cmix_x = nullptr, *v_first = nullptr;  // parts of one allocation (a device allocation costs 0.1 ms and more)
     size_t bytes = 0;
+    std::shared_ptr<StatePool> pool;
     CUtensorMap wkv_map;      // all layers' WKV states as one 2-D tensor [layers x slots x heads x 64][64] fp32 (TMA boxes of 64 rows x 32 columns)
     bool wkv_map_ok = false;  // encoded on first use
     void allocate(Model* m, int64_t slots);
@@ -134,6 +151,7 @@ struct Model {
     static constexpr int kPinRing = 4;
     void* pinned = nullptr;
     size_t pinned_bytes = 0;  // bytes per ring area
+    std::shared_ptr<StatePool> state_pool = std::make_shared<StatePool>();
     // pinned staging of a chunk's logits on their way to the caller (at most 128 rows), with an event per piece
     static constexpr int kOutParts = 32;
     float* pinned_out = nullptr;
@@ -153,7 +171,8 @@ struct Model {
     bool use_stream = true;  // one session: the row-owner weight-streaming kernel (RSV_NO_STREAM=1 sends it through the batched path)
     StreamCtx sctx;
     bool stream_available();
-    void run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bool argmax_feed, uint32_t* seq_dev, int* seq_cnt_dev, int seq_cap);
+    // host_token: the only token, known to the host (no copy)
+    void run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bool argmax_feed, uint32_t* seq_dev, int* seq_cnt_dev, int seq_cap, const uint32_t* host_token = nullptr);
     static std::unique_ptr<Model> create_bare(int device);  // stream + events only (operator-level entry points)
 
     static std::unique_ptr<Model> load(const std::string& path, int device);
@@ -164,6 +183,7 @@ struct Model {
     // Runs one packed step.  Input tokens are read from ws.tokens[r] (or ws.tok_list[*tok_pos * R + r] when
     // `use_cursor`).  With out_rows non-empty, logits land in ws.logits[o, V] in out_rows order.
     void forward_rows(State& st, const StepPlan& plan, bool use_cursor);
+    void judge_status(const int* sw);  // throws what the two status words say
     void check_status();
 };
 

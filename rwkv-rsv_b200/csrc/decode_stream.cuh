@@ -322,6 +322,9 @@ struct DsShared {
     int abort_flag;
     int abort_where;  // which wait gave up first (1 rows: full, 2 producer: empty, 3 grid barrier, 4 heads: full) | detail << 4
     uint32_t tok;
+    // Exchanged between the consumer warps, one array per use: 0, 1 row sums (LayerNorm; ||kk||^2 and bonus; arg-max), 2, 3 GroupNorm
+    // sums, 2, 5 operand maxima, 4 scales of a head's rank vectors.  An array may be written again only after a barrier that follows its
+    // last read; between a head's last sum (3) and the maxima of the next unit (2, 5) there is none.
     float red[6][16];
     int red_i[16];
     long long tsw[16];                       // per warp: exact sum of its fixed-point values
@@ -887,7 +890,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_stream_kernel(const __gr
                 am1 = warp_absmax(am1);
                 if (lane == 0) {
                     S->red[2][w] = am0;
-                    S->red[3][w] = am1;
+                    S->red[5][w] = am1;  // (not [3]: a head's last sum before this unit may still be being read there)
                 }
                 if (!(ok = !ds_consumer_sync_or(!ok))) break;
                 // the shift state this CTA owns: this phase's input is complete, so everybody has read the old one
@@ -895,7 +898,7 @@ __global__ void __launch_bounds__(kDsThreads, 1) decode_stream_kernel(const __gr
                     if (ph == 1) (P.tmix_x + lx)[r0o + wtid] = S->ts_own[wtid];
                     if (ph == 3) (P.cmix_x + lx)[r0o + wtid] = S->cs_own[wtid];
                 }
-                const int ex0 = ds_exponent(warp_absmax(S->red[2][lane & 15])), ex1 = ds_exponent(warp_absmax(S->red[3][lane & 15]));
+                const int ex0 = ds_exponent(warp_absmax(S->red[2][lane & 15])), ex1 = ds_exponent(warp_absmax(S->red[5][lane & 15]));
                 {
                     long long ts = 0;
 #pragma unroll 1

@@ -782,6 +782,24 @@ void rl_launch(Model& m, const char* name, const RlLaunch& L, int ctas, size_t s
 
 void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const RowTiles& t) {
     if (n < 1 || n > kRlMaxProb) throw std::runtime_error("rows_linear: too many problems in one launch");
+    {
+        // The kernel is compiled for one kind of int8 weights.  Matrices with a (scale, zero) per row next to others with one per group
+        // (a per-group file in which some rows happen to be uniform) go out in a launch of their own.
+        RlReq per_row[kRlMaxProb], rest[kRlMaxProb];
+        int nrow = 0, nrest = 0;
+        bool mixed = false;
+        for (int i = 0; i < n; ++i) {
+            if (rl_fmt(*reqs[i].W) == RL_I8)
+                per_row[nrow++] = reqs[i];
+            else
+                rest[nrest++] = reqs[i];
+            mixed = mixed || rl_fmt(*reqs[i].W) == RL_I8G;
+        }
+        if (mixed && nrow) {
+            run_rows_linear(m, name, per_row, nrow, t);
+            return run_rows_linear(m, name, rest, nrest, t);
+        }
+    }
     RlLaunch L;
     memset(&L, 0, sizeof(L));
     const bool build = reqs[0].op == nullptr;
@@ -823,7 +841,6 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
         kb_max = std::max(kb_max, P.kblocks);
         nt_max = std::max(nt_max, t.nt(P.fmt));
     }
-    if (grouped && row8) throw std::runtime_error("rows_linear: per-row and per-group int8 weights in one launch");
     if (grouped && t.rt > kRlMaxRowsG) throw std::runtime_error("rows_linear: row tile too large for per-group weights");
     L.nprob = n;
     L.R = t.R;
@@ -918,7 +935,6 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     const int C = cfg.n_embd, H = cfg.n_head, F = cfg.ffn_hidden, V = cfg.vocab, MIDS = cfg.mids(), NL = cfg.n_layer;
     if (R == 0) return;
     RSV_CUDA(cudaSetDevice(device));
-    const LayerW& L0 = layers[0];
     bool per_group = false, int8 = false;
     for (const LayerW& L : layers)
         for (const LinearW* W : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv}) {
@@ -927,8 +943,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         }
     // tw: the layer's launches with many weight tiles; t: the others, which would have too few tiles for the GPU with 128 rows each
     const RowTiles t = row_tiles(R, per_group, true), tw = row_tiles(R, per_group, int8), to = row_tiles(std::max(O, 1), rl_fmt(head) == RL_I8G, rl_fmt(head) == RL_I8);
-    // Operands of a layer; the matrices of one kind have the same format in every layer of the files the loader accepts, and where
-    // they do not, the operand is carved again.
+    // Operands of a layer, carved again for every layer (a matrix's format is its own); the head's follow the largest layer's.
     OperandCarver cv;
     struct LayerOps {
         RlOperandOut r, w, k, v, a, g, vr, mid[4], y, x2, h;
@@ -949,8 +964,12 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         o.h = cv.operand(t, rl_fmt(L.Wfv), F, nullptr, known_parts(F));
     };
     LayerOps ops;
-    carve_layer(L0, ops);
-    const size_t layer_bytes = cv.used;
+    size_t layer_bytes = 0;
+    for (const LayerW& L : layers) {
+        carve_layer(L, ops);
+        layer_bytes = std::max(layer_bytes, cv.used);
+    }
+    cv.used = layer_bytes;
     RlOperandOut head_op = cv.operand(to, rl_fmt(head), C);
     ensure_operand_memory(*this, cv.used);
     cv.base = ws.op_mem;
@@ -992,7 +1011,6 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     for (int l = 0; l < NL; ++l) {
         const LayerW& L = layers[l];
         carve_layer(L, ops);
-        if (cv.used > layer_bytes) throw std::runtime_error("layers of one model differ in their weight formats");
         float* tmix_x = st.tmix_x + l * lay_x;
         float* cmix_x = st.cmix_x + l * lay_x;
         float* wkv = st.wkv + l * lay_s;

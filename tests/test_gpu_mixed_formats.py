@@ -1,0 +1,71 @@
+"""Checkpoints whose matrices do not all have one format: the format is the tensor's, so any mix of fp16, int8 with one (scale, zero) per
+row and int8 with one per row and group loads and runs at every step size."""
+import os
+
+import numpy as np
+import pytest
+
+import orc
+import rwkv_rsv_b200 as rsv
+from checkpoint_files import read_safetensors, write_safetensors
+
+pytestmark = pytest.mark.gpu
+
+BIG = ("att.receptance", "att.key", "att.value", "att.output", "ffn.key", "ffn.value")
+SHAPE = dict(n_layer=3, n_embd=512, n_head=8, ffn_hidden=2048, vocab=1000, w_mid=32, a_mid=32, v_mid=16, g_mid=64)
+
+
+def _sources(tmp_path, **shape):
+    return {name: read_safetensors(rsv.write_synthetic(os.path.join(str(tmp_path), name + ".st"), "tiny", seed=0, quant=q, **shape))
+            for name, q in (("fp16", 0), ("int8", 1), ("int8g", 2))}
+
+
+def _take(dst, src, prefix):
+    """The matrix `prefix` (+ ".weight") of `dst` in the format it has in `src`."""
+    for key in [k for k in dst if k.startswith(prefix + ".weight")]:
+        del dst[key]
+    for key in src:
+        if key.startswith(prefix + ".weight"):
+            dst[key] = src[key]
+
+
+def _check(path, sizes, vocab):
+    b, o = rsv.ModelBuilder(path).build(), orc.OracleModel(path)
+    rng = np.random.default_rng(3)
+    try:
+        for n in sizes:
+            toks = rng.integers(0, vocab, size=n).astype(np.uint32)
+            b.reset()
+            o.reset()
+            lg, want = b.infer_seq(toks), o.forward(toks)
+            # fp32 through the layers in another summation order: a few ulps of the logits' scale per layer
+            assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n
+            assert np.abs(b.state_back() - o.state_back()).max() <= 1e-4 * max(1.0, float(np.abs(o.state_back()).max()))
+    finally:
+        b.state.close()
+        b.model.close()
+
+
+# which format each of the three layers has
+@pytest.mark.parametrize("layers", [("fp16", "int8", "int8"), ("int8", "fp16", "int8"), ("int8g", "int8", "fp16"), ("fp16", "int8g", "int8")])
+def test_layers_of_different_formats(tmp_path, layers):
+    src = _sources(tmp_path, **SHAPE)
+    out = dict(src["fp16"])
+    for i, fmt in enumerate(layers):
+        for m in BIG:
+            _take(out, src[fmt], f"blocks.{i}.{m}")
+    _check(write_safetensors(os.path.join(str(tmp_path), "mixed.st"), out), (1, 2, 3, 16, 64, 65, 130), SHAPE["vocab"])
+
+
+# a per-group file in which some matrices have the same (scale, zero) in every group of a row, so that they are rows with one: alone, and
+# next to an fp16 matrix in the same launch
+@pytest.mark.parametrize("uniform,half", [(("att.receptance",), ()), (("att.key", "att.value", "ffn.key"), ("att.receptance",)), ((), ("att.value",))])
+def test_uniform_matrices_in_a_per_group_file(tmp_path, uniform, half):
+    src = _sources(tmp_path, **SHAPE)
+    out = dict(src["int8g"])
+    for i in range(SHAPE["n_layer"]):
+        for m in uniform:
+            _take(out, src["int8"], f"blocks.{i}.{m}")
+        for m in half:
+            _take(out, src["fp16"], f"blocks.{i}.{m}")
+    _check(write_safetensors(os.path.join(str(tmp_path), "uniform.st"), out), (2, 33, 64), SHAPE["vocab"])

@@ -293,7 +293,8 @@ __global__ void __launch_bounds__(kLnMaxThreads) ln_operands_kernel(const __grid
 
 // ---- operands of activations another kernel left in fp32 ----------------------------------------------------------------------
 // Rows whose producer left maxima of |x| over `parts` parts of the row (amax[R][parts]): elementwise, grid (rows, ceil(K / 2048)); every
-// CTA leaves the exact sum of its part of the row (tsum[R][gridDim.y]).
+// CTA leaves the exact sum of its part of the row (tsum[R][gridDim.y]).  Elements between K and the end of the last block are written as
+// zeros: the weights there are zero-filled by the tensor map, and 0 x NaN (what another step left in the image) would not be.
 constexpr int kOpThreads = 256;
 __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* x, int ldx, int K, const float* amax, int parts, int rt,
                                                                    const __grid_constant__ RlOperandOut O) {
@@ -304,6 +305,9 @@ __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* 
     pdl_wait();
     float v[8];
     rl_load8(v, x + (size_t)r * ldx + (k0 < K ? k0 : 0));
+    if (k0 >= K)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = 0.f;
     float am = 0.f;
 #pragma unroll 1
     for (int i = threadIdx.x; i < parts; i += kOpThreads) am = fmaxf(am, __ldcg(amax + (size_t)r * parts + i));
@@ -313,7 +317,7 @@ __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* 
     am = redm[lane & (kOpThreads / 32 - 1)];
     const int ex = rl_scale_exp(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)))), kel = rl_kelems(O.fmt);
     int ts = 0;
-    if (k0 < K) ts = rl_put8(O.fmt, rl_tile(O, rt, r, k0 / kel), (r % rt) * rl_cols(O.fmt), k0 % kel, v, rl_mult(O.fmt, ex));
+    if (k0 < O.kblocks * kel) ts = rl_put8(O.fmt, rl_tile(O, rt, r, k0 / kel), (r % rt) * rl_cols(O.fmt), k0 % kel, v, rl_mult(O.fmt, ex));
     if (O.fmt != RL_F16) {
         const long long t16 = rl_group_sum(ts);
         if (O.fmt == RL_I8G) {
@@ -334,8 +338,7 @@ __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* 
 }
 
 // Short rows (the rank-space vectors; any length works): one warp per (row, matrix) finds the maximum, then converts.  Elements
-// between K and the end of the last block are written as zeros: the weights there are zero-filled by the tensor map, and 0 x NaN
-// would not be.
+// between K and the end of the last block are written as zeros, as above.
 struct OperandRowsArgs {
     const float* x[4];
     int ldx[4], K[4];

@@ -69,3 +69,15 @@ def test_uniform_matrices_in_a_per_group_file(tmp_path, uniform, half):
         for m in half:
             _take(out, src["fp16"], f"blocks.{i}.{m}")
     _check(write_safetensors(os.path.join(str(tmp_path), "uniform.st"), out), (2, 33, 64), SHAPE["vocab"])
+
+
+def test_padding_of_the_last_k_block(tmp_path):
+    """fp16 ffn.value whose K ends inside a block of 64, next to int8 matrices: what another step's operands left behind the K end must not
+    reach the products."""
+    shape = dict(SHAPE, n_layer=2)
+    src = _sources(tmp_path, **shape)
+    out = read_safetensors(rsv.write_synthetic(os.path.join(str(tmp_path), "f200.st"), "tiny", seed=0, quant=0, **dict(shape, ffn_hidden=200)))
+    for i in range(2):
+        for m in ("att.receptance", "att.key", "att.value", "att.output"):
+            _take(out, src["int8"], f"blocks.{i}.{m}")
+    _check(write_safetensors(os.path.join(str(tmp_path), "mixed.st"), out), (64, 2, 3, 5, 17, 130, 2, 33), shape["vocab"])

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
 #pragma unroll
     for (int q = 0; q < kScPer; ++q) {
         x[q] *= invT;
+        if (x[q] < -3.0e38f) x[q] = -1e30f;  // masked tokens (-inf, the lowest float) count as -1e30, so that a row of nothing else is drawn from uniformly
         if (q < nv) mx = fmaxf(mx, x[q]);
     }
 #pragma unroll
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
     float e[kScPer];
 #pragma unroll
     for (int q = 0; q < kScPer; ++q) {
-        e[q] = q < nv && !(x[q] < thr) ? expf(x[q] - mx) : 0.f;
+        e[q] = q < nv ? expf((x[q] < thr ? -1e30f : x[q]) - mx) : 0.f;
         ps += e[q];
     }
     ps = sc_block_sum(ps, sh.red);

@@ -543,8 +543,8 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_rows_kernel(const float
 // Specification = the general path of rwkv_sample(_batch) (src/backend_cuda.rs:3741-3769, 3835-3908,
 // 3923-3957, 3980-4006): top-k keeps everything >= the K-th largest value; top-p picks probabilities
 // from the largest down (at most 512 picks) until the running sum reaches top_p and keeps everything
-// >= the last pick; the draw is u = u01(seed) * sum(kept) and the first index, in vocabulary order,
-// whose running sum exceeds u.  The reference's 1<=top_k<=50 fast path accumulates top-p and the
+// >= the last pick; the draw is u = u01(seed) * sum(kept) and the first kept index, in vocabulary order,
+// whose running sum exceeds u (the last kept one where none does: u01 rounds to 1 for 128 of 2^32 seeds).  The reference's 1<=top_k<=50 fast path accumulates top-p and the
 // draw from the smallest kept probability (:3913-3922, :3962-3978), against its documented intent;
 // that variant is not reproduced — every top_k takes the path above.
 // Here the K-th largest value comes from a 4-pass radix select instead of K arg-max sweeps, the 512
@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
     __shared__ float s_list[kTopPMaxPicks];
     __shared__ int s_count;
     __shared__ float s_cut;
-    __shared__ int s_chosen;
+    __shared__ int s_chosen, s_last;
     const int row = blockIdx.x, tid = threadIdx.x;
     const int ent = row_map ? row_map[row] : row;  // entry of the per-session arrays (sampler rows, history, counters, tokens)
     const float* lg = logits + (size_t)row * V;
@@ -753,7 +753,10 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
     }
     __syncthreads();
     if ((tid & 31) == 31) red[tid >> 5] = incl;
-    if (tid == 0) s_chosen = V - 1;
+    if (tid == 0) {
+        s_chosen = V;
+        s_last = -1;
+    }
     __syncthreads();
     float wbase = 0.f, total2 = 0.f;
 #pragma unroll
@@ -763,17 +766,23 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
     }
     const float u = u01(seed) * total2;
     float acc = wbase + incl - csum;  // exclusive prefix of this thread's range
+    // only kept tokens are looked at: the sums of threads round differently, so one without kept tokens can start above u first
+    int last = -1;
     for (int i = i0; i < i1; ++i) {
         const float p = temp[i];
-        acc += (p < cutoff) ? 0.0f : p;
+        if (!(p > 0.0f) || p < cutoff) continue;
+        last = i;
+        acc += p;
         if (acc > u) {
             atomicMin(&s_chosen, i);
             break;
         }
     }
+    if (last >= 0) atomicMax(&s_last, last);
     __syncthreads();
     if (tid == 0) {
-        const uint32_t tok = (uint32_t)s_chosen;
+        // (total2 is NaN when a probability is: then no sum exceeds u, and the answer is V - 1)
+        const uint32_t tok = (uint32_t)(s_chosen < V ? s_chosen : s_last >= 0 && total2 == total2 ? s_last : V - 1);
         next_tok[ent] = tok;
         if (seq) {
             const int c = seq_cnt[ent];

@@ -32,7 +32,7 @@ struct ScShared {
     float local[kScList];     // this CTA's part of the collection (read by the others)
     int local_n;
     float xmax, xsum, xkept;  // this CTA's maximum, sum, kept sum (read by the others)
-    int xchosen;
+    int xchosen, xlast;       // this CTA's drawn token (V: none) and its last kept one (-1: none)
     float list[kScList];      // the collection, sorted (every CTA its own copy)
     float red[kScThreads / 32];
     uint32_t ured[kScThreads / 32];
@@ -325,7 +325,9 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
         cutoff = sh.cut;
     }
 
-    // ---- draw: first index, in vocabulary order, whose running sum exceeds u ----
+    // ---- draw: first kept index, in vocabulary order, whose running sum exceeds u ----
+    // Sums put together from different parts round differently, so a thread without kept tokens can start above what the one before it
+    // reached; only kept tokens are looked at.  Where no sum exceeds u (u = the total), the last kept token is the answer.
     float csum = 0.f;
 #pragma unroll
     for (int q = 0; q < kScPer; ++q) {
@@ -340,7 +342,10 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
     }
     __syncthreads();
     if ((tid & 31) == 31) sh.red[tid >> 5] = incl;
-    if (tid == 0) sh.chosen = V - 1;
+    if (tid == 0) {
+        sh.xchosen = V;
+        sh.xlast = -1;
+    }
     __syncthreads();
     float wbase = 0.f, kept = 0.f;
 #pragma unroll
@@ -359,20 +364,29 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
     }
     const float u = u01(seed) * total2;
     float acc = base + wbase + incl - csum;  // exclusive prefix of this thread's range
-    int mine = V - 1;
+    int mine = V, last = -1;
 #pragma unroll
     for (int q = 0; q < kScPer; ++q) {
         acc += e[q];
-        if (q < nv && acc > u && mine == V - 1) mine = i0 + q;
+        if (e[q] > 0.0f) {
+            last = i0 + q;
+            if (acc > u && mine == V) mine = i0 + q;
+        }
     }
-    if (mine < V - 1) atomicMin(&sh.chosen, mine);
-    __syncthreads();
-    if (tid == 0) sh.xchosen = sh.chosen;
+    if (mine < V) atomicMin(&sh.xchosen, mine);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if ((tid & 31) == 0 && last >= 0) atomicMax(&sh.xlast, last);
     sc_cluster_sync(S);
     if (rank == 0 && tid == 0) {
-        int tok = V - 1;
+        int tok = V;
 #pragma unroll 1
         for (int c = 0; c < S; ++c) tok = min(tok, (int)sc_remote_u32(&sh.xchosen, c));
+        if (tok == V) {
+            tok = -1;
+#pragma unroll 1
+            for (int c = 0; c < S; ++c) tok = max(tok, (int)sc_remote_u32(&sh.xlast, c));
+            if (tok < 0 || total2 != total2) tok = V - 1;  // nothing was kept, or a NaN among the probabilities
+        }
         next_tok[ent] = (uint32_t)tok;
         if (seq) {
             const int c = seq_cnt[ent];

@@ -1,4 +1,5 @@
-"""What the sampler does with masked tokens (-inf, the lowest float), in rows of one CTA, of a cluster and of the kernel for large vocabularies."""
+"""What the sampler promises whatever the rounding: a drawn token is one that top-k and top-p kept, masked rows are drawn from as ever,
+and any float pointer is a logits pointer."""
 import numpy as np
 import pytest
 
@@ -21,9 +22,89 @@ def _unmix(z):
     return (z - 0x9E3779B9) & m
 
 
+def _running_sums(p, ctas, threads, per):
+    """The kernels' fp32 prefix sums: start and end of every thread's range of `per` tokens, and the total."""
+    e = np.zeros(ctas * threads * per, f32)
+    e[:p.size] = p
+    e = e.reshape(ctas, threads // 32, 32, per)
+    csum = np.zeros(e.shape[:3], f32)
+    for q in range(per):
+        csum = csum + e[..., q]
+    incl = csum.copy()
+    for o in (1, 2, 4, 8, 16):
+        up = np.zeros_like(incl)
+        up[..., o:] = incl[..., :-o]
+        incl = np.where(np.arange(32) >= o, incl + up, incl)
+    warps = incl[..., 31]
+    wbase = np.zeros(warps.shape, f32)
+    for i in range(1, warps.shape[1]):
+        wbase[:, i] = wbase[:, i - 1] + warps[:, i - 1]
+    kept = wbase[:, -1] + warps[:, -1]
+    base = np.zeros(ctas, f32)
+    for c in range(1, ctas):
+        base[c] = base[c - 1] + kept[c - 1]
+    total = base[-1] + kept[-1]
+    start = ((base[:, None] + wbase)[..., None] + incl) - csum
+    end = start
+    for q in range(per):
+        end = end + e[..., q]
+    return start.ravel(), end.ravel(), csum.ravel() > 0, total
+
+
+def _seeds_between_steps(p, ctas, threads, per):
+    """Seeds whose u lies in a gap: at or above what every kept thread before it reached, below where a thread without kept tokens starts."""
+    start, end, has, total = _running_sums(p, ctas, threads, per)
+    seeds = []
+    reach = np.maximum.accumulate(np.where(has, end, f32(0)))
+    for t in np.nonzero(~has & (start > reach))[0]:
+        f = f32(reach[t] / total)
+        for _ in range(8):
+            f = np.nextafter(f, f32(0))
+        for _ in range(16):
+            if reach[t] <= f32(f * total) < start[t]:
+                z = int(np.float64(f) * 2 ** 32)
+                if z < 2 ** 32 and f32(z) == f32(np.float64(f) * 2 ** 32):
+                    seeds.append(_unmix(z))
+                    break
+            f = np.nextafter(f, f32(2))
+    return seeds
+
+
 def test_unmix_is_the_inverse():
     for z in (0, 1, 12345, 0x80000000, 0xFFFFFFFF):
         assert f32(orc.lib().orc_u01(_unmix(z))) == f32(f32(z) / f32(4294967296.0))
+
+
+# a row of one cluster of CTAs (8192 logits each), of one CTA of a cluster kernel, and of the kernel for larger vocabularies
+@pytest.mark.parametrize("v,ctas,threads,per", [(65536, 8, 512, 16), (8192, 1, 512, 16), (70000, 1, 1024, 69)])
+def test_drawn_tokens_were_kept(v, ctas, threads, per):
+    rng = np.random.default_rng(v)
+    logits, rows = [], []
+    for n in range(20, 400):
+        # n equally probable tokens; everything else is cut by top-k
+        lg = np.full(v, -100.0, f32)
+        lg[rng.choice(v - 1, n, replace=False)] = 0.0  # the last token is never kept
+        p = np.where(lg == 0, f32(1) / f32(n), f32(0)).astype(f32)
+        seeds = _seeds_between_steps(p, ctas, threads, per)[:2] + [_unmix(0xFFFFFFFF), _unmix(0)]  # and u = 1 and 0
+        for s in seeds:
+            logits.append(lg)
+            rows.append(orc.pack_sampler(seed=s, top_k=n, top_p=1.0))
+        if len(rows) >= 200:
+            break
+    logits = np.stack(logits)
+    got = rsv.op_sample(logits, np.stack(rows)).astype(np.int64)
+    bad = [(i, int(t)) for i, t in enumerate(got) if logits[i, t] != 0]
+    assert not bad, bad[:5]
+
+
+def test_drawn_tokens_of_a_nucleus_were_kept():
+    v, n = 16384, 1500
+    lg = (np.random.default_rng(5).standard_normal(v) * 4).astype(f32)
+    logits = np.broadcast_to(lg, (n, v))
+    got = rsv.op_sample(logits, np.stack([orc.pack_sampler(seed=s, top_p=0.7) for s in range(n)]))
+    p = np.sort(np.exp(np.float64(lg) - lg.max()) / np.exp(np.float64(lg) - lg.max()).sum())[::-1]
+    k = int(np.searchsorted(np.cumsum(p), 0.7)) + 2  # (one more: the kernel's fp32 sum may need another pick)
+    assert lg[got].min() >= np.sort(lg)[::-1][k]
 
 
 # Every logit below the sampler's floor: such tokens count as -1e30 and are then equally probable.  V = 5000 and 65536 are rows of a cluster,

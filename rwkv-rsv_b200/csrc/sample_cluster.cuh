@@ -291,9 +291,10 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
     // ---- softmax over what is kept ----
     float ps = 0.f;
     float e[kScPer];
+    const float below = expf(-1e30f - mx);  // what a token under the threshold counts: 0, but 1 in a row of masked tokens only
 #pragma unroll
     for (int q = 0; q < kScPer; ++q) {
-        e[q] = q < nv ? expf((x[q] < thr ? -1e30f : x[q]) - mx) : 0.f;
+        e[q] = q >= nv ? 0.f : x[q] < thr ? below : expf(x[q] - mx);  // (most warps have nothing above a top-k threshold and skip the rest)
         ps += e[q];
     }
     ps = sc_block_sum(ps, sh.red);

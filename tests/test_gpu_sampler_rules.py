@@ -1,5 +1,5 @@
-"""What the sampler promises whatever the rounding: a drawn token is one that top-k and top-p kept, masked rows are drawn from as ever,
-and any float pointer is a logits pointer."""
+"""What the sampler promises whatever the rounding: a drawn token is one that top-k and top-p kept, and masked tokens (-inf, the lowest
+float) are never drawn beside others.  Rows of one CTA, of a cluster and of the kernel for large vocabularies."""
 import numpy as np
 import pytest
 
@@ -131,3 +131,12 @@ def test_masked_tokens_are_not_drawn(v, k, top_p):
     got = rsv.op_sample(lg, rows)
     assert set(int(g) for g in got) <= set(int(a) for a in allowed)
     assert [int(g) for g in got[:8]] == [orc.sample(lg[s], seed=s, top_k=k, top_p=top_p, temperature=0.8) for s in range(8)]
+
+
+@pytest.mark.parametrize("v", [5000, 65536, 70000])
+def test_rows_with_a_nan_or_an_infinity(v):
+    # no sum of such a row exceeds u, so the answer is the last token, as on the CPU path
+    lg = np.random.default_rng(v).standard_normal((2, v)).astype(f32)
+    lg[0, 100], lg[1, 100] = np.nan, np.inf
+    got = rsv.op_sample(lg, np.stack([orc.pack_sampler(seed=s) for s in (1, 2)]))
+    assert [int(g) for g in got] == [v - 1, v - 1] == [orc.sample(lg[s], seed=s + 1) for s in range(2)]

@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
     const float* lg = logits + (size_t)row * V;
     const int i0 = rank * kScSeg + tid * kScPer;
     float x[kScPer];
-    if ((V & 3) == 0) {
+    if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(lg) & 15) == 0) {  // (a caller's device array need not start at 16 bytes)
 #pragma unroll
         for (int q = 0; q < kScPer / 4; ++q) {
             float4 t = make_float4(0.f, 0.f, 0.f, 0.f);

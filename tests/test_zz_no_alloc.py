@@ -58,6 +58,24 @@ def test_static_sampler_matches_allocating_entry_point_twice():
     assert np.array_equal(_static_sample(logits, srows, hist), want1)
 
 
+# logits that begin anywhere in the caller's array: the wide loads are for rows that start at 16 bytes
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows,V", [(1, 65536), (5, 4096), (3, 4099)])
+def test_static_sampler_takes_logits_at_any_offset(offset, rows, V):
+    import torch
+    logits = (np.random.default_rng(V + offset).standard_normal((rows, V)) * 2).astype(np.float32)
+    srows = np.stack([orc.pack_sampler(seed=3 + r, top_k=100, top_p=0.95) for r in range(rows)])
+    buf = torch.zeros(rows * V + 4, device="cuda")
+    buf[offset:offset + rows * V] = torch.from_numpy(logits.reshape(-1)).cuda()
+    sr, out = torch.from_numpy(srows).cuda(), torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    rc = rsv.native().rsv_op_sample_static(0, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.c_void_p(buf.data_ptr() + 4 * offset), rows, V,
+                                           ctypes.c_void_p(sr.data_ptr()), None, 0, ctypes.c_void_p(out.data_ptr()))
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), rsv.op_sample(logits, srows))
+
+
 def test_static_sampler_rejects_oversize_requests():
     rows, V = 17, 65536      # 17 * 65536 > 1,048,576
     with pytest.raises(rsv.RsvError, match="exceeds the static work area"):

@@ -1403,11 +1403,11 @@ void Model::run_stream(State& st, int slot, int n_tokens, bool tok_from_list, bo
     P.tok_from_list = host_token ? 2 : tok_from_list ? 1 : 0;
     P.tok0 = host_token ? *host_token : 0u;
     P.argmax_feed = argmax_feed ? 1 : 0;
-    P.epoch = sc.epoch;
-    sc.epoch += (uint32_t)n_tokens * (uint32_t)cfg.n_layer;
-    P.bar_base = sc.bar_base;
-    sc.bar_base += (unsigned)sc.grid * (unsigned)(argmax_feed ? n_tokens : n_tokens - 1);
-    LAUNCH(*this, "decode_stream") { dispatch_stream(sc.kl, P, sc.grid, sc.smem, stream, false); }
+    sc.seq.run((uint32_t)n_tokens * (uint32_t)cfg.n_layer, (unsigned)sc.grid * (unsigned)(argmax_feed ? n_tokens : n_tokens - 1), [&](uint32_t epoch, unsigned bar_base) {
+        P.epoch = epoch;
+        P.bar_base = bar_base;
+        LAUNCH(*this, "decode_stream") { dispatch_stream(sc.kl, P, sc.grid, sc.smem, stream, false); }
+    });
 }
 
 void Model::check_status() {
@@ -1423,9 +1423,8 @@ void Model::judge_status(const int* sw) {
         RSV_CUDA(cudaMemsetAsync(ws.status, 0, 2 * sizeof(int), stream));
         if ((s & 32) && sctx.exchange) {  // a launch that gave up left some of its exchanged values unwritten
             RSV_CUDA(cudaMemsetAsync(sctx.exchange, 0, sctx.exchange_bytes, stream));
-            sctx.epoch = 1;
             RSV_CUDA(cudaMemsetAsync(sctx.grid_bar, 0, 4, stream));
-            sctx.bar_base = 0;
+            sctx.seq = StreamSequence{};
         }
         if (s & 32) {
             static const char* const site[5] = {"a wait", "a chunk of weight rows", "room in the ring", "a grid barrier", "a chunk of a head's rows"};

@@ -12,6 +12,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "stream_sequence.hpp"
 
 namespace rsv {
 
@@ -79,8 +80,7 @@ struct StreamCtx {
     long long wslot = 0, hslot = 0;
     unsigned long long* exchange = nullptr;  // values the CTAs exchange (see decode_stream.cuh): xa, xb, yg, vfirst [C], rkv [3C], mid, then hbuf [F] words
     size_t exchange_bytes = 0;
-    uint32_t epoch = 1;                      // tag of the next launch's first layer
-    unsigned bar_base = 0;      // value of the grid barrier's counter when the next launch begins
+    StreamSequence seq;  // layer tags and barrier counts used so far
     float* cand_val = nullptr;
     int* cand_idx = nullptr;
     unsigned* grid_bar = nullptr;

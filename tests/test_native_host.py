@@ -1,0 +1,20 @@
+"""CPU checks of the engine's host-side parts that make no CUDA call of their own: small programs built with g++ and run here."""
+import os
+import subprocess
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "rwkv-rsv_b200", "csrc")
+
+
+def _run(tmp_path, name, *flags):
+    exe = tmp_path / name
+    r = subprocess.run(["g++", "-O1", "-std=c++17", "-pthread", "-I", CSRC, *flags, os.path.join(ROOT, "tests", "native", name + ".cpp"), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+    run = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert run.returncode == 0, run.stdout[-2000:]
+    return run.stdout
+
+
+def test_decode_launches_continue_after_one_that_failed(tmp_path):
+    assert "sequence ok" in _run(tmp_path, "stream_sequence_check")

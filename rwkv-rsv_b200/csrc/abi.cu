@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "engine.hpp"
+#include "parts_to_host.hpp"
 #include "rsv_b200.h"
 
 using namespace rsv;
@@ -126,43 +127,37 @@ constexpr int kMaxChunk = 512;  // rows per packed step on the chunk path
 class LogitsToHost {
   public:
     explicit LogitsToHost(Model& model) : m(model) {}
-    ~LogitsToHost() { join(); }
+    ~LogitsToHost() {
+        moves.join();
+        if (queued) cudaStreamSynchronize(m.stream);  // left by an exception: nothing writes to the caller's memory afterwards
+    }
     // queues the copy of `count` logits; returns while it is under way
     void start(float* dst, size_t count) {
-        join();  // the staging area is free again
+        moves.join();  // the staging area is free again
         cudaPointerAttributes at;
         const bool direct = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
         if (!direct) cudaGetLastError();
+        queued = true;
         if (direct || count < kSmall) {
             RSV_CUDA(cudaMemcpyAsync(dst, m.ws.logits, count * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
             return;
         }
         m.ensure_pinned_out(count * sizeof(float));
-        const size_t part = (count + kOutParts - 1) / kOutParts;
         for (int i = 0; i < kOutParts; ++i) {
-            const size_t at0 = std::min(count, i * part), n = std::min(count, at0 + part) - at0;
+            const size_t at0 = PartsToHost::part_begin(count, kOutParts, i), n = PartsToHost::part_begin(count, kOutParts, i + 1) - at0;
             if (n) RSV_CUDA(cudaMemcpyAsync(m.pinned_out + at0, m.ws.logits + at0, n * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
             RSV_CUDA(cudaEventRecord(m.out_ev[i], m.stream));
         }
         const int workers = (int)std::min<unsigned>(kWorkers, std::max(1u, std::thread::hardware_concurrency() / 2));
-        failed.assign((size_t)workers, 0);
-        for (int w = 0; w < workers; ++w)
-            threads.emplace_back([this, dst, count, part, w, workers] {
-                cudaSetDevice(m.device);
-                for (int i = w; i < kOutParts; i += workers) {
-                    if (cudaEventSynchronize(m.out_ev[i]) != cudaSuccess) {
-                        failed[(size_t)w] = 1;
-                        return;
-                    }
-                    const size_t at0 = std::min(count, i * part), n = std::min(count, at0 + part) - at0;
-                    memcpy(dst + at0, m.pinned_out + at0, n * sizeof(float));
-                }
-            });
+        Model& model = m;
+        moves.start(dst, m.pinned_out, count, kOutParts, workers,
+                    [&model](int i) { return cudaSetDevice(model.device) == cudaSuccess && cudaEventSynchronize(model.out_ev[i]) == cudaSuccess; });
     }
     void finish() {
-        join();
+        const bool all = moves.finish();
         RSV_CUDA(cudaStreamSynchronize(m.stream));
-        for (char f : failed) need(!f, "copy of the logits to the host failed");
+        queued = false;
+        need(all, "copy of the logits to the host failed");
     }
 
   private:
@@ -170,12 +165,8 @@ class LogitsToHost {
     static constexpr int kOutParts = Model::kOutParts;
     static constexpr unsigned kWorkers = 8;
     Model& m;
-    std::vector<std::thread> threads;
-    std::vector<char> failed;
-    void join() {
-        for (auto& t : threads) t.join();
-        threads.clear();
-    }
+    PartsToHost moves;
+    bool queued = false;
 };
 
 // chunked prefill of one session; out_mode 1: logits of the very last token in ws.logits[0,:];

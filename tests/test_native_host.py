@@ -18,3 +18,7 @@ def _run(tmp_path, name, *flags):
 
 def test_decode_launches_continue_after_one_that_failed(tmp_path):
     assert "sequence ok" in _run(tmp_path, "stream_sequence_check")
+
+
+def test_logits_that_arrive_in_parts(tmp_path):
+    assert "parts ok" in _run(tmp_path, "parts_to_host_check")

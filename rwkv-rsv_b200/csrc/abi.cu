@@ -121,6 +121,15 @@ void decode_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n) {
 
 constexpr int kMaxChunk = 512;  // rows per packed step on the chunk path
 
+// Memory the driver knows (pinned; or, though the interface asks for host arrays, managed or a device's) takes copies directly; only pageable
+// memory is the host's own to write.
+bool driver_knows(const void* p) {
+    cudaPointerAttributes at;
+    const bool known = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    if (!known) cudaGetLastError();
+    return known;
+}
+
 // Logits of a whole chunk to the caller's memory.  A copy to pageable memory runs at what one thread of the driver moves (201 x 65536
 // logits: 53 MB, 8 ms with the first touch of the pages); here the chunk goes to pinned memory in kOutParts pieces behind its forward
 // pass, and a few threads move each piece on as soon as it has arrived, while the GPU runs the next chunk.
@@ -134,12 +143,9 @@ class LogitsToHost {
     // queues the copy of `count` logits; returns while it is under way
     void start(float* dst, size_t count) {
         moves.join();  // the staging area is free again
-        cudaPointerAttributes at;
-        const bool direct = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
-        if (!direct) cudaGetLastError();
         queued = true;
-        if (direct || count < kSmall) {
-            RSV_CUDA(cudaMemcpyAsync(dst, m.ws.logits, count * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
+        if (count < kSmall || driver_knows(dst)) {
+            RSV_CUDA(cudaMemcpyAsync(dst, m.ws.logits, count * sizeof(float), cudaMemcpyDefault, m.stream));
             return;
         }
         m.ensure_pinned_out(count * sizeof(float));
@@ -193,14 +199,12 @@ void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int6
 }
 
 // One row of logits and the status words, through pinned memory: two copies and one wait instead of two waits (a copy to pageable memory
-// is one).  A caller's pinned array is written directly.
+// is one).  Memory the driver knows is written directly.
 void fetch_logits(Model& m, float* logits_out) {
     const size_t V = m.cfg.vocab;
-    cudaPointerAttributes at;
-    const bool direct = cudaPointerGetAttributes(&at, logits_out) == cudaSuccess && at.type == cudaMemoryTypeHost;
-    if (!direct) cudaGetLastError();
+    const bool direct = driver_knows(logits_out);
     m.ensure_pinned_out((V + 2) * sizeof(float));
-    RSV_CUDA(cudaMemcpyAsync(direct ? logits_out : m.pinned_out, m.ws.logits, V * sizeof(float), cudaMemcpyDeviceToHost, m.stream));
+    RSV_CUDA(cudaMemcpyAsync(direct ? logits_out : m.pinned_out, m.ws.logits, V * sizeof(float), cudaMemcpyDefault, m.stream));
     RSV_CUDA(cudaMemcpyAsync(m.pinned_out + V, m.ws.status, 2 * sizeof(int), cudaMemcpyDeviceToHost, m.stream));
     RSV_CUDA(cudaStreamSynchronize(m.stream));
     int sw[2];

@@ -43,3 +43,23 @@ def test_logits_of_every_position(bundle, n):
     pinned = torch.full((n, V), float("nan"), pin_memory=True)
     _full(b, toks, pinned.data_ptr())
     assert np.array_equal(pinned.numpy(), pageable)
+
+
+def test_logits_into_memory_of_the_device(bundle):
+    # the arrays are the host's by contract; a device array is a matter for the driver's copy and never for the host's own
+    import torch
+    b = bundle
+    toks = np.arange(70, dtype=np.uint32)
+    host = np.empty((70, V), np.float32)
+    _full(b, toks, host.ctypes.data)
+    dev = torch.zeros((70, V), device="cuda")
+    torch.cuda.synchronize()
+    _full(b, toks, dev.data_ptr())
+    assert np.array_equal(dev.cpu().numpy(), host)
+    one = torch.zeros(V, device="cuda")
+    torch.cuda.synchronize()
+    t = np.array([3], dtype=np.uint32)
+    b.reset()
+    assert rsv.native().rsv_infer_tokens(b.model._h, b.state._h, t.ctypes.data_as(ctypes.c_void_p), 1, ctypes.c_void_p(one.data_ptr())) == 0
+    b.reset()
+    assert np.array_equal(one.cpu().numpy(), b.infer_tokens(t))

@@ -88,7 +88,7 @@ void ensure_tok_list(Model& m, size_t n) {
         m.ws.tok_list = nullptr;
         m.ws.tok_list_cap = 0;
         size_t cap = std::max<size_t>(n, 1024);
-        RSV_CUDA(cudaMalloc(&m.ws.tok_list, cap * sizeof(uint32_t)));
+        RSV_CUDA(device_malloc(&m.ws.tok_list, cap * sizeof(uint32_t)));
         m.ws.tok_list_cap = cap;
     }
 }
@@ -238,8 +238,8 @@ std::unique_ptr<rsv_ticket> selfloop_submit(Model& m, State& st, const uint32_t*
     t.model = &m;
     t.batch = batch;
     t.n = n;
-    RSV_CUDA(cudaMalloc(&t.seq, (size_t)batch * n * sizeof(uint32_t)));
-    RSV_CUDA(cudaMalloc(&t.cnt, (size_t)batch * sizeof(int)));
+    RSV_CUDA(device_malloc(&t.seq, (size_t)batch * n * sizeof(uint32_t)));
+    RSV_CUDA(device_malloc(&t.cnt, (size_t)batch * sizeof(int)));
     RSV_CUDA(cudaMemsetAsync(t.seq, 0, (size_t)batch * n * sizeof(uint32_t), m.stream));
     RSV_CUDA(cudaMemsetAsync(t.cnt, 0, (size_t)batch * sizeof(int), m.stream));
     RSV_CUDA(cudaMemcpyAsync(m.ws.tokens, seeds, (size_t)batch * sizeof(uint32_t), cudaMemcpyHostToDevice, m.stream));
@@ -248,7 +248,7 @@ std::unique_ptr<rsv_ticket> selfloop_submit(Model& m, State& st, const uint32_t*
         // (src/gpu_model.rs:1738-1756); the kernel adds r itself from the slot's token counter.
         std::vector<float> rows((size_t)batch * 8);
         for (int64_t b = 0; b < batch; ++b) pack_sampler_row(&rows[(size_t)b * 8], *sp, seeds[b], 0);
-        RSV_CUDA(cudaMalloc(&t.sampler, rows.size() * sizeof(float)));
+        RSV_CUDA(device_malloc(&t.sampler, rows.size() * sizeof(float)));
         RSV_CUDA(cudaMemcpyAsync(t.sampler, rows.data(), rows.size() * sizeof(float), cudaMemcpyHostToDevice, m.stream));
         RSV_CUDA(cudaStreamSynchronize(m.stream));  // `rows` is a stack-lifetime pageable buffer
     }
@@ -600,8 +600,8 @@ int rsv_infer_sample(rsv_model* mh, rsv_state* s, const uint32_t* tokens, int64_
         pack_sampler_row(row, *sp, sp->seed, (uint32_t)nh);
         float* d_row = nullptr;
         uint32_t* d_hist = nullptr;
-        RSV_CUDA(cudaMalloc(&d_row, sizeof(row)));
-        if (nh) RSV_CUDA(cudaMalloc(&d_hist, (size_t)nh * sizeof(uint32_t)));
+        RSV_CUDA(device_malloc(&d_row, sizeof(row)));
+        if (nh) RSV_CUDA(device_malloc(&d_hist, (size_t)nh * sizeof(uint32_t)));
         int rc = guarded([&] {
             RSV_CUDA(cudaMemcpyAsync(d_row, row, sizeof(row), cudaMemcpyHostToDevice, m.stream));
             if (nh) RSV_CUDA(cudaMemcpyAsync(d_hist, history, (size_t)nh * sizeof(uint32_t), cudaMemcpyHostToDevice, m.stream));
@@ -645,7 +645,7 @@ static void prefill_batch(Model& m, State& st, const uint32_t* flat, const uint3
         }
     } guard{acc};
     if (mean_out) {
-        RSV_CUDA(cudaMalloc(&acc, (size_t)batch * C * 4));
+        RSV_CUDA(device_malloc(&acc, (size_t)batch * C * 4));
         RSV_CUDA(cudaMemsetAsync(acc, 0, (size_t)batch * C * 4, m.stream));
     }
     // Steps of at most kMaxChunk rows, shared between the sessions in proportion to what they have left.  The state update is sequential
@@ -777,7 +777,7 @@ int rsv_synchronize(rsv_model* m) {
 namespace {
 struct DevBuf {
     void* p = nullptr;
-    explicit DevBuf(size_t bytes) { RSV_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16))); }
+    explicit DevBuf(size_t bytes) { RSV_CUDA(device_malloc(&p, std::max<size_t>(bytes, 16))); }
     ~DevBuf() {
         if (p) cudaFree(p);
     }

@@ -170,7 +170,7 @@ struct Loader {
 
     void* dev_alloc(size_t bytes) {
         void* p = nullptr;
-        RSV_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
+        RSV_CUDA(device_malloc(&p, std::max<size_t>(bytes, 16)));
         m.allocs.push_back(p);
         m.weight_bytes += bytes;
         return p;
@@ -284,6 +284,7 @@ std::unique_ptr<Model> Model::load(const std::string& path, int device) {
     SafeTensorsFile st(path);
     auto m = std::make_unique<Model>();
     m->device = device;
+    m->state_pool = std::make_shared<StatePool>(device);
     Config& c = m->cfg;
     // hyper-parameters come from tensor shapes only (src/gpu_model.rs:406-444)
     int max_layer = -1;
@@ -388,8 +389,8 @@ std::unique_ptr<Model> Model::load(const std::string& path, int device) {
     m->pinned_bytes = 1 << 18;
     RSV_CUDA(cudaMallocHost(&m->pinned, m->pinned_bytes * Model::kPinRing));
     for (int i = 0; i < Model::kPinRing; ++i) RSV_CUDA(cudaEventCreateWithFlags(&m->pin_ev[i], cudaEventDisableTiming));
-    RSV_CUDA(cudaMalloc(&m->ws.status, 2 * sizeof(int)));
-    RSV_CUDA(cudaMalloc(&m->ws.tok_pos, sizeof(int)));
+    RSV_CUDA(device_malloc(&m->ws.status, 2 * sizeof(int)));
+    RSV_CUDA(device_malloc(&m->ws.tok_pos, sizeof(int)));
     RSV_CUDA(cudaMemsetAsync(m->ws.status, 0, 2 * sizeof(int), m->stream));
     RSV_CUDA(cudaMemsetAsync(m->ws.tok_pos, 0, sizeof(int), m->stream));
     return m;
@@ -407,13 +408,14 @@ std::unique_ptr<Model> Model::create_bare(int device) {
     if (prop.major != 10) throw std::runtime_error("this library is built for sm_100a (B200) only");
     auto m = std::make_unique<Model>();
     m->device = device;
+    m->state_pool = std::make_shared<StatePool>(device);
     m->num_sms = prop.multiProcessorCount;
     RSV_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
     RSV_CUDA(cudaEventCreate(&m->ev0));
     RSV_CUDA(cudaEventCreate(&m->ev1));
     RSV_CUDA(cudaEventCreate(&m->tev[0]));
     RSV_CUDA(cudaEventCreate(&m->tev[1]));
-    RSV_CUDA(cudaMalloc(&m->ws.status, 2 * sizeof(int)));
+    RSV_CUDA(device_malloc(&m->ws.status, 2 * sizeof(int)));
     RSV_CUDA(cudaMemsetAsync(m->ws.status, 0, 2 * sizeof(int), m->stream));
     return m;
 }
@@ -437,7 +439,7 @@ static void free_workspace(Workspace& w) {
 Model::~Model() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    state_pool->release(true);
+    if (state_pool) state_pool->release(true);
     free_workspace(ws);
     if (ws.status) cudaFree(ws.status);
     if (ws.tok_pos) cudaFree(ws.tok_pos);
@@ -460,33 +462,6 @@ Model::~Model() {
     if (stream) cudaStreamDestroy(stream);
 }
 
-float* StatePool::take(size_t bytes) {
-    std::lock_guard<std::mutex> lock(mu);
-    for (size_t i = 0; i < kept.size(); ++i)
-        if (kept[i].first == bytes) {
-            float* p = kept[i].second;
-            kept.erase(kept.begin() + (long)i);
-            return p;
-        }
-    return nullptr;
-}
-void StatePool::give(size_t bytes, float* p) {
-    std::lock_guard<std::mutex> lock(mu);
-    if (open && bytes <= kMostBytes) {
-        kept.emplace_back(bytes, p);
-        if (kept.size() <= kMost) return;
-        p = kept.front().second;
-        kept.erase(kept.begin());
-    }
-    cudaFree(p);
-}
-void StatePool::release(bool close) {
-    std::lock_guard<std::mutex> lock(mu);
-    for (auto& k : kept) cudaFree(k.second);
-    kept.clear();
-    if (close) open = false;
-}
-
 State::~State() {
     if (!wkv) return;
     cudaSetDevice(pool->device);
@@ -501,13 +476,11 @@ void State::allocate(Model* m, int64_t slots) {
     const size_t nx = aligned((size_t)c.n_layer * cap * c.n_embd), ns = aligned((size_t)c.n_layer * cap * c.n_head * kHeadSize * kHeadSize);
     bytes = (ns + 2 * nx + (size_t)cap * c.n_embd) * 4;
     pool = m->state_pool;
-    pool->device = m->device;
     wkv = pool->take(bytes);
-    if (!wkv && cudaMalloc(&wkv, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        wkv = nullptr;
-        pool->release(false);
-        RSV_CUDA(cudaMalloc(&wkv, bytes));
+    if (!wkv) {
+        float* p = nullptr;
+        RSV_CUDA(device_malloc(&p, bytes));
+        wkv = p;
     }
     tmix_x = wkv + ns;
     cmix_x = tmix_x + nx;
@@ -527,7 +500,7 @@ void Model::ensure_workspace(int rows, int outs, int segs) {
     segs = grow(segs, ws.segs);
     free_workspace(ws);
     const size_t C = cfg.n_embd, F = cfg.ffn_hidden, V = cfg.vocab, R = rows;
-    auto fa = [&](float*& p, size_t n) { RSV_CUDA(cudaMalloc(&p, std::max<size_t>(n, 4) * sizeof(float))); };
+    auto fa = [&](float*& p, size_t n) { RSV_CUDA(device_malloc(&p, std::max<size_t>(n, 4) * sizeof(float))); };
     fa(ws.x, R * C);
     fa(ws.x2, R * C);
     fa(ws.delta, R * C);
@@ -549,13 +522,13 @@ void Model::ensure_workspace(int rows, int outs, int segs) {
     fa(ws.staging_c, (size_t)segs * C);
     if (V > (size_t)kScMaxV) {  // the sampler of smaller vocabularies needs no work area
         fa(ws.samp_temp, (size_t)outs * V);
-        RSV_CUDA(cudaMalloc(&ws.samp_cnt, std::max<size_t>((size_t)outs * V, 4) * sizeof(uint32_t)));
+        RSV_CUDA(device_malloc(&ws.samp_cnt, std::max<size_t>((size_t)outs * V, 4) * sizeof(uint32_t)));
     }
-    RSV_CUDA(cudaMalloc(&ws.tokens, R * sizeof(uint32_t)));
+    RSV_CUDA(device_malloc(&ws.tokens, R * sizeof(uint32_t)));
     RSV_CUDA(cudaMemsetAsync(ws.tokens, 0, R * sizeof(uint32_t), stream));
-    RSV_CUDA(cudaMalloc(&ws.row_meta, R * sizeof(RowMeta)));
-    RSV_CUDA(cudaMalloc(&ws.seg_meta, (size_t)segs * sizeof(SegMeta)));
-    RSV_CUDA(cudaMalloc(&ws.out_rows, (size_t)std::max(outs, 1) * sizeof(int)));
+    RSV_CUDA(device_malloc(&ws.row_meta, R * sizeof(RowMeta)));
+    RSV_CUDA(device_malloc(&ws.seg_meta, (size_t)segs * sizeof(SegMeta)));
+    RSV_CUDA(device_malloc(&ws.out_rows, (size_t)std::max(outs, 1) * sizeof(int)));
     ws.rows = rows;
     ws.outs = outs;
     ws.segs = segs;
@@ -737,7 +710,7 @@ void ensure_operand_memory(Model& m, size_t bytes) {
     w.op_mem = nullptr;
     w.op_bytes = 0;
     const size_t nb = bytes + bytes / 4;
-    RSV_CUDA(cudaMalloc(&w.op_mem, nb));
+    RSV_CUDA(device_malloc(&w.op_mem, nb));
     RSV_CUDA(cudaMemsetAsync(w.op_mem, 0, nb, m.stream));
     w.op_bytes = nb;
 }
@@ -1300,7 +1273,7 @@ bool Model::stream_available() {
         d.k_k = Lw.k_k;
         d.k_a = Lw.k_a;
     }
-    RSV_CUDA(cudaMalloc(&sc.d_layers, dl.size() * sizeof(DsLayer)));
+    RSV_CUDA(device_malloc(&sc.d_layers, dl.size() * sizeof(DsLayer)));
     RSV_CUDA(cudaMemcpy(sc.d_layers, dl.data(), dl.size() * sizeof(DsLayer), cudaMemcpyHostToDevice));
     {
         // second copy of the weights in the order the kernel consumes them (a chunk = one bulk copy): region sizes = the largest CTA's
@@ -1309,8 +1282,8 @@ bool Model::stream_available() {
         if (!bind(head_e, head, nullptr)) return fail("the head of the checkpoint does not have the model's shape");
         sc.wslot = wslot;
         sc.hslot = hslot;
-        RSV_CUDA(cudaMalloc(&sc.wstream, (size_t)wslot * G * L));
-        RSV_CUDA(cudaMalloc(&sc.hstream, (size_t)hslot * G));
+        RSV_CUDA(device_malloc(&sc.wstream, (size_t)wslot * G * L));
+        RSV_CUDA(device_malloc(&sc.hstream, (size_t)hslot * G));
         DsParams Q;
         memset(&Q, 0, sizeof(Q));
         Q.layers = (const DsLayer*)sc.d_layers;
@@ -1331,11 +1304,11 @@ bool Model::stream_available() {
     }
     const size_t pairs = (size_t)7 * C + cfg.mids();
     sc.exchange_bytes = pairs * 8 + (size_t)F * 4;
-    RSV_CUDA(cudaMalloc(&sc.exchange, sc.exchange_bytes));
+    RSV_CUDA(device_malloc(&sc.exchange, sc.exchange_bytes));
     RSV_CUDA(cudaMemsetAsync(sc.exchange, 0, sc.exchange_bytes, stream));  // tag 0: no launch's
-    RSV_CUDA(cudaMalloc(&sc.cand_val, (size_t)G * 4));
-    RSV_CUDA(cudaMalloc(&sc.cand_idx, (size_t)G * 4));
-    RSV_CUDA(cudaMalloc(&sc.grid_bar, 4));
+    RSV_CUDA(device_malloc(&sc.cand_val, (size_t)G * 4));
+    RSV_CUDA(device_malloc(&sc.cand_idx, (size_t)G * 4));
+    RSV_CUDA(device_malloc(&sc.grid_bar, 4));
     RSV_CUDA(cudaMemsetAsync(sc.grid_bar, 0, 4, stream));
     P.layers = (const DsLayer*)sc.d_layers;
     P.head = ds_head_entry(shp, G);
@@ -1553,22 +1526,22 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
     Buf din[8], dpar[5], dstate, dy, dseg, dstatus;
     for (int i = 0; i < 8; ++i)
         if (in[i]) {
-            RSV_CUDA(cudaMalloc(&din[i].p, row_bytes));
+            RSV_CUDA(device_malloc(&din[i].p, row_bytes));
             RSV_CUDA(cudaMemcpy(din[i].p, in[i], row_bytes, cudaMemcpyHostToDevice));
         }
     for (int i = 0; i < 5; ++i) {
-        RSV_CUDA(cudaMalloc(&dpar[i].p, (size_t)C * 4));
+        RSV_CUDA(device_malloc(&dpar[i].p, (size_t)C * 4));
         RSV_CUDA(cudaMemcpy(dpar[i].p, par[i], (size_t)C * 4, cudaMemcpyHostToDevice));
     }
-    RSV_CUDA(cudaMalloc(&dstate.p, st_floats * 4));
+    RSV_CUDA(device_malloc(&dstate.p, st_floats * 4));
     RSV_CUDA(cudaMemcpy(dstate.p, state_host, st_floats * 4, cudaMemcpyHostToDevice));
-    RSV_CUDA(cudaMalloc(&dy.p, row_bytes));
+    RSV_CUDA(device_malloc(&dy.p, row_bytes));
     RSV_CUDA(cudaMemset(dy.p, 0, row_bytes));
     std::vector<SegMeta> segs((size_t)nseg);
     for (int s2 = 0; s2 < nseg; ++s2) segs[s2] = SegMeta{s2 * T, T, s2, 0};
-    RSV_CUDA(cudaMalloc(&dseg.p, segs.size() * sizeof(SegMeta)));
+    RSV_CUDA(device_malloc(&dseg.p, segs.size() * sizeof(SegMeta)));
     RSV_CUDA(cudaMemcpy(dseg.p, segs.data(), segs.size() * sizeof(SegMeta), cudaMemcpyHostToDevice));
-    RSV_CUDA(cudaMalloc(&dstatus.p, 8));
+    RSV_CUDA(device_malloc(&dstatus.p, 8));
     RSV_CUDA(cudaMemset(dstatus.p, 0, 8));
     const float *r = (const float*)din[0].p, *k = (const float*)din[1].p, *v = (const float*)din[2].p, *w = (const float*)din[3].p, *a = (const float*)din[4].p,
                 *g = (const float*)din[5].p, *vgate = (const float*)din[6].p, *vfirst = (const float*)din[7].p;
@@ -1631,8 +1604,8 @@ void engine_op_linear(Model& m, int path, int wtype, const void* w_host, const u
             ld.prepare_tc_f16(W);
         }
         if (path == 1 && wtype == W_INT8 && (!W.row_scaled() || M % kTcTileM)) throw std::runtime_error("op_linear: this matrix cannot take the tensor-core path (needs one scale/zero per row, M and K multiples of 128)");
-        RSV_CUDA(cudaMalloc(&dx, (size_t)R * K * 4));
-        RSV_CUDA(cudaMalloc(&dy, (size_t)R * M * 4));
+        RSV_CUDA(device_malloc(&dx, (size_t)R * K * 4));
+        RSV_CUDA(device_malloc(&dy, (size_t)R * M * 4));
         RSV_CUDA(cudaMemcpyAsync(dx, x_host, (size_t)R * K * 4, cudaMemcpyHostToDevice, m.stream));
         if (path == 1) {
             const RowTiles t = row_tiles(R, false, rl_fmt(W) == RL_I8);

@@ -12,6 +12,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "device_memory.hpp"
 #include "stream_sequence.hpp"
 
 namespace rsv {
@@ -96,20 +97,6 @@ struct KernelProf {
 
 struct Model;
 
-// Allocations of states that are gone, for the next ones of the same model (mapping device memory costs up to 4 ms): the last kMost of
-// at most kMostBytes each.  Shared by the model, which empties and closes it when it goes, and its states, which may outlive it.  All work
-// on a state goes through the model's stream, so the next user's clearing is ordered behind it.
-struct StatePool {
-    static constexpr size_t kMost = 2, kMostBytes = 512u << 20;
-    std::mutex mu;
-    std::vector<std::pair<size_t, float*>> kept;  // newest last
-    bool open = true;
-    int device = 0;
-    float* take(size_t bytes);
-    void give(size_t bytes, float* p);
-    void release(bool close);
-};
-
 // Session state: per layer tmix_x[cap,C], wkv[cap,H,N,N], cmix_x[cap,C], plus v_first[cap,C]
 // (src/gpu_model.rs:194-199, 3915-3963).  fp32 on the device, so back/load round-trips bit-exactly.
 struct State {
@@ -151,7 +138,7 @@ struct Model {
     static constexpr int kPinRing = 4;
     void* pinned = nullptr;
     size_t pinned_bytes = 0;  // bytes per ring area
-    std::shared_ptr<StatePool> state_pool = std::make_shared<StatePool>();
+    std::shared_ptr<StatePool> state_pool;
     // pinned staging of a chunk's logits on their way to the caller (at most 128 rows), with an event per piece
     static constexpr int kOutParts = 32;
     float* pinned_out = nullptr;

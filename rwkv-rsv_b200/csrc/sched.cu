@@ -177,12 +177,12 @@ int rsv_sched_new(rsv_model* mh, int64_t max_slots, int64_t chunk, int64_t max_r
         S->seq_cap = (int)max_new_cap;
         State& st = S->st;
         st.allocate(&m, max_slots);
-        RSV_CUDA(cudaMalloc(&S->slot_tok, (size_t)max_slots * 4));
-        RSV_CUDA(cudaMalloc(&S->slot_seq, (size_t)max_slots * max_new_cap * 4));
-        RSV_CUDA(cudaMalloc(&S->slot_cnt, (size_t)max_slots * 4));
-        RSV_CUDA(cudaMalloc(&S->slot_sampler, (size_t)max_slots * 32));
-        RSV_CUDA(cudaMalloc(&S->host_tok_dev, (size_t)max_rows * 4));
-        RSV_CUDA(cudaMalloc(&S->out_slot_dev, (size_t)max_rows * 4));
+        RSV_CUDA(device_malloc(&S->slot_tok, (size_t)max_slots * 4));
+        RSV_CUDA(device_malloc(&S->slot_seq, (size_t)max_slots * max_new_cap * 4));
+        RSV_CUDA(device_malloc(&S->slot_cnt, (size_t)max_slots * 4));
+        RSV_CUDA(device_malloc(&S->slot_sampler, (size_t)max_slots * 32));
+        RSV_CUDA(device_malloc(&S->host_tok_dev, (size_t)max_rows * 4));
+        RSV_CUDA(device_malloc(&S->out_slot_dev, (size_t)max_rows * 4));
         S->pinned_area = (size_t)max_rows * 8 + (size_t)max_slots * 32;
         RSV_CUDA(cudaMallocHost(&S->pinned, S->pinned_area * rsv_sched::kRing));
         for (auto& e : S->pin_ev) RSV_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

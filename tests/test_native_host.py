@@ -2,9 +2,12 @@
 import os
 import subprocess
 
+import pytest
+
 from conftest import ROOT
 
 CSRC = os.path.join(ROOT, "rwkv-rsv_b200", "csrc")
+CUDA_INCLUDE = "/usr/local/cuda/include"
 
 
 def _run(tmp_path, name, *flags):
@@ -22,3 +25,8 @@ def test_decode_launches_continue_after_one_that_failed(tmp_path):
 
 def test_logits_that_arrive_in_parts(tmp_path):
     assert "parts ok" in _run(tmp_path, "parts_to_host_check")
+
+
+@pytest.mark.skipif(not os.path.exists(CUDA_INCLUDE), reason="no CUDA headers")
+def test_memory_of_freed_states_is_given_back(tmp_path):
+    assert "device memory ok" in _run(tmp_path, "device_memory_check", "-I", CUDA_INCLUDE)

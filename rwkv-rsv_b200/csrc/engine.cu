@@ -874,10 +874,16 @@ bool rl_builds(const LinearW& W, const RowTiles& t) { return t.n == 1 && t.R <= 
 
 void launch_ln_operands(Model& m, const char* name, const LnOperandsArgs& A) {
     const int threads = std::max(kLnSumThreads, (int)round_up((size_t)(A.C / 8), 32));
-    if (threads > kLnMaxThreads) throw std::runtime_error("n_embd too large for the LayerNorm kernel");
     // few rows: a CTA per (row, output), each repeating the row statistics; as rows fill the GPU a CTA takes several outputs (more
     // than two CTAs per SM would have to wait for the predecessor's to leave)
     const int gy = std::max(1, std::min(A.nout, 2 * m.num_sms / std::max(A.R, 1)));
+    if (threads > kLnMaxThreads) {
+        LAUNCH(m, name) {
+            launch_pdl(m, ln_operands_wide_kernel, dim3(A.R + A.nseg, gy), dim3(kLnMaxThreads), 0, A);
+            check_launch("ln_operands_wide");
+        }
+        return;
+    }
     const size_t smem = (size_t)A.C * 4 * (A.rows ? 2 : 1);
     if (smem > 40 * 1024) RSV_CUDA(cudaFuncSetAttribute(ln_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 8 * kLnMaxThreads * 4));
     LAUNCH(m, name) {

@@ -142,7 +142,7 @@ struct LnOperandsArgs {
     int R, C, rt, nseg, nout;
     RlOperandOut out[7];
 };
-constexpr int kLnMaxThreads = 1024;  // n_embd up to 8192
+constexpr int kLnMaxThreads = 1024;  // n_embd up to 8192 (ln_operands_wide_kernel: any)
 constexpr int kLnSumThreads = 256;  // threads that take part in the row sums (the others only hold channels)
 // Sums of (x - c0) or (x - c0)^2 over the row in shared memory, and of the previous token's row when there is one: thread t adds
 // elements t, t + 256, ..., then shuffles, then the eight warps in order.  (The order is the same at every block size and number of rows.)
@@ -289,6 +289,144 @@ __global__ void __launch_bounds__(kLnMaxThreads) ln_operands_kernel(const __grid
             for (int i = 16; i > 0; i >>= 1) t += __shfl_xor_sync(0xffffffffu, t, i);
             if (lane == 0) A.out[o].tsum[r] = t;
         }
+}
+
+// The same for rows that do not fit the block's registers (n_embd above 8192): the row is read again from global memory (L2) for the statistics,
+// for every output's maximum and for its digits.  Same sums in the same order.  No model in use is this wide, so nothing is tuned here.
+__global__ void __launch_bounds__(kLnMaxThreads) ln_operands_wide_kernel(const __grid_constant__ LnOperandsArgs A) {
+    __shared__ float red[2][kLnSumThreads / 32], redm[32];
+    __shared__ long long redt[32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int C = A.C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    if ((int)blockIdx.x >= A.R) {  // commit CTAs
+        if (blockIdx.y == 0) {
+            const int sg = (int)blockIdx.x - A.R;
+            float* dst = A.commit_dst + (size_t)A.segs[sg].slot * C;
+            for (int i = tid; i < C; i += blockDim.x) dst[i] = __ldcg(A.commit_src + (size_t)sg * C + i);
+        }
+        return;
+    }
+    const int r = blockIdx.x, rloc = r % A.rt, rtile = r / A.rt;
+    RowMeta rm{0, 0, 0, 0};
+    if (A.rows) rm = A.rows[r];
+    const size_t row = A.row_map ? (size_t)A.row_map[r] : (size_t)r;
+    const bool shift = A.rows != nullptr, pln = shift && rm.has_prev;
+    const float *xr = A.x_in + row * C, *dr = A.delta ? A.delta + row * C : nullptr, *sr = shift ? A.shift_state + (size_t)rm.slot * C : nullptr;
+    auto load8 = [&](float (&v)[8], const float* x, const float* d, int k) {  // eight elements of a row with its pending residual
+        rl_load8(v, x + k);
+        if (d) {
+            float t[8];
+            rl_load8(t, d + k);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] += t[i];
+        }
+    };
+    if (A.x_out && blockIdx.y == 0)
+        for (int k = 8 * tid; k < C; k += 8 * blockDim.x) {
+            float v[8];
+            load8(v, xr, dr, k);
+            float4* o = reinterpret_cast<float4*>(A.x_out + row * C + k);
+            o[0] = make_float4(v[0], v[1], v[2], v[3]);
+            o[1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+    float mean[2] = {0.f, 0.f}, inv[2] = {0.f, 0.f};
+    for (int w = 0; w < (pln ? 2 : 1); ++w)
+        for (int pass = 0; pass < 2; ++pass) {
+            const float *x = xr - (size_t)w * C, *d = dr ? dr - (size_t)w * C : nullptr;
+            if (tid < kLnSumThreads) {
+                float a = 0.f;
+                for (int i = tid; i < C; i += kLnSumThreads) {
+                    const float v = __ldcg(x + i) + (d ? __ldcg(d + i) : 0.f), c = v - mean[w];
+                    a += pass ? c * c : v;
+                }
+                a = warp_sum(a);
+                if (lane == 0) red[pass][warp] = a;
+            }
+            __syncthreads();
+            float sum = 0.f;
+            for (int i = 0; i < kLnSumThreads / 32; ++i) sum += red[pass][i];
+            if (pass == 0)
+                mean[w] = sum / (float)C;
+            else
+                inv[w] = 1.0f / sqrtf(sum / (float)C + kLnEps);
+        }
+    // cur = LN of the row, and prev - cur, at channels k .. k + 7
+    auto normalised = [&](float (&x)[8], float (&xp)[8], int k) {
+        float lw[8], lb[8];
+        rl_load8(lw, A.lw + k);
+        rl_load8(lb, A.lb + k);
+        load8(x, xr, dr, k);
+        if (pln)
+            load8(xp, xr - C, dr ? dr - C : nullptr, k);
+        else if (shift)
+            rl_load8(xp, sr + k);
+        else
+            for (int i = 0; i < 8; ++i) xp[i] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            x[i] = (x[i] - mean[0]) * inv[0] * lw[i] + lb[i];
+            if (pln) xp[i] = (xp[i] - mean[1]) * inv[1] * lw[i] + lb[i];
+            xp[i] -= x[i];
+        }
+    };
+    if (shift && rm.is_last && blockIdx.y == 0)
+        for (int k = 8 * tid; k < C; k += 8 * blockDim.x) {
+            float x[8], xp[8];
+            normalised(x, xp, k);
+            float4* o = reinterpret_cast<float4*>(A.staging + (size_t)rm.seg * C + k);
+            o[0] = make_float4(x[0], x[1], x[2], x[3]);
+            o[1] = make_float4(x[4], x[5], x[6], x[7]);
+        }
+    for (int o = blockIdx.y; o < A.nout; o += gridDim.y) {
+        const RlOperandOut& O = A.out[o];
+        auto mixed = [&](float (&v)[8], int k) {
+            float xp[8];
+            normalised(v, xp, k);
+            if (O.mix) {
+                float mx[8];
+                rl_load8(mx, O.mix + k);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = v[i] + mx[i] * xp[i];
+            }
+        };
+        float am = 0.f;
+        for (int k = 8 * tid; k < C; k += 8 * blockDim.x) {
+            float v[8];
+            mixed(v, k);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(v[i]));
+        }
+        am = warp_absmax(am);
+        if (lane == 0) redm[warp] = am;
+        __syncthreads();
+        const int ex = rl_scale_exp(warp_absmax(lane < nw ? redm[lane] : 0.f)), fmt = O.fmt, kel = rl_kelems(fmt);
+        long long tot = 0;
+        for (int k0 = 0; k0 < C; k0 += 8 * blockDim.x) {  // (uniform trip count: the sums below are warp-wide)
+            const int k = k0 + 8 * tid;
+            int ts = 0;
+            if (k < C) {
+                float v[8];
+                mixed(v, k);
+                ts = rl_put8(fmt, O.img + ((size_t)rtile * O.kblocks + k / kel) * (size_t)(O.nt * 128), rloc * rl_cols(fmt), k % kel, v, rl_mult(fmt, ex));
+            }
+            if (fmt == RL_F16) continue;
+            const long long t16 = rl_group_sum(ts);
+            if (fmt == RL_I8G && k < C && (lane & 15) == 0) O.tgrp[(size_t)r * O.kblocks + k / 128] = (float)t16;
+            tot += t16 + __shfl_xor_sync(0xffffffffu, t16, 16);
+        }
+        if (lane == 0) redt[warp] = tot;
+        __syncthreads();
+        if (tid == 0) {
+            O.xscale[r] = rl_xscale(fmt, ex);
+            if (fmt == RL_I8) {
+                long long t = 0;
+                for (int i = 0; i < nw; ++i) t += redt[i];
+                O.tsum[r] = t;
+            }
+        }
+        __syncthreads();  // redm and redt are written again
+    }
 }
 
 // ---- operands of activations another kernel left in fp32 ----------------------------------------------------------------------

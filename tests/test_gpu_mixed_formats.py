@@ -81,3 +81,12 @@ def test_padding_of_the_last_k_block(tmp_path):
         for m in ("att.receptance", "att.key", "att.value", "att.output"):
             _take(out, src["int8"], f"blocks.{i}.{m}")
     _check(write_safetensors(os.path.join(str(tmp_path), "mixed.st"), out), (64, 2, 3, 5, 17, 130, 2, 33), shape["vocab"])
+
+
+@pytest.mark.parametrize("quant", [1, 2])
+def test_rows_wider_than_one_block(tmp_path, quant):
+    """n_embd above 8192: a row no longer fits the LayerNorm kernel's block of 1024 threads with eight channels each."""
+    shape = dict(n_layer=1, n_embd=8320, n_head=130, ffn_hidden=256, vocab=64, w_mid=16, a_mid=16, v_mid=16, g_mid=16)
+    path = rsv.write_synthetic(os.path.join(str(tmp_path), "wide.st"), "tiny", seed=0, quant=quant, **shape)
+    _check(path, (1, 3, 40), shape["vocab"])
+    os.remove(path)

@@ -443,9 +443,6 @@ __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* 
     pdl_wait();
     float v[8];
     rl_load8(v, x + (size_t)r * ldx + (k0 < K ? k0 : 0));
-    if (k0 >= K)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = 0.f;
     float am = 0.f;
 #pragma unroll 1
     for (int i = threadIdx.x; i < parts; i += kOpThreads) am = fmaxf(am, __ldcg(amax + (size_t)r * parts + i));
@@ -455,7 +452,13 @@ __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* 
     am = redm[lane & (kOpThreads / 32 - 1)];
     const int ex = rl_scale_exp(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(am)))), kel = rl_kelems(O.fmt);
     int ts = 0;
-    if (k0 < O.kblocks * kel) ts = rl_put8(O.fmt, rl_tile(O, rt, r, k0 / kel), (r % rt) * rl_cols(O.fmt), k0 % kel, v, rl_mult(O.fmt, ex));
+    if (k0 < K) ts = rl_put8(O.fmt, rl_tile(O, rt, r, k0 / kel), (r % rt) * rl_cols(O.fmt), k0 % kel, v, rl_mult(O.fmt, ex));
+    else if (O.fmt == RL_F16 && k0 < O.kblocks * 64) {  // (K of int8 weights is whole blocks)
+        uint8_t* col = rl_tile(O, rt, r, k0 / 64) + (r % rt) * 2 * 128;
+        const int chunk = (k0 % 64) / 8, n0 = (r % rt) * 2;
+        *reinterpret_cast<uint4*>(col + ((chunk ^ (n0 & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(col + 128 + ((chunk ^ ((n0 + 1) & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+    }
     if (O.fmt != RL_F16) {
         const long long t16 = rl_group_sum(ts);
         if (O.fmt == RL_I8G) {

@@ -386,6 +386,14 @@ std::unique_ptr<Model> Model::load(const std::string& path, int device) {
         L.g1 = ld.lowrank(p + "att.g1", C, c.g_mid);
         L.g2 = ld.lowrank(p + "att.g2", c.g_mid, C);
     }
+    auto same_formats = [&](const LayerW& a, const LayerW& b) {
+        const auto x = a.big(), y = b.big();
+        bool same = true;
+        for (size_t i = 0; i < x.size(); ++i) same = same && x[i]->wtype == y[i]->wtype && x[i]->row_scaled() == y[i]->row_scaled();
+        return same;
+    };
+    for (int i = 0; i < c.n_layer; ++i)
+        if (std::none_of(m->format_layers.begin(), m->format_layers.end(), [&](int j) { return same_formats(m->layers[j], m->layers[i]); })) m->format_layers.push_back(i);
     m->pinned_bytes = 1 << 18;
     RSV_CUDA(cudaMallocHost(&m->pinned, m->pinned_bytes * Model::kPinRing));
     for (int i = 0; i < Model::kPinRing; ++i) RSV_CUDA(cudaEventCreateWithFlags(&m->pin_ev[i], cudaEventDisableTiming));
@@ -915,8 +923,8 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     if (R == 0) return;
     RSV_CUDA(cudaSetDevice(device));
     bool per_group = false, int8 = false;
-    for (const LayerW& L : layers)
-        for (const LinearW* W : {&L.Wr, &L.Wk, &L.Wv, &L.Wo, &L.Wfk, &L.Wfv}) {
+    for (int i : format_layers)
+        for (const LinearW* W : layers[i].big()) {
             per_group = per_group || rl_fmt(*W) == RL_I8G;
             int8 = int8 || rl_fmt(*W) == RL_I8;
         }
@@ -944,8 +952,8 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     };
     LayerOps ops;
     size_t layer_bytes = 0;
-    for (const LayerW& L : layers) {
-        carve_layer(L, ops);
+    for (int i : format_layers) {
+        carve_layer(layers[i], ops);
         layer_bytes = std::max(layer_bytes, cv.used);
     }
     cv.used = layer_bytes;
@@ -1214,7 +1222,7 @@ bool Model::stream_available() {
     if (format_of(head) < 0) return fail("int8 head without scales");
     const int fmt = layers.empty() ? 0 : format_of(layers[0].Wr);
     for (const LayerW& Lw : layers)
-        for (const LinearW* W : {&Lw.Wr, &Lw.Wk, &Lw.Wv, &Lw.Wo, &Lw.Wfk, &Lw.Wfv})
+        for (const LinearW* W : Lw.big())
             if (format_of(*W) != fmt || fmt < 0) return fail("the big matrices of the layers differ in their weight format, or an int8 matrix has no scales");
     // the layout (row ownership, chunks, shared memory, every capacity of the kernel's tables) is pure arithmetic on the shape
     const DsShape shp{L, C, F, V, H, cfg.w_mid, cfg.a_mid, cfg.v_mid, cfg.g_mid, fmt, format_of(head)};

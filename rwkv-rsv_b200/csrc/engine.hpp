@@ -3,6 +3,7 @@
 // (src/gpu_model.rs:401-546, 868-1803, 1968-2543, 2911-3568) and its CudaBackend
 // (src/backend_cuda.rs).  One host thread drives one Model; all work goes to the model's stream.
 #pragma once
+#include <array>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -48,6 +49,7 @@ struct LayerW {
     LinearW Wr, Wk, Wv, Wo, Wfk, Wfv;
     LinearW w1, a1, v1, g1;  // rank-space projections, stored [mid, C] fp16
     LinearW w2, a2, v2, g2;  // back-projections, stored [C, mid] fp16
+    std::array<const LinearW*, 6> big() const { return {&Wr, &Wk, &Wv, &Wo, &Wfk, &Wfv}; }  // the matrices that have any format
 };
 
 struct Workspace {
@@ -130,6 +132,7 @@ struct Model {
     float *ln0_w = nullptr, *ln0_b = nullptr, *ln_out_w = nullptr, *ln_out_b = nullptr;
     LinearW head;
     std::vector<LayerW> layers;
+    std::vector<int> format_layers;  // the first layer of every combination of weight formats (one, as a rule)
     std::vector<void*> allocs;  // every weight allocation, freed in the destructor
     size_t weight_bytes = 0;
     Workspace ws;

@@ -740,11 +740,16 @@ struct RlReq {
 constexpr size_t kRlRingMax = 196 * 1024;  // stages of the persistent kernel, which has its SM to itself
 constexpr size_t kRlHalfSm = 109 * 1024;  // dynamic shared memory of a CTA that leaves room for a second one on its SM
 
+// Bytes of shared memory in which the CTAs of a split tile receive each other's partial sums.
+size_t rl_recv_bytes(int rt, int split) { return (size_t)split * ((rt + split - 1) / split) * kRlTileM * 8; }
 // How many CTAs share a tile's K.  The step's launches are short (few tiles, weights prefetched behind the previous kernel), so a
-// launch wants about one CTA per half SM and few K blocks per CTA, but no second wave.
-int rl_split(const Model& m, int jobs, int kb_min, int kb_max) {
+// launch wants about one CTA per half SM and few K blocks per CTA, but no second wave.  A split tile of more than 108 rows (fp16) takes a
+// whole SM, for the partial sums it receives; counted as half of one, r, k, v and rank projections of 256 rows (132 tiles, 2560 channels)
+// went out as two waves of 264 CTAs in 51 us, 33 unsplit.
+int rl_split(const Model& m, int jobs, int kb_min, int kb_max, int rt) {
+    auto slots = [&](int s) { return rl_recv_bytes(rt, s) + 1024 <= kRlHalfSm ? 2 * m.num_sms : m.num_sms; };
     int s = 1;
-    while (s < kRlMaxSplit && 2 * s <= kb_min && jobs * 2 * s <= 2 * m.num_sms && kb_max / s > 5) s *= 2;
+    while (s < kRlMaxSplit && 2 * s <= kb_min && jobs * 2 * s <= slots(2 * s) && kb_max / s > 5) s *= 2;
     return s;
 }
 
@@ -830,7 +835,7 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
     L.nt8 = t.nt8;
     L.nt16 = t.nt16;
     L.status = m.ws.status;
-    L.split = build ? 1 : rl_split(m, jobs, kb_min, kb_max);  // a kernel that builds its operands has to see whole rows
+    L.split = build ? 1 : rl_split(m, jobs, kb_min, kb_max, t.rt);  // a kernel that builds its operands has to see whole rows
     while ((1 << L.log_split) < L.split) ++L.log_split;
     L.f16_halves = grouped || row8;
     int nk = 0;
@@ -860,7 +865,7 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
         return;
     }
     const size_t stage = kRlABytes + (build ? 0 : (size_t)nt_max * 128), bbuf = build ? (size_t)nk * nt_max * 128 : 0, tg = grouped ? round_up((size_t)nk * t.rt * 4, 16) : 0;
-    const size_t recv = (size_t)L.split * ((t.rt + L.split - 1) / L.split) * kRlTileM * 8;  // partial sums reuse the ring
+    const size_t recv = L.split > 1 || grouped ? rl_recv_bytes(t.rt, L.split) : 0;  // partial sums reuse the ring
     int stages = std::min(nk, kRlMaxStages);
     while (stages > 2 && stages * stage + bbuf + tg + 1024 > kRlHalfSm) --stages;
     L.ring = (int)std::max(stages * stage, round_up(recv, 1024));

@@ -15,7 +15,8 @@
 // rows), so that a layer with few tiles still has every SM streaming and no partial sum goes through global memory (the kernel this
 // one replaces cut tiles between persistent CTAs and paid a global round trip, an atomic and a serial sum per cut tile).  A CTA takes
 // at most half an SM (<= 113 KB shared memory, <= 256 TMEM columns): two are resident, one loads while the other finishes, and the
-// next kernel of the step becomes resident early and requests its weights before the dependency wait.
+// next kernel of the step becomes resident early and requests its weights before the dependency wait.  (The exception: split tiles of
+// more than 108 rows of fp16 weights, whose partial sums take up to 128 KB; one of them is resident.)
 // What bounds it: at few rows the chain operand tiles (L2) -> products -> exchange -> store behind the dependency wait, the weights
 // are there already; at 64 rows the operand tiles' L2 traffic as well (a 128-row tile re-reads them all).
 //

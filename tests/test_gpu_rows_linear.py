@@ -51,3 +51,11 @@ def test_step_sizes_agree_with_the_cpu_path(tiny_paths, name):
         # fp32 through the layers in another summation order: a few ulps of the logits' scale per layer
         assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n
         assert np.abs(b.state_back() - o.state_back()).max() <= 1e-4 * max(1.0, float(np.abs(o.state_back()).max()))
+
+
+# fp16 tiles of up to 108 rows share an SM when K is split, larger ones have it to themselves; m = 2048: few tiles, which are split; 9600: as many
+# tiles as a launch of one CTA per SM holds, which are not; 704: a tile of fewer than 16 K blocks, which no persistent CTA takes
+@pytest.mark.parametrize("rows", [210, 216, 217, 256])
+@pytest.mark.parametrize("m,k", [(2048, 2560), (9600, 1536), (9600, 704)])
+def test_linear_fp16_tiles_that_need_a_whole_sm(rows, m, k):
+    test_linear_tile_edges(rows, m, k, False)

@@ -231,5 +231,5 @@ def test_7b_int8_matches_oracle():
 
 def test_3b_per_group_int8_matches_oracle():
     # the reference's own container (one scale and zero per row and group of 128 weights) at the 3B shape: the one-launch decode
-    # kernel rescales every group inside its multiply loop; prefill runs on the weight-streaming SIMT kernel
+    # kernel rescales every group inside its multiply loop; prefill runs on the tensor cores with a fresh accumulator per group
     _short_parity(_checkpoint("3b", "int8g"), n_prompt=6, n_stream=16, chunk_tokens=64)

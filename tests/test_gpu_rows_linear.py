@@ -31,11 +31,39 @@ def test_linear_tile_edges(rows, m, k, int8):
     assert np.all(np.abs(got - want) <= bound + 1e-30), float((np.abs(got - want) / bound).max())
 
 
-# enough tiles that K is not split and two CTAs share a tile of 256 weight rows: full and ragged row tiles, an odd number of 128-row
-# weight tiles, the last of them partly or wholly past the end
+# several row tiles of few K blocks, one CTA per tile (int8: K unsplit; fp16: split over two): full and ragged row tiles, an odd number of weight
+# tiles, a partial last one
 @pytest.mark.parametrize("rows,m,k,int8", [(513, 2560, 1024, True), (640, 2688, 384, True), (513, 2560, 704, False), (577, 2570, 640, False)])
-def test_linear_tiles_of_a_cta_pair(rows, m, k, int8):
+def test_linear_several_row_tiles(rows, m, k, int8):
     test_linear_tile_edges(rows, m, k, int8)
+
+
+# The persistent kernel: several row tiles, more tiles than SMs (so that K is not split), 16 K blocks and more, int8 or fp16 tiles of more than 64
+# rows.  129: three tiles of 43 rows (no multiple of 4); 201: the last tile is one row shorter; 4033: the last tile is a single row; 10250
+# and 9640 weight rows: a partial last weight tile; 257, 513 and 1025 rows of fp16: ragged last tiles of 85, 101 and 113 rows
+@pytest.mark.parametrize("rows,m,k,int8", [(129, 10240, 2560, True), (201, 10240, 2560, True), (4033, 384, 2048, True), (257, 10250, 1088, False), (513, 10250, 1088, False),
+                                           (1025, 9640, 1024, False)])
+def test_linear_persistent_tiles(rows, m, k, int8):
+    test_linear_tile_edges(rows, m, k, int8)
+
+
+# The same kernel as a step uses it: int8 next to fp16 problems in one launch, rank projections that are partial weight tiles, the maxima of
+# ffn.key's outputs (8200: its last weight tile has eight rows), row tiles of 44, 51, 65 and 86 rows
+@pytest.mark.parametrize("quant,ffn", [(1, 8192), (0, 8200)])
+def test_step_of_persistent_tiles_agrees_with_the_cpu_path(tmp_path, quant, ffn):
+    p = rsv.write_synthetic(str(tmp_path / "m.st"), "tiny", seed=0, quant=quant, n_layer=1, n_embd=2048, n_head=32, ffn_hidden=ffn, vocab=300, w_mid=24, a_mid=40,
+                            v_mid=8, g_mid=72)
+    b, o = rsv.ModelBuilder(p).build(), orc.OracleModel(p)
+    for n in (130, 201, 257):
+        toks = np.random.default_rng(n).integers(0, 300, size=n).astype(np.uint32)
+        b.reset()
+        o.reset()
+        lg, want = b.infer_seq(toks), o.forward(toks)
+        # fp32 through the layer in another summation order: a few ulps of the logits' scale
+        assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n
+        assert np.abs(b.state_back() - o.state_back()).max() <= 1e-4 * max(1.0, float(np.abs(o.state_back()).max()))
+    b.state.close()
+    b.model.close()
 
 
 @pytest.mark.parametrize("name", ["fp16", "int8", "int8g"])

@@ -31,16 +31,14 @@ struct CudaError : std::runtime_error {
 
 enum WType : int { W_F16 = 0, W_INT8 = 1 };
 
-// Epilogues of the weight-streaming linear kernel.  `acc` is the fp32 dot product for (row r, output m).
+// Epilogues of the linear layers.  `acc` is the dot product for (row r, output m).
 enum Epi : int {
     EPI_STORE = 0,         // y = acc
-    EPI_ADD = 1,           // y += acc                                   (residual)
-    EPI_RELU2 = 2,         // y = max(acc,0)^2                           (ffn.key)
-    EPI_TANH = 3,          // y = tanh(acc)                              (decay adapter, rank space)
-    EPI_SIGMOID = 4,       // y = sigmoid(acc)                           (gate adapter, rank space)
-    EPI_DECAY = 5,         // y = exp(-sigmoid(acc + bias[m]) / sqrt(e)) (w)
-    EPI_SIGMOID_BIAS = 6,  // y = sigmoid(acc + bias[m])                 (a)
-    EPI_VLERP = 7,         // y = y + sigmoid(acc + bias[m]) * (aux[r,m] - y)   (v <- lerp(v, v_first, gate))
+    EPI_RELU2 = 1,         // y = max(acc,0)^2                           (ffn.key)
+    EPI_TANH = 2,          // y = tanh(acc)                              (decay adapter, rank space)
+    EPI_SIGMOID = 3,       // y = sigmoid(acc)                           (gate adapter, rank space)
+    EPI_DECAY = 4,         // y = exp(-sigmoid(acc + bias[m]) / sqrt(e)) (w)
+    EPI_SIGMOID_BIAS = 5,  // y = sigmoid(acc + bias[m])                 (a, v gate)
 };
 
 // Row r of a packed step: which session slot it belongs to and how it chains to its neighbours.

@@ -586,21 +586,8 @@ void Model::upload_plan(const StepPlan& plan) {
 // ------------------------------------------------------------------------------------------------
 namespace {
 
-struct LinReq {
-    const LinearW* W;
-    const float* x;
-    int ldx;
-    float* y;
-    int ldy;
-    int epi;
-    const float* bias = nullptr;
-    const float* aux = nullptr;
-    int ldaux = 0;
-    float* y2 = nullptr;
-};
-
 template <int RT>
-void launch_linear_rt(Model& m, const LinGroup& g, int nblk, int R, size_t smem) {
+void launch_linear_rt(Model& m, const LinProb& P, int nblk, int R, size_t smem) {
     static bool configured[8] = {false};
     int dev = m.device & 7;
     if (!configured[dev]) {
@@ -608,58 +595,35 @@ void launch_linear_rt(Model& m, const LinGroup& g, int nblk, int R, size_t smem)
         configured[dev] = true;
     }
     dim3 grid(nblk, (R + RT - 1) / RT);
-    linear_rows_kernel<RT><<<grid, kLinWarps * 32, smem, m.stream>>>(g, R);
+    linear_rows_kernel<RT><<<grid, kLinWarps * 32, smem, m.stream>>>(P, R);
     check_launch("linear_rows");
 }
 
-void run_linear_simt(Model& m, const char* name, const LinReq* reqs, int n, int R) {
-    LinGroup g;
-    memset(&g, 0, sizeof(g));
-    g.n = n;
-    int total_rows = 0, kmax = 0;
-    bool any_i8 = false;
-    for (int i = 0; i < n; ++i) {
-        total_rows += reqs[i].W->M;
-        kmax = std::max(kmax, reqs[i].W->K);
-        any_i8 = any_i8 || reqs[i].W->wtype == W_INT8;
-    }
+void run_linear_simt(Model& m, const char* name, const LinearW& W, const float* x, float* y, int R) {
+    LinProb P;
+    memset(&P, 0, sizeof(P));
+    P.w = W.w;
+    P.sz = W.sz;
+    P.x = x;
+    P.y = y;
+    P.M = W.M;
+    P.K = W.K;
+    P.wtype = W.wtype;
     // rows per CTA: aim for a few waves over 148 SMs, but amortise the x staging
     const int unit = kLinWarps * kLinWR;
-    int rpb = (total_rows / (148 * 4)) / unit * unit;
-    rpb = std::min(std::max(rpb, unit), 8 * unit);
-    int blk = 0;
-    for (int i = 0; i < n; ++i) {
-        const LinReq& q = reqs[i];
-        LinProb& P = g.p[i];
-        P.w = q.W->w;
-        P.sz = q.W->sz;
-        P.x = q.x;
-        P.y = q.y;
-        P.y2 = q.y2;
-        P.bias = q.bias;
-        P.aux = q.aux;
-        P.M = q.W->M;
-        P.K = q.W->K;
-        P.ldx = q.ldx;
-        P.ldy = q.ldy;
-        P.ldaux = q.ldaux;
-        P.wtype = q.W->wtype;
-        P.epi = q.epi;
-        P.rows_per_blk = rpb;
-        P.blk0 = blk;
-        blk += (P.M + rpb - 1) / rpb;
-    }
-    auto smem_for = [&](int rt) { return (size_t)rt * kmax * 4 + (any_i8 ? (size_t)rt * (kmax / 16) * 4 : 0); };
+    P.rows_per_blk = std::min(std::max((W.M / (148 * 4)) / unit * unit, unit), 8 * unit);
+    const int blk = (W.M + P.rows_per_blk - 1) / P.rows_per_blk;
+    auto smem_for = [&](int rt) { return (size_t)rt * W.K * 4 + (W.wtype == W_INT8 ? (size_t)rt * (W.K / 16) * 4 : 0); };
     int rt = R >= 4 ? 4 : (R >= 2 ? 2 : 1);
     while (rt > 1 && smem_for(rt) > 200 * 1024) rt >>= 1;
     if (smem_for(rt) > 200 * 1024) throw std::runtime_error("linear: inner dimension too large for the shared-memory tile");
     LAUNCH(m, name) {
         if (rt == 4)
-            launch_linear_rt<4>(m, g, blk, R, smem_for(4));
+            launch_linear_rt<4>(m, P, blk, R, smem_for(4));
         else if (rt == 2)
-            launch_linear_rt<2>(m, g, blk, R, smem_for(2));
+            launch_linear_rt<2>(m, P, blk, R, smem_for(2));
         else
-            launch_linear_rt<1>(m, g, blk, R, smem_for(1));
+            launch_linear_rt<1>(m, P, blk, R, smem_for(1));
     }
 }
 
@@ -1645,8 +1609,7 @@ void engine_op_linear(Model& m, int path, int wtype, const void* w_host, const u
             RlReq q = {&W, &A.out[0], dy, M, EPI_STORE};
             run_rows_linear(m, "op_linear", &q, 1, t);
         } else {
-            LinReq q = {&W, dx, K, dy, M, EPI_STORE};
-            run_linear_simt(m, "op_linear_simt", &q, 1, R);
+            run_linear_simt(m, "op_linear_simt", W, dx, dy, R);
         }
         RSV_CUDA(cudaMemcpyAsync(y_host, dy, (size_t)R * M * 4, cudaMemcpyDeviceToHost, m.stream));
         m.check_status();

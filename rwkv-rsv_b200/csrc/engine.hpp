@@ -122,8 +122,6 @@ struct StepPlan {
     bool multi_row_segments = false;
 };
 
-enum class PostOp { None, Argmax };
-
 struct Model {
     int device = 0;
     cudaStream_t stream = nullptr;

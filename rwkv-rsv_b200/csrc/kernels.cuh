@@ -90,70 +90,31 @@ __global__ void commit_shift_kernel(const float* __restrict__ staging, const Seg
 }
 
 // ------------------------------------------------------------------------------------------------
-// Weight-streaming linear layer, SIMT form: y[r, m] = epi( sum_k W[m,k] * x[r,k] ).
-// Stands in for gemv_f16, gemv_variant(_mb), gemv_(int8_)rkv_stage1(_batch), gemv_lowrank_chain4(_batch),
-// rwkv_dequant_int8 + GEMM + rwkv_gemm_epilogue (src/backend_cuda.rs:1421-1498, 1665-1986, 2772-3554,
-// 4195-4227, 4580-4633).  Differences by design: fp32 accumulation (the reference accumulates in half2),
+// Weight-streaming linear layer, SIMT form: y[r, m] = sum_k W[m,k] * x[r,k]; the second implementation behind rsv_op_linear, in
+// fp32 throughout (the forward path runs on rows_linear.cuh and decode_stream.cuh).
+// Stands in for gemv_f16, gemv_variant(_mb) and rwkv_dequant_int8 + GEMM (src/backend_cuda.rs:1421-1498, 3229-3554, 4195-4227).
+// Differences by design: fp32 accumulation (the reference accumulates in half2),
 // the int8 dequant w = scale*q + zero (src/model.rs:234-252) is applied per group of 128 in factored
 // form  sum_g [ scale_g * sum_{k in g} q_k x_k  +  zero_g * sum_{k in g} x_k ],  and one warp owns an
-// output element so its reduction order is fixed.
-// A launch runs up to 8 independent problems (r/k/v plus the four rank-space projections of a layer
-// go out together).  Every weight byte is read once per tile of RT rows.
+// output element so its reduction order is fixed.  Every weight byte is read once per tile of RT rows.
 // ------------------------------------------------------------------------------------------------
 constexpr int kLinWarps = 8;
 constexpr int kLinWR = 2;  // output rows a warp carries at a time
 struct LinProb {
     const void* w;       // fp16 [M,K] or u8 [M,K]
     const uint32_t* sz;  // int8 only: [M, K/128] words, fp16 scale (low half) | fp16 zero (high half)
-    const float* x;      // [R, ldx]
-    float* y;            // [R, ldy]
-    float* y2;           // optional second copy of the output (EPI_STORE only)
-    const float* bias;   // [M]     (EPI_DECAY, EPI_SIGMOID_BIAS, EPI_VLERP)
-    const float* aux;    // [R, ldaux] (EPI_VLERP)
-    int M, K, ldx, ldy, ldaux, wtype, epi;
+    const float* x;      // [R, K]
+    float* y;            // [R, M]
+    int M, K, wtype;
     int rows_per_blk;  // output rows per CTA, multiple of kLinWarps*kLinWR
-    int blk0;          // first blockIdx.x of this problem
 };
-struct LinGroup {
-    LinProb p[8];
-    int n;
-};
-
-__device__ __forceinline__ void lin_epilogue(const LinProb& P, int r, int m, float acc) {
-    float* yp = P.y + (size_t)r * P.ldy + m;
-    switch (P.epi) {
-        case EPI_STORE:
-            *yp = acc;
-            if (P.y2) P.y2[(size_t)r * P.ldy + m] = acc;
-            break;
-        case EPI_ADD: *yp += acc; break;
-        case EPI_RELU2: {
-            float t = fmaxf(acc, 0.f);
-            *yp = t * t;
-            break;
-        }
-        case EPI_TANH: *yp = tanhf(acc); break;
-        case EPI_SIGMOID: *yp = sigmoidf_(acc); break;
-        case EPI_DECAY: *yp = expf(sigmoidf_(acc + P.bias[m]) * kDecayScale); break;
-        case EPI_SIGMOID_BIAS: *yp = sigmoidf_(acc + P.bias[m]); break;
-        case EPI_VLERP: {
-            float v = *yp;
-            float gate = sigmoidf_(acc + P.bias[m]);
-            *yp = v + gate * (P.aux[(size_t)r * P.ldaux + m] - v);
-            break;
-        }
-    }
-}
 
 // x tile in shared memory: element k of row rr lives in float4 slot [(rr*JPC + j) * nchunk + c] with
 // c = k / CH (the chunk one lane consumes per step), j = (k % CH) / 4.  Consecutive lanes read
 // consecutive float4 slots, so the reads are bank-conflict free.
 template <int RT>
-__global__ void __launch_bounds__(kLinWarps * 32) linear_rows_kernel(const __grid_constant__ LinGroup g, int R) {
+__global__ void __launch_bounds__(kLinWarps * 32) linear_rows_kernel(const __grid_constant__ LinProb P, int R) {
     extern __shared__ float4 smem4[];
-    int pi = 0;
-    while (pi + 1 < g.n && (int)blockIdx.x >= g.p[pi + 1].blk0) ++pi;
-    const LinProb& P = g.p[pi];
     const int K = P.K, M = P.M;
     const bool i8 = P.wtype == W_INT8;
     const int CH = i8 ? 16 : 8, JPC = CH / 4;
@@ -166,7 +127,7 @@ __global__ void __launch_bounds__(kLinWarps * 32) linear_rows_kernel(const __gri
     for (int idx = threadIdx.x; idx < RT * k4; idx += kLinWarps * 32) {
         const int rr = idx / k4, f = idx - rr * k4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r0 + rr < R) v = *reinterpret_cast<const float4*>(P.x + (size_t)(r0 + rr) * P.ldx + (size_t)f * 4);
+        if (r0 + rr < R) v = *reinterpret_cast<const float4*>(P.x + (size_t)(r0 + rr) * K + (size_t)f * 4);
         xs[(rr * JPC + (f % JPC)) * nchunk + f / JPC] = v;
     }
     __syncthreads();
@@ -185,7 +146,7 @@ __global__ void __launch_bounds__(kLinWarps * 32) linear_rows_kernel(const __gri
     }
 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int mblk = ((int)blockIdx.x - P.blk0) * P.rows_per_blk;
+    const int mblk = (int)blockIdx.x * P.rows_per_blk;
     const int mend = min(M, mblk + P.rows_per_blk);
     for (int m0 = mblk + wid * kLinWR; m0 < mend; m0 += kLinWarps * kLinWR) {
         float acc[kLinWR][RT];
@@ -289,7 +250,7 @@ __global__ void __launch_bounds__(kLinWarps * 32) linear_rows_kernel(const __gri
 #pragma unroll
             for (int rr = 0; rr < RT; ++rr) {
                 const float v = warp_sum(acc[a][rr]);
-                if (lane == 0 && (a == 0 || has1) && r0 + rr < R) lin_epilogue(P, r0 + rr, m0 + a, v);
+                if (lane == 0 && (a == 0 || has1) && r0 + rr < R) P.y[(size_t)(r0 + rr) * M + m0 + a] = v;
             }
     }
 }

@@ -31,7 +31,7 @@ def test_linear_tile_edges(rows, m, k, int8):
     assert np.all(np.abs(got - want) <= bound + 1e-30), float((np.abs(got - want) / bound).max())
 
 
-# several row tiles of few K blocks, one CTA per tile (int8: K unsplit; fp16: split over two): full and ragged row tiles, an odd number of weight
+# several row tiles of few K blocks, a CTA or (the first fp16 shape) a pair that splits K per tile: full and ragged row tiles, an odd number of weight
 # tiles, a partial last one
 @pytest.mark.parametrize("rows,m,k,int8", [(513, 2560, 1024, True), (640, 2688, 384, True), (513, 2560, 704, False), (577, 2570, 640, False)])
 def test_linear_several_row_tiles(rows, m, k, int8):

@@ -801,12 +801,8 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
     L.status = m.ws.status;
     L.split = build ? 1 : rl_split(m, jobs, kb_min, kb_max, t.rt);  // a kernel that builds its operands has to see whole rows
     while ((1 << L.log_split) < L.split) ++L.log_split;
-    L.f16_halves = grouped || row8;
     int nk = 0;
-    for (int i = 0; i < n; ++i) {
-        const int sk = L.p[i].fmt == RL_F16 && L.f16_halves ? std::min(L.split, 2) : L.split;
-        nk = std::max(nk, (L.p[i].kblocks + sk - 1) / sk);
-    }
+    for (int i = 0; i < n; ++i) nk = std::max(nk, (L.p[i].kblocks + L.split - 1) / L.split);
     // Several full row tiles that fill the GPU without splitting K: the persistent kernel.  A tile of fewer than 16 K blocks is all
     // epilogue (the rank back-projections: 30 us at 512 rows with a CTA per tile, 34 persistent), and fp16 tiles of 64 rows leave half of
     // the matrix instruction's columns out.

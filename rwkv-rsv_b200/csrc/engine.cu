@@ -634,18 +634,42 @@ void run_linear_simt(Model& m, const char* name, const LinearW& W, const float* 
 // weights pass through L2 half as often.
 struct RowTiles {
     int R = 0, rt = 0, n = 0, nt8 = 0, nt16 = 0;
+    bool turns = false;  // cut for the persistent kernel (fit_turns): K is not split
     int nt(int fmt) const { return fmt == RL_F16 ? nt16 : nt8; }
     size_t image_bytes(int fmt, int K) const { return (size_t)n * ((K + rl_kelems(fmt) - 1) / rl_kelems(fmt)) * nt(fmt) * 128; }
 };
-RowTiles row_tiles(int R, bool per_group, bool int8) {
+RowTiles cut_rows(int R, int n) {
     RowTiles t;
     t.R = R;
-    const int most = per_group ? kRlMaxRowsG : int8 || R <= kRlMaxRowsF ? kRlMaxRows : kRlMaxRowsF;
-    t.n = (R + most - 1) / most;
-    t.rt = (R + t.n - 1) / t.n;
+    t.rt = (R + n - 1) / n;
+    t.n = (R + t.rt - 1) / t.rt;
     t.nt8 = (int)round_up((size_t)t.rt * rl_cols(RL_I8), 16);
     t.nt16 = (int)round_up((size_t)t.rt * rl_cols(RL_F16), 16);
     return t;
+}
+RowTiles row_tiles(int R, bool per_group, bool int8) {
+    const int most = per_group ? kRlMaxRowsG : int8 || R <= kRlMaxRowsF ? kRlMaxRows : kRlMaxRowsF;
+    return cut_rows(R, (R + most - 1) / most);
+}
+// The row tiles of a launch with more tiles than SMs, which the persistent kernel takes in turns: `mt` weight tiles, at least `kb` blocks of K, fmt
+// the format of most of them.  A turn lasts as long as its K blocks take to arrive (an SM draws about 70 bytes per cycle from L2: 16 KB of weights and 128
+// bytes per operand column), so the cut with the least turns x (columns + 128) is taken, the largest tiles among equals.  512 rows, 10240 -> 2560
+// channels: 160 tiles of 64 rows are two turns on 148 SMs and took 59 us, 260 tiles of 40 rows are two shorter ones, 49 us; 2560 -> 2560: 24 and 17 us.  fp16
+// layers of 512 rows leave the kernel with a CTA per 64-row tile this way.  Fewer than 32 rows would leave the matrix instruction too narrow.
+RowTiles fit_turns(const RowTiles& t, int mt, int kb, int fmt, int sms) {
+    if (t.n < 2 || fmt == RL_I8G || mt * t.n <= sms || kb < 16) return t;
+    const int cols = rl_cols(fmt), most = fmt == RL_F16 ? kRlMaxRowsF : kRlMaxRows;
+    RowTiles best = t;
+    long long cost = -1;
+    for (int n = (t.R + most - 1) / most; n <= (t.R + 31) / 32; ++n) {
+        const RowTiles c = cut_rows(t.R, n);
+        const long long turns = ((long long)mt * c.n + sms - 1) / sms, now = turns * (round_up((size_t)c.rt * cols, 16) + 128);
+        if (cost >= 0 && now >= cost) continue;
+        cost = now;
+        best = c;
+    }
+    best.turns = true;
+    return best;
 }
 int rl_fmt(const LinearW& W) { return W.wtype != W_INT8 ? RL_F16 : W.row_scaled() ? RL_I8 : RL_I8G; }
 
@@ -799,14 +823,15 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
     L.nt8 = t.nt8;
     L.nt16 = t.nt16;
     L.status = m.ws.status;
-    L.split = build ? 1 : rl_split(m, jobs, kb_min, kb_max, t.rt);  // a kernel that builds its operands has to see whole rows
+    L.split = build || t.turns ? 1 : rl_split(m, jobs, kb_min, kb_max, t.rt);  // a kernel that builds its operands has to see whole rows
     while ((1 << L.log_split) < L.split) ++L.log_split;
     int nk = 0;
     for (int i = 0; i < n; ++i) nk = std::max(nk, (L.p[i].kblocks + L.split - 1) / L.split);
     // Several full row tiles that fill the GPU without splitting K: the persistent kernel.  A tile of fewer than 16 K blocks is all
     // epilogue (the rank back-projections: 30 us at 512 rows with a CTA per tile, 34 persistent), and fp16 tiles of 64 rows leave half of
-    // the matrix instruction's columns out.
-    if (!build && !grouped && t.n > 1 && L.split == 1 && kb_min >= 16 && (row8 || t.rt > kRlMaxRows)) {
+    // the matrix instruction's columns out.  One row tile and more weight tiles than two CTAs per SM take at once (the vocabulary head: 512 of them, 336 MB):
+    // the second set of CTAs would start its ring from nothing; 3 rows 75 us, persistent 58, 64 rows 83 and 63.
+    if (!build && !grouped && (t.turns || (L.split == 1 && kb_min >= 16 && (t.n > 1 ? row8 || t.rt > kRlMaxRows : jobs > 2 * m.num_sms)))) {
         const size_t st = kRlABytes + (size_t)nt_max * 128;
         L.nt_max = nt_max;
         L.ring = (int)(std::min<size_t>(kRlMaxStages, kRlRingMax / st) * st);
@@ -819,7 +844,7 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
             configured[m.device & 15] = true;
         }
         LAUNCH(m, name) {
-            launch_pdl(m, rows_linear_persistent_kernel, dim3(std::min(jobs, m.num_sms)), dim3(kRlThreads), bytes, L, jobs);
+            launch_pdl(m, rows_linear_persistent_kernel, dim3(std::min(jobs, m.num_sms)), dim3(kRlPThreads), bytes, L, jobs);
             check_launch("rows_linear_persistent");
         }
         return;
@@ -895,6 +920,12 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         }
     // tw: the layer's launches with many weight tiles; t: the others, which would have too few tiles for the GPU with 128 rows each
     const RowTiles t = row_tiles(R, per_group, true), tw = row_tiles(R, per_group, int8), to = row_tiles(std::max(O, 1), rl_fmt(head) == RL_I8G, rl_fmt(head) == RL_I8);
+    // ... cut again where a launch takes several turns of the GPU
+    const int fmt = per_group ? RL_I8G : int8 ? RL_I8 : RL_F16, mtc = (C + kRlTileM - 1) / kRlTileM, mtf = (F + kRlTileM - 1) / kRlTileM;
+    int mtr = 3 * mtc;
+    for (int mid : {cfg.w_mid, cfg.a_mid, cfg.g_mid, cfg.v_mid}) mtr += (mid + kRlTileM - 1) / kRlTileM;
+    const int kbc = (C + rl_kelems(fmt) - 1) / rl_kelems(fmt);
+    const RowTiles tr = fit_turns(tw, mtr, kbc, fmt, num_sms), tk = fit_turns(tw, mtf, kbc, fmt, num_sms), tn = fit_turns(t, mtc, kbc, fmt, num_sms);
     // Operands of a layer, carved again for every layer (a matrix's format is its own); the head's follow the largest layer's.
     OperandCarver cv;
     struct LayerOps {
@@ -902,18 +933,18 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     };
     auto carve_layer = [&](const LayerW& L, LayerOps& o) {
         cv.used = 0;
-        o.r = cv.operand(tw, rl_fmt(L.Wr), C, L.x_r);
-        o.k = cv.operand(tw, rl_fmt(L.Wk), C, L.x_k);
-        o.v = cv.operand(tw, rl_fmt(L.Wv), C, L.x_v);
-        o.w = cv.operand(tw, RL_F16, C, L.x_w);
-        o.a = cv.operand(tw, RL_F16, C, L.x_a);
-        o.g = cv.operand(tw, RL_F16, C, L.x_g);
-        o.vr = rl_fmt(L.Wv) == RL_F16 ? o.v : cv.operand(tw, RL_F16, C, L.x_v);
+        o.r = cv.operand(tr, rl_fmt(L.Wr), C, L.x_r);
+        o.k = cv.operand(tr, rl_fmt(L.Wk), C, L.x_k);
+        o.v = cv.operand(tr, rl_fmt(L.Wv), C, L.x_v);
+        o.w = cv.operand(tr, RL_F16, C, L.x_w);
+        o.a = cv.operand(tr, RL_F16, C, L.x_a);
+        o.g = cv.operand(tr, RL_F16, C, L.x_g);
+        o.vr = rl_fmt(L.Wv) == RL_F16 ? o.v : cv.operand(tr, RL_F16, C, L.x_v);
         const int mids[4] = {cfg.w_mid, cfg.a_mid, cfg.g_mid, cfg.v_mid};
         for (int i = 0; i < 4; ++i) o.mid[i] = cv.operand(t, RL_F16, mids[i]);
-        o.y = cv.operand(t, rl_fmt(L.Wo), C, nullptr, known_parts(C));
-        o.x2 = cv.operand(tw, rl_fmt(L.Wfk), C, L.ffn_x_k);
-        o.h = cv.operand(t, rl_fmt(L.Wfv), F, nullptr, known_parts(F));
+        o.y = cv.operand(tn, rl_fmt(L.Wo), C, nullptr, known_parts(C));
+        o.x2 = cv.operand(tk, rl_fmt(L.Wfk), C, L.ffn_x_k);
+        o.h = cv.operand(tn, rl_fmt(L.Wfv), F, nullptr, known_parts(F));
     };
     LayerOps ops;
     size_t layer_bytes = 0;
@@ -955,7 +986,6 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         A.segs = ws.seg_meta;
         A.R = R;
         A.C = C;
-        A.rt = tw.rt;
         A.nseg = from ? S : 0;
         return A;
     };
@@ -971,6 +1001,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
             const RlOperandOut* out[7] = {&ops.r, &ops.k, &ops.v, &ops.w, &ops.a, &ops.g, &ops.vr};
             const bool shared_v = ops.vr.img == ops.v.img;
             A.nout = l == 0 || shared_v ? 6 : 7;
+            A.rt = tr.rt;
             for (int i = 0; i < A.nout; ++i) A.out[i] = *out[i];
             launch_ln_operands(*this, "ln_shift6", A);
         }
@@ -994,7 +1025,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
                 {&L.g1, &ops.g, mg, MIDS, EPI_SIGMOID},
                 {&L.v1, &ops.vr, mv, MIDS, EPI_STORE},
             };
-            run_rows_linear(*this, "linear_rkv_rank", q, l == 0 ? 6 : 7, tw);
+            run_rows_linear(*this, "linear_rkv_rank", q, l == 0 ? 6 : 7, tr);
             // back-projections: decay w, a, gate g and (layers > 0) the v-lerp gate
             const int nb = l == 0 ? 3 : 4;
             const LinearW* Wb[4] = {&L.w2, &L.a2, &L.g2, &L.v2};
@@ -1079,14 +1110,15 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         }
         // a linear layer on activations whose row maxima their producer collected
         auto linear_known = [&](const char* name, RlReq q, const float* x, int ldx, const float* amax, int parts, const RlOperandOut& op) {
-            launch_operand_known(*this, x, ldx, q.W->K, amax, parts, t, op);
+            launch_operand_known(*this, x, ldx, q.W->K, amax, parts, tn, op);
             q.op = &op;
-            run_rows_linear(*this, name, &q, 1, t);
+            run_rows_linear(*this, name, &q, 1, tn);
         };
         linear_known("linear_att_out", RlReq{&L.Wo, nullptr, ws.delta, C, EPI_STORE}, ws.yg, C, ws.ymax, yparts, ops.y);
         pending = ws.delta;
         {
             LnOperandsArgs A = ln_args(L.ln2_w, L.ln2_b, cmix_x, ws.staging_c, ws.staging_t, tmix_x);
+            A.rt = tk.rt;
             A.nout = 1;
             A.out[0] = ops.x2;
             launch_ln_operands(*this, "ln_shift1", A);
@@ -1096,7 +1128,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         {
             RlReq q = {&L.Wfk, &ops.x2, ws.h, F, EPI_RELU2};
             q.ymax = ws.hmax;
-            run_rows_linear(*this, "linear_ffn_key", &q, 1, tw);
+            run_rows_linear(*this, "linear_ffn_key", &q, 1, tk);
         }
         linear_known("linear_ffn_value", RlReq{&L.Wfv, nullptr, ws.delta, C, EPI_STORE}, ws.h, F, ws.hmax, (F + kRlTileM - 1) / kRlTileM, ops.h);
         pending = ws.delta;

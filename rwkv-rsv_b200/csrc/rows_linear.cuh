@@ -41,6 +41,9 @@ namespace rsv {
 constexpr int kRlThreads = 320;
 constexpr int kRlEpiWarps = 8;
 constexpr int kRlEpiThreads = 32 * kRlEpiWarps;
+constexpr int kRlPEpiWarps = 16;  // of the persistent kernel
+constexpr int kRlPEpiThreads = 32 * kRlPEpiWarps;
+constexpr int kRlPThreads = 64 + kRlPEpiThreads;
 constexpr int kRlTileM = 128;
 constexpr int kRlABytes = kRlTileM * 128;
 constexpr int kRlMaxRows = 64;    // activation rows of a tile with int8 weights, or few rows
@@ -92,7 +95,10 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                  "r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void rl_epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kRlEpiThreads) : "memory"); }
+template <int THREADS = kRlEpiThreads>
+__device__ __forceinline__ void rl_epi_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+}
 
 // Four outputs at a time (independent chains), one piece of code for all epilogues (bias is 0 where there is none).
 __device__ __forceinline__ void rl_activate4(int epi, float (&a)[4], float bias) {
@@ -150,11 +156,12 @@ __device__ __forceinline__ RlOut rl_out(const RlProb& P, int r0, int nr, int m, 
     return o;
 }
 // The sums of a tile whose K was not split, from tensor memory through the thread's registers to the output, rows rl .. rl + 3 at a time
-// (`half`: the two warps of a lane quarter take turns).  What bounds this is instructions: 8192 outputs on eight warps.
+// (`turn`: the WARPS / 4 warps of a lane quarter take turns).  What bounds this is the latency of its instructions: a warp issues one in eight cycles.
+template <int WARPS>
 __device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t taddr, const float* s_xs, const double2* s_xt, float* s_ymax, double ws, double wz, bool mok,
-                                          int half, int lane) {
+                                          int turn, int lane) {
 #pragma unroll 1
-    for (int rl = 4 * half; rl < o.nr; rl += 8) {
+    for (int rl = 4 * turn; rl < o.nr; rl += WARPS) {
         float a[4];
         if (f16) {
             uint32_t v[8];
@@ -483,7 +490,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     const double wsd = ws, wzd = wz;
     if (go && direct) {
         const RlOut out = rl_out(P, r0, nr, m, bias);
-        rl_finish(out, BUILD || fmt == RL_F16, taddr, s_xs, s_xt, s_ymax[quarter], wsd, wzd, mok, half, lane);
+        rl_finish<kRlEpiWarps>(out, BUILD || fmt == RL_F16, taddr, s_xs, s_xt, s_ymax[quarter], wsd, wzd, mok, half, lane);
     } else if (!BUILD && go) {
         // this CTA's share of the rows: slices added in order, scaled, activated, stored (four rows at a time per thread)
         const int mine = nr > rank ? (nr - rank + S - 1) >> sh : 0;
@@ -553,8 +560,10 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
 // activation rows in turn, whole K.  One ring of stages runs through all of them and there are two accumulators, so the tensor core
 // works on the next tile while the epilogue warps finish the last one.  With a CTA per tile (two resident) both CTAs of an SM ran in
 // step: of a tile's 22 us at K = 2560 the tensor core worked 13 at 85 % of its rate, the rest was the first loads and the epilogue.
-// Measured, 2560 x 10240 (ffn.key): int8, 1024 rows 139 -> 94 us, 512 rows 82 -> 56 us.  What bounds it: the products (0.3 us per K block
-// and SM of 0.27 at the nominal rate), then the last turn, in which some SMs have no tile.
+// Measured, 2560 x 10240 (ffn.key): int8, 1024 rows 139 -> 94 us, 512 rows 82 -> 56 us (46 with sixteen epilogue warps: eight took longer over a tile
+// than the tensor core over its 20 K blocks).  What bounds it: the traffic of a K block, 48 KB from L2 for 512 cycles of products (an SM draws about 70
+// bytes per cycle; the copies alone take 85 % of the time, the products alone 75 %).  Tried without gain: four producer threads, six stages instead
+// of four, weights asked into L2 a turn ahead.
 struct RlCursor {
     int job, pi, kb, nk, mt, ntile;
     __device__ __forceinline__ void set(const RlLaunch& L, int j) {
@@ -567,7 +576,7 @@ struct RlCursor {
         nk = L.p[pi].kblocks;
     }
 };
-__global__ void __launch_bounds__(kRlThreads, 1) rows_linear_persistent_kernel(const __grid_constant__ RlLaunch L, int jobs) {
+__global__ void __launch_bounds__(kRlPThreads, 1) rows_linear_persistent_kernel(const __grid_constant__ RlLaunch L, int jobs) {
     extern __shared__ __align__(1024) uint8_t rl_raw[];
     __shared__ __align__(8) uint64_t full[kRlMaxStages], empty[kRlMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
@@ -581,14 +590,16 @@ __global__ void __launch_bounds__(kRlThreads, 1) rows_linear_persistent_kernel(c
     const uint32_t stage_bytes = (uint32_t)(kRlABytes + L.nt_max * 128), acc_cols = (uint32_t)L.tmem_cols / 2;
     const uint32_t NS = min((uint32_t)kRlMaxStages, (uint32_t)L.ring / stage_bytes);
     uint32_t filled = 0;
+    uint64_t pol = 0;
     if (threadIdx.x == 0) {
+        pol = L.n_tiles == 1 ? l2_evict_first_policy() : l2_evict_normal_policy();  // (see above)
         for (int i = 0; i < kRlMaxStages; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], kRlEpiWarps);
+            mbar_init(&acc_empty[i], kRlPEpiWarps);
         }
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -600,7 +611,7 @@ __global__ void __launch_bounds__(kRlThreads, 1) rows_linear_persistent_kernel(c
         for (; filled < NS && c.job < jobs; ++filled) {
             const int fmt = L.p[c.pi].fmt;
             mbar_expect_tx(&full[filled], kRlABytes + (uint32_t)(fmt == RL_F16 ? L.nt16 : L.nt8) * 128u);
-            tma_load_2d(&L.amap[c.pi], &full[filled], smem + (size_t)filled * stage_bytes, c.kb * rl_kelems(fmt), c.mt * kRlTileM);
+            tma_load_2d_hint(&L.amap[c.pi], &full[filled], smem + (size_t)filled * stage_bytes, c.kb * rl_kelems(fmt), c.mt * kRlTileM, pol);
             if (++c.kb == c.nk) {
                 if (c.job + G >= jobs) {
                     ++filled;
@@ -643,7 +654,7 @@ __global__ void __launch_bounds__(kRlThreads, 1) rows_linear_persistent_kernel(c
                             break;
                         }
                         mbar_expect_tx(&full[s], kRlABytes + bbytes);
-                        tma_load_2d(&L.amap[c.pi], &full[s], dst, kb * kel, c.mt * kRlTileM);
+                        tma_load_2d_hint(&L.amap[c.pi], &full[s], dst, kb * kel, c.mt * kRlTileM, pol);
                     }
                     bulk_load(dst + kRlABytes, bsrc, bbytes, &full[s]);
                     if (++s == NS) {
@@ -692,7 +703,7 @@ __global__ void __launch_bounds__(kRlThreads, 1) rows_linear_persistent_kernel(c
             if (ok) tc_commit_elect(&acc_full[it & 1u]);
         }
     } else {
-        const int et = threadIdx.x - 64, half = ((warp - 2) >> 2) & 1, quarter = warp & 3, ml = quarter * 32 + lane;
+        const int et = threadIdx.x - 64, turn = (warp - 2) >> 2, quarter = warp & 3, ml = quarter * 32 + lane;
         uint32_t it = 0;
         pdl_wait();
         // every warp runs every turn (the block barriers below): after a time-out without waiting and without output
@@ -720,17 +731,17 @@ __global__ void __launch_bounds__(kRlThreads, 1) rows_linear_persistent_kernel(c
                     s_xt[et] = make_double2((double)xs, rl_ll2d(t));
                 }
             }
-            rl_epi_sync();
+            rl_epi_sync<kRlPEpiThreads>();
             if (!*abort_flag) mbar_wait_parked(&acc_full[it & 1u], (it >> 1) & 1u, abort_flag);
             tc_fence_after();
             if (!__any_sync(0xffffffffu, *abort_flag)) {
                 const RlOut out = rl_out(P, r0, nr, m, bias);
-                rl_finish(out, P.fmt == RL_F16, tmem + ((uint32_t)(quarter * 32) << 16) + (it & 1u) * acc_cols, s_xs, s_xt, s_ymax[quarter], (double)ws, (double)wz, mok, half, lane);
+                rl_finish<kRlPEpiWarps>(out, P.fmt == RL_F16, tmem + ((uint32_t)(quarter * 32) << 16) + (it & 1u) * acc_cols, s_xs, s_xt, s_ymax[quarter], (double)ws, (double)wz, mok, turn, lane);
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[it & 1u]);
-            rl_epi_sync();
+            rl_epi_sync<kRlPEpiThreads>();
             if (P.ymax && et < nr)
                 P.ymax[(size_t)(r0 + et) * ((P.M + kRlTileM - 1) / kRlTileM) + c.mt] = fmaxf(fmaxf(s_ymax[0][et], s_ymax[1][et]), fmaxf(s_ymax[2][et], s_ymax[3][et]));
         }

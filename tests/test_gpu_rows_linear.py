@@ -87,3 +87,29 @@ def test_step_sizes_agree_with_the_cpu_path(tiny_paths, name):
 @pytest.mark.parametrize("m,k", [(2048, 2560), (9600, 1536), (9600, 704)])
 def test_linear_fp16_tiles_that_need_a_whole_sm(rows, m, k):
     test_linear_tile_edges(rows, m, k, False)
+
+
+# One row tile and more weight tiles than two CTAs per SM hold (a vocabulary head): the persistent kernel with a single row tile; 38016 and 38100: 297
+# and 298 weight tiles, the last of 84 rows
+@pytest.mark.parametrize("rows,m,k,int8", [(1, 38016, 1024, False), (3, 38100, 1088, False), (64, 38016, 2048, True)])
+def test_linear_persistent_with_one_row_tile(rows, m, k, int8):
+    test_linear_tile_edges(rows, m, k, int8)
+
+
+# 449 rows and more of 2560 channels are more 64-row tiles than SMs in every launch of a layer: the rows are cut again for the turns of the persistent
+# kernel, differently for wide and narrow layers (att.output and ffn.value: 37 to 40 rows of int8, 65 and more of fp16)
+@pytest.mark.parametrize("quant", [0, 1])
+def test_step_of_rows_cut_for_turns_agrees_with_the_cpu_path(tmp_path, quant):
+    p = rsv.write_synthetic(str(tmp_path / "m.st"), "tiny", seed=1, quant=quant, n_layer=1, n_embd=2560, n_head=40, ffn_hidden=5120, vocab=300, w_mid=24, a_mid=40,
+                            v_mid=8, g_mid=72)
+    b, o = rsv.ModelBuilder(p).build(), orc.OracleModel(p)
+    for n in (449, 512):
+        toks = np.random.default_rng(n).integers(0, 300, size=n).astype(np.uint32)
+        b.reset()
+        o.reset()
+        lg, want = b.infer_seq(toks), o.forward(toks)
+        # fp32 through the layer in another summation order: a few ulps of the logits' scale
+        assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n
+        assert np.abs(b.state_back() - o.state_back()).max() <= 1e-4 * max(1.0, float(np.abs(o.state_back()).max()))
+    b.state.close()
+    b.model.close()

@@ -11,7 +11,7 @@
 #include "sample_cluster.cuh"
 #include "decode_stream_layout.hpp"
 #include "wkv_rows.cuh"
-#include "wkv_seq.cuh"
+#include "wkv_chunk.cuh"
 
 namespace rsv {
 
@@ -429,7 +429,7 @@ std::unique_ptr<Model> Model::create_bare(int device) {
 }
 
 static void free_workspace(Workspace& w) {
-    void* ptrs[] = {w.x, w.x2, w.delta, w.r, w.k, w.v, w.w, w.a, w.g, w.yg, w.xb, w.mid, w.h, w.vfirst, w.logits, w.staging_t, w.staging_c, w.ymax, w.hmax, w.tokens, w.row_meta, w.seg_meta, w.out_rows, w.samp_temp, w.samp_cnt};
+    void* ptrs[] = {w.wkv_tmp, w.x, w.x2, w.delta, w.r, w.k, w.v, w.w, w.a, w.g, w.yg, w.xb, w.mid, w.h, w.vfirst, w.logits, w.staging_t, w.staging_c, w.ymax, w.hmax, w.tokens, w.row_meta, w.seg_meta, w.out_rows, w.samp_temp, w.samp_cnt};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     int* status = w.status;
@@ -571,7 +571,12 @@ void Model::upload_plan(const StepPlan& plan) {
     memcpy(p, plan.rows.data(), R * sizeof(RowMeta));
     RSV_CUDA(cudaMemcpyAsync(ws.row_meta, p, R * sizeof(RowMeta), cudaMemcpyHostToDevice, stream));
     p += R * sizeof(RowMeta);
-    memcpy(p, plan.segs.data(), S * sizeof(SegMeta));
+    SegMeta* sm = reinterpret_cast<SegMeta*>(p);
+    for (int i = 0, chunks = 0; i < S; ++i) {
+        sm[i] = plan.segs[i];
+        sm[i].pad = chunks;
+        chunks += wkv_chunks_of(sm[i].len);
+    }
     RSV_CUDA(cudaMemcpyAsync(ws.seg_meta, p, S * sizeof(SegMeta), cudaMemcpyHostToDevice, stream));
     p += S * sizeof(SegMeta);
     if (O) {
@@ -889,6 +894,37 @@ void launch_ln_operands(Model& m, const char* name, const LnOperandsArgs& A) {
         check_launch("ln_operands");
     }
 }
+// How many chunks of sixteen tokens a step's segments make if they take the matrix form of the WKV (wkv_chunk.cuh says when it is the faster one): all
+// of them long, and few enough that the chunk kernel's CTAs have an SM each.  0: token by token.
+int wkv_step_chunks(const SegMeta* segs, int nseg, int H, int sms) {
+    if (2 * H * nseg > sms) return 0;
+    int n = 0;
+    for (int i = 0; i < nseg; ++i) {
+        if (segs[i].len < kWcMinLen) return 0;
+        n += wkv_chunks_of(segs[i].len);
+    }
+    return n;
+}
+void ensure_wkv_memory(Model& m, size_t bytes) {
+    Workspace& w = m.ws;
+    if (bytes <= w.wkv_bytes) return;
+    RSV_CUDA(cudaStreamSynchronize(m.stream));
+    if (w.wkv_tmp) cudaFree(w.wkv_tmp);
+    w.wkv_tmp = nullptr;
+    w.wkv_bytes = 0;
+    RSV_CUDA(device_malloc(&w.wkv_tmp, bytes));
+    w.wkv_bytes = bytes;
+}
+// The raw y of a step in matrix form (wkv7_finish_kernel follows).
+void launch_wkv_chunks(Model& m, const WkvArgs& A, int chunks) {
+    static bool configured[16] = {false};
+    if (!configured[m.device & 15]) {
+        RSV_CUDA(cudaFuncSetAttribute(wkv7_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWcSmemBytes));
+        configured[m.device & 15] = true;
+    }
+    launch_pdl(m, wkv7_prepare_kernel, dim3(A.H, chunks), dim3(kWcPrepThreads), 0, A);
+    launch_pdl(m, wkv7_chunk_kernel, dim3(2 * A.H, A.nseg), dim3(kWcThreads), kWcSmemBytes, A);
+}
 int known_parts(int K) { return (K + 8 * kOpThreads - 1) / (8 * kOpThreads); }
 void launch_operand_known(Model& m, const float* x, int ldx, int K, const float* amax, int parts, const RowTiles& t, const RlOperandOut& o) {
     LAUNCH(m, "operand_known") {
@@ -990,6 +1026,8 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         return A;
     };
     float* vgate_buf = ws.xb;
+    const int chunks = plan.multi_row_segments ? wkv_step_chunks(plan.segs.data(), S, H, num_sms) : 0;
+    ensure_wkv_memory(*this, (size_t)chunks * H * kWcFloats * sizeof(float));
     for (int l = 0; l < NL; ++l) {
         const LayerW& L = layers[l];
         carve_layer(L, ops);
@@ -1066,7 +1104,9 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
             if (plan.multi_row_segments) {
                 // prefill chunks: vectors built by preparation warps, only state-dependent work in the per-token chain (wkv_seq.cuh)
                 // few (head, segment) pairs: a head over two CTAs
-                if (H * S <= num_sms) {
+                if (chunks > 0) {
+                    launch_wkv_chunks(*this, WkvArgs{ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, L.k_k, L.k_a, wkv, l == 0 ? st.v_first : nullptr, ws.yg, ws.wkv_tmp, S, H, C, ws.status}, chunks);
+                } else if (H * S <= num_sms) {
                     // Where every CTA can have an SM to itself it asks for more than half of the shared memory, so that no two share one:
                     // they would start in pairs as the predecessor's CTAs leave, and a pair takes a third longer (512 tokens, 40 heads).
                     const size_t alone = 2 * H * S <= num_sms ? 120 * 1024 : 0;
@@ -1534,7 +1574,7 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
             if (p) cudaFree(p);
         }
     };
-    Buf din[8], dpar[5], dstate, dy, dseg, dstatus;
+    Buf din[8], dpar[5], dstate, dy, dseg, dstatus, dtmp;
     for (int i = 0; i < 8; ++i)
         if (in[i]) {
             RSV_CUDA(device_malloc(&din[i].p, row_bytes));
@@ -1564,7 +1604,17 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
     cudaDeviceProp prop;
     RSV_CUDA(cudaGetDeviceProperties(&prop, device));
     const int sms = prop.multiProcessorCount, n_items = H * nseg;
-    if (variant == 0) variant = T > 1 ? (n_items <= sms ? 3 : 4) : (n_items >= 4 * sms ? 2 : 1);
+    if (variant < 0 || variant > 4) throw std::runtime_error("wkv7: variant must be 0 (automatic), 1 (token kernel), 2 (row-per-lane kernel), 3 or 4 (sequence kernel, head over two CTAs / one CTA)");
+    // automatic: what a step runs.  A step's decays are exp(-sigmoid / sqrt(e)) > 0.54; products of sixteen others (which only this entry point can be given)
+    // may underflow: those go token by token.
+    constexpr int kChunked = 5;
+    int chunks = 0;
+    if (variant == 0) {
+        chunks = T > 1 ? wkv_step_chunks(segs.data(), nseg, H, sms) : 0;
+        for (size_t i = 0; i < (size_t)R * C && chunks; ++i)
+            if (!(in[3][i] >= 0.5f && in[3][i] <= 1.0f)) chunks = 0;
+        variant = chunks ? kChunked : T > 1 ? (n_items <= sms ? 3 : 4) : (n_items >= 4 * sms ? 2 : 1);
+    }
     if (variant == 1) {
         wkv7_kernel<<<dim3(H, nseg), kWkvThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C, nullptr);
     } else if (variant == 2) {
@@ -1573,16 +1623,22 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
         RSV_CUDA(cudaFuncSetAttribute(wkv7_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWrSmemBytes));
         const int ctas = std::min((n_items + kWrPairs - 1) / kWrPairs, sms);
         wkv7_rows_kernel<<<ctas, kWrThreads, kWrSmemBytes>>>(map, 0LL, sm, n_items, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, nullptr, yg, H, C, status, nullptr);
-    } else if (variant == 3 || variant == 4) {
-        if (variant == 3)
+    } else {
+        if (variant == kChunked) {
+            for (int s2 = 0, before = 0; s2 < nseg; before += wkv_chunks_of(T), ++s2) segs[s2].pad = before;
+            RSV_CUDA(cudaMemcpy(dseg.p, segs.data(), segs.size() * sizeof(SegMeta), cudaMemcpyHostToDevice));
+            RSV_CUDA(device_malloc(&dtmp.p, (size_t)chunks * H * kWcFloats * sizeof(float)));
+            RSV_CUDA(cudaDeviceSynchronize());  // (the launches below go to a stream of their own)
+            auto m = Model::create_bare(device);
+            launch_wkv_chunks(*m, WkvArgs{sm, r, k, v, vgate, vfirst, w, a, k_k, k_a, state, nullptr, yg, (float*)dtmp.p, nseg, H, C, status}, chunks);
+            RSV_CUDA(cudaStreamSynchronize(m->stream));
+        } else if (variant == 3)
             wkv7_seq_kernel<2><<<dim3(2 * H, nseg), kWsThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C, status);
         else
             wkv7_seq_kernel<4><<<dim3(H, nseg), kWsThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C, status);
         check_launch("wkv7_seq");
         wkv7_finish_kernel<<<(R * H + kWsFinishThreads / 32 - 1) / (kWsFinishThreads / 32), kWsFinishThreads>>>(r, k, v, vgate, vfirst, a, g, k_a, r_k, lnx_w, lnx_b, yg,
                                                                                                               R, H, C, nullptr);
-    } else {
-        throw std::runtime_error("wkv7: variant must be 0 (automatic), 1 (token kernel), 2 (row-per-lane kernel), 3 or 4 (sequence kernel, head over two CTAs / one CTA)");
     }
     check_launch("wkv7");
     RSV_CUDA(cudaDeviceSynchronize());

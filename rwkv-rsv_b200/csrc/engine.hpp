@@ -61,6 +61,8 @@ struct Workspace {
     // operands of the tensor-core layers (operands.cuh) with their scales and sums, carved per step from one block
     uint8_t* op_mem = nullptr;
     size_t op_bytes = 0;
+    float* wkv_tmp = nullptr;  // a step's WKV chunks (wkv_chunk.cuh)
+    size_t wkv_bytes = 0;
     float *ymax = nullptr, *hmax = nullptr;  // [rows][parts] maxima of the time-mix output (per head) and of the ffn hidden vector (per M tile)
     float* samp_temp = nullptr;      // [outs, V] sampler work area
     uint32_t* samp_cnt = nullptr;    // [outs, V] penalty histogram

@@ -12,7 +12,8 @@
 //                    equal logits, or a large k) the bits of the k-th largest are found by four 8-bit radix passes instead.
 //   top-p            a walk over the sorted list (k <= 512: the top-k list serves both)
 //   draw             prefix sums in vocabulary order: thread, block, cluster
-// Measured, 65536 logits, one row: top-k 50 + top-p 25 us (218 before), top-p alone 43 us.
+// Measured, 65536 logits: one row, top-k 50 + top-p 23 us (218 in one CTA, 24 before the walk below took eight entries at a time and the sort dropped block
+// barriers within a warp); 1024 rows of top-p alone 1.09 ms (1.51).
 #pragma once
 #include "kernels.cuh"
 #include "tc_ptx.cuh"
@@ -33,7 +34,7 @@ struct ScShared {
     int local_n;
     float xmax, xsum, xkept;  // this CTA's maximum, sum, kept sum (read by the others)
     int xchosen, xlast;       // this CTA's drawn token (V: none) and its last kept one (-1: none)
-    float list[kScList];      // the collection, sorted (every CTA its own copy)
+    alignas(16) float list[kScList];  // the collection, sorted (every CTA its own copy)
     float red[kScThreads / 32];
     uint32_t ured[kScThreads / 32];
     int cross, before;        // bin that holds the k-th largest; elements in the bins before it
@@ -262,7 +263,8 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
             while (np < n) np <<= 1;
             for (int i = at + tid; i < np; i += kScThreads) sh.list[i] = i < n ? kth : -INFINITY;
             __syncthreads();
-            // bitonic sort, descending (np <= 1024: a pair per thread)
+            // bitonic sort, descending (np <= 1024: a pair per thread).  Pairs up to 32 apart stay within the 64 entries of a warp: steps that follow
+            // each other there need no block barrier (15 of the 55 steps of 1024 entries do).
 #pragma unroll 1
             for (int kk = 2; kk <= np; kk <<= 1)
 #pragma unroll 1
@@ -276,8 +278,12 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
                             sh.list[b] = va;
                         }
                     }
-                    __syncthreads();
+                    if (j > 32 || (j == 1 && kk >= 64))  // (the next step is kk's, j / 2 apart, or after j = 1 that of 2 kk, kk apart)
+                        __syncthreads();
+                    else
+                        __syncwarp();
                 }
+            __syncthreads();
             kth = sh.list[K - 1];
             // entries >= kth: all of them are in the list
             const int lim = min(n, kTopPMaxPicks);
@@ -313,8 +319,18 @@ __global__ void __launch_bounds__(kScThreads, 2) sample_cluster_kernel(const flo
         __syncthreads();
         if (tid == 0) {
             // picks from the largest down until the sum reaches top_p (at most 512); past the list only zeros follow
+            // Eight at a time while their sum stays under top_p (the same additions in the same order; the chain is an addition per pick instead of a read, an
+            // addition, a comparison and a branch)
             float cum = 0.0f, cut = 0.0f;
             int c = 0;
+#pragma unroll 1
+            for (; c + 8 <= m; c += 8) {
+                const float4 p = *reinterpret_cast<const float4*>(&sh.list[c]), q = *reinterpret_cast<const float4*>(&sh.list[c + 4]);
+                const float t = (((((((cum + p.x) + p.y) + p.z) + p.w) + q.x) + q.y) + q.z) + q.w;
+                if (!(t < top_p)) break;
+                cum = t;
+                cut = q.w;
+            }
             for (; c < m && cum < top_p; ++c) {
                 cut = sh.list[c];
                 cum += cut;

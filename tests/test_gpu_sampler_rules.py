@@ -140,3 +140,28 @@ def test_rows_with_a_nan_or_an_infinity(v):
     lg[0, 100], lg[1, 100] = np.nan, np.inf
     got = rsv.op_sample(lg, np.stack([orc.pack_sampler(seed=s) for s in (1, 2)]))
     assert [int(g) for g in got] == [v - 1, v - 1] == [orc.sample(lg[s], seed=s + 1) for s in range(2)]
+
+
+# The top-p walk takes eight entries of the sorted list at a time until their sum reaches top_p: the last kept token at the ends of such a group, the list's
+# own end (512), and lists of one warp's and of several warps' entries
+@pytest.mark.parametrize("kept,top_k", [(1, 0), (7, 0), (8, 0), (9, 0), (16, 0), (17, 0), (65, 0), (512, 0), (8, 8), (13, 13), (9, 40), (33, 50), (700, 0)])
+def test_top_p_keeps_exactly_the_largest_that_reach_it(kept, top_k):
+    rng = np.random.default_rng(kept)
+    V, rows = 4096, 400
+    order = rng.permutation(V)
+    logits = np.empty(V, np.float32)
+    logits[order] = -1e-3 * np.arange(V, dtype=np.float32)  # nearly flat: every kept token is drawn sooner or later
+    p = np.exp(logits[order].astype(np.float64))
+    if top_k:
+        p[top_k:] = 0.0
+    p /= p.sum()
+    top_p = float(min(0.999999, p[:kept].sum() - 0.5 * p[kept - 1]))
+    got = rsv.op_sample(np.repeat(logits[None], rows, 0), np.stack([orc.pack_sampler(seed=77 * r + 1, top_p=top_p, top_k=top_k) for r in range(rows)])).astype(np.int64)
+    rank = np.empty(V, np.int64)
+    rank[order] = np.arange(V)
+    ranks, n = rank[got], min(kept, 512)  # (at most 512 picks)
+    assert ranks.max() <= n - 1
+    if n <= 17:
+        assert set(ranks.tolist()) == set(range(n))
+    else:
+        assert ranks.max() >= 0.9 * n - 1

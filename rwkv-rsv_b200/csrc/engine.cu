@@ -634,48 +634,6 @@ void run_linear_simt(Model& m, const char* name, const LinearW& W, const float* 
 
 
 // ---- tensor-core path ---------------------------------------------------------------------------
-// Row tiles of a step, of equal size: at most 64 activation rows each (32 with per-group int8 weights).  With fp16 weights alone and more
-// than 128 rows a tile has up to 128: its two columns per row then fill the matrix instruction as four per row of 64 do, and the
-// weights pass through L2 half as often.
-struct RowTiles {
-    int R = 0, rt = 0, n = 0, nt8 = 0, nt16 = 0;
-    bool turns = false;  // cut for the persistent kernel (fit_turns): K is not split
-    int nt(int fmt) const { return fmt == RL_F16 ? nt16 : nt8; }
-    size_t image_bytes(int fmt, int K) const { return (size_t)n * ((K + rl_kelems(fmt) - 1) / rl_kelems(fmt)) * nt(fmt) * 128; }
-};
-RowTiles cut_rows(int R, int n) {
-    RowTiles t;
-    t.R = R;
-    t.rt = (R + n - 1) / n;
-    t.n = (R + t.rt - 1) / t.rt;
-    t.nt8 = (int)round_up((size_t)t.rt * rl_cols(RL_I8), 16);
-    t.nt16 = (int)round_up((size_t)t.rt * rl_cols(RL_F16), 16);
-    return t;
-}
-RowTiles row_tiles(int R, bool per_group, bool int8) {
-    const int most = per_group ? kRlMaxRowsG : int8 || R <= kRlMaxRowsF ? kRlMaxRows : kRlMaxRowsF;
-    return cut_rows(R, (R + most - 1) / most);
-}
-// The row tiles of a launch with more tiles than SMs, which the persistent kernel takes in turns: `mt` weight tiles, at least `kb` blocks of K, fmt
-// the format of most of them.  A turn lasts as long as its K blocks take to arrive (an SM draws about 70 bytes per cycle from L2: 16 KB of weights and 128
-// bytes per operand column), so the cut with the least turns x (columns + 128) is taken, the largest tiles among equals.  512 rows, 10240 -> 2560
-// channels: 160 tiles of 64 rows are two turns on 148 SMs and took 59 us, 260 tiles of 40 rows are two shorter ones, 49 us; 2560 -> 2560: 24 and 17 us.  fp16
-// layers of 512 rows leave the kernel with a CTA per 64-row tile this way.  Fewer than 32 rows would leave the matrix instruction too narrow.
-RowTiles fit_turns(const RowTiles& t, int mt, int kb, int fmt, int sms) {
-    if (t.n < 2 || fmt == RL_I8G || mt * t.n <= sms || kb < 16) return t;
-    const int cols = rl_cols(fmt), most = fmt == RL_F16 ? kRlMaxRowsF : kRlMaxRows;
-    RowTiles best = t;
-    long long cost = -1;
-    for (int n = (t.R + most - 1) / most; n <= (t.R + 31) / 32; ++n) {
-        const RowTiles c = cut_rows(t.R, n);
-        const long long turns = ((long long)mt * c.n + sms - 1) / sms, now = turns * (round_up((size_t)c.rt * cols, 16) + 128);
-        if (cost >= 0 && now >= cost) continue;
-        cost = now;
-        best = c;
-    }
-    best.turns = true;
-    return best;
-}
 int rl_fmt(const LinearW& W) { return W.wtype != W_INT8 ? RL_F16 : W.row_scaled() ? RL_I8 : RL_I8G; }
 
 // Carves a step's operands out of one block of device memory.
@@ -961,7 +919,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     int mtr = 3 * mtc;
     for (int mid : {cfg.w_mid, cfg.a_mid, cfg.g_mid, cfg.v_mid}) mtr += (mid + kRlTileM - 1) / kRlTileM;
     const int kbc = (C + rl_kelems(fmt) - 1) / rl_kelems(fmt);
-    const RowTiles tr = fit_turns(tw, mtr, kbc, fmt, num_sms), tk = fit_turns(tw, mtf, kbc, fmt, num_sms), tn = fit_turns(t, mtc, kbc, fmt, num_sms);
+    const RowTiles tr = fit_turns(tw, mtr, kbc, fmt, num_sms, R + S), tk = fit_turns(tw, mtf, kbc, fmt, num_sms, R + S), tn = fit_turns(t, mtc, kbc, fmt, num_sms, 0);
     // Operands of a layer, carved again for every layer (a matrix's format is its own); the head's follow the largest layer's.
     OperandCarver cv;
     struct LayerOps {

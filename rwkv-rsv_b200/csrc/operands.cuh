@@ -11,17 +11,11 @@
 // weight row) or per group of 128 (tgrp; one per weight row and group).
 #pragma once
 #include "kernels.cuh"
+#include "row_tiles.hpp"
 
 namespace rsv {
 
-enum RlFmt : int { RL_F16 = 0, RL_I8 = 1, RL_I8G = 2 };  // fp16; int8 with one (scale, zero) per row; int8 with one per row and group of 128
-constexpr int kRlDigits = 4;
 constexpr int kRlP = 7 * kRlDigits - 1;  // fixed-point bits
-
-// columns an activation row takes in an operand tile
-__host__ __device__ inline int rl_cols(int fmt) { return fmt == RL_F16 ? 2 : kRlDigits; }
-// K elements in a 128-byte block
-__host__ __device__ inline int rl_kelems(int fmt) { return fmt == RL_F16 ? 64 : 128; }
 
 // smallest ex with 2^ex >= amax (0 for an all-zero or non-finite row)
 __device__ __forceinline__ int rl_scale_exp(float amax) {

@@ -46,9 +46,6 @@ constexpr int kRlPEpiThreads = 32 * kRlPEpiWarps;
 constexpr int kRlPThreads = 64 + kRlPEpiThreads;
 constexpr int kRlTileM = 128;
 constexpr int kRlABytes = kRlTileM * 128;
-constexpr int kRlMaxRows = 64;    // activation rows of a tile with int8 weights, or few rows
-constexpr int kRlMaxRowsF = 128;  // the same for fp16 weights and many rows (256 columns of operand either way)
-constexpr int kRlMaxRowsG = 32;   // the same for per-group weights: two accumulators are in use, and fp32 sums in registers
 constexpr int kRlMaxProb = 8;
 constexpr int kRlMaxStages = 8;
 constexpr int kRlMaxSplit = 8;

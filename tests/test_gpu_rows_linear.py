@@ -97,7 +97,7 @@ def test_linear_persistent_with_one_row_tile(rows, m, k, int8):
 
 
 # 449 rows and more of 2560 channels are more 64-row tiles than SMs in every launch of a layer: the rows are cut again for the turns of the persistent
-# kernel, differently for wide and narrow layers (att.output and ffn.value: 37 to 40 rows of int8, 65 and more of fp16)
+# kernel, differently for wide and narrow layers (att.output and ffn.value: 35 and 40 rows of int8, 65 and 74 of fp16)
 @pytest.mark.parametrize("quant", [0, 1])
 def test_step_of_rows_cut_for_turns_agrees_with_the_cpu_path(tmp_path, quant):
     p = rsv.write_synthetic(str(tmp_path / "m.st"), "tiny", seed=1, quant=quant, n_layer=1, n_embd=2560, n_head=40, ffn_hidden=5120, vocab=300, w_mid=24, a_mid=40,
@@ -111,5 +111,33 @@ def test_step_of_rows_cut_for_turns_agrees_with_the_cpu_path(tmp_path, quant):
         # fp32 through the layer in another summation order: a few ulps of the logits' scale
         assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n
         assert np.abs(b.state_back() - o.state_back()).max() <= 1e-4 * max(1.0, float(np.abs(o.state_back()).max()))
+    b.state.close()
+    b.model.close()
+
+
+# The smallest steps whose rows are cut again (10240 ffn channels): ffn.key of int8 weights has three tiles of 22 to 43 rows up to 128 rows; fp16 keeps its
+# 64-row tiles there for one segment, has one tile where every row is a segment (93 rows and more), and three tiles from 129 rows on
+@pytest.mark.parametrize("quant", [0, 1])
+def test_small_steps_cut_for_turns_agree_with_the_cpu_path(tmp_path, quant):
+    p = rsv.write_synthetic(str(tmp_path / "m.st"), "tiny", seed=2, quant=quant, n_layer=1, n_embd=2560, n_head=40, ffn_hidden=10240, vocab=300, w_mid=24, a_mid=40,
+                            v_mid=8, g_mid=72)
+    b, o = rsv.ModelBuilder(p).build(), orc.OracleModel(p)
+    for n in (65, 80, 97, 128, 129, 193):
+        toks = np.random.default_rng(n).integers(0, 300, size=n).astype(np.uint32)
+        b.reset()
+        o.reset()
+        lg, want = b.infer_seq(toks), o.forward(toks)
+        # fp32 through the layer in another summation order: a few ulps of the logits' scale
+        assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n
+        assert np.abs(b.state_back() - o.state_back()).max() <= 1e-4 * max(1.0, float(np.abs(o.state_back()).max()))
+    for n in (65, 112, 128):
+        toks = np.random.default_rng(n).integers(0, 300, size=n).astype(np.uint32)
+        st = b.model.create_batch_state(n)
+        got = b.model.forward_seq_batch_mean_hidden(st, [toks[i:i + 1] for i in range(n)])
+        st.close()
+        for i in range(0, n, 7):
+            o.reset()
+            want = o.mean_hidden(toks[i:i + 1])
+            assert float(np.sqrt(np.mean((got[i] - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), (n, i)
     b.state.close()
     b.model.close()

@@ -27,6 +27,10 @@ def test_logits_that_arrive_in_parts(tmp_path):
     assert "parts ok" in _run(tmp_path, "parts_to_host_check")
 
 
+def test_rows_are_cut_into_no_more_turns_than_the_widest_tiles_need(tmp_path):
+    assert "row tiles ok" in _run(tmp_path, "row_tiles_check")
+
+
 @pytest.mark.skipif(not os.path.exists(CUDA_INCLUDE), reason="no CUDA headers")
 def test_memory_of_freed_states_is_given_back(tmp_path):
     assert "device memory ok" in _run(tmp_path, "device_memory_check", "-I", CUDA_INCLUDE)

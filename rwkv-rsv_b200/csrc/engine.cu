@@ -717,6 +717,19 @@ void rl_launch(Model& m, const char* name, const RlLaunch& L, int ctas, size_t s
     }
 }
 
+template <int WARPS>
+void rl_launch_persistent(Model& m, const char* name, const RlLaunch& L, int jobs, size_t smem) {
+    static bool configured[16] = {false};
+    if (!configured[m.device & 15]) {
+        RSV_CUDA(cudaFuncSetAttribute(rows_linear_persistent_kernel<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRlRingMax + 1024));
+        configured[m.device & 15] = true;
+    }
+    LAUNCH(m, name) {
+        launch_pdl(m, rows_linear_persistent_kernel<WARPS>, dim3(std::min(jobs, m.num_sms)), dim3(rl_persistent_threads(WARPS)), smem, L, jobs);
+        check_launch("rows_linear_persistent");
+    }
+}
+
 void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const RowTiles& t) {
     if (n < 1 || n > kRlMaxProb) throw std::runtime_error("rows_linear: too many problems in one launch");
     {
@@ -801,15 +814,13 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
         L.tmem_cols = 64;
         while (L.tmem_cols < 2 * nt_max) L.tmem_cols *= 2;
         const size_t bytes = L.ring + 1024;
-        static bool configured[16] = {false};
-        if (!configured[m.device & 15]) {
-            RSV_CUDA(cudaFuncSetAttribute(rows_linear_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRlRingMax + 1024));
-            configured[m.device & 15] = true;
-        }
-        LAUNCH(m, name) {
-            launch_pdl(m, rows_linear_persistent_kernel, dim3(std::min(jobs, m.num_sms)), dim3(kRlPThreads), bytes, L, jobs);
-            check_launch("rows_linear_persistent");
-        }
+        // Several narrow tiles of few rows: eight epilogue warps keep up with the products, and beside sixteen (46 of 64 K registers) the CTAs of the next kernel, which
+        // converts the outputs of up to 118 rows, would not all be resident early (a layer of 72 int8 rows, 2560 channels: 112.0 us with sixteen, 110.4 with
+        // eight; 112 rows 140.4 and 138.1, 128 the same, 160 rows 166.2 and 168.8).
+        if (t.n > 1 && t.R <= 2 * kRlMaxRows)
+            rl_launch_persistent<8>(m, name, L, jobs, bytes);
+        else
+            rl_launch_persistent<16>(m, name, L, jobs, bytes);
         return;
     }
     const size_t stage = kRlABytes + (build ? 0 : (size_t)nt_max * 128), bbuf = build ? (size_t)nk * nt_max * 128 : 0, tg = grouped ? round_up((size_t)nk * t.rt * 4, 16) : 0;

@@ -41,9 +41,7 @@ namespace rsv {
 constexpr int kRlThreads = 320;
 constexpr int kRlEpiWarps = 8;
 constexpr int kRlEpiThreads = 32 * kRlEpiWarps;
-constexpr int kRlPEpiWarps = 16;  // of the persistent kernel
-constexpr int kRlPEpiThreads = 32 * kRlPEpiWarps;
-constexpr int kRlPThreads = 64 + kRlPEpiThreads;
+constexpr int rl_persistent_threads(int epi_warps) { return 64 + 32 * epi_warps; }
 constexpr int kRlTileM = 128;
 constexpr int kRlABytes = kRlTileM * 128;
 constexpr int kRlMaxProb = 8;
@@ -573,7 +571,8 @@ struct RlCursor {
         nk = L.p[pi].kblocks;
     }
 };
-__global__ void __launch_bounds__(kRlPThreads, 1) rows_linear_persistent_kernel(const __grid_constant__ RlLaunch L, int jobs) {
+template <int WARPS>
+__global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_persistent_kernel(const __grid_constant__ RlLaunch L, int jobs) {
     extern __shared__ __align__(1024) uint8_t rl_raw[];
     __shared__ __align__(8) uint64_t full[kRlMaxStages], empty[kRlMaxStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
@@ -596,7 +595,7 @@ __global__ void __launch_bounds__(kRlPThreads, 1) rows_linear_persistent_kernel(
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
-            mbar_init(&acc_empty[i], kRlPEpiWarps);
+            mbar_init(&acc_empty[i], WARPS);
         }
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -728,17 +727,17 @@ __global__ void __launch_bounds__(kRlPThreads, 1) rows_linear_persistent_kernel(
                     s_xt[et] = make_double2((double)xs, rl_ll2d(t));
                 }
             }
-            rl_epi_sync<kRlPEpiThreads>();
+            rl_epi_sync<32 * WARPS>();
             if (!*abort_flag) mbar_wait_parked(&acc_full[it & 1u], (it >> 1) & 1u, abort_flag);
             tc_fence_after();
             if (!__any_sync(0xffffffffu, *abort_flag)) {
                 const RlOut out = rl_out(P, r0, nr, m, bias);
-                rl_finish<kRlPEpiWarps>(out, P.fmt == RL_F16, tmem + ((uint32_t)(quarter * 32) << 16) + (it & 1u) * acc_cols, s_xs, s_xt, s_ymax[quarter], (double)ws, (double)wz, mok, turn, lane);
+                rl_finish<WARPS>(out, P.fmt == RL_F16, tmem + ((uint32_t)(quarter * 32) << 16) + (it & 1u) * acc_cols, s_xs, s_xt, s_ymax[quarter], (double)ws, (double)wz, mok, turn, lane);
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[it & 1u]);
-            rl_epi_sync<kRlPEpiThreads>();
+            rl_epi_sync<32 * WARPS>();
             if (P.ymax && et < nr)
                 P.ymax[(size_t)(r0 + et) * ((P.M + kRlTileM - 1) / kRlTileM) + c.mt] = fmaxf(fmaxf(s_ymax[0][et], s_ymax[1][et]), fmaxf(s_ymax[2][et], s_ymax[3][et]));
         }

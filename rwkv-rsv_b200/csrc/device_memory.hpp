@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <initializer_list>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -95,5 +96,43 @@ cudaError_t device_malloc(T** p, size_t bytes) {
     }
     return e;
 }
+
+// A work area that grows and that its user can do without: where the device is full, reserve() says so instead of throwing.
+class SpareArea {
+  public:
+    // At least `bytes`, with a quarter on top where there is room for it, so that needs that creep up reallocate a few times only.  `idle` waits for the work
+    // on the memory that the area has.  Its contents are lost when it grows.
+    template <typename Idle>
+    bool reserve(size_t bytes, Idle&& idle) {
+        if (bytes <= size) return true;
+        if (p) idle();
+        release();
+        for (size_t want : {bytes + bytes / 4, bytes}) {
+            const cudaError_t e = device_malloc(&p, want);
+            if (e == cudaSuccess) {
+                size = want;
+                return true;
+            }
+            p = nullptr;
+            if (e != cudaErrorMemoryAllocation) return false;  // (an earlier failure of the device: the next call that checks reports it)
+            cudaGetLastError();
+        }
+        return false;
+    }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        size = 0;
+    }
+    template <typename T>
+    T* as() const {
+        return static_cast<T*>(p);
+    }
+    size_t bytes() const { return size; }
+
+  private:
+    void* p = nullptr;
+    size_t size = 0;
+};
 
 }  // namespace rsv

@@ -45,19 +45,23 @@ struct LaunchScope {
 // stream is still running and synchronises with it through pdl_wait().  Only kernels that call pdl_wait() before they
 // touch anything an earlier kernel of the step produces are launched this way.
 template <typename... KArgs, typename... Args>
-static void launch_pdl(Model& m, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+static void launch_pdl_on(cudaStream_t stream, bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = m.stream;
+    cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = m.use_pdl ? 1 : 0;
+    cfg.numAttrs = pdl ? 1 : 0;
     RSV_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(std::forward<Args>(args))...));
+}
+template <typename... KArgs, typename... Args>
+static void launch_pdl(Model& m, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+    launch_pdl_on(m.stream, m.use_pdl, kernel, grid, block, smem, std::forward<Args>(args)...);
 }
 
 // The same as a launch of thread-block clusters of `cluster` CTAs.
@@ -429,7 +433,7 @@ std::unique_ptr<Model> Model::create_bare(int device) {
 }
 
 static void free_workspace(Workspace& w) {
-    void* ptrs[] = {w.wkv_tmp, w.x, w.x2, w.delta, w.r, w.k, w.v, w.w, w.a, w.g, w.yg, w.xb, w.mid, w.h, w.vfirst, w.logits, w.staging_t, w.staging_c, w.ymax, w.hmax, w.tokens, w.row_meta, w.seg_meta, w.out_rows, w.samp_temp, w.samp_cnt};
+    void* ptrs[] = {w.x, w.x2, w.delta, w.r, w.k, w.v, w.w, w.a, w.g, w.yg, w.xb, w.mid, w.h, w.vfirst, w.logits, w.staging_t, w.staging_c, w.ymax, w.hmax, w.tokens, w.row_meta, w.seg_meta, w.out_rows, w.samp_temp, w.samp_cnt};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     int* status = w.status;
@@ -442,6 +446,7 @@ static void free_workspace(Workspace& w) {
     w.tok_list_cap = keep.tok_list_cap;
     w.op_mem = keep.op_mem;
     w.op_bytes = keep.op_bytes;
+    w.wkv_tmp = keep.wkv_tmp;
 }
 
 Model::~Model() {
@@ -453,8 +458,8 @@ Model::~Model() {
     if (ws.tok_pos) cudaFree(ws.tok_pos);
     if (ws.tok_list) cudaFree(ws.tok_list);
     for (void* p : allocs) cudaFree(p);
-    for (void* p : {(void*)ws.op_mem})
-        if (p) cudaFree(p);
+    if (ws.op_mem) cudaFree(ws.op_mem);
+    ws.wkv_tmp.release();
     for (void* p : {sctx.d_layers, sctx.wstream, sctx.hstream, (void*)sctx.exchange, (void*)sctx.cand_val, (void*)sctx.cand_idx, (void*)sctx.grid_bar})
         if (p) cudaFree(p);
     if (pinned) cudaFreeHost(pinned);
@@ -874,25 +879,19 @@ int wkv_step_chunks(const SegMeta* segs, int nseg, int H, int sms) {
     }
     return n;
 }
-void ensure_wkv_memory(Model& m, size_t bytes) {
-    Workspace& w = m.ws;
-    if (bytes <= w.wkv_bytes) return;
-    RSV_CUDA(cudaStreamSynchronize(m.stream));
-    if (w.wkv_tmp) cudaFree(w.wkv_tmp);
-    w.wkv_tmp = nullptr;
-    w.wkv_bytes = 0;
-    RSV_CUDA(device_malloc(&w.wkv_tmp, bytes));
-    w.wkv_bytes = bytes;
+// Scratch for that many chunks; false where the device has no room for it (the step then goes token by token, which needs none).
+bool reserve_wkv_chunks(Model& m, int chunks) {
+    return m.ws.wkv_tmp.reserve((size_t)chunks * m.cfg.n_head * kWcFloats * sizeof(float), [&] { RSV_CUDA(cudaStreamSynchronize(m.stream)); });
 }
 // The raw y of a step in matrix form (wkv7_finish_kernel follows).
-void launch_wkv_chunks(Model& m, const WkvArgs& A, int chunks) {
+void launch_wkv_chunks(int device, cudaStream_t stream, bool pdl, const WkvArgs& A, int chunks) {
     static bool configured[16] = {false};
-    if (!configured[m.device & 15]) {
+    if (!configured[device & 15]) {
         RSV_CUDA(cudaFuncSetAttribute(wkv7_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWcSmemBytes));
-        configured[m.device & 15] = true;
+        configured[device & 15] = true;
     }
-    launch_pdl(m, wkv7_prepare_kernel, dim3(A.H, chunks), dim3(kWcPrepThreads), 0, A);
-    launch_pdl(m, wkv7_chunk_kernel, dim3(2 * A.H, A.nseg), dim3(kWcThreads), kWcSmemBytes, A);
+    launch_pdl_on(stream, pdl, wkv7_prepare_kernel, dim3(A.H, chunks), dim3(kWcPrepThreads), 0, A);
+    launch_pdl_on(stream, pdl, wkv7_chunk_kernel, dim3(2 * A.H, A.nseg), dim3(kWcThreads), kWcSmemBytes, A);
 }
 int known_parts(int K) { return (K + 8 * kOpThreads - 1) / (8 * kOpThreads); }
 void launch_operand_known(Model& m, const float* x, int ldx, int K, const float* amax, int parts, const RowTiles& t, const RlOperandOut& o) {
@@ -908,6 +907,13 @@ void launch_operand_rows(Model& m, const OperandRowsArgs& A) {
     }
 }
 }  // namespace
+
+void Model::reserve_prompt_scratch(int rows, int segs, int chunk) {
+    segs = std::min(segs, num_sms / (2 * std::max(cfg.n_head, 1)));
+    rows = (int)std::min<int64_t>(rows, (int64_t)segs * chunk);
+    if (segs < 1 || std::min(rows, chunk) < kWcMinLen) return;
+    reserve_wkv_chunks(*this, rows / kWcT + segs);  // (every segment may end in a part of a chunk)
+}
 
 // ------------------------------------------------------------------------------------------------
 // the packed forward step (one token per row), Appendix-style data flow of src/model.rs:396-516
@@ -963,6 +969,8 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
     cv.base = ws.op_mem;
     cv.used = layer_bytes;
     head_op = cv.operand(to, rl_fmt(head), C);
+    int chunks = plan.multi_row_segments ? wkv_step_chunks(plan.segs.data(), S, H, num_sms) : 0;
+    if (chunks && !reserve_wkv_chunks(*this, chunks)) chunks = 0;
 
     LAUNCH(*this, "embed_ln0") {
         embed_ln0_kernel<<<R, kRowThreads, 0, stream>>>(emb, ln0_w, ln0_b, use_cursor ? ws.tok_list : ws.tokens, use_cursor ? ws.tok_pos : nullptr, R, C, V,
@@ -995,8 +1003,6 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
         return A;
     };
     float* vgate_buf = ws.xb;
-    const int chunks = plan.multi_row_segments ? wkv_step_chunks(plan.segs.data(), S, H, num_sms) : 0;
-    ensure_wkv_memory(*this, (size_t)chunks * H * kWcFloats * sizeof(float));
     for (int l = 0; l < NL; ++l) {
         const LayerW& L = layers[l];
         carve_layer(L, ops);
@@ -1074,7 +1080,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
                 // prefill chunks: vectors built by preparation warps, only state-dependent work in the per-token chain (wkv_seq.cuh)
                 // few (head, segment) pairs: a head over two CTAs
                 if (chunks > 0) {
-                    launch_wkv_chunks(*this, WkvArgs{ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, L.k_k, L.k_a, wkv, l == 0 ? st.v_first : nullptr, ws.yg, ws.wkv_tmp, S, H, C, ws.status}, chunks);
+                    launch_wkv_chunks(device, stream, use_pdl, WkvArgs{ws.seg_meta, ws.r, ws.k, ws.v, vgate, ws.vfirst, ws.w, ws.a, L.k_k, L.k_a, wkv, l == 0 ? st.v_first : nullptr, ws.yg, ws.wkv_tmp.as<float>(), S, H, C, ws.status}, chunks);
                 } else if (H * S <= num_sms) {
                     // Where every CTA can have an SM to itself it asks for more than half of the shared memory, so that no two share one:
                     // they would start in pairs as the predecessor's CTAs leave, and a pair takes a third longer (512 tokens, 40 heads).
@@ -1582,6 +1588,11 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
         chunks = T > 1 ? wkv_step_chunks(segs.data(), nseg, H, sms) : 0;
         for (size_t i = 0; i < (size_t)R * C && chunks; ++i)
             if (!(in[3][i] >= 0.5f && in[3][i] <= 1.0f)) chunks = 0;
+        if (chunks && device_malloc(&dtmp.p, (size_t)chunks * H * kWcFloats * sizeof(float)) != cudaSuccess) {
+            dtmp.p = nullptr;
+            cudaGetLastError();
+            chunks = 0;
+        }
         variant = chunks ? kChunked : T > 1 ? (n_items <= sms ? 3 : 4) : (n_items >= 4 * sms ? 2 : 1);
     }
     if (variant == 1) {
@@ -1596,11 +1607,7 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
         if (variant == kChunked) {
             for (int s2 = 0, before = 0; s2 < nseg; before += wkv_chunks_of(T), ++s2) segs[s2].pad = before;
             RSV_CUDA(cudaMemcpy(dseg.p, segs.data(), segs.size() * sizeof(SegMeta), cudaMemcpyHostToDevice));
-            RSV_CUDA(device_malloc(&dtmp.p, (size_t)chunks * H * kWcFloats * sizeof(float)));
-            RSV_CUDA(cudaDeviceSynchronize());  // (the launches below go to a stream of their own)
-            auto m = Model::create_bare(device);
-            launch_wkv_chunks(*m, WkvArgs{sm, r, k, v, vgate, vfirst, w, a, k_k, k_a, state, nullptr, yg, (float*)dtmp.p, nseg, H, C, status}, chunks);
-            RSV_CUDA(cudaStreamSynchronize(m->stream));
+            launch_wkv_chunks(device, nullptr, false, WkvArgs{sm, r, k, v, vgate, vfirst, w, a, k_k, k_a, state, nullptr, yg, (float*)dtmp.p, nseg, H, C, status}, chunks);
         } else if (variant == 3)
             wkv7_seq_kernel<2><<<dim3(2 * H, nseg), kWsThreads>>>(sm, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, state, nullptr, yg, H, C, status);
         else

@@ -61,8 +61,7 @@ struct Workspace {
     // operands of the tensor-core layers (operands.cuh) with their scales and sums, carved per step from one block
     uint8_t* op_mem = nullptr;
     size_t op_bytes = 0;
-    float* wkv_tmp = nullptr;  // a step's WKV chunks (wkv_chunk.cuh)
-    size_t wkv_bytes = 0;
+    SpareArea wkv_tmp;  // a step's WKV chunks (wkv_chunk.cuh)
     float *ymax = nullptr, *hmax = nullptr;  // [rows][parts] maxima of the time-mix output (per head) and of the ffn hidden vector (per M tile)
     float* samp_temp = nullptr;      // [outs, V] sampler work area
     uint32_t* samp_cnt = nullptr;    // [outs, V] penalty histogram
@@ -169,6 +168,8 @@ struct Model {
     ~Model();
 
     void ensure_workspace(int rows, int outs, int segs);
+    // WKV scratch for steps of up to `rows` rows in up to `segs` segments of up to `chunk` tokens; where there is no room such steps run without it
+    void reserve_prompt_scratch(int rows, int segs, int chunk);
     void upload_plan(const StepPlan& plan);
     // Runs one packed step.  Input tokens are read from ws.tokens[r] (or ws.tok_list[*tok_pos * R + r] when
     // `use_cursor`).  With out_rows non-empty, logits land in ws.logits[o, V] in out_rows order.

@@ -105,6 +105,26 @@ int main() {
         g_device = 1;
     }
     g_device = 0;
+    {
+        // a work area: slack, no reallocation below its size, the exact size where the slack does not fit, and a refusal instead of an error
+        SpareArea area;
+        int waits = 0;
+        auto idle = [&] { ++waits; };
+        CHECK(area.reserve(100 * MB, idle) && area.bytes() == 125 * MB && waits == 0, "first growth");
+        void* first = area.as<void>();
+        CHECK(area.reserve(125 * MB, idle) && area.as<void>() == first && waits == 0, "an area that was large enough moved");
+        CHECK(area.reserve(900 * MB, idle) && area.bytes() == 900 * MB && waits == 1 && g_free[0] == 100 * MB, "the exact size was not taken where the slack does not fit");
+        CHECK(!area.reserve(1100 * MB, idle) && area.bytes() == 0 && !area.as<void>() && waits == 2 && g_free[0] == 1000 * MB, "refused, and the old memory kept");
+        CHECK(area.reserve(200 * MB, idle) && area.bytes() == 250 * MB, "no use after a refusal");
+        area.release();
+        area.release();
+        auto pool = std::make_shared<StatePool>(0);
+        float* q = nullptr;
+        CHECK(device_malloc(&q, 500 * MB) == cudaSuccess, "no memory for a state");
+        pool->give(500 * MB, q);
+        CHECK(area.reserve(600 * MB, idle) && area.bytes() == 750 * MB, "the memory of freed states was not given back for it");
+        area.release();
+    }
     CHECK(g_free[0] == 1000 * MB, "%zu bytes of device 0 lost", 1000 * MB - g_free[0]);
     if (!bad) std::printf("device memory ok\n");
     return bad != 0;

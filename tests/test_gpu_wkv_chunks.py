@@ -61,3 +61,18 @@ def test_other_decays_go_token_by_token():
     y, s = rsv.op_wkv7(variant=0, **d)
     ref, sref = rsv.op_wkv7(variant=3, **d)
     assert np.array_equal(y, ref) and np.array_equal(s, sref) and np.isfinite(s).all()
+
+
+# The scratch of a prompt's chunks grows with the prompt: lengths up and down, against the same prompts in steps that are too short for the matrix form
+def test_prompts_of_growing_length(tmp_path):
+    b = rsv.ModelBuilder(rsv.write_synthetic(str(tmp_path / "m.st"), "tiny", seed=3)).build()
+    for n in (320, 336, 400, 512, 330, 511):
+        toks = np.random.default_rng(n).integers(0, 4096, size=n).astype(np.uint32)
+        b.reset()
+        lg = b.infer_chunked(toks, 512)
+        b.reset()
+        want = b.infer_chunked(toks, 256)
+        # fp32 through the layers in another summation order: a few ulps of the logits' scale per layer
+        assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n
+    b.state.close()
+    b.model.close()

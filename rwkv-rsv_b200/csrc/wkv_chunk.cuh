@@ -11,9 +11,11 @@
 // The triangular system does not involve the state, so it is solved for the right-hand sides kk^ and B v beforehand:
 //   u = S0 K + UV,  y = S0 R + YV   with   K = (1 - A)^-1 kk^,  UV = (1 - A)^-1 B v,  R = r^ + E K,  YV = E UV + F v.
 // Precision.  A model's decays lie in (0.545, 1] (exp(-sigmoid / sqrt(e))), so 1 / W stays below 1.7e4 and only products with W_t / W_s <= 1 are ever
-// summed.  Everything is fp32 but the running products and the joining of the products' 16-column sums (double).  Against the recurrence in 64 bits (512 tokens,
-// normal inputs) the state is off by 7.3e-8 relative and y by 1.04e-7, token by token in fp32 by 7.3e-8 and 0.99e-7; the sums are cut into short chains for that
-// (in the products, even and odd terms in the solution): 1.01e-7 and 1.85e-7 without.
+// summed.  Everything is fp32 but the running products and the joining of the products' 16-column sums (double), and the sums are cut into short chains (in the
+// products, even and odd terms in the solution; the state takes the sums of a chunk over u and over v, two roundings instead of seventeen).  Against the
+// recurrence in 64 bits (320 and 512 tokens, 8 heads, normal inputs; 1e-7 relative, token by token in fp32 in brackets):
+//   decays uniform in (0.545, 1): y 1.24 (1.30), state 0.72 (0.73);  all 0.545: 1.32 (1.50), 0.64 (0.67);  0.999 to 1: 1.67 (2.38), 1.65 (3.19);
+//   those of a random model: 1.36 (1.42), 1.02 (1.12).
 //
 //   wkv7_prepare_kernel  one CTA per (head, chunk), all chunks of the step at once: the vectors and K, R, UV, YV of a chunk -> scratch
 //   wkv7_chunk_kernel    two CTAs per (head, segment), 32 state rows each, chunk after chunk: two products with the state per chunk
@@ -345,17 +347,10 @@ __global__ void __launch_bounds__(kWcThreads) wkv7_chunk_kernel(const __grid_con
             }
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kWcConsumers) : "memory");
-        // ---- S = S0 diag(W) + sum u b + v k ----
+        // ---- S = S0 diag(W) + (sum u b + sum v k): the old state is rounded once per chunk, whatever its size against the sums ----
         const float *bz = X + kWcX + 16 * wc + 4 * lc, *kz = bz + T * 64, *vr = X + kWcHeadFloats + T * kWcRows + 4 * lr, *ur = us + 4 * lr;
         const float4 W = *reinterpret_cast<const float4*>(X + kWcX + kWcZ + 16 * wc + 4 * lc);
-        float D[4][4] = {};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            S[i][0] *= W.x;
-            S[i][1] *= W.y;
-            S[i][2] *= W.z;
-            S[i][3] *= W.w;
-        }
+        float B[4][4] = {}, D[4][4] = {};
 #pragma unroll
         for (int s = 0; s < T; ++s) {
             const float4 u = *reinterpret_cast<const float4*>(ur + s * kWcRows), v = *reinterpret_cast<const float4*>(vr + s * kWcRows);
@@ -363,10 +358,10 @@ __global__ void __launch_bounds__(kWcThreads) wkv7_chunk_kernel(const __grid_con
             const float uu[4] = {u.x, u.y, u.z, u.w}, vv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                S[i][0] = fmaf(uu[i], b.x, S[i][0]);
-                S[i][1] = fmaf(uu[i], b.y, S[i][1]);
-                S[i][2] = fmaf(uu[i], b.z, S[i][2]);
-                S[i][3] = fmaf(uu[i], b.w, S[i][3]);
+                B[i][0] = fmaf(uu[i], b.x, B[i][0]);
+                B[i][1] = fmaf(uu[i], b.y, B[i][1]);
+                B[i][2] = fmaf(uu[i], b.z, B[i][2]);
+                B[i][3] = fmaf(uu[i], b.w, B[i][3]);
                 D[i][0] = fmaf(vv[i], k.x, D[i][0]);
                 D[i][1] = fmaf(vv[i], k.y, D[i][1]);
                 D[i][2] = fmaf(vv[i], k.z, D[i][2]);
@@ -374,9 +369,12 @@ __global__ void __launch_bounds__(kWcThreads) wkv7_chunk_kernel(const __grid_con
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) S[i][j] += D[i][j];
+        for (int i = 0; i < 4; ++i) {
+            S[i][0] = fmaf(S[i][0], W.x, B[i][0]) + D[i][0];
+            S[i][1] = fmaf(S[i][1], W.y, B[i][1]) + D[i][1];
+            S[i][2] = fmaf(S[i][2], W.z, B[i][2]) + D[i][2];
+            S[i][3] = fmaf(S[i][3], W.w, B[i][3]) + D[i][3];
+        }
         __syncwarp();  // every lane has read the stage and the piece
         if (lane == 0) mbar_arrive(&empty[sl]);
     }

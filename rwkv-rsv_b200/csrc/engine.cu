@@ -887,11 +887,11 @@ bool reserve_wkv_chunks(Model& m, int chunks) {
 void launch_wkv_chunks(int device, cudaStream_t stream, bool pdl, const WkvArgs& A, int chunks) {
     static bool configured[16] = {false};
     if (!configured[device & 15]) {
-        RSV_CUDA(cudaFuncSetAttribute(wkv7_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWcSmemBytes));
+        RSV_CUDA(cudaFuncSetAttribute(wkv7_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWcSmemAlone));
         configured[device & 15] = true;
     }
     launch_pdl_on(stream, pdl, wkv7_prepare_kernel, dim3(A.H, chunks), dim3(kWcPrepThreads), 0, A);
-    launch_pdl_on(stream, pdl, wkv7_chunk_kernel, dim3(2 * A.H, A.nseg), dim3(kWcThreads), kWcSmemBytes, A);
+    launch_pdl_on(stream, pdl, wkv7_chunk_kernel, dim3(2 * A.H, A.nseg), dim3(kWcThreads), kWcSmemAlone, A);
 }
 int known_parts(int K) { return (K + 8 * kOpThreads - 1) / (8 * kOpThreads); }
 void launch_operand_known(Model& m, const float* x, int ldx, int K, const float* amax, int parts, const RowTiles& t, const RlOperandOut& o) {

@@ -21,16 +21,19 @@
 //   wkv7_chunk_kernel    two CTAs per (head, segment), 32 state rows each, chunk after chunk: two products with the state per chunk
 // GroupNorm, bonus and gate follow in wkv7_finish_kernel (wkv_seq.cuh).
 // What bounds it: shared memory.  A 16-byte read of a warp takes four cycles however many lanes want the same bytes; a chunk's products are 112 of them
-// per warp (a lane's tile is four rows x eight tokens, then four rows x four columns), 1800 cycles of the 3600 a chunk takes; the rest is the
-// chain products, barrier, sums, barrier, products.  512 tokens, 40 heads: 61 us and 27 to prepare; token by token 130.  201 tokens: 29 + 14 and 55.  4 x 128
-// tokens: 43 + 27 and 63, so several segments, which fill the GPU without it, stay with wkv7_seq_kernel.
+// per warp (a lane's tile is four rows x eight tokens, then four rows x four columns), 1800 cycles of the 3400 a chunk takes; the rest is the
+// chain products, barrier, sums, barrier, products.  512 tokens, 40 heads: 56 us and 27 to prepare; token by token 130.  201 tokens: 25 + 14 and 51.
+// A CTA asks for more than half of the shared memory, so that no two share an SM: what they need (103 KB) leaves room for two, and they were placed in pairs as the
+// predecessor's CTAs left, in some runs and not in others (320 tokens 58 us always, 512 tokens 57 or 90; alone 36 and 56).
 #pragma once
 #include "wkv_seq.cuh"
 
 namespace rsv {
 
 constexpr int kWcT = 16;       // tokens of a chunk
-constexpr int kWcMinLen = 320;  // tokens of the shortest segment: a layer (3B shape, int8) takes as long either way at 256, at 384 about 298 us token by token and 280, at 512 385 and 345
+// Tokens of the shortest segment.  A layer in us, token by token and in chunks (8, 40 and 64 heads): 96 tokens 84.8 and 86.1, 128.2 and 133.0, 178.4 and 185.6; 128 tokens
+// 98.0 and 96.6, 147.3 and 145.5, 204.3 and 204.9; 160 tokens 108.9 and 100.7, 166.9 and 162.2, 255.3 and 251.9; 256 tokens 138 and 120, 227 and 209, 320 and 309.
+constexpr int kWcMinLen = 160;
 constexpr int kWcRows = 32;    // state rows of a CTA
 constexpr int kWcXStride = 68;  // floats between the rows of K and R: eight lanes read eight rows, 16 bytes each, from different banks
 constexpr int kWcConsumers = 128;
@@ -45,6 +48,8 @@ constexpr int kWcStageFloats = kWcHeadFloats + kWcPart;
 constexpr int kWcSStride = 20;  // floats between rows of a warp's 32 x 16 piece of the state
 constexpr int kWcSumStride = 40;  // floats between the tokens of the warps' sums
 constexpr size_t kWcSmemBytes = (size_t)(kWcStages * kWcStageFloats + 4 * 2 * kWcT * kWcSumStride + 4 * kWcRows * kWcSStride + kWcT * kWcRows) * 4 + 128;
+constexpr size_t kWcSmemAlone = 120 * 1024;  // (see above)
+static_assert(kWcSmemBytes <= kWcSmemAlone);
 
 __host__ __device__ inline int wkv_chunks_of(int len) { return (len + kWcT - 1) / kWcT; }
 

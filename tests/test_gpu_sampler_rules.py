@@ -147,7 +147,8 @@ def test_rows_with_a_nan_or_an_infinity(v):
 @pytest.mark.parametrize("kept,top_k", [(1, 0), (7, 0), (8, 0), (9, 0), (16, 0), (17, 0), (65, 0), (512, 0), (8, 8), (13, 13), (9, 40), (33, 50), (700, 0)])
 def test_top_p_keeps_exactly_the_largest_that_reach_it(kept, top_k):
     rng = np.random.default_rng(kept)
-    V, rows = 4096, 400
+    V, n = 4096, min(kept, 512)  # (at most 512 picks)
+    rows = 400 if kept <= 33 else 24 * n  # the least likely of n kept tokens goes undrawn in 24 n draws with probability e^-18
     order = rng.permutation(V)
     logits = np.empty(V, np.float32)
     logits[order] = -1e-3 * np.arange(V, dtype=np.float32)  # nearly flat: every kept token is drawn sooner or later
@@ -159,9 +160,4 @@ def test_top_p_keeps_exactly_the_largest_that_reach_it(kept, top_k):
     got = rsv.op_sample(np.repeat(logits[None], rows, 0), np.stack([orc.pack_sampler(seed=77 * r + 1, top_p=top_p, top_k=top_k) for r in range(rows)])).astype(np.int64)
     rank = np.empty(V, np.int64)
     rank[order] = np.arange(V)
-    ranks, n = rank[got], min(kept, 512)  # (at most 512 picks)
-    assert ranks.max() <= n - 1
-    if n <= 17:
-        assert set(ranks.tolist()) == set(range(n))
-    else:
-        assert ranks.max() >= 0.9 * n - 1
+    assert set(rank[got].tolist()) == set(range(n))

@@ -50,7 +50,8 @@ struct RowMeta {
 };
 // A segment = consecutive rows of one session (1 row for decode, up to the chunk length for prefill).
 struct SegMeta {
-    int start, len, slot, pad;  // pad: chunks of sixteen tokens (wkv_chunk.cuh) in the segments before, filled in when a plan is uploaded
+    int start, len, slot;
+    int chunk0;  // chunks of sixteen tokens (wkv_chunk.cuh) in the segments before: filled in when a plan is uploaded
 };
 
 // Programmatic dependent launch.  A kernel launched with the programmatic-stream-serialization attribute may start

@@ -579,7 +579,7 @@ void Model::upload_plan(const StepPlan& plan) {
     SegMeta* sm = reinterpret_cast<SegMeta*>(p);
     for (int i = 0, chunks = 0; i < S; ++i) {
         sm[i] = plan.segs[i];
-        sm[i].pad = chunks;
+        sm[i].chunk0 = chunks;
         chunks += wkv_chunks_of(sm[i].len);
     }
     RSV_CUDA(cudaMemcpyAsync(ws.seg_meta, p, S * sizeof(SegMeta), cudaMemcpyHostToDevice, stream));
@@ -1605,7 +1605,7 @@ void engine_op_wkv7(int device, int variant, int nseg, int T, int H, const float
         wkv7_rows_kernel<<<ctas, kWrThreads, kWrSmemBytes>>>(map, 0LL, sm, n_items, r, k, v, vgate, vfirst, w, a, g, k_k, k_a, r_k, lnx_w, lnx_b, nullptr, yg, H, C, status, nullptr);
     } else {
         if (variant == kChunked) {
-            for (int s2 = 0, before = 0; s2 < nseg; before += wkv_chunks_of(T), ++s2) segs[s2].pad = before;
+            for (int s2 = 0, before = 0; s2 < nseg; before += wkv_chunks_of(T), ++s2) segs[s2].chunk0 = before;
             RSV_CUDA(cudaMemcpy(dseg.p, segs.data(), segs.size() * sizeof(SegMeta), cudaMemcpyHostToDevice));
             launch_wkv_chunks(device, nullptr, false, WkvArgs{sm, r, k, v, vgate, vfirst, w, a, k_k, k_a, state, nullptr, yg, (float*)dtmp.p, nseg, H, C, status}, chunks);
         } else if (variant == 3)

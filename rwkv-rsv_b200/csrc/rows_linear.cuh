@@ -84,12 +84,6 @@ __device__ __forceinline__ void cluster_sync_all() {
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// untiled bulk copy global -> shared memory of this CTA (16-byte aligned addresses and size)
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes),
-                 "r"(smem_u32(bar))
-                 : "memory");
-}
 template <int THREADS = kRlEpiThreads>
 __device__ __forceinline__ void rl_epi_sync() {
     asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");

@@ -55,7 +55,7 @@ __host__ __device__ inline int wkv_chunks_of(int len) { return (len + kWcT - 1) 
 
 // The inputs of the WKV kernels of a step (token rows [R, C]) and the head parameters [C].
 struct WkvArgs {
-    const SegMeta* segs;  // pad: chunks of the segments before
+    const SegMeta* segs;  // chunk0: chunks of the segments before
     const float *r, *k, *v, *vgate, *vfirst, *w, *a;
     const float *k_k, *k_a;
     float *state, *v_first_state, *yg, *tmp;
@@ -90,11 +90,11 @@ __global__ void __launch_bounds__(kWcPrepThreads, 5) wkv7_prepare_kernel(const _
     int lo = 0, hi = P.nseg;  // the last segment with at most `chunk` chunks before it
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (P.segs[mid].pad <= chunk) lo = mid;
+        if (P.segs[mid].chunk0 <= chunk) lo = mid;
         else hi = mid;
     }
     const SegMeta sg = P.segs[lo];
-    const int t0 = (chunk - sg.pad) * T, nt = min(T, sg.len - t0);
+    const int t0 = (chunk - sg.chunk0) * T, nt = min(T, sg.len - t0);
     const int c = tid & (N - 1), half = tid >> 6, hc = h * N, C = P.C;  // thread: channel c, tokens 8 half .. 8 half + 7
     const float kkc = P.k_k[hc + c], kac = P.k_a[hc + c];
     pdl_wait();
@@ -239,12 +239,6 @@ __global__ void __launch_bounds__(kWcPrepThreads, 5) wkv7_prepare_kernel(const _
     }
 }
 
-__device__ __forceinline__ void wc_bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes),
-                 "r"(smem_u32(bar))
-                 : "memory");
-}
-
 // Grid (2 H, segments).  Four consumer warps, one producer.  Warp wc has columns 16 wc .. 16 wc + 15 of the CTA's 32 rows, in registers (four rows x
 // four columns per lane) and, for the products with K and R, in shared memory.
 __global__ void __launch_bounds__(kWcThreads) wkv7_chunk_kernel(const __grid_constant__ WkvArgs P) {
@@ -283,7 +277,7 @@ __global__ void __launch_bounds__(kWcThreads) wkv7_chunk_kernel(const __grid_con
     if (wc == 4) {
         // ---- producer: chunk n -> stage n mod 3 ----
         if (lane == 0) {
-            const float* src = pdl_fresh(P.tmp) + ((size_t)sg.pad * H + h) * kWcFloats;
+            const float* src = pdl_fresh(P.tmp) + ((size_t)sg.chunk0 * H + h) * kWcFloats;
             int n = 0;
 #pragma unroll 1
             for (; n < nc; ++n, src += (size_t)H * kWcFloats) {
@@ -291,8 +285,8 @@ __global__ void __launch_bounds__(kWcThreads) wkv7_chunk_kernel(const __grid_con
                 if (n >= kWcStages && !mbar_wait(&empty[sl], (uint32_t)(n / kWcStages - 1) & 1u, abort_flag)) break;
                 float* dst = stage + sl * kWcStageFloats;
                 mbar_expect_tx(&full[sl], kWcStageFloats * 4);
-                wc_bulk_load(dst, src, kWcHeadFloats * 4, &full[sl]);
-                wc_bulk_load(dst + kWcHeadFloats, src + kWcHeadFloats + part * kWcPart, kWcPart * 4, &full[sl]);
+                bulk_load(dst, src, kWcHeadFloats * 4, &full[sl]);
+                bulk_load(dst + kWcHeadFloats, src + kWcHeadFloats + part * kWcPart, kWcPart * 4, &full[sl]);
             }
             if (*abort_flag)  // copies in flight land before the CTA may exit
                 for (int m = max(0, n - kWcStages); m < n; ++m)

@@ -47,7 +47,7 @@
 // than a fifth; and nothing should spill: with the shared memory taken, the threads' stacks do not fit L1 and every spill is an L2 round
 // trip (0.07 ms of a token's 1.40 with 128 bytes of spills; up to 2560 channels nothing does, the 4096-channel instantiation spills as much).
 // Measured per token at 2560 channels, 32 layers, 65536 rows of vocabulary: int8 1.30 ms (3.0 GB: 0.47 ms at copy bandwidth), fp16
-// 1.81 ms; 1.49 and 1.90 ms with a grid barrier after every phase and a tile of rows per warp; int8 per group 1.53 ms.  512 channels, 12 layers:
+// 1.81 ms; 1.49 and 1.90 ms with a grid barrier after every phase and a tile of rows per warp; int8 per group 1.53 ms.  512 channels, 4 layers:
 // 0.09 ms (0.13).  4096 channels, 32 layers: int8 2.47 ms.
 // All waits are bounded; on expiry bit 5 of the status word is set (and the word after it says which wait), every role drains its copies in flight and exits.
 #pragma once

@@ -18,7 +18,7 @@
 // next kernel of the step becomes resident early and requests its weights before the dependency wait.  (The exception: split tiles of
 // more than 108 rows of fp16 weights, whose partial sums take up to 128 KB; one of them is resident.)
 // All problems of a launch are cut alike.  (fp16 rank projections next to int8 matrices were cut in two at most: twenty K blocks through a ring of
-// five were the longest chain of the launch with r, k and v; 3 rows, 2560 channels, 32 layers: a step of 1.73 ms, now 1.66.)
+// five were the longest chain of the launch with r, k and v; 3 rows, 2560 channels, 32 layers: a step of 1.74 ms, now 1.67.)
 // What bounds it: at few rows the chain operand tiles (L2) -> products -> exchange -> store behind the dependency wait, the weights
 // are there already; at 64 rows the operand tiles' L2 traffic as well (a 128-row tile re-reads them all).
 //
@@ -545,14 +545,16 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     }
 }
 
-// Many rows (several row tiles; per-row int8 and fp16 weights): one persistent CTA per SM takes tiles of 128 weight rows x up to 64
-// activation rows in turn, whole K.  One ring of stages runs through all of them and there are two accumulators, so the tensor core
-// works on the next tile while the epilogue warps finish the last one.  With a CTA per tile (two resident) both CTAs of an SM ran in
+// Several row tiles (per-row int8 weights; fp16 weights in tiles of more than 64 rows or cut for turns), and heads of one row tile: one persistent CTA per SM takes tiles of 128
+// weight rows x up to 64 activation rows (fp16: 128) in turn, whole K.  One ring of stages runs through all of them and there are two accumulators, so the
+// tensor core works on the next tile while the epilogue warps finish the last one.  With a CTA per tile (two resident) both CTAs of an SM ran in
 // step: of a tile's 22 us at K = 2560 the tensor core worked 13 at 85 % of its rate, the rest was the first loads and the epilogue.
-// Measured, 2560 x 10240 (ffn.key): int8, 1024 rows 139 -> 94 us, 512 rows 82 -> 56 us (46 with sixteen epilogue warps: eight took longer over a tile
-// than the tensor core over its 20 K blocks).  What bounds it: the traffic of a K block, 48 KB from L2 for 512 cycles of products (an SM draws about 70
-// bytes per cycle; the copies alone take 85 % of the time, the products alone 75 %).  Tried without gain: four producer threads, six stages instead
-// of four, weights asked into L2 a turn ahead.
+// Measured, 2560 x 10240 (ffn.key), int8: 1024 rows 139 us with a CTA per tile, now 80; 512 rows 82 and 44.  Sixteen epilogue warps: eight took longer over a
+// tile than the tensor core over its 20 K blocks (512 rows 48; up to 128 rows there are eight all the same, see the launch).
+// What bounds it: no part alone.  512 rows with parts switched off (us): ffn.key 46, copies alone 35, products and epilogue alone 40; ffn.value 49, 43 and 37.  Without
+// the operands' copies, over half of the traffic, 45 and 48; with one matrix instruction of four 41 and 42; without the epilogue 41 and 44.  The tensor
+// pipe is active in 41 to 63 % of an SM's cycles; copies and products meet in shared memory, and a turn's start and last epilogue are not covered.  Tried
+// without gain: four producer threads, six stages instead of four, weights asked into L2 a turn ahead.
 struct RlCursor {
     int job, pi, kb, nk, mt, ntile;
     __device__ __forceinline__ void set(const RlLaunch& L, int j) {

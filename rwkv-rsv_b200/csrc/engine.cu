@@ -851,7 +851,7 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
 bool rl_builds(const LinearW& W, const RowTiles& t) { return t.n == 1 && t.R <= 16 && rl_fmt(W) == RL_F16 && (size_t)((W.K + 63) / 64) * t.nt16 * 128 <= 44 * 1024; }
 
 void launch_ln_operands(Model& m, const char* name, const LnOperandsArgs& A) {
-    const int threads = std::max(kLnSumThreads, (int)round_up((size_t)(A.C / 8), 32));
+    const int threads = (int)round_up((size_t)(A.C / 8), 32);
     // few rows: a CTA per (row, output), each repeating the row statistics; as rows fill the GPU a CTA takes several outputs (more
     // than two CTAs per SM would have to wait for the predecessor's to leave)
     const int gy = std::max(1, std::min(A.nout, 2 * m.num_sms / std::max(A.R, 1)));
@@ -862,10 +862,9 @@ void launch_ln_operands(Model& m, const char* name, const LnOperandsArgs& A) {
         }
         return;
     }
-    const size_t smem = (size_t)A.C * 4 * (A.rows ? 2 : 1);
-    if (smem > 40 * 1024) RSV_CUDA(cudaFuncSetAttribute(ln_operands_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 8 * kLnMaxThreads * 4));
+    void (*kernel)(LnOperandsArgs) = threads <= 320 ? ln_operands_kernel<320, 3> : threads <= 512 ? ln_operands_kernel<512, 2> : ln_operands_kernel<kLnMaxThreads, 1>;
     LAUNCH(m, name) {
-        launch_pdl(m, ln_operands_kernel, dim3(A.R + A.nseg, gy), dim3(threads), smem, A);
+        launch_pdl(m, kernel, dim3(A.R + A.nseg, gy), dim3(threads), 0, A);
         check_launch("ln_operands");
     }
 }

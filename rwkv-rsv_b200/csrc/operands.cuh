@@ -123,6 +123,10 @@ __device__ __forceinline__ long long rl_group_sum(int ts) {
 // segment's first row still has to read the old one; the CTAs past the rows commit the staging area of the block before this one.
 // What bounds it: at few rows the chain load -> mean -> variance -> row maximum -> digits (block-wide reductions); it writes operands instead of fp32 because the
 // conversion in a kernel of its own cost a second launch and a second such chain (8 rows, n_embd 2560: 11.0 + 9.2 us for the two kernels it replaces, CUDA events around each).
+// Cycles after the dependency wait at 3 rows: loads 1500, two sums of 700, normalising 700, maxima 360, digits 1800, sum of digits 500; 512 rows of six
+// outputs are bound by the digits.  The row stays in registers (in shared memory the sums took 1.4 us, and the kernel's 20 KB kept the next launch's CTAs
+// off its SMs) and the outputs' maxima meet behind one barrier: 2560 channels, exclusive us in the step, 3 rows 4.6 -> 4.3, 512 rows and one
+// output 15.2 -> 13.2, six outputs 27.3 -> 26.0.
 struct LnOperandsArgs {
     const float *x_in, *delta;
     float* x_out;
@@ -137,38 +141,34 @@ struct LnOperandsArgs {
     RlOperandOut out[7];
 };
 constexpr int kLnMaxThreads = 1024;  // n_embd up to 8192 (ln_operands_wide_kernel: any)
-constexpr int kLnSumThreads = 256;  // threads that take part in the row sums (the others only hold channels)
-// Sums of (x - c0) or (x - c0)^2 over the row in shared memory, and of the previous token's row when there is one: thread t adds
-// elements t, t + 256, ..., then shuffles, then the eight warps in order.  (The order is the same at every block size and number of rows.)
-template <bool SQUARE>
-__device__ __forceinline__ void ln_row_sums(const float* rows, int nrows, int C, const float (&c0)[2], float (&sum)[2], float (*red)[kLnSumThreads / 32]) {
-    if (threadIdx.x < kLnSumThreads) {
-#pragma unroll 1
-        for (int w = 0; w < nrows; ++w) {
-            const float* row = rows + (size_t)w * C + threadIdx.x;
-            const float c = w ? c0[1] : c0[0];
-            float a = 0.f;
-#pragma unroll 5
-            for (int i = threadIdx.x; i < C; i += kLnSumThreads, row += kLnSumThreads) {
-                const float d = *row - c;
-                a += SQUARE ? d * d : *row;
-            }
-            a = warp_sum(a);
-            if ((threadIdx.x & 31) == 0) red[w][threadIdx.x >> 5] = a;
-        }
+constexpr int kLnSumThreads = 256;  // the wide kernel: threads that take part in the row sums
+// Sums over the block of a (the row) and, where `two`, of b (the previous token's row): shuffles, then every warp adds the warps' sums.  The order depends on
+// the row's length alone, so a row gives the same bits as itself and as somebody's previous token, whatever the step.
+__device__ __forceinline__ void ln_block_sums(float& a, float& b, bool two, float (&red)[2][32], int warp, int lane, int nw) {
+    a = warp_sum(a);
+    if (two) b = warp_sum(b);
+    if (lane == 0) {
+        red[0][warp] = a;
+        red[1][warp] = b;
     }
     __syncthreads();
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        sum[w] = 0.f;
-        if (w < nrows)
-#pragma unroll
-            for (int i = 0; i < kLnSumThreads / 32; ++i) sum[w] += red[w][i];
-    }
+    a = warp_sum(lane < nw ? red[0][lane] : 0.f);
+    if (two) b = warp_sum(lane < nw ? red[1][lane] : 0.f);
 }
-__global__ void __launch_bounds__(kLnMaxThreads) ln_operands_kernel(const __grid_constant__ LnOperandsArgs A) {
-    extern __shared__ __align__(16) float ln_rows_smem[];  // the row and the previous token's
-    __shared__ float red[2][2][kLnSumThreads / 32];
+__device__ __forceinline__ float ln_sum8(const float (&v)[8]) { return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])); }
+__device__ __forceinline__ float ln_square8(const float (&v)[8]) {
+    float q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = v[i] * v[i];
+    return ln_sum8(q);
+}
+__device__ __forceinline__ void ln_weights8(float (&v)[8], const float* p) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p + 4));
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+template <int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __grid_constant__ LnOperandsArgs A) {
+    __shared__ float red[2][2][32];
     __shared__ float redm[7][32];
     __shared__ long long redt[7][32];
     pdl_launch_dependents();
@@ -192,20 +192,21 @@ __global__ void __launch_bounds__(kLnMaxThreads) ln_operands_kernel(const __grid
     const bool shift = A.rows != nullptr, pln = shift && rm.has_prev;
     // weights: requested before the dependency wait
     float lw[8], lb[8], mx[8];
-    rl_load8(lw, A.lw + kc);
-    rl_load8(lb, A.lb + kc);
-    const float* mix = A.out[blockIdx.y].mix;
-    if (mix) rl_load8(mx, mix + kc);
+    ln_weights8(lw, A.lw + kc);
+    ln_weights8(lb, A.lb + kc);
+    const int o0 = blockIdx.y, step = gridDim.y;
+    if (A.out[o0].mix) ln_weights8(mx, A.out[o0].mix + kc);
     const int rloc = r % A.rt, rtile = r / A.rt;
     pdl_wait();
     const float* xr = A.x_in + row * C + kc;
     const float* dr = A.delta ? A.delta + row * C + kc : nullptr;
-    float x[8], xp[8], d[8];
+    float x[8], xp[8];
     rl_load8(x, xr);
 #pragma unroll
     for (int i = 0; i < 8; ++i) xp[i] = 0.f;
     if (shift) rl_load8(xp, pln ? xr - C : A.shift_state + (size_t)rm.slot * C + kc);
     if (dr) {
+        float d[8];
         rl_load8(d, dr);
 #pragma unroll
         for (int i = 0; i < 8; ++i) x[i] += d[i];
@@ -215,53 +216,56 @@ __global__ void __launch_bounds__(kLnMaxThreads) ln_operands_kernel(const __grid
             for (int i = 0; i < 8; ++i) xp[i] += d[i];
         }
     }
-    float* xs = ln_rows_smem;
-    if (on) {
-        const float4 a = make_float4(x[0], x[1], x[2], x[3]), b = make_float4(x[4], x[5], x[6], x[7]);
-        *reinterpret_cast<float4*>(xs + k0) = a;
-        *reinterpret_cast<float4*>(xs + k0 + 4) = b;
-        if (pln) {
-            *reinterpret_cast<float4*>(xs + C + k0) = make_float4(xp[0], xp[1], xp[2], xp[3]);
-            *reinterpret_cast<float4*>(xs + C + k0 + 4) = make_float4(xp[4], xp[5], xp[6], xp[7]);
-        }
-        if (A.x_out && blockIdx.y == 0) {
-            float4* o = reinterpret_cast<float4*>(A.x_out + row * C + k0);
-            o[0] = a;
-            o[1] = b;
-        }
+    if (A.x_out && on && o0 == 0) {
+        float4* o = reinterpret_cast<float4*>(A.x_out + row * C + k0);
+        o[0] = make_float4(x[0], x[1], x[2], x[3]);
+        o[1] = make_float4(x[4], x[5], x[6], x[7]);
     }
-    __syncthreads();
-    float mean[2] = {0.f, 0.f}, var[2];
-    ln_row_sums<false>(xs, pln ? 2 : 1, C, mean, var, red[0]);
-    mean[0] = var[0] / (float)C;
-    mean[1] = var[1] / (float)C;
-    ln_row_sums<true>(xs, pln ? 2 : 1, C, mean, var, red[1]);
-    const float inv = 1.0f / sqrtf(var[0] / (float)C + kLnEps), pinv = 1.0f / sqrtf(var[1] / (float)C + kLnEps);
+    float s0 = on ? ln_sum8(x) : 0.f, s1 = on ? ln_sum8(xp) : 0.f;
+    ln_block_sums(s0, s1, pln, red[0], warp, lane, nw);
+    s0 /= (float)C;
+    s1 /= (float)C;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        x[i] = (x[i] - mean[0]) * inv * lw[i] + lb[i];                    // cur
-        if (pln) xp[i] = (xp[i] - mean[1]) * pinv * lw[i] + lb[i];  // prev
-        xp[i] -= x[i];                                              // prev - cur
+        x[i] -= s0;
+        if (pln) xp[i] -= s1;
     }
-    if (shift && rm.is_last && on && blockIdx.y == 0) {
+    s0 = on ? ln_square8(x) : 0.f;
+    s1 = on ? ln_square8(xp) : 0.f;
+    ln_block_sums(s0, s1, pln, red[1], warp, lane, nw);
+    s0 = 1.0f / sqrtf(s0 / (float)C + kLnEps);
+    s1 = 1.0f / sqrtf(s1 / (float)C + kLnEps);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        x[i] = x[i] * s0 * lw[i] + lb[i];                  // cur
+        if (pln) xp[i] = xp[i] * s1 * lw[i] + lb[i];  // prev
+        xp[i] -= x[i];                                     // prev - cur
+    }
+    if (shift && rm.is_last && on && o0 == 0) {
         float4* o = reinterpret_cast<float4*>(A.staging + (size_t)rm.seg * C + k0);
         o[0] = make_float4(x[0], x[1], x[2], x[3]);
         o[1] = make_float4(x[4], x[5], x[6], x[7]);
     }
+    // the outputs' maxima, behind one barrier
 #pragma unroll 1
-    for (int o = blockIdx.y; o < A.nout; o += gridDim.y) {
-        const RlOperandOut& O = A.out[o];
-        if (o != (int)blockIdx.y && O.mix) rl_load8(mx, O.mix + kc);
-        float v[8], am = 0.f;
+    for (int o = o0; o < A.nout; o += step) {
+        const float* mix = A.out[o].mix;
+        if (o != o0 && mix) ln_weights8(mx, mix + kc);
+        float am = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] = O.mix ? x[i] + mx[i] * xp[i] : x[i];
-            am = fmaxf(am, fabsf(v[i]));
-        }
+        for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(mix ? x[i] + mx[i] * xp[i] : x[i]));
         am = warp_absmax(on ? am : 0.f);
         if (lane == 0) redm[o][warp] = am;
-        __syncthreads();
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int o = o0; o < A.nout; o += step) {
+        const RlOperandOut& O = A.out[o];
+        if (o0 + step < A.nout && O.mix) ln_weights8(mx, O.mix + kc);
         const int ex = rl_scale_exp(warp_absmax(lane < nw ? redm[o][lane] : 0.f)), fmt = O.fmt, lk = fmt == RL_F16 ? 6 : 7;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = O.mix ? x[i] + mx[i] * xp[i] : x[i];
         int ts = 0;
         if (on)
             ts = rl_put8(fmt, O.img + ((size_t)rtile * O.kblocks + (k0 >> lk)) * (size_t)(O.nt * 128), rloc * rl_cols(fmt), k0 & ((1 << lk) - 1), v, rl_mult(fmt, ex));
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(kLnMaxThreads) ln_operands_kernel(const __grid
     __syncthreads();
 #pragma unroll 1
     for (int o = warp; o < A.nout; o += nw)
-        if (o % (int)gridDim.y == (int)blockIdx.y && A.out[o].fmt == RL_I8) {
+        if (o % step == o0 && A.out[o].fmt == RL_I8) {
             long long t = lane < nw ? redt[o][lane] : 0;
 #pragma unroll
             for (int i = 16; i > 0; i >>= 1) t += __shfl_xor_sync(0xffffffffu, t, i);

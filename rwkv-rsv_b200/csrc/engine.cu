@@ -1029,16 +1029,18 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
             float* ma = mw + cfg.w_mid;
             float* mv = ma + cfg.a_mid;
             float* mg = mv + cfg.v_mid;
-            RlReq q[7] = {
-                {&L.Wr, &ops.r, ws.r, C, EPI_STORE},
-                {&L.Wk, &ops.k, ws.k, C, EPI_STORE},
-                {&L.Wv, &ops.v, ws.v, C, EPI_STORE, nullptr, l == 0 ? ws.vfirst : nullptr},
+            // The rank projections come first: an fp16 row has twice the K blocks of an int8 one, and the last few clusters of the launch find room only when
+            // the LayerNorm's CTAs leave (3 rows, 2560 int8 channels: the launch 8.2 -> 6.4 us, a layer 46.6 -> 44.8).
+            const RlReq q[7] = {
+                {&L.v1, &ops.vr, mv, MIDS, EPI_STORE},  // (layers > 0)
                 {&L.w1, &ops.w, mw, MIDS, EPI_TANH},
                 {&L.a1, &ops.a, ma, MIDS, EPI_STORE},
                 {&L.g1, &ops.g, mg, MIDS, EPI_SIGMOID},
-                {&L.v1, &ops.vr, mv, MIDS, EPI_STORE},
+                {&L.Wr, &ops.r, ws.r, C, EPI_STORE},
+                {&L.Wk, &ops.k, ws.k, C, EPI_STORE},
+                {&L.Wv, &ops.v, ws.v, C, EPI_STORE, nullptr, l == 0 ? ws.vfirst : nullptr},
             };
-            run_rows_linear(*this, "linear_rkv_rank", q, l == 0 ? 6 : 7, tr);
+            run_rows_linear(*this, "linear_rkv_rank", q + (l == 0), 7 - (l == 0), tr);
             // back-projections: decay w, a, gate g and (layers > 0) the v-lerp gate
             const int nb = l == 0 ? 3 : 4;
             const LinearW* Wb[4] = {&L.w2, &L.a2, &L.g2, &L.v2};

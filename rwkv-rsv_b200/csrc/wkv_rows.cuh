@@ -6,7 +6,9 @@
 //   * everything an item needs arrives through one mbarrier, requested as soon as the previous item's copy is in registers: the 16 KB state as two TMA boxes (64 rows x 128
 //     bytes, SWIZZLE_128B: a lane reads its 128-byte row segment chunk by chunk without bank conflicts), the first token's
 //     eight input vectors and the head's five parameter vectors as 256-byte bulk copies.  No load of an iteration depends on
-//     another load: with the memory system loaded a dependent global load costs microseconds per item;
+//     another load: with the memory system loaded a dependent global load costs microseconds per item.  The first item's state and
+//     parameters, which no kernel of the step writes, are requested before the dependency wait (16 sessions of 40 heads 9.4 -> 8.2 us, 64
+//     20.6 -> 18.2);
 //   * the updated rows leave through a staging tile and TMA stores;
 //   * six warp pairs per CTA walk their own item streams (a head's chain of reductions and barriers is long and a thread holds
 //     64 state registers, so the pairs are what hides latency: 96 KB of state reads in flight per SM); they share nothing but
@@ -20,6 +22,10 @@ namespace rsv {
 
 constexpr int kWrPairs = 6;
 constexpr int kWrThreads = 64 * kWrPairs;
+// From how many (session, head) pairs per SM on a step takes this kernel.  Its pairs go in rounds of six per SM, 5.8 us each, and its shared memory keeps the
+// next kernels' CTAs, which would fetch weights meanwhile, off the SM.  A layer of 40 heads and 2560 int8 channels with wkv7_kernel and with this
+// one (us): 16 sessions 57.8 and 58.0, 20 63.5 and 62.9, 24 67.1 and 70.1, 32 74.6 and 76.8, 40 85.1 and 84.6.
+constexpr int kWrItemsPerSm = 10;
 constexpr int kWrStages = 1;               // load stages per pair (plus one staging tile for the stores)
 constexpr int kWrTileFloats = 64 * 32;     // one TMA box: 64 rows x 32 columns
 constexpr int kWrStateBytes = 2 * kWrTileFloats * 4;
@@ -67,6 +73,32 @@ __global__ void __launch_bounds__(kWrThreads, 1) wkv7_rows_kernel(const __grid_c
     }
     __syncthreads();
     pdl_launch_dependents();
+    const int nvec = vgate ? kWrVecs : kWrVecs - 2;
+    // segment descriptors run three items ahead in registers: the leader's copy addresses must not wait for a load of their own
+    auto meta_of = [&](int n) { return n < my_items ? segs[(first + n * stride) / H] : SegMeta{0, 0, 0, 0}; };
+    auto issue_state = [&](int n, const SegMeta& sg) {  // the pair's leader only: what no kernel of this step writes
+        const int st = n % kWrStages, item = first + n * stride, h = item % H;
+        const int y = (int)(row0 + ((long long)sg.slot * H + h) * N);
+        uint64_t* bar = &full[pair * kWrStages + st];
+        uint8_t* dst = my + (size_t)st * kWrStageBytes;
+        float* vdst = reinterpret_cast<float*>(dst + kWrStateBytes);
+        mbar_expect_tx(bar, (uint32_t)(kWrStateBytes + nvec * 256));
+        tma_load_2d(&smap, bar, dst, 0, y);
+        tma_load_2d(&smap, bar, dst + kWrTileFloats * 4, 32, y);
+        const float* pr[5] = {k_k, k_a, r_k, lnx_w, lnx_b};
+        for (int i = 0; i < 5; ++i) bulk_load_256(vdst + (8 + i) * N, pr[i] + (size_t)h * N, bar);
+    };
+    auto issue_vectors = [&](int n, const SegMeta& sg) {  // ... and the vectors that the kernels before leave
+        const int st = n % kWrStages, h = (first + n * stride) % H;
+        float* vdst = reinterpret_cast<float*>(my + (size_t)st * kWrStageBytes + kWrStateBytes);
+        const size_t hb = (size_t)sg.start * C + (size_t)h * N;
+        const float* in[8] = {r, k, v, w, a, g, vgate, vfirst};
+        for (int i = 0; i < (vgate ? 8 : 6); ++i) bulk_load_256(vdst + i * N, in[i] + hb, &full[pair * kWrStages + st]);
+    };
+    SegMeta sg0 = meta_of(0), sg1 = meta_of(1), sg2 = meta_of(2);
+    // the first items' states are requested before the dependency wait
+    if (leader)
+        for (int n = 0; n < min(kWrStages, my_items); ++n) issue_state(n, n ? sg1 : sg0);
     pdl_wait();  // the input vectors come from the predecessor kernels
     r = pdl_fresh(r);
     k = pdl_fresh(k);
@@ -76,29 +108,8 @@ __global__ void __launch_bounds__(kWrThreads, 1) wkv7_rows_kernel(const __grid_c
     w = pdl_fresh(w);
     a = pdl_fresh(a);
     g = pdl_fresh(g);
-    const int nvec = vgate ? kWrVecs : kWrVecs - 2;
-    // segment descriptors run three items ahead in registers: the leader's copy addresses must not wait for a load of their own
-    auto meta_of = [&](int n) { return n < my_items ? segs[(first + n * stride) / H] : SegMeta{0, 0, 0, 0}; };
-    auto issue_load = [&](int n, const SegMeta& sg) {  // the pair's leader only
-        const int st = n % kWrStages, item = first + n * stride, h = item % H;
-        const int y = (int)(row0 + ((long long)sg.slot * H + h) * N);
-        uint64_t* bar = &full[pair * kWrStages + st];
-        uint8_t* dst = my + (size_t)st * kWrStageBytes;
-        float* vdst = reinterpret_cast<float*>(dst + kWrStateBytes);
-        mbar_expect_tx(bar, (uint32_t)(kWrStateBytes + nvec * 256));
-        tma_load_2d(&smap, bar, dst, 0, y);
-        tma_load_2d(&smap, bar, dst + kWrTileFloats * 4, 32, y);
-        const size_t hb = (size_t)sg.start * C + (size_t)h * N;
-        const float* in[8] = {r, k, v, w, a, g, vgate, vfirst};
-        for (int i = 0; i < (vgate ? 8 : 6); ++i) bulk_load_256(vdst + i * N, in[i] + hb, bar);
-        const float* pr[5] = {k_k, k_a, r_k, lnx_w, lnx_b};
-        for (int i = 0; i < 5; ++i) bulk_load_256(vdst + (8 + i) * N, pr[i] + (size_t)h * N, bar);
-    };
-    SegMeta sg0 = meta_of(0), sg1 = meta_of(1), sg2 = meta_of(2);
-    if (leader) {
-        if (my_items > 0) issue_load(0, sg0);
-        if (kWrStages > 1 && my_items > 1) issue_load(1, sg1);
-    }
+    if (leader)
+        for (int n = 0; n < min(kWrStages, my_items); ++n) issue_vectors(n, n ? sg1 : sg0);
     float* sv = svec + (size_t)pair * 5 * N;  // both warps of the pair write the same five vectors (identical values) and read them back
     float* pred = red + pair * 4;
     for (int n = 0; n < my_items; ++n) {
@@ -139,7 +150,10 @@ __global__ void __launch_bounds__(kWrThreads, 1) wkv7_rows_kernel(const __grid_c
         const float rkc0 = vs[10 * N + lane], rkc1 = vs[10 * N + lane + 32], gw = vs[11 * N + rr], gb = vs[12 * N + rr];
         // the stage is free once both warps hold its contents: the data of item n + 2 may land in it
         wr_pair_sync(pair);
-        if (leader && n + kWrStages < my_items) issue_load(n + kWrStages, kWrStages == 1 ? sg1 : sg2);
+        if (leader && n + kWrStages < my_items) {
+            issue_state(n + kWrStages, kWrStages == 1 ? sg1 : sg2);
+            issue_vectors(n + kWrStages, kWrStages == 1 ? sg1 : sg2);
+        }
         for (int t = 0; t < sg.len; ++t) {
             const size_t hb = (size_t)(sg.start + t) * C + hc;
             WkvIn nx = cur;

@@ -121,6 +121,24 @@ __device__ __forceinline__ float rl_rowmax4(const float (&a)[4], bool mine, int 
 }
 // exact integer (|q| < 2^51) -> double without the slow 64-bit conversion
 __device__ __forceinline__ double rl_ll2d(long long q) { return __longlong_as_double(0x4338000000000000LL + q) - 6755399441055744.0; }
+// An int8 output from the exact sum Q = sum_k q_k t_k and 128 T, T = sum_k t_k: xs (ws Q + wz T), rounded once.  Files quantised symmetrically around code 128 have
+// wz = -128 ws (`sym`, the same for a warp): then it is xs ws (Q - 128 T), the integer in a multiple of 2^23 and 23 bits, whose products meet before the
+// rounding (exact but for 2^-25 up to |Q - 128 T| < 2^47, typically 2^37).  In fp64, which other files take, the arithmetic holds the tensor pipe up: 512 rows of
+// 2560 -> 10240 45.4 us, without any arithmetic 38.6.
+struct RlScale {
+    float ws, wz;
+    bool sym;
+};
+__device__ __forceinline__ RlScale rl_scale(float ws, float wz) { return RlScale{ws, wz, (bool)__all_sync(0xffffffffu, wz == -128.0f * ws)}; }
+__device__ __forceinline__ float rl_value8(const RlScale& w, float xs, long long q, long long t128) {
+    if (w.sym) {
+        const long long d = q - t128;
+        const float hi = (float)(int)(d >> 23), lo = __uint_as_float(0x4B000000u | ((uint32_t)d & 0x7FFFFFu)) - 8388608.0f, w23 = w.ws * 8388608.0f;
+        const float p = w23 * hi;
+        return xs * (p + fmaf(w.ws, lo, fmaf(w23, hi, -p)));
+    }
+    return (float)((double)xs * ((double)w.ws * rl_ll2d(q) + (double)w.wz * (rl_ll2d(t128) * 0.0078125)));
+}
 __device__ __forceinline__ long long rl_digits2q(int i0, int i1, int i2, int i3) {
     return ((long long)i0 * 128 + i1) * 16384 + ((long long)i2 * 128 + i3);
 }
@@ -147,7 +165,7 @@ __device__ __forceinline__ RlOut rl_out(const RlProb& P, int r0, int nr, int m, 
 // The sums of a tile whose K was not split, from tensor memory through the thread's registers to the output, rows rl .. rl + 3 at a time
 // (`turn`: the WARPS / 4 warps of a lane quarter take turns).  What bounds this is the latency of its instructions: a warp issues one in eight cycles.
 template <int WARPS>
-__device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t taddr, const float* s_xs, const double2* s_xt, float* s_ymax, double ws, double wz, bool mok,
+__device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t taddr, const float* s_xs, const long long* s_t, float* s_ymax, const RlScale& w, bool mok,
                                           int turn, int lane) {
 #pragma unroll 1
     for (int rl = 4 * turn; rl < o.nr; rl += WARPS) {
@@ -161,10 +179,7 @@ __device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t tad
             uint32_t v[16];
             tmem_ld16(taddr + 4 * rl, v);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const double2 xt = s_xt[rl + i];
-                a[i] = (float)(xt.x * (ws * rl_ll2d(rl_digits2q((int)v[4 * i], (int)v[4 * i + 1], (int)v[4 * i + 2], (int)v[4 * i + 3])) + wz * xt.y));
-            }
+            for (int i = 0; i < 4; ++i) a[i] = rl_value8(w, s_xs[rl + i], rl_digits2q((int)v[4 * i], (int)v[4 * i + 1], (int)v[4 * i + 2], (int)v[4 * i + 3]), s_t[rl + i]);
         }
         rl_activate4(o.epi, a, o.bias);
         const int left = o.nr - rl;
@@ -199,7 +214,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     __shared__ float s_xs[kRlMaxRowsF];
-    __shared__ double2 s_xt[kRlMaxRows];  // int8: the row's scale, and its sum of fixed-point values
+    __shared__ long long s_t[kRlMaxRows];  // int8: 128 x the row's sum of fixed-point values
     __shared__ float s_ymax[4][kRlMaxRowsF];  // per lane quarter (32 weight rows)
     uint8_t* smem = (uint8_t*)(((uintptr_t)rl_raw + 1023) & ~(uintptr_t)1023);
     volatile int* abort_flag = &s_abort;
@@ -393,7 +408,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
                     long long t = 0;
 #pragma unroll 1
                     for (int i = 0; i < P.tparts; ++i) t += __ldcg(P.tsum + (size_t)(r0 + et) * P.tparts + i);
-                    s_xt[et] = make_double2((double)s_xs[et], rl_ll2d(t));
+                    s_t[et] = 128 * t;
                 }
             }
             if (grouped)
@@ -476,10 +491,10 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     if (S > 1) cluster_sync_all();
     else if (GROUPED && epi && !direct) rl_epi_sync();
     const int epi_op = P.epi;
-    const double wsd = ws, wzd = wz;
+    const RlScale w8{ws, wz, false};  // (no products run beside this: fp64 is the shorter chain, 3 rows of att.output 4.7 us and 5.0)
     if (go && direct) {
         const RlOut out = rl_out(P, r0, nr, m, bias);
-        rl_finish<kRlEpiWarps>(out, BUILD || fmt == RL_F16, taddr, s_xs, s_xt, s_ymax[quarter], wsd, wzd, mok, half, lane);
+        rl_finish<kRlEpiWarps>(out, BUILD || fmt == RL_F16, taddr, s_xs, s_t, s_ymax[quarter], w8, mok, half, lane);
     } else if (!BUILD && go) {
         // this CTA's share of the rows: slices added in order, scaled, activated, stored (four rows at a time per thread)
         const int mine = nr > rank ? (nr - rank + S - 1) >> sh : 0;
@@ -513,11 +528,11 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
             } else {
                 long long q[4] = {0, 0, 0, 0};
 #pragma unroll 1
-                for (int s = 0; s < S; ++s, src += stride)
+                for (int s = 0; s < S; s += 2, src += 2 * stride)  // (S is 2, 4 or 8 here)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) q[i] += (long long)src[off[i]];
+                    for (int i = 0; i < 4; ++i) q[i] += (long long)src[off[i]] + (long long)src[stride + off[i]];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[i] = (float)(s_xt[r[i]].x * (wsd * rl_ll2d(q[i]) + wzd * s_xt[r[i]].y));
+                for (int i = 0; i < 4; ++i) a[i] = rl_value8(w8, s_xs[r[i]], q[i], s_t[r[i]]);
             }
             rl_activate4(epi_op, a, bias);
 #pragma unroll
@@ -551,10 +566,12 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
 // step: of a tile's 22 us at K = 2560 the tensor core worked 13 at 85 % of its rate, the rest was the first loads and the epilogue.
 // Measured, 2560 x 10240 (ffn.key), int8: 1024 rows 139 us with a CTA per tile, now 80; 512 rows 82 and 44.  Sixteen epilogue warps: eight took longer over a
 // tile than the tensor core over its 20 K blocks (512 rows 48; up to 128 rows there are eight all the same, see the launch).
-// What bounds it: no part alone.  512 rows with parts switched off (us): ffn.key 46, copies alone 35, products and epilogue alone 40; ffn.value 49, 43 and 37.  Without
-// the operands' copies, over half of the traffic, 45 and 48; with one matrix instruction of four 41 and 42; without the epilogue 41 and 44.  The tensor
-// pipe is active in 41 to 63 % of an SM's cycles; copies and products meet in shared memory, and a turn's start and last epilogue are not covered.  Tried
-// without gain: four producer threads, six stages instead of four, weights asked into L2 a turn ahead.
+// What bounds it: the products, at the clock that the power limit leaves them (1.75 GHz), and what gets in their way.  512 rows with parts switched off (us): ffn.key
+// 41.7, products alone 31, without the copies 34, without the epilogue 37; ffn.value 44 to 48, 37, 40 and 44.  The loop that issues products is a function of its own: inside
+// the kernel's control flow it took 600 cycles a K block whose products take 480, as a function those 480 (a bare ring of barriers and products
+// does too); with the fp32 epilogue (rl_value8) ffn.key 43.7 -> 41.5 us, ffn.value 47.8 -> 43.9, r, k, v and rank projections 40.8 -> 38.9, at 1024 rows ffn.key 79.8 -> 74.5.
+// Tried without gain: four producer threads, six stages instead of four, weights asked into L2 a turn ahead, one warp that waits for an accumulator and wakes
+// the others, the next stage's barrier tried ahead.
 struct RlCursor {
     int job, pi, kb, nk, mt, ntile;
     __device__ __forceinline__ void set(const RlLaunch& L, int j) {
@@ -567,6 +584,26 @@ struct RlCursor {
         nk = L.p[pi].kblocks;
     }
 };
+// The products of one tile: K block after K block through the ring (position s, parity par) into the accumulator at d.
+template <bool I8>
+__device__ __forceinline__ bool rl_mma_tile(uint64_t* full, uint64_t* empty, uint32_t& s, uint32_t& par, uint32_t NS, int nk, uint32_t smem_addr, uint32_t stage_bytes, uint32_t d,
+                                            uint32_t idesc, volatile int* abort_flag) {
+#pragma unroll 1
+    for (int kb = 0; kb < nk; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag))) return false;
+        tc_fence_after();
+        const uint32_t a_addr = smem_addr + s * stage_bytes;
+        const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + kRlABytes);
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<I8>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb == 0 && k4 == 0) ? 0u : 1u);
+        tc_commit_elect(&empty[s]);
+        if (++s == NS) {
+            s = 0;
+            par ^= 1u;
+        }
+    }
+    return true;
+}
 template <int WARPS>
 __global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_persistent_kernel(const __grid_constant__ RlLaunch L, int jobs) {
     extern __shared__ __align__(1024) uint8_t rl_raw[];
@@ -574,7 +611,7 @@ __global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_p
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     __shared__ float s_xs[kRlMaxRowsF];
-    __shared__ double2 s_xt[kRlMaxRows];
+    __shared__ long long s_t[kRlMaxRows];
     __shared__ float s_ymax[4][kRlMaxRowsF];
     uint8_t* smem = (uint8_t*)(((uintptr_t)rl_raw + 1023) & ~(uintptr_t)1023);
     volatile int* abort_flag = &s_abort;
@@ -672,26 +709,9 @@ __global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_p
             const int fmt = L.p[c.pi].fmt, nr = min(L.rt, L.R - c.ntile * L.rt);
             const uint32_t idesc = tc_idesc(fmt != RL_F16, (nr * rl_cols(fmt) + 15) & ~15), d = tmem + (it & 1u) * acc_cols;
             ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[it & 1u], ((it >> 1) & 1u) ^ 1u, abort_flag));
-#pragma unroll 1
-            for (int kb = 0; kb < c.nk && ok; ++kb) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag));
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a_addr = smem_addr + s * stage_bytes;
-                const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + kRlABytes);
-                if (fmt != RL_F16) {
-#pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<true>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb == 0 && k4 == 0) ? 0u : 1u);
-                } else {
-#pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<false>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb == 0 && k4 == 0) ? 0u : 1u);
-                }
-                tc_commit_elect(&empty[s]);
-                if (++s == NS) {
-                    s = 0;
-                    par ^= 1u;
-                }
-            }
+            if (ok)
+                ok = fmt != RL_F16 ? rl_mma_tile<true>(full, empty, s, par, NS, c.nk, smem_addr, stage_bytes, d, idesc, abort_flag)
+                                   : rl_mma_tile<false>(full, empty, s, par, NS, c.nk, smem_addr, stage_bytes, d, idesc, abort_flag);
             if (ok) tc_commit_elect(&acc_full[it & 1u]);
         }
     } else {
@@ -720,15 +740,16 @@ __global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_p
                     long long t = 0;
 #pragma unroll 1
                     for (int i = 0; i < P.tparts; ++i) t += __ldcg(P.tsum + (size_t)(r0 + et) * P.tparts + i);
-                    s_xt[et] = make_double2((double)xs, rl_ll2d(t));
+                    s_t[et] = 128 * t;
                 }
             }
+            const RlScale w8 = rl_scale(ws, wz);
             rl_epi_sync<32 * WARPS>();
             if (!*abort_flag) mbar_wait_parked(&acc_full[it & 1u], (it >> 1) & 1u, abort_flag);
             tc_fence_after();
             if (!__any_sync(0xffffffffu, *abort_flag)) {
                 const RlOut out = rl_out(P, r0, nr, m, bias);
-                rl_finish<WARPS>(out, P.fmt == RL_F16, tmem + ((uint32_t)(quarter * 32) << 16) + (it & 1u) * acc_cols, s_xs, s_xt, s_ymax[quarter], (double)ws, (double)wz, mok, turn, lane);
+                rl_finish<WARPS>(out, P.fmt == RL_F16, tmem + ((uint32_t)(quarter * 32) << 16) + (it & 1u) * acc_cols, s_xs, s_t, s_ymax[quarter], w8, mok, turn, lane);
             }
             tc_fence_before();
             __syncwarp();

@@ -47,6 +47,27 @@ def test_linear_persistent_tiles(rows, m, k, int8):
     test_linear_tile_edges(rows, m, k, int8)
 
 
+# ... with (scale, zero) pairs that are not symmetric around code 128 in every row, in one row of a tile, or with codes and activations at their limits (the integer
+# sums reach 2^47)
+@pytest.mark.parametrize("kind", ["asymmetric", "one row", "limits"])
+def test_linear_persistent_zero_points(kind):
+    rows, m, k = 513, 2560, 10240 if kind == "limits" else 2560
+    rng = np.random.default_rng(len(kind))
+    x = np.ones((rows, k), np.float32) if kind == "limits" else rng.standard_normal((rows, k)).astype(np.float32)
+    idx = rng.integers(0, 2, size=(m, 1), dtype=np.uint8) * np.full((1, k), 255, np.uint8) if kind == "limits" else rng.integers(0, 256, size=(m, k), dtype=np.uint8)
+    scale = (rng.random((m, 1)) * 0.01 + 0.001).astype(np.float16)
+    zero = (-128.0 * scale.astype(np.float32)).astype(np.float16)
+    if kind == "asymmetric":
+        zero = (rng.standard_normal((m, 1)) * 0.3).astype(np.float16)
+    elif kind == "one row":
+        zero[200] = 0.25
+    sz = np.ascontiguousarray(np.repeat((zero.view(np.uint16).astype(np.uint32) << 16) | scale.view(np.uint16).astype(np.uint32), k // 128, axis=1))
+    got, w = rsv.op_linear(x, idx, sz, path=1), orc.dequant_int8(idx, sz).astype(np.float64)
+    want = x.astype(np.float64) @ w.T
+    bound = 2.0 ** -27 * np.abs(x).max(1, keepdims=True) * np.abs(w).sum(1)[None, :] + 2.0 ** -23 * np.abs(want)  # (as above)
+    assert np.all(np.abs(got - want) <= bound + 1e-30), float((np.abs(got - want) / bound).max())
+
+
 # The same kernel as a step uses it: int8 next to fp16 problems in one launch, rank projections that are partial weight tiles, the maxima of
 # ffn.key's outputs (8200: its last weight tile has eight rows), row tiles of 44, 51, 65 and 86 rows
 @pytest.mark.parametrize("quant,ffn", [(1, 8192), (0, 8200)])

@@ -829,7 +829,7 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
             rl_launch_persistent<16>(m, name, L, jobs, bytes);
         return;
     }
-    const size_t stage = kRlABytes + (build ? 0 : (size_t)nt_max * 128), bbuf = build ? (size_t)nk * nt_max * 128 : 0, tg = grouped ? round_up((size_t)nk * t.rt * 4, 16) : 0;
+    const size_t stage = kRlABytes + (build ? 0 : (size_t)nt_max * 128), bbuf = build ? (size_t)nk * nt_max * 128 : 0, tg = grouped ? round_up(((size_t)nk * rl_group_rows(t.rt) + kRlMaxRowsG) * 4, 16) : 0;  // (sums of rows past the end are read)
     const size_t recv = L.split > 1 || grouped ? rl_recv_bytes(t.rt, L.split) : 0;  // partial sums reuse the ring
     int stages = std::min(nk, kRlMaxStages);
     while (stages > 2 && stages * stage + bbuf + tg + 1024 > kRlHalfSm) --stages;
@@ -837,7 +837,7 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
     const size_t smem = L.ring + bbuf + tg + 1024;
     if (smem > 200 * 1024) throw std::runtime_error("rows_linear: operands do not fit in shared memory");
     int cols = 32;
-    while (cols < (grouped ? 2 * t.nt8 : nt_max)) cols *= 2;
+    while (cols < std::max(grouped ? 2 * rl_group_cols(t.nt8) : 0, nt_max)) cols *= 2;
     L.tmem_cols = cols;
     if (build)
         rl_launch<false, true>(m, name, L, jobs, smem);

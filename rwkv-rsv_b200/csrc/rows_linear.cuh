@@ -121,6 +121,11 @@ __device__ __forceinline__ float rl_rowmax4(const float (&a)[4], bool mine, int 
 }
 // exact integer (|q| < 2^51) -> double without the slow 64-bit conversion
 __device__ __forceinline__ double rl_ll2d(long long q) { return __longlong_as_double(0x4338000000000000LL + q) - 6755399441055744.0; }
+// Per-group weights: columns between the two accumulators (read 32 at a time), and floats between the blocks' activation sums in shared memory.
+__host__ __device__ constexpr int rl_group_cols(int nt) { return (nt + 31) / 32 * 32; }
+__host__ __device__ constexpr int rl_group_rows(int rt) { return (rt + 3) / 4 * 4; }
+// A digit's sum over a group, |i| <= 2^21, as fp32 (the conversion instruction runs at an eighth of this)
+__device__ __forceinline__ float rl_small2f(uint32_t i) { return __uint_as_float(0x4B400000u + i) - 12582912.0f; }
 // An int8 output from the exact sum Q = sum_k q_k t_k and 128 T, T = sum_k t_k: xs (ws Q + wz T), rounded once.  Files quantised symmetrically around code 128 have
 // wz = -128 ws (`sym`, the same for a warp): then it is xs ws (Q - 128 T), the integer in a multiple of 2^23 and 23 bits, whose products meet before the
 // rounding (exact but for 2^-25 up to |Q - 128 T| < 2^47, typically 2^37).  In fp64, which other files take, the arithmetic holds the tensor pipe up: 512 rows of
@@ -204,6 +209,49 @@ __device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t tad
     }
 }
 
+// The products of one tile: K block after K block through the ring (position s, parity par) into the accumulator at d.
+template <bool I8>
+__device__ __forceinline__ bool rl_mma_tile(uint64_t* full, uint64_t* empty, uint32_t& s, uint32_t& par, uint32_t NS, int nk, uint32_t smem_addr, uint32_t stage_bytes, uint32_t d,
+                                            uint32_t idesc, volatile int* abort_flag) {
+#pragma unroll 1
+    for (int kb = 0; kb < nk; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag))) return false;
+        tc_fence_after();
+        const uint32_t a_addr = smem_addr + s * stage_bytes;
+        const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + kRlABytes);
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<I8>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb == 0 && k4 == 0) ? 0u : 1u);
+        tc_commit_elect(&empty[s]);
+        if (++s == NS) {
+            s = 0;
+            par ^= 1u;
+        }
+    }
+    return true;
+}
+// The same for per-group weights: block j into accumulator j mod 2 (acc_cols apart), handed to the epilogue warps block by block.
+__device__ __forceinline__ bool rl_mma_groups(uint64_t* full, uint64_t* empty, uint64_t* acc_full, uint64_t* acc_empty, uint32_t NS, int nk, uint32_t smem_addr, uint32_t stage_bytes, uint32_t tmem,
+                                              uint32_t acc_cols, uint32_t idesc, volatile int* abort_flag) {
+    uint32_t s = 0, par = 0;
+#pragma unroll 1
+    for (int j = 0; j < nk; ++j) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag))) return false;
+        if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[j & 1], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_flag))) return false;
+        tc_fence_after();
+        const uint32_t a_addr = smem_addr + s * stage_bytes, d = tmem + (uint32_t)(j & 1) * acc_cols;
+        const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + kRlABytes);
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<true>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, k4 ? 1u : 0u);
+        tc_commit_elect(&acc_full[j & 1]);
+        tc_commit_elect(&empty[s]);
+        if (++s == NS) {
+            s = 0;
+            par ^= 1u;
+        }
+    }
+    return true;
+}
+
 // GROUPED: the launch's int8 problems have per-group weights (RL_I8G), else RL_I8; fp16 problems may be in either kind of launch.
 // BUILD (fp16 problems with short rows, not split along K): the operands are built here from fp32 activations, straight into shared
 // memory; a kernel of its own would cost more than every CTA converting the few rows again.
@@ -255,6 +303,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
         pol = L.n_tiles == 1 ? l2_evict_first_policy() : l2_evict_normal_policy();
 #pragma unroll 1
         for (int j = 0; j < nk; ++j) {
+            if (grouped && (P.M & 3) == 0) l2_prefetch(P.szt + (size_t)(kb0 + j) * P.M + mt * kRlTileM, (uint32_t)min(kRlTileM, P.M - mt * kRlTileM) * 4u);
             if (j < NS) {
                 mbar_expect_tx(&full[j], kRlABytes + bbytes);
                 tma_load_2d_hint(&L.amap[pi], &full[j], smem + (size_t)j * stage_bytes, (kb0 + j) * kel, mt * kRlTileM, pol);
@@ -304,39 +353,33 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (the warp runs convergently, one elected lane issues) ----------------
-        const uint32_t idesc = tc_idesc(fmt != RL_F16, (ncols + 15) & ~15);
-        const uint32_t smem_addr = smem_u32(smem), bbuf = smem_addr + (uint32_t)L.ring;
+        const uint32_t idesc = tc_idesc(fmt != RL_F16, (ncols + 15) & ~15), smem_addr = smem_u32(smem);
         uint32_t s = 0, par = 0;
-        bool ok = true;
+        bool ok;
         if (BUILD) {
+            const uint32_t bbuf = smem_addr + (uint32_t)L.ring;
             ok = __all_sync(0xffffffffu, mbar_wait(&b_ready, 0u, abort_flag));
             tc_fence_after();
-        }
 #pragma unroll 1
-        for (int j = 0; j < nk && ok; ++j) {
-            if (grouped) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[j & 1], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_flag));
+            for (int j = 0; j < nk && ok; ++j) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag));
                 if (!ok) break;
-            }
-            ok = __all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag));
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t a_addr = smem_addr + s * (uint32_t)stage_bytes, b_addr = BUILD ? bbuf + (uint32_t)(j * NT * 128) : a_addr + kRlABytes;
-            const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(b_addr);
-            const uint32_t d = tmem + (grouped ? (uint32_t)((j & 1) * NT) : 0u);
-            if (!BUILD && fmt != RL_F16) {
+                tc_fence_after();
+                const uint64_t adesc = tc_smem_desc(smem_addr + s * (uint32_t)stage_bytes), bdesc = tc_smem_desc(bbuf + (uint32_t)(j * NT * 128));
 #pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<true>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, ((grouped || j == 0) && k4 == 0) ? 0u : 1u);
-            } else {
-#pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<false>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (j == 0 && k4 == 0) ? 0u : 1u);
+                for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<false>(tmem, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (j == 0 && k4 == 0) ? 0u : 1u);
+                tc_commit_elect(&empty[s]);
+                if (++s == (uint32_t)NS) {
+                    s = 0;
+                    par ^= 1u;
+                }
             }
-            tc_commit_elect(&empty[s]);
-            if (grouped) tc_commit_elect(&acc_full[j & 1]);
-            if (++s == (uint32_t)NS) {
-                s = 0;
-                par ^= 1u;
-            }
+        } else if (grouped) {
+            ok = rl_mma_groups(full, empty, acc_full, acc_empty, (uint32_t)NS, nk, smem_addr, (uint32_t)stage_bytes, tmem, rl_group_cols(NT), idesc, abort_flag);
+        } else if (fmt != RL_F16) {
+            ok = rl_mma_tile<true>(full, empty, s, par, (uint32_t)NS, nk, smem_addr, (uint32_t)stage_bytes, tmem, idesc, abort_flag);
+        } else {
+            ok = rl_mma_tile<false>(full, empty, s, par, (uint32_t)NS, nk, smem_addr, (uint32_t)stage_bytes, tmem, idesc, abort_flag);
         }
         if (!grouped && ok) tc_commit_elect(&acc_full[0]);
     }
@@ -347,8 +390,10 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     const int sh = L.log_split, slots = (nr + S - 1) >> sh;
     const uint32_t recv = smem_u32(smem);
     float ws = 0.f, wz = 0.f, bias = 0.f;
-    constexpr int kGChunks = kRlMaxRowsG / 4 / 2;  // 16-column chunks (four activation rows) per warp
-    float gacc[GROUPED ? kGChunks : 1][4];
+    constexpr int kGChunks = kRlMaxRowsG / 8 / 2;  // 32-column chunks (eight activation rows) per warp
+    float gacc[GROUPED ? kGChunks : 1][8];
+    const int tg_rows = rl_group_rows(L.rt);
+    uint32_t z0 = 0, z1 = 0;  // grouped: (scale, zero) words of the next two groups
     if (epi) {
         if (mok) {
             if (!BUILD && fmt == RL_I8) {
@@ -356,8 +401,12 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
                 wz = P.wzero[m];
             }
             if (P.bias) bias = P.bias[m];
+            if (grouped) {
+                z0 = __ldg(P.szt + (size_t)kb0 * P.M + m);
+                if (nk > 1) z1 = __ldg(P.szt + (size_t)(kb0 + 1) * P.M + m);
+            }
         }
-        float* s_tg = reinterpret_cast<float*>(smem + L.ring);  // grouped: [nk][rt]
+        float* s_tg = reinterpret_cast<float*>(smem + L.ring);  // grouped: [nk][tg_rows]
         pdl_wait();
         if (BUILD) {
             // a warp per row: find the maximum, convert; elements past K are zeros (the tensor map fills the weights there with zeros)
@@ -412,46 +461,59 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
                 }
             }
             if (grouped)
-#pragma unroll 1
+#pragma unroll 4
                 for (int i = et; i < nk * nr; i += kRlEpiThreads) {
                     const int r = i / nk, kb = i - r * nk;
-                    s_tg[kb * L.rt + r] = __ldcg(P.tgrp + (size_t)(r0 + r) * P.kblocks + kb0 + kb);
+                    s_tg[kb * tg_rows + r] = __ldcg(P.tgrp + (size_t)(r0 + r) * P.kblocks + kb0 + kb);
                 }
         }
         rl_epi_sync();
         if (grouped) {
             // ---- per group: digit sums -> fp32, times the group's scale, plus zero x the group's activation sum ----
+            // What bounds it: at few rows the way of a group's word from memory (one group ahead, behind the wait and not in L2: 3 rows of 2560 channels
+            // a layer 60.1 us; two ahead, the first two before the wait, all of them asked into L2 with the weights 54.4; 16 rows 72.6 and 67.1),
+            // at many rows the instructions of the sums (201 rows 271 us with both halves of a sum through the conversion unit and 16 columns a load, 246 now).
 #pragma unroll
             for (int c = 0; c < (GROUPED ? kGChunks : 1); ++c)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) gacc[c][i] = 0.f;
-            uint32_t z = mok ? __ldg(P.szt + (size_t)kb0 * P.M + m) : 0u;
-#pragma unroll 1
-            for (int j = 0; j < nk; ++j) {
-                const uint32_t zc = z;
-                if (j + 1 < nk && mok) z = __ldg(P.szt + (size_t)(kb0 + j + 1) * P.M + m);
-                const float gs = __half2float(__ushort_as_half((unsigned short)(zc & 0xFFFFu))), gz = __half2float(__ushort_as_half((unsigned short)(zc >> 16)));
-                if (!__all_sync(0xffffffffu, mbar_wait_parked(&acc_full[j & 1], ((uint32_t)j >> 1) & 1u, abort_flag))) break;
+                for (int i = 0; i < 8; ++i) gacc[c][i] = 0.f;
+            auto group = [&](int j, uint32_t& z) -> bool {
+                const float gs = __half2float(__ushort_as_half((unsigned short)(z & 0xFFFFu))), gz = __half2float(__ushort_as_half((unsigned short)(z >> 16)));
+                if (j + 2 < nk && mok) z = __ldg(P.szt + (size_t)(kb0 + j + 2) * P.M + m);
+                if (!__all_sync(0xffffffffu, mbar_wait_parked(&acc_full[j & 1], ((uint32_t)j >> 1) & 1u, abort_flag))) return false;
                 tc_fence_after();
-                const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((j & 1) * NT);
+                const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((j & 1) * rl_group_cols(NT));
 #pragma unroll
                 for (int c = 0; c < (GROUPED ? kGChunks : 1); ++c) {
-                    const int c0 = (2 * c + half) * 16;
-                    if (c0 < ncols) {
-                        uint32_t v[16];
-                        tmem_ld16(taddr + c0, v);
+                    const int c0 = (2 * c + half) * 32;
+                    if (c0 < ncols) {  // (rows past the end of the tile: sums of nothing, never sent)
+                        uint32_t v[32];
+                        tmem_ld32(taddr + c0, v);
+                        const float4* tg = reinterpret_cast<const float4*>(s_tg + j * tg_rows + (c0 >> 2));
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            // |digit sum| <= 2^21: pairs combine exactly in 32 bits, the two halves of Q in one fp32 fma
-                            const int hi = (int)v[4 * i] * 128 + (int)v[4 * i + 1], lo = (int)v[4 * i + 2] * 128 + (int)v[4 * i + 3];
-                            const float q = fmaf((float)hi, 16384.0f, (float)lo);
-                            gacc[c][i] = fmaf(gs, q, fmaf(gz, s_tg[j * L.rt + min((c0 >> 2) + i, nr - 1)], gacc[c][i]));
+                        for (int h = 0; h < 2; ++h) {
+                            const float4 t4 = tg[h];
+                            const float t[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                // |digit sum| <= 2^21: two halves of two digits each, their weighted sum in one fp32 fma.  One half through the conversion unit,
+                                // the other beside it (both through it were its whole time: 464 cycles for 29 rows of a block, whose products take 256).
+                                const uint32_t* d = v + 16 * h + 4 * i;
+                                const float hi = fmaf(rl_small2f(d[0]), 128.0f, rl_small2f(d[1])), lo = (float)((int)d[2] * 128 + (int)d[3]);
+                                gacc[c][4 * h + i] = fmaf(gs, fmaf(hi, 16384.0f, lo), fmaf(gz, t[i], gacc[c][4 * h + i]));
+                            }
                         }
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[j & 1]);
+                return true;
+            };
+#pragma unroll 1
+            for (int j = 0; j < nk; j += 2) {  // (two groups, so that a word is two groups on its way)
+                if (!group(j, z0)) break;
+                if (j + 1 < nk && !group(j + 1, z1)) break;
             }
         } else {
             mbar_wait_parked(&acc_full[0], 0u, abort_flag);  // a time-out shows in the abort flag
@@ -472,7 +534,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
 #pragma unroll
             for (int c = 0; c < (GROUPED ? kGChunks : 1); ++c)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) send((2 * c + half) * 4 + i, (unsigned long long)__float_as_uint(gacc[c][i]));
+                for (int i = 0; i < 8; ++i) send((2 * c + half) * 8 + i, (unsigned long long)__float_as_uint(gacc[c][i]));
         } else {
 #pragma unroll 1
             for (int c0 = half * 16; c0 < ncols; c0 += 32) {
@@ -584,26 +646,6 @@ struct RlCursor {
         nk = L.p[pi].kblocks;
     }
 };
-// The products of one tile: K block after K block through the ring (position s, parity par) into the accumulator at d.
-template <bool I8>
-__device__ __forceinline__ bool rl_mma_tile(uint64_t* full, uint64_t* empty, uint32_t& s, uint32_t& par, uint32_t NS, int nk, uint32_t smem_addr, uint32_t stage_bytes, uint32_t d,
-                                            uint32_t idesc, volatile int* abort_flag) {
-#pragma unroll 1
-    for (int kb = 0; kb < nk; ++kb) {
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], par, abort_flag))) return false;
-        tc_fence_after();
-        const uint32_t a_addr = smem_addr + s * stage_bytes;
-        const uint64_t adesc = tc_smem_desc(a_addr), bdesc = tc_smem_desc(a_addr + kRlABytes);
-#pragma unroll
-        for (int k4 = 0; k4 < 4; ++k4) tc_mma_elect<I8>(d, adesc + (uint64_t)(k4 * 2), bdesc + (uint64_t)(k4 * 2), idesc, (kb == 0 && k4 == 0) ? 0u : 1u);
-        tc_commit_elect(&empty[s]);
-        if (++s == NS) {
-            s = 0;
-            par ^= 1u;
-        }
-    }
-    return true;
-}
 template <int WARPS>
 __global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_persistent_kernel(const __grid_constant__ RlLaunch L, int jobs) {
     extern __shared__ __align__(1024) uint8_t rl_raw[];

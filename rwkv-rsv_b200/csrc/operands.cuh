@@ -190,12 +190,15 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
     if (A.rows) rm = A.rows[r];
     const size_t row = A.row_map ? (size_t)A.row_map[r] : (size_t)r;
     const bool shift = A.rows != nullptr, pln = shift && rm.has_prev;
-    // weights: requested before the dependency wait
+    // few rows: weights requested before the dependency wait; many: where they are used, so that a fourth block has registers on its SM
+    constexpr bool EARLY = BLOCKS < 4;
     float lw[8], lb[8], mx[8];
-    ln_weights8(lw, A.lw + kc);
-    ln_weights8(lb, A.lb + kc);
     const int o0 = blockIdx.y, step = gridDim.y;
-    if (A.out[o0].mix) ln_weights8(mx, A.out[o0].mix + kc);
+    if (EARLY) {
+        ln_weights8(lw, A.lw + kc);
+        ln_weights8(lb, A.lb + kc);
+        if (A.out[o0].mix) ln_weights8(mx, A.out[o0].mix + kc);
+    }
     const int rloc = r % A.rt, rtile = r / A.rt;
     pdl_wait();
     const float* xr = A.x_in + row * C + kc;
@@ -235,6 +238,10 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
     ln_block_sums(s0, s1, pln, red[1], warp, lane, nw);
     s0 = 1.0f / sqrtf(s0 / (float)C + kLnEps);
     s1 = 1.0f / sqrtf(s1 / (float)C + kLnEps);
+    if (!EARLY) {
+        ln_weights8(lw, A.lw + kc);
+        ln_weights8(lb, A.lb + kc);
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         x[i] = x[i] * s0 * lw[i] + lb[i];                  // cur
@@ -250,7 +257,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
 #pragma unroll 1
     for (int o = o0; o < A.nout; o += step) {
         const float* mix = A.out[o].mix;
-        if (o != o0 && mix) ln_weights8(mx, mix + kc);
+        if ((!EARLY || o != o0) && mix) ln_weights8(mx, mix + kc);
         float am = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(mix ? x[i] + mx[i] * xp[i] : x[i]));
@@ -261,7 +268,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
 #pragma unroll 1
     for (int o = o0; o < A.nout; o += step) {
         const RlOperandOut& O = A.out[o];
-        if (o0 + step < A.nout && O.mix) ln_weights8(mx, O.mix + kc);
+        if ((!EARLY || o0 + step < A.nout) && O.mix) ln_weights8(mx, O.mix + kc);
         const int ex = rl_scale_exp(warp_absmax(lane < nw ? redm[o][lane] : 0.f)), fmt = O.fmt, lk = fmt == RL_F16 ? 6 : 7;
         float v[8];
 #pragma unroll

@@ -120,6 +120,9 @@ void decode_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n) {
 }
 
 constexpr int kMaxChunk = 512;  // rows per packed step on the chunk path
+// ... whose logits are all wanted (256 x 65536 of them are 67 MB on the device and in pinned memory).  Chunks of 128 hid the copy of one behind the next, but a layer of
+// 201 rows takes 250 us and of 128 and 73 rows 199 and 150.
+constexpr int kMaxScored = 256;
 
 // Memory the driver knows (pinned; or, though the interface asks for host arrays, managed or a device's) takes copies directly; only pageable
 // memory is the host's own to write.
@@ -183,7 +186,7 @@ void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int6
     need(n >= 1, "empty token list");
     check_tokens(m, tokens, n);
     RSV_CUDA(cudaSetDevice(m.device));
-    const int64_t cs = std::max<int64_t>(1, std::min<int64_t>(chunk <= 0 ? kMaxChunk : chunk, out_mode == 2 ? 128 : kMaxChunk));
+    const int64_t cs = std::max<int64_t>(1, std::min<int64_t>(chunk <= 0 ? kMaxChunk : chunk, out_mode == 2 ? kMaxScored : kMaxChunk));
     const size_t V = m.cfg.vocab;
     LogitsToHost out(m);
     for (int64_t off = 0; off < n; off += cs) {

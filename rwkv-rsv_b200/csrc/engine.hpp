@@ -141,7 +141,7 @@ struct Model {
     void* pinned = nullptr;
     size_t pinned_bytes = 0;  // bytes per ring area
     std::shared_ptr<StatePool> state_pool;
-    // pinned staging of a chunk's logits on their way to the caller (at most 128 rows), with an event per piece
+    // pinned staging of a chunk's logits on their way to the caller (at most 256 rows), with an event per piece
     static constexpr int kOutParts = 32;
     float* pinned_out = nullptr;
     size_t pinned_out_bytes = 0;

@@ -862,9 +862,9 @@ void launch_ln_operands(Model& m, const char* name, const LnOperandsArgs& A) {
         }
         return;
     }
-    // more blocks than three per SM: a fourth, with fewer registers (512 rows, 2560 int8 channels: 13.2 -> 11.6 us, six outputs 25.8 -> 24.0, fp16 22.6 -> 18.9; at 444 and fewer three are
-    // one wave and no slower)
-    void (*kernel)(LnOperandsArgs) = threads <= 320 ? ((A.R + A.nseg) * gy > 3 * m.num_sms ? ln_operands_kernel<320, 4> : ln_operands_kernel<320, 3>) : threads <= 512 ? ln_operands_kernel<512, 2> : ln_operands_kernel<kLnMaxThreads, 1>;
+    // more blocks of rows than three per SM: a fourth, with fewer registers (512 rows, 2560 int8 channels: 13.2 -> 11.6 us, six outputs 25.8 -> 24.0, fp16 22.6 -> 18.9; with fewer, three are
+    // one wave and the faster ones, 64 sessions 9.2 us and 10.6; the blocks that commit a segment's shift state do not count)
+    void (*kernel)(LnOperandsArgs) = threads <= 320 ? (A.R * gy > 3 * m.num_sms ? ln_operands_kernel<320, 4> : ln_operands_kernel<320, 3>) : threads <= 512 ? ln_operands_kernel<512, 2> : ln_operands_kernel<kLnMaxThreads, 1>;
     LAUNCH(m, name) {
         launch_pdl(m, kernel, dim3(A.R + A.nseg, gy), dim3(threads), 0, A);
         check_launch("ln_operands");

@@ -21,6 +21,9 @@
 // five were the longest chain of the launch with r, k and v; 3 rows, 2560 channels, 32 layers: a step of 1.74 ms, now 1.67.)
 // What bounds it: at few rows the chain operand tiles (L2) -> products -> exchange -> store behind the dependency wait, the weights
 // are there already; at 64 rows the operand tiles' L2 traffic as well (a 128-row tile re-reads them all).
+// In cycles after the wait (3 rows, att.output and ffn.value split in 4 and 8): operand tiles and products 3800 and 5400, two cluster barriers and the partial sums
+// between them 2150 and 2500, their addition and the outputs 1500 and 1800; 64 rows, ffn.key split in two: 12000, 5900 and 6000.  Tried without gain: partial
+// sums counted by an mbarrier of their receiver instead of the barriers (3 rows 47.0 -> 49.8 us a layer), the epilogue run once on nothing before the wait.
 //
 // Code size is part of the design.  The kernels of a layer run for a few microseconds each, in turn, on every SM; 32 KB of code run at
 // an instruction per cycle, up to 128 KB at a third of that, more at less than a fifth (measured with straight-line kernels), and a

@@ -27,7 +27,7 @@ def _full(b, toks, out_ptr):
         raise rsv.RsvError(rsv.native().rsv_last_error().decode())
 
 
-# 63 / 64: below and at the size that is staged; 201: two staged chunks; 140: a staged chunk, then a small one; 300: three chunks in turn
+# 63 / 64: below and at the size that is staged; 140, 201: one staged chunk; 300: a staged chunk, then a small one
 @pytest.mark.parametrize("n", [1, 63, 64, 140, 201, 300])
 def test_logits_of_every_position(bundle, n):
     import torch
@@ -43,6 +43,12 @@ def test_logits_of_every_position(bundle, n):
     pinned = torch.full((n, V), float("nan"), pin_memory=True)
     _full(b, toks, pinned.data_ptr())
     assert np.array_equal(pinned.numpy(), pageable)
+
+
+# passes are 256 positions: up to the last one, one more, and three staged chunks in turn
+@pytest.mark.parametrize("n", [255, 256, 257, 600])
+def test_logits_of_every_position_around_a_pass(bundle, n):
+    test_logits_of_every_position(bundle, n)
 
 
 def test_logits_into_memory_of_the_device(bundle):

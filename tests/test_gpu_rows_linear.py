@@ -47,6 +47,12 @@ def test_linear_persistent_tiles(rows, m, k, int8):
     test_linear_tile_edges(rows, m, k, int8)
 
 
+# ... and tiles of few K blocks once there are four turns of them: a ragged last row tile (1025 rows are 17 tiles of 61, 1024 of fp16 weights eight of 128), a partial last weight tile
+@pytest.mark.parametrize("rows,m,k,int8", [(1025, 5120, 512, True), (1025, 9610, 320, False), (1024, 9600, 64, False)])
+def test_linear_persistent_short_rows(rows, m, k, int8):
+    test_linear_tile_edges(rows, m, k, int8)
+
+
 # ... with (scale, zero) pairs that are not symmetric around code 128 in every row, in one row of a tile, or with codes and activations at their limits (the integer
 # sums reach 2^47)
 @pytest.mark.parametrize("kind", ["asymmetric", "one row", "limits"])
@@ -162,3 +168,28 @@ def test_small_steps_cut_for_turns_agree_with_the_cpu_path(tmp_path, quant):
             assert float(np.sqrt(np.mean((got[i] - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), (n, i)
     b.state.close()
     b.model.close()
+
+
+# 444 rows are three LayerNorm blocks per SM of 148, 445 more than that (a block with fewer registers)
+def test_steps_around_three_layernorm_blocks_per_sm(tiny_paths):
+    b, o = rsv.ModelBuilder(tiny_paths["int8"]).build(), orc.OracleModel(tiny_paths["int8"])
+    rng = np.random.default_rng(11)
+    for n in (443, 444, 445):
+        toks = rng.integers(0, b.info().num_vocab, size=n).astype(np.uint32)
+        b.reset()
+        o.reset()
+        lg, want = b.infer_seq(toks), o.forward(toks)
+        assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n  # (as above)
+
+
+# 184 sessions of 8 heads go to the WKV kernel of one block per pair, 186 to the one that streams pairs (the line is ten pairs per SM: 185)
+def test_sessions_around_the_wkv_line(tiny_paths):
+    m = rsv.ModelBuilder(tiny_paths["int8"]).build().model
+    seeds = np.random.default_rng(5).integers(0, m.info().num_vocab, size=186).astype(np.uint32)
+
+    def stream(part):
+        s = m.create_batch_state(len(part))
+        return m.collect_sample_selfloop_batch(m.submit_sample_selfloop_batch(s, part, 6, None))
+
+    few = np.concatenate([stream(seeds[i:i + 31]) for i in range(0, 186, 31)])
+    assert np.array_equal(stream(seeds), few) and np.array_equal(stream(seeds[:184]), few[:184])

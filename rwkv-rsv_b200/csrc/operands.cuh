@@ -123,7 +123,7 @@ __device__ __forceinline__ long long rl_group_sum(int ts) {
 // segment's first row still has to read the old one; the CTAs past the rows commit the staging area of the block before this one.
 // What bounds it: at few rows the chain load -> mean -> variance -> row maximum -> digits (block-wide reductions); it writes operands instead of fp32 because the
 // conversion in a kernel of its own cost a second launch and a second such chain (8 rows, n_embd 2560: 11.0 + 9.2 us for the two kernels it replaces, CUDA events around each).
-// Cycles after the dependency wait at 3 rows: loads 1500, two sums of 700, normalising 700, maxima 360, digits 1800, sum of digits 500; 512 rows of six
+// Cycles after the dependency wait at 3 rows: loads 1500, two sums of 700, normalising 700, maxima 360, digits 1800, sum of digits 500 (in 64-bit shuffles; two integer reductions now, here and in operand_known_kernel: a layer of 3 rows 44.6 -> 44.1 us, 16 58.4 -> 57.6); 512 rows of six
 // outputs are bound by the digits.  The row stays in registers (in shared memory the sums took 1.4 us, and the kernel's 20 KB kept the next launch's CTAs
 // off its SMs) and the outputs' maxima meet behind one barrier: 2560 channels, exclusive us in the step, 3 rows 4.6 -> 4.3, 512 rows and one
 // output 15.2 -> 13.2, six outputs 27.3 -> 26.0.
@@ -170,7 +170,7 @@ template <int THREADS, int BLOCKS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __grid_constant__ LnOperandsArgs A) {
     __shared__ float red[2][2][32];
     __shared__ float redm[7][32];
-    __shared__ long long redt[7][32];
+    __shared__ int2 redt[7][32];  // per output and warp: low 16 bits and the rest of the fixed-point sums, added up
     pdl_launch_dependents();
     const int C = A.C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     if ((int)blockIdx.x >= A.R) {  // commit CTAs
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
             if (on && (lane & 15) == 0) O.tgrp[(size_t)r * O.kblocks + k0 / 128] = (float)t16;
         } else if (fmt == RL_I8) {
             const int lo = __reduce_add_sync(0xffffffffu, ts & 0xFFFF), hi = __reduce_add_sync(0xffffffffu, ts >> 16);
-            if (lane == 0) redt[o][warp] = (long long)hi * 65536 + lo;
+            if (lane == 0) redt[o][warp] = make_int2(lo, hi);
         }
         if (tid == 0) O.xscale[r] = rl_xscale(fmt, ex);
     }
@@ -289,10 +289,9 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
 #pragma unroll 1
     for (int o = warp; o < A.nout; o += nw)
         if (o % step == o0 && A.out[o].fmt == RL_I8) {
-            long long t = lane < nw ? redt[o][lane] : 0;
-#pragma unroll
-            for (int i = 16; i > 0; i >>= 1) t += __shfl_xor_sync(0xffffffffu, t, i);
-            if (lane == 0) A.out[o].tsum[r] = t;
+            const int2 t = lane < nw ? redt[o][lane] : make_int2(0, 0);
+            const int lo = __reduce_add_sync(0xffffffffu, t.x), hi = __reduce_add_sync(0xffffffffu, t.y);
+            if (lane == 0) A.out[o].tsum[r] = (long long)hi * 65536 + lo;
         }
 }
 
@@ -441,7 +440,7 @@ __global__ void __launch_bounds__(kLnMaxThreads) ln_operands_wide_kernel(const _
 constexpr int kOpThreads = 256;
 __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* x, int ldx, int K, const float* amax, int parts, int rt,
                                                                    const __grid_constant__ RlOperandOut O) {
-    __shared__ long long red[kOpThreads / 32];
+    __shared__ int2 red[kOpThreads / 32];
     __shared__ float redm[kOpThreads / 32];
     pdl_launch_dependents();
     const int r = blockIdx.x, k0 = ((int)blockIdx.y * kOpThreads + (int)threadIdx.x) * 8, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -464,20 +463,17 @@ __global__ void __launch_bounds__(kOpThreads) operand_known_kernel(const float* 
         *reinterpret_cast<uint4*>(col + ((chunk ^ (n0 & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
         *reinterpret_cast<uint4*>(col + 128 + ((chunk ^ ((n0 + 1) & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
     }
-    if (O.fmt != RL_F16) {
+    if (O.fmt == RL_I8G) {
         const long long t16 = rl_group_sum(ts);
-        if (O.fmt == RL_I8G) {
-            if (k0 < K && (lane & 15) == 0) O.tgrp[(size_t)r * O.kblocks + k0 / 128] = (float)t16;
-        } else {
-            const long long t32 = t16 + __shfl_xor_sync(0xffffffffu, t16, 16);
-            if (lane == 0) red[warp] = t32;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                long long t = 0;
-#pragma unroll 1
-                for (int i = 0; i < kOpThreads / 32; ++i) t += red[i];
-                O.tsum[(size_t)r * gridDim.y + blockIdx.y] = t;
-            }
+        if (k0 < K && (lane & 15) == 0) O.tgrp[(size_t)r * O.kblocks + k0 / 128] = (float)t16;
+    } else if (O.fmt == RL_I8) {
+        const int lo = __reduce_add_sync(0xffffffffu, ts & 0xFFFF), hi = __reduce_add_sync(0xffffffffu, ts >> 16);
+        if (lane == 0) red[warp] = make_int2(lo, hi);
+        __syncthreads();
+        if (warp == 0) {
+            const int2 t = lane < kOpThreads / 32 ? red[lane] : make_int2(0, 0);
+            const int l = __reduce_add_sync(0xffffffffu, t.x), h = __reduce_add_sync(0xffffffffu, t.y);
+            if (lane == 0) O.tsum[(size_t)r * gridDim.y + blockIdx.y] = (long long)h * 65536 + l;
         }
     }
     if (blockIdx.y == 0 && threadIdx.x == 0) O.xscale[r] = rl_xscale(O.fmt, ex);

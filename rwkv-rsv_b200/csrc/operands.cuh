@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
 }
 
 // The same for rows that do not fit the block's registers (n_embd above 8192): the row is read again from global memory (L2) for the statistics,
-// for every output's maximum and for its digits.  Same sums in the same order.  No model in use is this wide, so nothing is tuned here.
+// for every output's maximum and for its digits.  Its sums have an order of their own, which also depends on the length of a row alone.  No model in use is this wide, so nothing is tuned here.
 __global__ void __launch_bounds__(kLnMaxThreads) ln_operands_wide_kernel(const __grid_constant__ LnOperandsArgs A) {
     __shared__ float red[2][kLnSumThreads / 32], redm[32];
     __shared__ long long redt[32];

@@ -5,8 +5,8 @@
 //
 // Arithmetic.  Weights are never converted: the u8 codes q are the A operand of tcgen05.mma.kind::i8 as they sit in HBM, the
 // activation row is four columns of signed base-128 digits of its fixed-point value t (operands.cuh).  The tensor core returns exact
-// int32 sums; Q = sum_j 128^(3-j) I_j = sum_k q_k t_k, y = e 2^-27 (s Q + z sum_k t_k): no rounding but the one of t, no dependence on
-// how K is split.  Files with one (scale, zero) per group of 128 weights (the reference's own) get a fresh accumulator per K block of
+// int32 sums; Q = sum_j 128^(3-j) I_j = sum_k q_k t_k, y = e 2^-27 (s Q + z sum_k t_k): no rounding but the one of t and the one of y, so
+// no dependence on how K is split or on the other rows.  (Sums of more than 53 bits pass through fp64 in some kernels, which can turn a tie of the last rounding.)  Files with one (scale, zero) per group of 128 weights (the reference's own) get a fresh accumulator per K block of
 // 128 bytes = one group: the epilogue warps fold s_g Q_g + z_g T_g into fp32 registers while the next group is multiplied.  fp16
 // weights use kind::f16 with hi + lo halves of the activations.
 //
@@ -129,22 +129,23 @@ __host__ __device__ constexpr int rl_group_cols(int nt) { return (nt + 31) / 32 
 __host__ __device__ constexpr int rl_group_rows(int rt) { return (rt + 3) / 4 * 4; }
 // A digit's sum over a group, |i| <= 2^21, as fp32 (the conversion instruction runs at an eighth of this)
 __device__ __forceinline__ float rl_small2f(uint32_t i) { return __uint_as_float(0x4B400000u + i) - 12582912.0f; }
-// An int8 output from the exact sum Q = sum_k q_k t_k and 128 T, T = sum_k t_k: xs (ws Q + wz T), rounded once.  Files quantised symmetrically around code 128 have
-// wz = -128 ws (`sym`, the same for a warp): then it is xs ws (Q - 128 T), the integer in a multiple of 2^23 and 23 bits, whose products meet before the
-// rounding (exact but for 2^-25 up to |Q - 128 T| < 2^47, typically 2^37).  In fp64, which other files take, the arithmetic holds the tensor pipe up: 512 rows of
-// 2560 -> 10240 45.4 us, without any arithmetic 38.6.
+// An int8 output from the exact sum Q = sum_k q_k t_k and 128 T, T = sum_k t_k: xs (ws Q + wz T), xs a power of two, rounded to fp32 once.  Files quantised symmetrically around
+// code 128 have wz = -128 ws (`sym`): the sum is ws (Q - 128 T), and with the fp16 number ws = mant x unit, |mant| < 2^11 and the unit a power of two,
+// (Q - 128 T) mant is an integer (under 2^63 for K < 2^16), which the conversion to fp32 rounds.  In fp64, which other files take and which holds sums of up to 53 bits, the
+// arithmetic holds the tensor pipe up: 512 rows of 2560 -> 10240 45.4 us, without any arithmetic 38.6, as integers 41.0 (as two fp32 halves, which lost the last
+// bit of some sums and more of small negative ones, 40.8).
 struct RlScale {
-    float ws, wz;
+    float ws, wz, unit;
+    int mant;
     bool sym;
 };
-__device__ __forceinline__ RlScale rl_scale(float ws, float wz) { return RlScale{ws, wz, (bool)__all_sync(0xffffffffu, wz == -128.0f * ws)}; }
+__device__ __forceinline__ RlScale rl_scale(float ws, float wz) {
+    const uint32_t b = __float_as_uint(ws), e = (b >> 23) & 0xFFu;
+    const int mant = ws == 0.f ? 0 : (int)((b & 0x7FFFFFu) | 0x800000u) >> 13;
+    return RlScale{ws, wz, __uint_as_float((e > 10u ? e - 10u : 1u) << 23), (int)b < 0 ? -mant : mant, wz == -128.0f * ws && (mant == 0 || (e > 10u && e < 255u && !(b & 0x1FFFu)))};
+}
 __device__ __forceinline__ float rl_value8(const RlScale& w, float xs, long long q, long long t128) {
-    if (w.sym) {
-        const long long d = q - t128;
-        const float hi = (float)(int)(d >> 23), lo = __uint_as_float(0x4B000000u | ((uint32_t)d & 0x7FFFFFu)) - 8388608.0f, w23 = w.ws * 8388608.0f;
-        const float p = w23 * hi;
-        return xs * (p + fmaf(w.ws, lo, fmaf(w23, hi, -p)));
-    }
+    if (w.sym) return xs * (w.unit * (float)((q - t128) * w.mant));
     return (float)((double)xs * ((double)w.ws * rl_ll2d(q) + (double)w.wz * (rl_ll2d(t128) * 0.0078125)));
 }
 __device__ __forceinline__ long long rl_digits2q(int i0, int i1, int i2, int i3) {
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     if (S > 1) cluster_sync_all();
     else if (GROUPED && epi && !direct) rl_epi_sync();
     const int epi_op = P.epi;
-    const RlScale w8{ws, wz, false};  // (no products run beside this: fp64 is the shorter chain, 3 rows of att.output 4.7 us and 5.0)
+    const RlScale w8{ws, wz, 0.f, 0, false};  // (no products run beside this: fp64 is the shorter chain, 3 rows of att.output 4.7 us and 5.0)
     if (go && direct) {
         const RlOut out = rl_out(P, r0, nr, m, bias);
         rl_finish<kRlEpiWarps>(out, BUILD || fmt == RL_F16, taddr, s_xs, s_t, s_ymax[quarter], w8, mok, half, lane);
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
 // What bounds it: the products, at the clock that the power limit leaves them (1.75 GHz), and what gets in their way.  512 rows with parts switched off (us): ffn.key
 // 41.7, products alone 31, without the copies 34, without the epilogue 37; ffn.value 44 to 48, 37, 40 and 44.  The loop that issues products is a function of its own: inside
 // the kernel's control flow it took 600 cycles a K block whose products take 480, as a function those 480 (a bare ring of barriers and products
-// does too); with the fp32 epilogue (rl_value8) ffn.key 43.7 -> 41.5 us, ffn.value 47.8 -> 43.9, r, k, v and rank projections 40.8 -> 38.9, at 1024 rows ffn.key 79.8 -> 74.5.
+// does too); with that and the integer epilogue (rl_value8) ffn.key 42.0 -> 41.0 us, ffn.value 45.6 -> 44.3, r, k, v and rank projections 40.8 -> 39.5, at 1024 rows ffn.key 75.6 -> 72.2.
 // Tried without gain: four producer threads, six stages instead of four, weights asked into L2 a turn ahead, one warp that waits for an accumulator and wakes
 // the others, the next stage's barrier tried ahead.
 struct RlCursor {

@@ -74,6 +74,38 @@ def test_linear_persistent_zero_points(kind):
     assert np.all(np.abs(got - want) <= bound + 1e-30), float((np.abs(got - want) / bound).max())
 
 
+def _int8_words(scale, zero, groups):
+    word = (zero.view(np.uint16).astype(np.uint32) << 16) | scale.view(np.uint16).astype(np.uint32)
+    return np.ascontiguousarray(np.repeat(word[:, None], groups, axis=1))
+
+
+# An int8 output is the exact sum, rounded once, whichever kernel takes its row (2 and 16 rows: split along K where K is long; 513: the persistent one).  The activations are whole
+# numbers of at most 20 bits times a power of two, so that their fixed-point values are exact, and the products with the scales fit fp64.
+@pytest.mark.parametrize("kind", ["ordinary", "small sums", "limits", "one row"])
+@pytest.mark.parametrize("rows", [2, 16, 513])
+def test_int8_sums_are_rounded_once(rows, kind):
+    m, k = 2560, 10240 if kind == "limits" else 2560
+    rng = np.random.default_rng(rows + len(kind))
+    x = rng.integers(-(1 << 20), 1 << 20, size=(rows, k)).astype(np.float64)
+    idx = rng.integers(0, 256, size=(m, k), dtype=np.uint8)
+    if kind == "small sums":  # a large activation against the code of zero, and a few of the smallest: sums of both signs down to one step of the fixed point
+        x = np.where(rng.random((rows, k)) < 4 / k, rng.integers(-3, 4, size=(rows, k)), 0).astype(np.float64)
+        x[:, 0] = 1 << 26
+        idx[:, 0] = 128
+    elif kind == "limits":
+        x = np.where(rng.random((rows, 1)) < 0.5, 1.0, -1.0) * ((1 << 20) - rng.integers(0, 9, size=(rows, k)))
+        idx = (255 * rng.integers(0, 2, size=(m, 1)) + np.zeros((1, k))).astype(np.uint8)
+    scale = (rng.integers(1024, 2048, size=m) * 2.0 ** -14).astype(np.float16)  # 11 bits
+    scale[:4] = [0.0, 2.0 ** -24, -0.0078125, 511.0] if kind in ("ordinary", "small sums") else scale[:4]
+    zero = (-128.0 * scale.astype(np.float32)).astype(np.float16)
+    if kind == "one row":
+        zero[200] = 0.25
+    got = rsv.op_linear((x * 2.0 ** -9).astype(np.float32), idx, _int8_words(scale, zero, k // 128), path=1)
+    q, t = x @ idx.astype(np.float64).T, x.sum(1)[:, None]  # (whole numbers under 2^43)
+    want = (q * scale.astype(np.float64) + t * zero.astype(np.float64)) * 2.0 ** -9
+    assert np.array_equal(got, want.astype(np.float32)), (int((got != want.astype(np.float32)).sum()), float(np.abs(got / np.where(want == 0, 1, want) - 1).max()))
+
+
 # The same kernel as a step uses it: int8 next to fp16 problems in one launch, rank projections that are partial weight tiles, the maxima of
 # ffn.key's outputs (8200: its last weight tile has eight rows), row tiles of 44, 51, 65 and 86 rows
 @pytest.mark.parametrize("quant,ffn", [(1, 8192), (0, 8200)])

@@ -129,24 +129,38 @@ __host__ __device__ constexpr int rl_group_cols(int nt) { return (nt + 31) / 32 
 __host__ __device__ constexpr int rl_group_rows(int rt) { return (rt + 3) / 4 * 4; }
 // A digit's sum over a group, |i| <= 2^21, as fp32 (the conversion instruction runs at an eighth of this)
 __device__ __forceinline__ float rl_small2f(uint32_t i) { return __uint_as_float(0x4B400000u + i) - 12582912.0f; }
-// An int8 output from the exact sum Q = sum_k q_k t_k and 128 T, T = sum_k t_k: xs (ws Q + wz T), xs a power of two, rounded to fp32 once.  Files quantised symmetrically around
-// code 128 have wz = -128 ws (`sym`): the sum is ws (Q - 128 T), and with the fp16 number ws = mant x unit, |mant| < 2^11 and the unit a power of two,
-// (Q - 128 T) mant is an integer (under 2^63 for K < 2^16), which the conversion to fp32 rounds.  In fp64, which other files take and which holds sums of up to 53 bits, the
-// arithmetic holds the tensor pipe up: 512 rows of 2560 -> 10240 45.4 us, without any arithmetic 38.6, as integers 41.0 (as two fp32 halves, which lost the last
-// bit of some sums and more of small negative ones, 40.8).
+// An int8 output from the exact sum Q = sum_k q_k t_k and the row's T = sum_k t_k: xs (ws Q + wz T), xs a power of two, rounded to fp32 once.  The scales are fp16
+// numbers: with ws = ms unit and wz = mz unit in whole numbers (ms < 2^11, |mz| < 2^19, the unit a power of two with the sign of ws) ms Q + mz T is an
+// integer, under 2^63 for K < 2^16, which the conversion to fp32 rounds (`whole`).  That covers zero points of one to 256 steps of the codes, and none.  fp64 takes the
+// others; it holds sums of up to 53 bits.
+// In fp64 the arithmetic holds the tensor pipe up.  512 rows of 2560 -> 10240, us: files symmetric around code 128 42.0 and as integers 41.0 (as two fp32 halves, which lost
+// the last bit of some sums and more of small negative ones, 40.8), zero points of 96 steps 47.5 and 41.0; 1024 rows of those 84.2 and 72.2.
 struct RlScale {
     float ws, wz, unit;
-    int mant;
-    bool sym;
+    uint32_t ms;
+    int mz;
+    bool whole;
 };
 __device__ __forceinline__ RlScale rl_scale(float ws, float wz) {
-    const uint32_t b = __float_as_uint(ws), e = (b >> 23) & 0xFFu;
-    const int mant = ws == 0.f ? 0 : (int)((b & 0x7FFFFFu) | 0x800000u) >> 13;
-    return RlScale{ws, wz, __uint_as_float((e > 10u ? e - 10u : 1u) << 23), (int)b < 0 ? -mant : mant, wz == -128.0f * ws && (mant == 0 || (e > 10u && e < 255u && !(b & 0x1FFFu)))};
+    const uint32_t bs = __float_as_uint(ws), bz = __float_as_uint(wz), e = (bs >> 23) & 0xFFu;
+    const uint32_t ms = ws == 0.f ? 0u : ((bs & 0x7FFFFFu) | 0x800000u) >> 13, mz = wz == 0.f ? 0u : ((bz & 0x7FFFFFu) | 0x800000u) >> 13;
+    const int up = mz ? (int)((bz >> 23) & 0xFFu) - (int)e : 0;
+    RlScale w;
+    w.ws = ws;
+    w.wz = wz;
+    w.ms = ms;
+    w.whole = (ms | mz) == 0u || (e > 10u && e < 255u && up >= 0 && up <= 8 && !((bs | bz) & 0x1FFFu));
+    w.unit = __uint_as_float((bs & 0x80000000u) | (w.whole && ms ? (e - 10u) << 23 : 0u));
+    w.mz = w.whole ? (int)(mz << up) : 0;
+    if ((int)(bs ^ bz) < 0) w.mz = -w.mz;
+    return w;
 }
-__device__ __forceinline__ float rl_value8(const RlScale& w, float xs, long long q, long long t128) {
-    if (w.sym) return xs * (w.unit * (float)((q - t128) * w.mant));
-    return (float)((double)xs * ((double)w.ws * rl_ll2d(q) + (double)w.wz * (rl_ll2d(t128) * 0.0078125)));
+struct RlSum8 {  // of a row of activations: T, and as fp64
+    long long t;
+    double td;
+};
+__device__ __forceinline__ float rl_value8(const RlScale& w, float xs, long long q, const RlSum8& row) {
+    return xs * (w.whole ? w.unit * (float)(q * (long long)w.ms + row.t * w.mz) : (float)((double)w.ws * rl_ll2d(q) + (double)w.wz * row.td));
 }
 __device__ __forceinline__ long long rl_digits2q(int i0, int i1, int i2, int i3) {
     return ((long long)i0 * 128 + i1) * 16384 + ((long long)i2 * 128 + i3);
@@ -174,7 +188,7 @@ __device__ __forceinline__ RlOut rl_out(const RlProb& P, int r0, int nr, int m, 
 // The sums of a tile whose K was not split, from tensor memory through the thread's registers to the output, rows rl .. rl + 3 at a time
 // (`turn`: the WARPS / 4 warps of a lane quarter take turns).  What bounds this is the latency of its instructions: a warp issues one in eight cycles.
 template <int WARPS>
-__device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t taddr, const float* s_xs, const long long* s_t, float* s_ymax, const RlScale& w, bool mok,
+__device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t taddr, const float* s_xs, const RlSum8* s_t, float* s_ymax, const RlScale& w, bool mok,
                                           int turn, int lane) {
 #pragma unroll 1
     for (int rl = 4 * turn; rl < o.nr; rl += WARPS) {
@@ -266,7 +280,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     __shared__ float s_xs[kRlMaxRowsF];
-    __shared__ long long s_t[kRlMaxRows];  // int8: 128 x the row's sum of fixed-point values
+    __shared__ RlSum8 s_t[kRlMaxRows];  // int8
     __shared__ float s_ymax[4][kRlMaxRowsF];  // per lane quarter (32 weight rows)
     uint8_t* smem = (uint8_t*)(((uintptr_t)rl_raw + 1023) & ~(uintptr_t)1023);
     volatile int* abort_flag = &s_abort;
@@ -461,7 +475,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
                     long long t = 0;
 #pragma unroll 1
                     for (int i = 0; i < P.tparts; ++i) t += __ldcg(P.tsum + (size_t)(r0 + et) * P.tparts + i);
-                    s_t[et] = 128 * t;
+                    s_t[et] = RlSum8{t, rl_ll2d(t)};
                 }
             }
             if (grouped)
@@ -557,7 +571,7 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
     if (S > 1) cluster_sync_all();
     else if (GROUPED && epi && !direct) rl_epi_sync();
     const int epi_op = P.epi;
-    const RlScale w8{ws, wz, 0.f, 0, false};  // (no products run beside this: fp64 is the shorter chain, 3 rows of att.output 4.7 us and 5.0)
+    const RlScale w8{ws, wz, 0.f, 0u, 0, false};  // (no products run beside this: fp64 is the shorter chain, a layer of 3 rows 44.0 us and 44.8, 64 rows 103.7 and 104.6)
     if (go && direct) {
         const RlOut out = rl_out(P, r0, nr, m, bias);
         rl_finish<kRlEpiWarps>(out, BUILD || fmt == RL_F16, taddr, s_xs, s_t, s_ymax[quarter], w8, mok, half, lane);
@@ -657,7 +671,7 @@ __global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_p
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort;
     __shared__ float s_xs[kRlMaxRowsF];
-    __shared__ long long s_t[kRlMaxRows];
+    __shared__ RlSum8 s_t[kRlMaxRows];  // int8
     __shared__ float s_ymax[4][kRlMaxRowsF];
     uint8_t* smem = (uint8_t*)(((uintptr_t)rl_raw + 1023) & ~(uintptr_t)1023);
     volatile int* abort_flag = &s_abort;
@@ -786,7 +800,7 @@ __global__ void __launch_bounds__(rl_persistent_threads(WARPS), 1) rows_linear_p
                     long long t = 0;
 #pragma unroll 1
                     for (int i = 0; i < P.tparts; ++i) t += __ldcg(P.tsum + (size_t)(r0 + et) * P.tparts + i);
-                    s_t[et] = 128 * t;
+                    s_t[et] = RlSum8{t, rl_ll2d(t)};
                 }
             }
             const RlScale w8 = rl_scale(ws, wz);

@@ -81,7 +81,7 @@ def _int8_words(scale, zero, groups):
 
 # An int8 output is the exact sum, rounded once, whichever kernel takes its row (2 and 16 rows: split along K where K is long; 513: the persistent one).  The activations are whole
 # numbers of at most 20 bits times a power of two, so that their fixed-point values are exact, and the products with the scales fit fp64.
-@pytest.mark.parametrize("kind", ["ordinary", "small sums", "limits", "one row"])
+@pytest.mark.parametrize("kind", ["ordinary", "small sums", "limits", "asymmetric", "one row"])
 @pytest.mark.parametrize("rows", [2, 16, 513])
 def test_int8_sums_are_rounded_once(rows, kind):
     m, k = 2560, 10240 if kind == "limits" else 2560
@@ -98,7 +98,10 @@ def test_int8_sums_are_rounded_once(rows, kind):
     scale = (rng.integers(1024, 2048, size=m) * 2.0 ** -14).astype(np.float16)  # 11 bits
     scale[:4] = [0.0, 2.0 ** -24, -0.0078125, 511.0] if kind in ("ordinary", "small sums") else scale[:4]
     zero = (-128.0 * scale.astype(np.float32)).astype(np.float16)
-    if kind == "one row":
+    if kind == "asymmetric":
+        # zero points of under a step of the codes, of 100 to 155 steps, and of up to 1000
+        zero = np.choose(np.arange(m) % 3, [rng.integers(-2048, 2048, size=m) * 2.0 ** -14, -rng.uniform(100, 155, size=m) * scale, rng.uniform(-60, 60, size=m)]).astype(np.float16)
+    elif kind == "one row":
         zero[200] = 0.25
     got = rsv.op_linear((x * 2.0 ** -9).astype(np.float32), idx, _int8_words(scale, zero, k // 128), path=1)
     q, t = x @ idx.astype(np.float64).T, x.sum(1)[:, None]  # (whole numbers under 2^43)

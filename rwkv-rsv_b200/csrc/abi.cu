@@ -120,9 +120,11 @@ void decode_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n) {
 }
 
 constexpr int kMaxChunk = 512;  // rows per packed step on the chunk path
-// ... whose logits are all wanted (256 x 65536 of them are 67 MB on the device and in pinned memory).  Chunks of 128 hid the copy of one behind the next, but a layer of
-// 201 rows takes 250 us and of 128 and 73 rows 199 and 150.
-constexpr int kMaxScored = 256;
+// ... whose logits are all wanted (256 x 65536 of them are 67 MB on the device and in pinned memory).  Passes of 128 hide the copy of one behind the next, but two of them take
+// longer than a large one.  Texts of 129, 201, 256, 257 and 600 tokens, 3B shape, whole call in ms, in passes of 128 and of 256: int8 7.4 and 7.0, 10.8 and 9.0, 12.4 and
+// 10.7, 13.3 and 10.6, 29.7 and 23.4; fp16 8.1 and 7.0, 11.1 and 9.5, 12.7 and 10.2, 13.9 and 11.2, 30.4 and 24.0; int8 per group 9.6 and 9.7, 13.5 and 10.9,
+// 16.1 and 14.4, 17.0 and 14.4, 37.7 and 31.5.  128 remain for devices that have no room for more.
+constexpr int kMaxScored = 256, kShortScored = 128;
 
 // Memory the driver knows (pinned; or, though the interface asks for host arrays, managed or a device's) takes copies directly; only pageable
 // memory is the host's own to write.
@@ -142,6 +144,10 @@ class LogitsToHost {
     ~LogitsToHost() {
         moves.join();
         if (queued) cudaStreamSynchronize(m.stream);  // left by an exception: nothing writes to the caller's memory afterwards
+    }
+    // the staging area, before anything is queued
+    void reserve(const float* dst, size_t count) {
+        if (count >= kSmall && !driver_knows(dst)) m.ensure_pinned_out(count * sizeof(float));
     }
     // queues the copy of `count` logits; returns while it is under way
     void start(float* dst, size_t count) {
@@ -189,15 +195,16 @@ void prefill_tokens(Model& m, State& st, const uint32_t* tokens, int64_t n, int6
     const int64_t cs = std::max<int64_t>(1, std::min<int64_t>(chunk <= 0 ? kMaxChunk : chunk, out_mode == 2 ? kMaxScored : kMaxChunk));
     const size_t V = m.cfg.vocab;
     LogitsToHost out(m);
-    for (int64_t off = 0; off < n; off += cs) {
-        const int T = (int)std::min<int64_t>(cs, n - off);
+    in_passes(n, cs, out_mode == 2 ? std::min<int64_t>(cs, kShortScored) : cs, [&m] { return m.launches; }, [&](int64_t off, int64_t rows) {
+        const int T = (int)rows;
         const bool last = off + T >= n;
         StepPlan p = chunk_plan(0, T, out_mode == 2 ? 2 : (last && out_mode == 1 ? 1 : 0));
+        if (out_mode == 2 && off == 0) out.reserve(all_out, (size_t)T * V);
         m.upload_plan(p);
         RSV_CUDA(cudaMemcpyAsync(m.ws.tokens, tokens + off, (size_t)T * sizeof(uint32_t), cudaMemcpyHostToDevice, m.stream));
         m.forward_rows(st, p, false);
         if (out_mode == 2) out.start(all_out + (size_t)off * V, (size_t)T * V);
-    }
+    });
     if (out_mode == 2) out.finish();
 }
 

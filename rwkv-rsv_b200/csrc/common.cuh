@@ -8,6 +8,8 @@
 #include <stdexcept>
 #include <string>
 
+#include "cuda_error.hpp"
+
 namespace rsv {
 
 // Numerical constants of the reference's CPU path (src/model.rs:6-8, :438).
@@ -16,18 +18,6 @@ constexpr float kGnEps = 64.0e-5f;
 constexpr float kL2Eps = 1.0e-12f;
 constexpr float kDecayScale = -0.60653065971263342f;  // -1/sqrt(e)
 constexpr int kHeadSize = 64;                         // the only head size RWKV-7 checkpoints use
-
-struct CudaError : std::runtime_error {
-    using std::runtime_error::runtime_error;
-};
-
-#define RSV_CUDA(expr)                                                                                              \
-    do {                                                                                                            \
-        cudaError_t _e = (expr);                                                                                    \
-        if (_e != cudaSuccess)                                                                                      \
-            throw ::rsv::CudaError(std::string(#expr) + " failed: " + cudaGetErrorString(_e) + " (" __FILE__ ":" + \
-                                   std::to_string(__LINE__) + ")");                                                 \
-    } while (0)
 
 enum WType : int { W_F16 = 0, W_INT8 = 1 };
 

@@ -542,16 +542,17 @@ void Model::ensure_workspace(int rows, int outs, int segs) {
     RSV_CUDA(device_malloc(&ws.row_meta, R * sizeof(RowMeta)));
     RSV_CUDA(device_malloc(&ws.seg_meta, (size_t)segs * sizeof(SegMeta)));
     RSV_CUDA(device_malloc(&ws.out_rows, (size_t)std::max(outs, 1) * sizeof(int)));
-    ws.rows = rows;
-    ws.outs = outs;
-    ws.segs = segs;
     const size_t need = R * sizeof(RowMeta) + (size_t)segs * sizeof(SegMeta) + (size_t)outs * sizeof(int) + R * sizeof(uint32_t) + 256;
     if (need > pinned_bytes) {
         cudaFreeHost(pinned);
         pinned = nullptr;
+        pinned_bytes = 0;
+        RSV_CUDA(cudaMallocHost(&pinned, need * 2 * kPinRing));
         pinned_bytes = need * 2;
-        RSV_CUDA(cudaMallocHost(&pinned, pinned_bytes * kPinRing));
     }
+    ws.rows = rows;  // (last: an allocation that failed leaves a workspace of no rows)
+    ws.outs = outs;
+    ws.segs = segs;
 }
 
 void Model::ensure_pinned_out(size_t bytes) {

@@ -34,3 +34,8 @@ def test_rows_are_cut_into_no_more_turns_than_the_widest_tiles_need(tmp_path):
 @pytest.mark.skipif(not os.path.exists(CUDA_INCLUDE), reason="no CUDA headers")
 def test_memory_of_freed_states_is_given_back(tmp_path):
     assert "device memory ok" in _run(tmp_path, "device_memory_check", "-I", CUDA_INCLUDE)
+
+
+@pytest.mark.skipif(not os.path.exists(CUDA_INCLUDE), reason="no CUDA headers")
+def test_scored_texts_take_shorter_passes_where_memory_is_short(tmp_path):
+    assert "passes ok" in _run(tmp_path, "passes_check", "-I", CUDA_INCLUDE)

@@ -863,9 +863,12 @@ void launch_ln_operands(Model& m, const char* name, const LnOperandsArgs& A) {
         }
         return;
     }
-    // more blocks of rows than three per SM: a fourth, with fewer registers (512 rows, 2560 int8 channels: 13.2 -> 11.6 us, six outputs 25.8 -> 24.0, fp16 22.6 -> 18.9; with fewer, three are
-    // one wave and the faster ones, 64 sessions 9.2 us and 10.6; the blocks that commit a segment's shift state do not count)
-    void (*kernel)(LnOperandsArgs) = threads <= 320 ? (A.R * gy > 3 * m.num_sms ? ln_operands_kernel<320, 4> : ln_operands_kernel<320, 3>) : threads <= 512 ? ln_operands_kernel<512, 2> : ln_operands_kernel<kLnMaxThreads, 1>;
+    // Up to 2560 channels there are two variants (ln_operands_kernel says which rows each is for).  The blocks that commit a segment's shift state do not count.
+    void (*kernel)(LnOperandsArgs) = ln_operands_kernel<kLnMaxThreads, 1>;
+    if (threads <= 320)
+        kernel = A.R * gy > ln_resident_blocks(threads) * m.num_sms ? ln_operands_kernel<320, 4> : ln_operands_kernel<320, 3>;
+    else if (threads <= 512)
+        kernel = ln_operands_kernel<512, 2>;
     LAUNCH(m, name) {
         launch_pdl(m, kernel, dim3(A.R + A.nseg, gy), dim3(threads), 0, A);
         check_launch("ln_operands");

@@ -166,6 +166,11 @@ __device__ __forceinline__ void ln_weights8(float (&v)[8], const float* p) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p + 4));
     v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
+// Blocks of the variant with 64 registers a thread (<320, 3>) that an SM holds.  While all rows' blocks are resident at once it is the faster one: the weights are
+// there when they are needed.  With more rows the variant with 48 registers, which loads them where it uses them, fits more blocks beside one another: 512 int8 rows of
+// 2560 channels 14.3 us and 11.6, six outputs 26.4 and 23.8; but 448 rows of 2048 channels (256 threads, four blocks) 10.1 and 11.7, 19.3 and 23.4, 640 rows 13.7 and
+// 12.1, 25.6 and 23.9; 1024 rows of 512 channels (64 threads, sixteen blocks) 5.9 and 6.3, 19.6 and 23.7.
+constexpr int ln_resident_blocks(int threads) { return 1024 / threads; }
 template <int THREADS, int BLOCKS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __grid_constant__ LnOperandsArgs A) {
     __shared__ float red[2][2][32];
@@ -190,7 +195,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
     if (A.rows) rm = A.rows[r];
     const size_t row = A.row_map ? (size_t)A.row_map[r] : (size_t)r;
     const bool shift = A.rows != nullptr, pln = shift && rm.has_prev;
-    // few rows: weights requested before the dependency wait; many: where they are used, so that a fourth block has registers on its SM
+    // weights before the dependency wait, or where they are used (see above)
     constexpr bool EARLY = BLOCKS < 4;
     float lw[8], lb[8], mx[8];
     const int o0 = blockIdx.y, step = gridDim.y;

@@ -90,3 +90,12 @@ def test_rows_wider_than_one_block(tmp_path, quant):
     path = rsv.write_synthetic(os.path.join(str(tmp_path), "wide.st"), "tiny", seed=0, quant=quant, **shape)
     _check(path, (1, 3, 40), shape["vocab"])
     os.remove(path)
+
+
+# ... and rows of 4160 and 8192 channels, which a block of 520 and of 1024 threads holds, also with more rows than are resident at once
+@pytest.mark.parametrize("n_embd,sizes", [(4160, (1, 3, 40, 445)), (8192, (3, 40))])
+def test_rows_of_one_large_block(tmp_path, n_embd, sizes):
+    shape = dict(n_layer=1, n_embd=n_embd, n_head=n_embd // 64, ffn_hidden=256, vocab=64, w_mid=16, a_mid=16, v_mid=16, g_mid=16)
+    path = rsv.write_synthetic(os.path.join(str(tmp_path), "block.st"), "tiny", seed=0, quant=0 if n_embd % 128 else 1, **shape)
+    _check(path, sizes, shape["vocab"])
+    os.remove(path)

@@ -205,9 +205,10 @@ def test_small_steps_cut_for_turns_agree_with_the_cpu_path(tmp_path, quant):
     b.model.close()
 
 
-# 444 rows are three LayerNorm blocks per SM of 148, 445 more than that (a block with fewer registers)
-def test_steps_around_three_layernorm_blocks_per_sm(tiny_paths):
-    b, o = rsv.ModelBuilder(tiny_paths["int8"]).build(), orc.OracleModel(tiny_paths["int8"])
+# 444 rows of 2560 channels are three LayerNorm blocks per SM of 148, 445 more than that (a block with fewer registers)
+def test_steps_around_three_layernorm_blocks_per_sm(tmp_path):
+    p = rsv.write_synthetic(str(tmp_path / "m.st"), "tiny", seed=3, quant=1, n_layer=1, n_embd=2560, n_head=40, ffn_hidden=1024, vocab=300, w_mid=24, a_mid=40, v_mid=16, g_mid=56)
+    b, o = rsv.ModelBuilder(p).build(), orc.OracleModel(p)
     rng = np.random.default_rng(11)
     for n in (443, 444, 445):
         toks = rng.integers(0, b.info().num_vocab, size=n).astype(np.uint32)
@@ -215,6 +216,8 @@ def test_steps_around_three_layernorm_blocks_per_sm(tiny_paths):
         o.reset()
         lg, want = b.infer_seq(toks), o.forward(toks)
         assert float(np.sqrt(np.mean((lg - want) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(want).max())), n  # (as above)
+    b.state.close()
+    b.model.close()
 
 
 # 184 sessions of 8 heads go to the WKV kernel of one block per pair, 186 to the one that streams pairs (the line is ten pairs per SM: 185)

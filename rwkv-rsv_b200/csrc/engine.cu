@@ -1106,7 +1106,7 @@ void Model::forward_rows(State& st, const StepPlan& plan, bool use_cursor) {
                 }
                 launch_pdl(*this, wkv7_finish_kernel, dim3((R * H + kWsFinishThreads / 32 - 1) / (kWsFinishThreads / 32)), dim3(kWsFinishThreads), 0, ws.r, ws.k,
                            ws.v, vgate, ws.vfirst, ws.a, ws.g, L.k_a, L.r_k, L.lnx_w, L.lnx_b, ws.yg, R, H, C, ws.ymax);
-            } else if (n_items >= kWrItemsPerSm * num_sms) {
+            } else if (wr_pays(n_items, num_sms)) {
                 // many (session, head) pairs: one state row per lane, states staged by TMA (wkv_rows.cuh)
                 const size_t rows_total = (size_t)cfg.n_layer * st.cap * H * kHeadSize;
                 if (rows_total >= (1ull << 31)) throw std::runtime_error("state too large for the 32-bit row coordinate of its tensor map");

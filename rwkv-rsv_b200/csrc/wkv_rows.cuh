@@ -7,8 +7,7 @@
 //     bytes, SWIZZLE_128B: a lane reads its 128-byte row segment chunk by chunk without bank conflicts), the first token's
 //     eight input vectors and the head's five parameter vectors as 256-byte bulk copies.  No load of an iteration depends on
 //     another load: with the memory system loaded a dependent global load costs microseconds per item.  The first item's state and
-//     parameters, which no kernel of the step writes, are requested before the dependency wait (16 sessions of 40 heads 9.4 -> 8.2 us, 64
-//     20.6 -> 18.2);
+//     parameters, which no kernel of the step writes, are requested before the dependency wait (64 sessions of 40 heads 20.6 -> 18.2 us);
 //   * the updated rows leave through a staging tile and TMA stores;
 //   * six warp pairs per CTA walk their own item streams (a head's chain of reductions and barriers is long and a thread holds
 //     64 state registers, so the pairs are what hides latency: 96 KB of state reads in flight per SM); they share nothing but
@@ -22,10 +21,15 @@ namespace rsv {
 
 constexpr int kWrPairs = 6;
 constexpr int kWrThreads = 64 * kWrPairs;
-// From how many (session, head) pairs per SM on a step takes this kernel.  Its pairs go in rounds of six per SM, 5.8 us each, and its shared memory keeps the
-// next kernels' CTAs, which would fetch weights meanwhile, off the SM.  A layer of 40 heads and 2560 int8 channels with wkv7_kernel and with this
-// one (us): 16 sessions 57.8 and 58.0, 20 63.5 and 62.9, 24 67.1 and 70.1, 32 74.6 and 76.8, 40 85.1 and 84.6.
-constexpr int kWrItemsPerSm = 10;
+// Whether a step of `items` (session, head) pairs takes this kernel.  Its pairs go in rounds of six per SM, 5.7 us each, however few there are in the last one, and its shared
+// memory keeps the next kernels' CTAs, which would fetch weights meanwhile, off the SM (2 to 3 us); wkv7_kernel takes 1.5 us per pair and SM.  So its rounds
+// have to be full to five sixths on the average, or four at least.  A layer of 40 heads and 2560 int8 channels with wkv7_kernel and with this one (us): 16 sessions 57.9 and
+// 58.0, 20 64.1 and 63.2, 24 67.7 and 70.3, 32 74.6 and 77.7, 38 83.5 and 81.1, 44 90.1 and 87.3, 46 94.3 and 93.8, 52 99.4 and 100.7, 56 102.8 and 104.1,
+// 60 107.8 and 102.6, 72 112.0 and 107.3; fp16: 20 73.8 and 73.7, 24 76.0 and 79.0, 38 92.6 and 90.8, 48 101.9 and 103.9, 56 108.1 and 106.1.
+inline bool wr_pays(long long items, int sms) {
+    const long long rounds = (items + (long long)kWrPairs * sms - 1) / ((long long)kWrPairs * sms);
+    return rounds > 3 || items >= 5 * rounds * sms;
+}
 constexpr int kWrStages = 1;               // load stages per pair (plus one staging tile for the stores)
 constexpr int kWrTileFloats = 64 * 32;     // one TMA box: 64 rows x 32 columns
 constexpr int kWrStateBytes = 2 * kWrTileFloats * 4;

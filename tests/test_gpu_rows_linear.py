@@ -220,6 +220,27 @@ def test_steps_around_three_layernorm_blocks_per_sm(tmp_path):
     b.model.close()
 
 
+# Eight heads: steps on either side of the lines between the two WKV kernels (five and six pairs per SM, ten and twelve, fifteen and eighteen; 148 SMs) give the tokens and states of the
+# same sessions in batches of 31, which stay below all of them
+@pytest.mark.parametrize("sessions", [(92, 93), (111, 112), (184, 185), (222, 223), (277, 278), (333, 334)])
+def test_sessions_around_the_wkv_lines(tiny_paths, sessions):
+    m = rsv.ModelBuilder(tiny_paths["int8"]).build().model
+    seeds = np.random.default_rng(5).integers(0, m.info().num_vocab, size=sessions[1]).astype(np.uint32)
+
+    def stream(part):
+        s = m.create_batch_state(len(part))
+        toks = m.collect_sample_selfloop_batch(m.submit_sample_selfloop_batch(s, part, 6, None))
+        return toks, [s.slot_back(i) for i in range(len(part))]
+
+    parts = [stream(seeds[i:i + 31]) for i in range(0, len(seeds), 31)]
+    few, states = np.concatenate([t for t, _ in parts]), [x for _, p in parts for x in p]
+    for n in sessions:
+        toks, got = stream(seeds[:n])
+        assert np.array_equal(toks, few[:n])
+        for i in range(n):
+            assert float(np.sqrt(np.mean((got[i] - states[i]) ** 2))) <= 64 * 2.0 ** -24 * max(1.0, float(np.abs(states[i]).max())), (n, i)  # (as above)
+
+
 # 184 sessions of 8 heads go to the WKV kernel of one block per pair, 186 to the one that streams pairs (the line is ten pairs per SM: 185)
 def test_sessions_around_the_wkv_line(tiny_paths):
     m = rsv.ModelBuilder(tiny_paths["int8"]).build().model

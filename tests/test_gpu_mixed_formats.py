@@ -99,3 +99,12 @@ def test_rows_of_one_large_block(tmp_path, n_embd, sizes):
     path = rsv.write_synthetic(os.path.join(str(tmp_path), "block.st"), "tiny", seed=0, quant=0 if n_embd % 128 else 1, **shape)
     _check(path, sizes, shape["vocab"])
     os.remove(path)
+
+
+# Per-group weights at the edges of their kernel: one group a row, odd numbers of them (also where K is split), 80; full and ragged row tiles of up to 32 rows; a vocabulary head whose
+# last weight tile is partial and whose rows are no multiple of four
+@pytest.mark.parametrize("n_embd,ffn,vocab", [(128, 128, 301), (384, 1408, 200), (640, 10240, 130)])
+def test_groups_at_the_edges_of_a_tile(tmp_path, n_embd, ffn, vocab):
+    shape = dict(n_layer=2, n_embd=n_embd, n_head=n_embd // 64, ffn_hidden=ffn, vocab=vocab, w_mid=16, a_mid=24, v_mid=16, g_mid=40)
+    path = rsv.write_synthetic(os.path.join(str(tmp_path), "g.st"), "tiny", seed=0, quant=2, quant_head=True, **shape)
+    _check(path, (1, 2, 3, 7, 8, 9, 29, 31, 32, 33, 65, 130), vocab)

@@ -123,10 +123,13 @@ __device__ __forceinline__ long long rl_group_sum(int ts) {
 // segment's first row still has to read the old one; the CTAs past the rows commit the staging area of the block before this one.
 // What bounds it: at few rows the chain load -> mean -> variance -> row maximum -> digits (block-wide reductions); it writes operands instead of fp32 because the
 // conversion in a kernel of its own cost a second launch and a second such chain (8 rows, n_embd 2560: 11.0 + 9.2 us for the two kernels it replaces, CUDA events around each).
-// Cycles after the dependency wait at 3 rows: loads 1500, two sums of 700, normalising 700, maxima 360, digits 1800, sum of digits 500 (in 64-bit shuffles; two integer reductions now, here and in operand_known_kernel: a layer of 3 rows 44.6 -> 44.1 us, 16 58.4 -> 57.6); 512 rows of six
-// outputs are bound by the digits.  The row stays in registers (in shared memory the sums took 1.4 us, and the kernel's 20 KB kept the next launch's CTAs
-// off its SMs) and the outputs' maxima meet behind one barrier: 2560 channels, exclusive us in the step, 3 rows 4.6 -> 4.3, 512 rows and one
-// output 15.2 -> 13.2, six outputs 27.3 -> 26.0.
+// Cycles after the dependency wait at 3 rows: loads 1500, two sums of 700, normalising 700, maxima 360, digits 1800, sum of digits 500 (in 64-bit shuffles; two integer reductions
+// now, here and in operand_known_kernel: a layer of 3 rows 44.6 -> 44.1 us, 16 58.4 -> 57.6); 512 rows of six outputs are bound by the digits.  The row stays in registers: in shared
+// memory the sums took 1.4 us, and the kernel's 20 KB kept the next launch's CTAs off its SMs.  The outputs go one by one with a barrier each, the next one's mix
+// vector on its way meanwhile; with all maxima behind one barrier every value was computed twice and every mix vector read twice, which cost more than the barriers, most of all
+// in narrow models.  Exclusive us in the step, one output and six, with the row in shared memory, one barrier, as it is: 2560 channels 512 rows 15.2 27.4, 11.6 23.8, 11.0
+// 21.3, 1024 rows 25.8 45.3, 23.7 43.1, 22.4 38.5; 1024 channels 512 rows 7.9 15.2, 7.9 19.2, 7.6 17.1, 256 rows 7.2 12.1, 6.4 10.4, 6.1 8.3.
+// The variants with 64 registers spill one of them, which costs nothing that shows.
 struct LnOperandsArgs {
     const float *x_in, *delta;
     float* x_out;
@@ -167,9 +170,9 @@ __device__ __forceinline__ void ln_weights8(float (&v)[8], const float* p) {
     v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
 // Blocks of the variant with 64 registers a thread (<320, 3>) that an SM holds.  While all rows' blocks are resident at once it is the faster one: the weights are
-// there when they are needed.  With more rows the variant with 48 registers, which loads them where it uses them, fits more blocks beside one another: 512 int8 rows of
-// 2560 channels 14.3 us and 11.6, six outputs 26.4 and 23.8; but 448 rows of 2048 channels (256 threads, four blocks) 10.1 and 11.7, 19.3 and 23.4, 640 rows 13.7 and
-// 12.1, 25.6 and 23.9; 1024 rows of 512 channels (64 threads, sixteen blocks) 5.9 and 6.3, 19.6 and 23.7.
+// there when they are needed.  With more rows the variant with 48 registers, which loads them where it uses them, fits more blocks beside one another: one output and six,
+// 512 int8 rows of 2560 channels 12.6 22.6 us and 11.0 21.3; but 384 rows 9.1 17.1 and 10.8 21.1; 592 rows of 2048 channels (256 threads, four blocks) 11.8 18.7 and 11.1
+// 21.3, 640 rows 13.2 22.5 and 11.8 21.3; 1024 rows of 512 channels (64 threads, sixteen blocks) 5.8 17.4 and 6.0 21.1.
 constexpr int ln_resident_blocks(int threads) { return 1024 / threads; }
 template <int THREADS, int BLOCKS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __grid_constant__ LnOperandsArgs A) {
@@ -258,26 +261,22 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) ln_operands_kernel(const __gr
         o[0] = make_float4(x[0], x[1], x[2], x[3]);
         o[1] = make_float4(x[4], x[5], x[6], x[7]);
     }
-    // the outputs' maxima, behind one barrier
-#pragma unroll 1
-    for (int o = o0; o < A.nout; o += step) {
-        const float* mix = A.out[o].mix;
-        if ((!EARLY || o != o0) && mix) ln_weights8(mx, mix + kc);
-        float am = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) am = fmaxf(am, fabsf(mix ? x[i] + mx[i] * xp[i] : x[i]));
-        am = warp_absmax(on ? am : 0.f);
-        if (lane == 0) redm[o][warp] = am;
-    }
-    __syncthreads();
+    // output by output; the next one's mix vector is on its way meanwhile
+    if (!EARLY && A.out[o0].mix) ln_weights8(mx, A.out[o0].mix + kc);
 #pragma unroll 1
     for (int o = o0; o < A.nout; o += step) {
         const RlOperandOut& O = A.out[o];
-        if ((!EARLY || o0 + step < A.nout) && O.mix) ln_weights8(mx, O.mix + kc);
-        const int ex = rl_scale_exp(warp_absmax(lane < nw ? redm[o][lane] : 0.f)), fmt = O.fmt, lk = fmt == RL_F16 ? 6 : 7;
-        float v[8];
+        float v[8], am = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = O.mix ? x[i] + mx[i] * xp[i] : x[i];
+        for (int i = 0; i < 8; ++i) {
+            v[i] = O.mix ? x[i] + mx[i] * xp[i] : x[i];
+            am = fmaxf(am, fabsf(v[i]));
+        }
+        if (o + step < A.nout && A.out[o + step].mix) ln_weights8(mx, A.out[o + step].mix + kc);
+        am = warp_absmax(on ? am : 0.f);
+        if (lane == 0) redm[o][warp] = am;
+        __syncthreads();
+        const int ex = rl_scale_exp(warp_absmax(lane < nw ? redm[o][lane] : 0.f)), fmt = O.fmt, lk = fmt == RL_F16 ? 6 : 7;
         int ts = 0;
         if (on)
             ts = rl_put8(fmt, O.img + ((size_t)rtile * O.kblocks + (k0 >> lk)) * (size_t)(O.nt * 128), rloc * rl_cols(fmt), k0 & ((1 << lk) - 1), v, rl_mult(fmt, ex));

@@ -811,7 +811,8 @@ void run_rows_linear(Model& m, const char* name, const RlReq* reqs, int n, const
     for (int i = 0; i < n; ++i) nk = std::max(nk, (L.p[i].kblocks + L.split - 1) / L.split);
     // Several full row tiles that fill the GPU without splitting K: the persistent kernel.  Not for tiles of fewer than 16 K blocks, which are all epilogue: the rank
     // back-projections take 8.7 us at 128 rows with a CTA per tile and 13.8 persistent, 13.8 and 14.1 at 256, 15.9 and 16.0 at 384; from four turns on persistent is the
-    // faster one, 21.8 and 19.8 at 512 rows, 38.6 and 32.9 at 1024; nor for fp16 tiles of 64 rows that were not cut for turns: they
+    // faster one, 21.8 and 19.8 at 512 rows, 38.6 and 32.9 at 1024, and so it is with the tiles of 32 rows of per-group files, 16.0 and 14.0 at 256 rows, 27.4 and 23.9 at 512, 50.6
+    // and 44.7 at 1024; nor for fp16 tiles of 64 rows that were not cut for turns: they
     // leave half of the matrix instruction's columns out.  One row tile and more weight tiles than two CTAs per SM take at once (the vocabulary head: 512 of them, 336 MB):
     // the second set of CTAs would start its ring from nothing; 3 rows 75 us, persistent 56, 64 rows 83 and 63.
     if (!build && !grouped && (t.turns || (kb_max <= 8 && jobs >= 4 * m.num_sms) || (L.split == 1 && kb_min >= 16 && (t.n > 1 ? row8 || t.rt > kRlMaxRows : jobs > 2 * m.num_sms)))) {

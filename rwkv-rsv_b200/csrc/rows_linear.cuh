@@ -488,9 +488,9 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
         rl_epi_sync();
         if (grouped) {
             // ---- per group: digit sums -> fp32, times the group's scale, plus zero x the group's activation sum ----
-            // What bounds it: at few rows the way of a group's word from memory (one group ahead, behind the wait and not in L2: 3 rows of 2560 channels
-            // a layer 60.1 us; two ahead, the first two before the wait, all of them asked into L2 with the weights 54.4; 16 rows 72.6 and 67.1),
-            // at many rows the instructions of the sums (201 rows 271 us with both halves of a sum through the conversion unit and 16 columns a load, 246 now).
+            // What bounds it: at few rows the way of a group's word from memory, at many the instructions of the sums.  The words come two groups ahead, the first two before
+            // the wait, all of them asked into L2 with the weights; an accumulator is read 32 columns at a time (16 before) and one half of a sum does not go through the
+            // conversion unit: a layer of 3 rows of 2560 channels 60.2 -> 54.0 us, of 16 75.2 -> 66.6, a prompt of 201 rows 272 -> 249.
 #pragma unroll
             for (int c = 0; c < (GROUPED ? kGChunks : 1); ++c)
 #pragma unroll
@@ -644,10 +644,10 @@ __global__ void __launch_bounds__(kRlThreads, 2) rows_linear_kernel(const __grid
 // weight rows x up to 64 activation rows (fp16: 128) in turn, whole K.  One ring of stages runs through all of them and there are two accumulators, so the
 // tensor core works on the next tile while the epilogue warps finish the last one.  With a CTA per tile (two resident) both CTAs of an SM ran in
 // step: of a tile's 22 us at K = 2560 the tensor core worked 13 at 85 % of its rate, the rest was the first loads and the epilogue.
-// Measured, 2560 x 10240 (ffn.key), int8: 1024 rows 139 us with a CTA per tile, now 80; 512 rows 82 and 44.  Sixteen epilogue warps: eight took longer over a
+// Measured, 2560 x 10240 (ffn.key), int8: 1024 rows 139 us with a CTA per tile, now 72; 512 rows 82 and 41.  Sixteen epilogue warps: eight took longer over a
 // tile than the tensor core over its 20 K blocks (512 rows 48; up to 128 rows there are eight all the same, see the launch).
 // What bounds it: the products, at the clock that the power limit leaves them (1.75 GHz), and what gets in their way.  512 rows with parts switched off (us): ffn.key
-// 41.7, products alone 31, without the copies 34, without the epilogue 37; ffn.value 44 to 48, 37, 40 and 44.  The loop that issues products is a function of its own: inside
+// 41.7, products alone 31, without the copies 34, without the epilogue 37; ffn.value 48.0, 37, 40 and 44 (that GPU's; 44.3 on another, whose clock was higher).  The loop that issues products is a function of its own: inside
 // the kernel's control flow it took 600 cycles a K block whose products take 480, as a function those 480 (a bare ring of barriers and products
 // does too); with that and the integer epilogue (rl_value8) ffn.key 42.0 -> 41.0 us, ffn.value 45.6 -> 44.3, r, k, v and rank projections 40.8 -> 39.5, at 1024 rows ffn.key 75.6 -> 72.2.
 // Tried without gain: four producer threads, six stages instead of four, weights asked into L2 a turn ahead, one warp that waits for an accumulator and wakes

@@ -193,6 +193,7 @@ __device__ __forceinline__ void rl_finish(const RlOut& o, bool f16, uint32_t tad
 #pragma unroll 1
     for (int rl = 4 * turn; rl < o.nr; rl += WARPS) {
         float a[4];
+        __syncwarp();  // (the loads below want the whole warp, whose lanes may take either form of rl_value8)
         if (f16) {
             uint32_t v[8];
             tmem_ld8(taddr + 2 * rl, v);
